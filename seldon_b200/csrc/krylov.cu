@@ -35,6 +35,7 @@ namespace sb2 {
 
 int precond_apply(const sb2_precond* M, bool trans, const double* r, double* z,
                   cudaStream_t s);
+int precond_check(const sb2_precond* M, cudaStream_t s);
 
 constexpr int NT = kSpmvThreads;
 
@@ -4492,6 +4493,7 @@ static int host_solve(int which, const sb2_csr* A, const sb2_precond* M, double*
   else if (which == kQmrs) SB2_TRY(host_qmrsym(o, x, b, prm, it, V, &init_failed));
   else if (which == kSymm) SB2_TRY(host_symmlq(o, x, b, prm, it, V, &init_failed));
   else SB2_TRY(host_gmres(o, x, b, prm, it, V, &init_failed));
+  SB2_TRY(precond_check(M, s));
   SB2_CUDA_TRY(cudaStreamSynchronize(s));
   res->init_failed = init_failed;
   res->nb_iter = init_failed ? 0 : it.nb_iter;
@@ -4896,6 +4898,7 @@ static int pcg_solve(const sb2_csr* A, const sb2_precond* M, double* x, const do
     SB2_TRY(chain_pcg(S, n, PrecondLaunch{M, false}, x, b, work, st, part, dh, dhi, hcap,
                       prm->tol, prm->max_iter, prm->init_guess_null, s, &o));
   }
+  SB2_TRY(precond_check(M, s));
   const int nh = std::min(o.hist_len, std::max(hist_cap, 0));
   if (hist && nh > 0) SB2_CUDA_TRY(cudaMemcpy(hist, dh, sizeof(double) * nh, cudaMemcpyDeviceToHost));
   if (hist_it && nh > 0) SB2_CUDA_TRY(cudaMemcpy(hist_it, dhi, sizeof(int) * nh, cudaMemcpyDeviceToHost));

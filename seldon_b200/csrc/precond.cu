@@ -2,11 +2,10 @@
 //
 // SOR reproduces the reference's strictly sequential sweeps
 // (Relaxation_MatVect.cxx:41-95 RowSparse, :176-298 RowSymSparse) bit for
-// bit: rows are grouped into wavefront levels such that every value a row
-// reads is the one the sequential order would have read (true dependencies on
-// already-updated rows AND anti-dependencies on rows that must still hold
-// their old value), and each row repeats the reference's own operation order
-// with separately rounded products.
+// bit: a sweep writes its values into a vector of its own, so a row reads the
+// updated rows there and the others in the vector the sweep started from,
+// and each row repeats the reference's own operation order with separately
+// rounded products.
 //
 // The ILUT apply runs Seldon's SolveLU (computation/solver/SparseSolver.cxx:
 // 533-611 and 852-882) on a factor computed on the host.  Its loops are
@@ -14,14 +13,16 @@
 // (x_c -= v * x_i for each entry of row i).  Every sweep is put in gather
 // form: target j collects its updates in the order the sequential loop
 // would have applied them (the scatter sources in increasing or decreasing
-// row order, each row's entries in stored order), and the rows are grouped
-// into levels on their dependencies.  Each row then repeats the reference's
-// own operations with separately rounded products, so the result is the
-// reference's bit for bit.
+// row order, each row's entries in stored order).  Each row then repeats the
+// reference's own operations with separately rounded products, so the result
+// is the reference's bit for bit.
+//
+// Both run as persistent launches whose rows wait for the values they read
+// (sweep.cuh).  Only the device factorization of ILU(0) runs level by level.
 #include <algorithm>
 #include <vector>
 
-#include "sb2_internal.cuh"
+#include "sweep.cuh"
 
 namespace sb2 {
 
@@ -39,8 +40,7 @@ struct LevelPlan {
   }
 };
 
-static int upload_plan(const std::vector<int>& level, int n, LevelPlan* P,
-                       std::vector<int>* order = nullptr) {
+static int upload_plan(const std::vector<int>& level, int n, LevelPlan* P) {
   int nlev = 0;
   for (int i = 0; i < n; i++) nlev = std::max(nlev, level[i] + 1);
   P->nlev = nlev;
@@ -53,37 +53,11 @@ static int upload_plan(const std::vector<int>& level, int n, LevelPlan* P,
   SB2_CUDA_TRY(cudaMalloc(&P->d_lvl, sizeof(int) * (nlev + 1)));
   SB2_CUDA_TRY(cudaMemcpy(P->d_rows, rows.data(), sizeof(int) * std::max(n, 1), cudaMemcpyHostToDevice));
   SB2_CUDA_TRY(cudaMemcpy(P->d_lvl, P->h_lvl.data(), sizeof(int) * (nlev + 1), cudaMemcpyHostToDevice));
-  if (order) order->assign(rows.begin(), rows.begin() + n);
   return SB2_OK;
 }
 
-// Levels of a sequential sweep over rows in `order` (forward: increasing,
-// backward: decreasing).  Row j reads x(k) for every stored k: it must come
-// after k when k precedes j in the sweep (k is read updated) and before k
-// when k follows j (k is read old).
-static void sweep_levels(int n, const int* ptr, const int* ind, bool forward,
-                         std::vector<int>& level) {
-  level.assign(n, 0);
-  std::vector<int> req(n, 0);
-  for (int s = 0; s < n; s++) {
-    const int j = forward ? s : n - 1 - s;
-    int lev = req[j];
-    for (int k = ptr[j]; k < ptr[j + 1]; k++) {
-      const int c = ind[k];
-      const bool before = forward ? (c < j) : (c > j);
-      if (before) lev = std::max(lev, level[c] + 1);
-    }
-    level[j] = lev;
-    for (int k = ptr[j]; k < ptr[j + 1]; k++) {
-      const int c = ind[k];
-      const bool after = forward ? (c > j) : (c < j);
-      if (after) req[c] = std::max(req[c], lev + 1);
-    }
-  }
-}
-
-// Levels of a triangular solve: row j depends on the entries of `ptr/ind`
-// on the solved side (lower: c < j, upper: c > j).
+// Levels of a sweep: row j depends on the entries of `ptr/ind` on the side
+// already swept (lower: c < j, upper: c > j).
 static void tri_levels(int n, const int* ptr, const int* ind, bool lower,
                        std::vector<int>& level) {
   level.assign(n, 0);
@@ -105,106 +79,6 @@ static void tri_levels(int n, const int* ptr, const int* ind, bool lower,
 // the CTA's own stores, and across launches every write is visible.
 __device__ __forceinline__ double ldx(const double* p) { return *p; }
 
-// RowSparse sweep, one row (Relaxation_MatVect.cxx:69-77 / :83-91).
-struct RowSparseSor {
-  const int* ptr; const int* ind; const double* val; const double* diag;
-  const double* b; double* x; double omega;
-  __device__ void operator()(int j) const {
-    double temp = 0.0;
-    const double ajj = diag[j];
-    for (int k = ptr[j]; k < ptr[j + 1]; k++) temp = add_rn(temp, mul_rn(val[k], ldx(x + ind[k])));
-    const double xj = ldx(x + j);
-    temp = add_rn(__dsub_rn(b[j], temp), mul_rn(ajj, xj));
-    x[j] = add_rn(mul_rn(__dsub_rn(1.0, omega), xj), __ddiv_rn(mul_rn(omega, temp), ajj));
-  }
-};
-
-__device__ __forceinline__ double sym_diag(const int* uptr, const int* uind, const double* uval, int j) {
-  double ajj = 0.0;
-  for (int k = uptr[j]; k < uptr[j + 1]; k++)
-    if (uind[k] == j) ajj = add_rn(ajj, uval[k]);
-  return ajj;
-}
-
-// RowSymSparse forward, first loop (Relaxation_MatVect.cxx:214-230):
-// t_j = ((1-w)/w * ajj) * x_j + (b_j - sum_{p != j} a_jp x_p), x read old.
-struct SymFwd1 {
-  const int* uptr; const int* uind; const double* uval;
-  const double* b; const double* x; double* t; double omega;
-  __device__ void operator()(int j) const {
-    double temp = 0.0, ajj = 0.0;
-    for (int k = uptr[j]; k < uptr[j + 1]; k++) {
-      const int p = uind[k];
-      if (p == j) ajj = add_rn(ajj, uval[k]);
-      else temp = add_rn(temp, mul_rn(uval[k], ldx(x + p)));
-    }
-    temp = __dsub_rn(b[j], temp);
-    const double c = __ddiv_rn(__dsub_rn(1.0, omega), omega);
-    t[j] = add_rn(mul_rn(mul_rn(c, ajj), ldx(x + j)), temp);
-  }
-};
-
-// RowSymSparse forward, second loop as a gather (:232-249): x_j =
-// (t_j - a_{k1 j} x_{k1} - a_{k2 j} x_{k2} ...) * (w / ajj), k increasing.
-// fptr/find/fval: the full row, whose entries with column < j come first in
-// increasing column order (they mirror the strict upper part).
-struct SymFwd2 {
-  const int* fptr; const int* find; const double* fval;
-  const int* uptr; const int* uind; const double* uval;
-  const double* t; double* x; double omega;
-  __device__ void operator()(int j) const {
-    double v = t[j];
-    for (int k = fptr[j]; k < fptr[j + 1]; k++) {
-      const int c = find[k];
-      if (c >= j) break;
-      v = __dsub_rn(v, mul_rn(fval[k], ldx(x + c)));
-    }
-    const double ajj = sym_diag(uptr, uind, uval, j);
-    x[j] = mul_rn(v, __ddiv_rn(omega, ajj));
-  }
-};
-
-// RowSymSparse backward, first loop (:257-276): y_j = sum_{k<j} a_kj x_k (old x,
-// increasing k); t_j = (((1-w)/w * ajj) * x_j + b_j) - y_j.
-struct SymBwd1 {
-  const int* fptr; const int* find; const double* fval;
-  const int* uptr; const int* uind; const double* uval;
-  const double* b; const double* x; double* t; double omega;
-  __device__ void operator()(int j) const {
-    double y = 0.0;
-    for (int k = fptr[j]; k < fptr[j + 1]; k++) {
-      const int c = find[k];
-      if (c >= j) break;
-      y = add_rn(y, mul_rn(fval[k], ldx(x + c)));
-    }
-    const double ajj = sym_diag(uptr, uind, uval, j);
-    const double c0 = __ddiv_rn(__dsub_rn(1.0, omega), omega);
-    t[j] = __dsub_rn(add_rn(mul_rn(mul_rn(c0, ajj), ldx(x + j)), b[j]), y);
-  }
-};
-
-// RowSymSparse backward, second loop (:278-294): x_j = ((t_j - sum_{p != j}
-// a_jp x_p) * w) / ajj, rows decreasing, stored order.
-struct SymBwd2 {
-  const int* uptr; const int* uind; const double* uval;
-  const double* t; double* x; double omega;
-  __device__ void operator()(int j) const {
-    double temp = 0.0, ajj = 0.0;
-    for (int k = uptr[j]; k < uptr[j + 1]; k++) {
-      const int p = uind[k];
-      if (p == j) ajj = add_rn(ajj, uval[k]);
-      else temp = add_rn(temp, mul_rn(uval[k], ldx(x + p)));
-    }
-    x[j] = __ddiv_rn(mul_rn(__dsub_rn(t[j], temp), omega), ajj);
-  }
-};
-
-template <class Op>
-__global__ void rows_kernel(int n, Op op) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < n) op(j);
-}
-
 template <class Op>
 __global__ void level_kernel(int begin, int end, const int* __restrict__ rows, Op op) {
   int i = begin + blockIdx.x * blockDim.x + threadIdx.x;
@@ -220,42 +94,6 @@ __global__ void __launch_bounds__(1024) level_single_cta(int nlev, const int* __
     __syncthreads();
   }
 }
-
-// The same kernels for ops that take the position in level order.
-template <class Op>
-__global__ void level_kernel_pos(int begin, int end, Op op) {
-  int i = begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < end) op(i);
-}
-
-template <class Op>
-__global__ void __launch_bounds__(1024) level_single_cta_pos(int nlev, const int* __restrict__ lvl,
-                                                             Op op) {
-  for (int l = 0; l < nlev; l++) {
-    for (int i = lvl[l] + threadIdx.x; i < lvl[l + 1]; i += blockDim.x) op(i);
-    __syncthreads();
-  }
-}
-
-// x_j = (x_j * pre_j - v_1 x_{c1} - v_2 x_{c2} - ...) * post_j, the
-// subtractions in the listed order (pre/post may be null), for a gather
-// sweep whose update lists are stored in level order: position i
-// holds row rows[i] and its list ptr[i]..ptr[i+1], so the row id, the list
-// bounds and (through them) the entries load without waiting on each other.
-struct GatherSubPacked {
-  const int* rows; const int* ptr; const int* ind; const double* val;
-  const double* pre; const double* post; double* x;
-  __device__ void operator()(int i) const {
-    const int j = rows[i];
-    const int e = ptr[i + 1];
-    double v = ldx(x + j);
-    if (pre) v = mul_rn(v, pre[j]);
-    for (int k = ptr[i]; k < e; k++) v = __dsub_rn(v, mul_rn(val[k], ldx(x + ind[k])));
-    if (post) v = mul_rn(v, post[j]);
-    x[j] = v;
-  }
-};
-
 
 // One row of GetIlu0 (IlutPreconditioning.cxx:1115-1176) or, with
 // `modified`, of GetMilu0 (:1178-1243), in place on the CSR values: rows
@@ -298,22 +136,6 @@ struct Ilu0Row {
   }
 };
 
-// out[idx[i]] = in[i]
-__global__ void perm_scatter_kernel(int n, const int* __restrict__ idx,
-                                    const double* __restrict__ in, double* __restrict__ out) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    out[idx[i]] = in[i];
-}
-
-// out[i] = in[idx[i]]
-__global__ void perm_gather_kernel(int n, const int* __restrict__ idx,
-                                   const double* __restrict__ in, double* __restrict__ out) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    out[i] = in[idx[i]];
-}
-
 __global__ void jacobi_kernel(int n, const double* __restrict__ r,
                               const double* __restrict__ d, double* __restrict__ z) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -322,12 +144,12 @@ __global__ void jacobi_kernel(int n, const double* __restrict__ r,
 }
 #endif
 
-constexpr int kSorSingleCtaMaxN = 65536;
+constexpr int kSingleCtaMaxN = 65536;
 
 template <class Op>
 static int run_levels(const LevelPlan& P, int n, const Op& op, cudaStream_t s) {
   if (n == 0 || P.nlev == 0) return SB2_OK;
-  if (n <= kSorSingleCtaMaxN) {
+  if (n <= kSingleCtaMaxN) {
     level_single_cta<Op><<<1, 1024, 0, s>>>(P.nlev, P.d_lvl, P.d_rows, op);
   } else {
     for (int l = 0; l < P.nlev; l++) {
@@ -339,46 +161,21 @@ static int run_levels(const LevelPlan& P, int n, const Op& op, cudaStream_t s) {
   return SB2_OK;
 }
 
-template <class Op>
-static int run_levels_pos(const LevelPlan& P, int n, const Op& op, cudaStream_t s) {
-  if (n == 0 || P.nlev == 0) return SB2_OK;
-  if (n <= kSorSingleCtaMaxN) {
-    level_single_cta_pos<Op><<<1, 1024, 0, s>>>(P.nlev, P.d_lvl, op);
-  } else {
-    for (int l = 0; l < P.nlev; l++) {
-      const int cnt = P.h_lvl[l + 1] - P.h_lvl[l];
-      level_kernel_pos<Op><<<(cnt + 255) / 256, 256, 0, s>>>(P.h_lvl[l], P.h_lvl[l + 1], op);
-    }
-  }
-  SB2_CUDA_TRY(cudaGetLastError());
-  return SB2_OK;
-}
-
-template <class Op>
-static int run_rows(int n, const Op& op, cudaStream_t s) {
-  if (n == 0) return SB2_OK;
-  rows_kernel<Op><<<(n + 255) / 256, 256, 0, s>>>(n, op);
-  SB2_CUDA_TRY(cudaGetLastError());
-  return SB2_OK;
-}
-
 }  // namespace sb2
 
 namespace sb2 {
-// One triangular sweep in gather form: the rows' update lists, stored in
-// level order (list i belongs to row lv.d_rows[i]), and the levels.
+// One triangular sweep in gather form: the rows' update lists, stored in the
+// order the rows are taken.
 struct GatherSweep {
-  int* d_ptr = nullptr;
   int* d_ind = nullptr;
   double* d_val = nullptr;
-  LevelPlan lv;
+  SweepPlan plan;
   void release() {
-    cudaFree(d_ptr);
     cudaFree(d_ind);
     cudaFree(d_val);
-    d_ptr = d_ind = nullptr;
+    d_ind = nullptr;
     d_val = nullptr;
-    lv.release();
+    plan.release();
   }
 };
 }  // namespace sb2
@@ -389,31 +186,21 @@ struct sb2_precond {
   double omega = 1.0;
   int nb_iter = 1;
   int symmetric = 1;
-  // SOR schedules: general forward/backward sweeps, or for symmetric storage
-  // the lower (forward) and upper (backward) triangular solves.
-  sb2::LevelPlan fwd, bwd;
-  double* d_t = nullptr;  // scratch of the symmetric sweeps and of ILUT
+  sb2::SweepGrid grid;      // row blocks and work vectors of the sweeps
+  sb2::SweepPlan fwd, bwd;  // SOR
+  double* d_sdiag = nullptr;  // SOR, symmetric storage: diagonal of each stored row
   std::mutex mu;
   bool planned = false;
-  // ILUT: order, storage, permutations, 1/U(i,i) or 1/D(i), and the sweeps
-  // (unsymmetric: L forward, U backward, U^T forward, L^T backward;
-  // symmetric: L forward through the transposed rows, L^T backward)
+  // ILUT: order, storage, permutations (and the inverse of the row one),
+  // 1/U(i,i) or 1/D(i), and the sweeps (unsymmetric: L forward, U backward,
+  // U^T forward, L^T backward; symmetric: L forward through the transposed
+  // rows, L^T backward)
   int n_ilu = 0;
   int ilu_sym = 0;
-  int* d_prow = nullptr;
+  int* d_iprow = nullptr;
   int* d_pcol = nullptr;
   double* d_dinv = nullptr;
   sb2::GatherSweep s_lf, s_ub, s_utf, s_ltb;
-  // Applies with one launch per level, recorded once per (r, z, direction)
-  // as CUDA graphs and replayed (the Krylov drivers reuse their buffers).
-  struct Recorded {
-    const double* r;
-    double* z;
-    bool trans;
-    cudaGraphExec_t exec;
-  };
-  std::vector<Recorded> graphs;
-  cudaStream_t cap_stream = nullptr;
 };
 
 namespace sb2 {
@@ -423,69 +210,83 @@ static int plan_sor(sb2_precond* M) {
   if (M->planned) return SB2_OK;
   const sb2_csr* A = M->A;
   const int n = A->m;
-  const CsrArrays& src = A->sym ? A->upper : A->full;
-  std::vector<int> ptr(n + 1), ind(src.nnz);
-  SB2_CUDA_TRY(cudaMemcpy(ptr.data(), src.d_ptr, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost));
-  if (src.nnz) SB2_CUDA_TRY(cudaMemcpy(ind.data(), src.d_ind, sizeof(int) * src.nnz, cudaMemcpyDeviceToHost));
-  std::vector<int> level;
-  if (!A->sym) {
-    sweep_levels(n, ptr.data(), ind.data(), true, level);
-    SB2_TRY(upload_plan(level, n, &M->fwd));
-    sweep_levels(n, ptr.data(), ind.data(), false, level);
-    SB2_TRY(upload_plan(level, n, &M->bwd));
-  } else {
-    // forward second loop = lower solve (dependencies c < j of the full
-    // pattern); backward second loop = upper solve on the stored rows.
-    const CsrArrays& f = A->full;
-    std::vector<int> fptr(n + 1), find(f.nnz);
-    SB2_CUDA_TRY(cudaMemcpy(fptr.data(), f.d_ptr, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost));
-    if (f.nnz) SB2_CUDA_TRY(cudaMemcpy(find.data(), f.d_ind, sizeof(int) * f.nnz, cudaMemcpyDeviceToHost));
-    tri_levels(n, fptr.data(), find.data(), true, level);
-    SB2_TRY(upload_plan(level, n, &M->fwd));
-    tri_levels(n, ptr.data(), ind.data(), false, level);
-    SB2_TRY(upload_plan(level, n, &M->bwd));
-    SB2_CUDA_TRY(cudaMalloc(&M->d_t, sizeof(double) * std::max(n, 1)));
+  const CsrArrays& f = A->full;
+  std::vector<int> ptr(n + 1), ind(f.nnz), uptr, uind;
+  SB2_CUDA_TRY(cudaMemcpy(ptr.data(), f.d_ptr, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost));
+  if (f.nnz) SB2_CUDA_TRY(cudaMemcpy(ind.data(), f.d_ind, sizeof(int) * f.nnz, cudaMemcpyDeviceToHost));
+  if (A->sym) {
+    const CsrArrays& u = A->upper;
+    uptr.resize(n + 1);
+    uind.resize(u.nnz);
+    SB2_CUDA_TRY(cudaMemcpy(uptr.data(), u.d_ptr, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost));
+    if (u.nnz) SB2_CUDA_TRY(cudaMemcpy(uind.data(), u.d_ind, sizeof(int) * u.nnz, cudaMemcpyDeviceToHost));
+  }
+  SB2_TRY(make_sweep_grid(n, &M->grid));
+  auto span = [&](int, int j) {
+    if (!A->sym) return make_int4(ptr[j], ptr[j + 1], 0, 0);
+    // the mirrored entries come first in the expanded row
+    const int stored = uptr[j + 1] - uptr[j];
+    return make_int4(uptr[j], uptr[j + 1], ptr[j], ptr[j + 1] - stored);
+  };
+  std::vector<int> level, order;
+  tri_levels(n, ptr.data(), ind.data(), true, level);
+  SB2_TRY(make_sweep_plan(M->grid, level, &M->fwd, order, span));
+  if (A->sym) tri_levels(n, uptr.data(), uind.data(), false, level);
+  else tri_levels(n, ptr.data(), ind.data(), false, level);
+  SB2_TRY(make_sweep_plan(M->grid, level, &M->bwd, order, span));
+  if (A->sym) {
+    // values of symmetric storage never change (sb2_csr_set_values)
+    const CsrArrays& u = A->upper;
+    SB2_CUDA_TRY(cudaMalloc(&M->d_sdiag, sizeof(double) * std::max(n, 1)));
+    if (n > 0) {
+      sym_diag_kernel<<<std::min((n + 255) / 256, 1184), 256>>>(n, u.d_ptr, u.d_ind, u.d_val, M->d_sdiag);
+      SB2_CUDA_TRY(cudaGetLastError());
+      SB2_CUDA_TRY(cudaDeviceSynchronize());
+    }
   }
   M->planned = true;
   return SB2_OK;
 }
 
-// SOR(A, X, B, omega, iter, type_ssor) on device, in place on x, once the
-// level plans and the diagonal exist (sor_apply makes them).
-static int sor_run(sb2_precond* M, double* x, const double* b, double omega,
-                   int iter, int type_ssor, cudaStream_t s) {
-  const sb2_csr* A = M->A;
-  const int n = A->m;
-  if (!A->sym) {
-    SB2_TRY(ensure_diag(A));
-    RowSparseSor op{A->full.d_ptr, A->full.d_ind, A->full.d_val, A->d_diag, b, x, omega};
-    if (type_ssor % 2 == 0)
-      for (int i = 0; i < iter; i++) SB2_TRY(run_levels(M->fwd, n, op, s));
-    if (type_ssor % 3 == 0)
-      for (int i = 0; i < iter; i++) SB2_TRY(run_levels(M->bwd, n, op, s));
-    return SB2_OK;
-  }
-  const CsrArrays& u = A->upper;
-  const CsrArrays& f = A->full;
-  if (type_ssor % 2 == 0)
-    for (int i = 0; i < iter; i++) {
-      SB2_TRY(run_rows(n, SymFwd1{u.d_ptr, u.d_ind, u.d_val, b, x, M->d_t, omega}, s));
-      SB2_TRY(run_levels(M->fwd, n,
-                         SymFwd2{f.d_ptr, f.d_ind, f.d_val, u.d_ptr, u.d_ind, u.d_val, M->d_t, x, omega}, s));
-    }
-  if (type_ssor % 3 == 0)
-    for (int i = 0; i < iter; i++) {
-      SB2_TRY(run_rows(n, SymBwd1{f.d_ptr, f.d_ind, f.d_val, u.d_ptr, u.d_ind, u.d_val, b, x, M->d_t, omega}, s));
-      SB2_TRY(run_levels(M->bwd, n, SymBwd2{u.d_ptr, u.d_ind, u.d_val, M->d_t, x, omega}, s));
-    }
-  return SB2_OK;
-}
-
-static int sor_apply(sb2_precond* M, double* x, const double* b, double omega,
+// SOR(A, X, B, omega, iter, type_ssor) on the device: the sweeps from x0
+// (null: zero) into x, two a launch.  x0 is null or x itself.
+static int sor_apply(sb2_precond* M, const double* x0, double* x, const double* b, double omega,
                      int iter, int type_ssor, cudaStream_t s) {
   SB2_TRY(plan_sor(M));
-  if (!M->A->sym) SB2_TRY(ensure_diag(M->A));
-  return sor_run(M, x, b, omega, iter, type_ssor, s);
+  const sb2_csr* A = M->A;
+  const int n = A->m;
+  if (!A->sym) SB2_TRY(ensure_diag(A));
+  const SweepGrid& G = M->grid;
+  const int nf = type_ssor % 2 == 0 ? std::max(iter, 0) : 0;
+  const int total = nf + (type_ssor % 3 == 0 ? std::max(iter, 0) : 0);
+  const int launches = (total + 1) / 2;
+  const double* cur = x0;
+  for (int l = 0, done = 0; l < launches; l++, done += 2) {
+    const bool two = done + 1 < total;
+    const bool fwd[2] = {done < nf, done + 1 < nf};
+    const SweepPlan* const plan[2] = {fwd[0] ? &M->fwd : &M->bwd, fwd[1] ? &M->fwd : &M->bwd};
+    // targets alternate between x and a work vector, so that none is the
+    // vector its launch starts from; from zero the last one is x
+    const bool into_x = x0 ? l % 2 == 1 : (launches - 1 - l) % 2 == 0;
+    double* last = into_x ? x : G.d_new[1];
+    double* out0 = two ? G.d_new[0] : last;
+    double* out1 = two ? last : nullptr;
+    if (A->sym) {
+      const CsrArrays &u = A->upper, &f = A->full;
+      SB2_TRY(launch_sweeps(G, plan, fwd, out0, out1,
+                            SymmetricSor{u.d_ind, u.d_val, f.d_ind, f.d_val, M->d_sdiag, b, cur, omega,
+                                         (1.0 - omega) / omega}, s));
+    } else {
+      const CsrArrays& f = A->full;
+      SB2_TRY(launch_sweeps(G, plan, fwd, out0, out1,
+                            GeneralSor{f.d_ind, f.d_val, A->d_diag, b, cur, omega, 1.0 - omega}, s));
+    }
+    cur = last;
+  }
+  if (launches == 0 && !x0) SB2_CUDA_TRY(cudaMemsetAsync(x, 0, sizeof(double) * n, s));
+  if (launches > 0 && cur != x)
+    SB2_CUDA_TRY(cudaMemcpyAsync(x, cur, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+  return SB2_OK;
 }
 
 // Levels of a gather sweep: row j waits for every row it reads; rows are
@@ -502,27 +303,25 @@ static void gather_levels(int n, const std::vector<int>& ptr, const std::vector<
   }
 }
 
-static int upload_sweep(int n, const std::vector<int>& ptr, const std::vector<int>& ind,
-                        const std::vector<double>& val, bool ascending, GatherSweep* S) {
+static int upload_sweep(const SweepGrid& G, const std::vector<int>& ptr,
+                        const std::vector<int>& ind, const std::vector<double>& val,
+                        bool ascending, GatherSweep* S) {
   std::vector<int> level, order;
-  gather_levels(n, ptr, ind, ascending, level);
-  SB2_TRY(upload_plan(level, n, &S->lv, &order));
-  // the lists in level order
-  std::vector<int> pptr(n + 1, 0), pind;
+  gather_levels(G.n, ptr, ind, ascending, level);
+  // the lists in the order the rows are taken
+  std::vector<int> pind;
   std::vector<double> pval;
   pind.reserve(ind.size());
   pval.reserve(val.size());
-  for (int i = 0; i < n; i++) {
-    const int j = order[i];
+  SB2_TRY(make_sweep_plan(G, level, &S->plan, order, [&](int, int j) {
+    const int k0 = (int)pind.size();
     pind.insert(pind.end(), ind.begin() + ptr[j], ind.begin() + ptr[j + 1]);
     pval.insert(pval.end(), val.begin() + ptr[j], val.begin() + ptr[j + 1]);
-    pptr[i + 1] = (int)pind.size();
-  }
+    return make_int4(k0, (int)pind.size(), 0, 0);
+  }));
   const size_t nz = pind.size();
-  SB2_CUDA_TRY(cudaMalloc(&S->d_ptr, sizeof(int) * (n + 1)));
   SB2_CUDA_TRY(cudaMalloc(&S->d_ind, sizeof(int) * std::max<size_t>(nz, 1)));
   SB2_CUDA_TRY(cudaMalloc(&S->d_val, sizeof(double) * std::max<size_t>(nz, 1)));
-  SB2_CUDA_TRY(cudaMemcpy(S->d_ptr, pptr.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice));
   if (nz) {
     SB2_CUDA_TRY(cudaMemcpy(S->d_ind, pind.data(), sizeof(int) * nz, cudaMemcpyHostToDevice));
     SB2_CUDA_TRY(cudaMemcpy(S->d_val, pval.data(), sizeof(double) * nz, cudaMemcpyHostToDevice));
@@ -572,6 +371,8 @@ static int plan_ilut(sb2_precond* M, int n, const int* fp, const int* fi, const 
     if (fp[i + 1] < fp[i]) return SB2_ERR_INVALID_CSR;
   if (!is_permutation(n, prow) || (!M->ilu_sym && !is_permutation(n, pcol)))
     return SB2_ERR_INVALID_VALUE;
+  SB2_TRY(make_sweep_grid(n, &M->grid));
+  const SweepGrid& G = M->grid;
   std::vector<double> dinv(n);
   std::vector<int> ptr, ind;
   std::vector<double> val;
@@ -592,8 +393,8 @@ static int plan_ilut(sb2_precond* M, int n, const int* fp, const int* fi, const 
       bptr[i + 1] = (int)bind.size();
     }
     fwd.flatten(ptr, ind, val);
-    SB2_TRY(upload_sweep(n, ptr, ind, val, true, &M->s_lf));
-    SB2_TRY(upload_sweep(n, bptr, bind, bval, false, &M->s_ub));
+    SB2_TRY(upload_sweep(G, ptr, ind, val, true, &M->s_lf));
+    SB2_TRY(upload_sweep(G, bptr, bind, bval, false, &M->s_ub));
   } else {
     // row i: L part (columns < i), then 1/U(i,i), then the U part
     std::vector<int> lptr(n + 1, 0), lind, uptr(n + 1, 0), uind;
@@ -622,21 +423,23 @@ static int plan_ilut(sb2_precond* M, int n, const int* fp, const int* fi, const 
     }
     for (int i = n - 1; i >= 0; i--)  // L^T: x(k) -= L(i,k) x(i), i decreasing
       for (int k = fp[i]; k < dpos[i]; k++) ltb.add(fi[k], i, fv[k]);
-    SB2_TRY(upload_sweep(n, lptr, lind, lval, true, &M->s_lf));
-    SB2_TRY(upload_sweep(n, uptr, uind, uval, false, &M->s_ub));
+    SB2_TRY(upload_sweep(G, lptr, lind, lval, true, &M->s_lf));
+    SB2_TRY(upload_sweep(G, uptr, uind, uval, false, &M->s_ub));
     utf.flatten(ptr, ind, val);
-    SB2_TRY(upload_sweep(n, ptr, ind, val, true, &M->s_utf));
+    SB2_TRY(upload_sweep(G, ptr, ind, val, true, &M->s_utf));
     ltb.flatten(ptr, ind, val);
-    SB2_TRY(upload_sweep(n, ptr, ind, val, false, &M->s_ltb));
+    SB2_TRY(upload_sweep(G, ptr, ind, val, false, &M->s_ltb));
   }
+  std::vector<int> iprow(n);
+  for (int i = 0; i < n; i++) iprow[prow[i]] = i;
   SB2_CUDA_TRY(cudaMalloc(&M->d_dinv, sizeof(double) * std::max(n, 1)));
-  SB2_CUDA_TRY(cudaMalloc(&M->d_prow, sizeof(int) * std::max(n, 1)));
-  SB2_CUDA_TRY(cudaMalloc(&M->d_pcol, sizeof(int) * std::max(n, 1)));
-  SB2_CUDA_TRY(cudaMalloc(&M->d_t, sizeof(double) * std::max(n, 1)));
+  SB2_CUDA_TRY(cudaMalloc(&M->d_iprow, sizeof(int) * std::max(n, 1)));
   SB2_CUDA_TRY(cudaMemcpy(M->d_dinv, dinv.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
-  SB2_CUDA_TRY(cudaMemcpy(M->d_prow, prow, sizeof(int) * n, cudaMemcpyHostToDevice));
-  SB2_CUDA_TRY(cudaMemcpy(M->d_pcol, M->ilu_sym ? prow : pcol, sizeof(int) * n,
-                          cudaMemcpyHostToDevice));
+  SB2_CUDA_TRY(cudaMemcpy(M->d_iprow, iprow.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
+  if (!M->ilu_sym) {
+    SB2_CUDA_TRY(cudaMalloc(&M->d_pcol, sizeof(int) * std::max(n, 1)));
+    SB2_CUDA_TRY(cudaMemcpy(M->d_pcol, pcol, sizeof(int) * n, cudaMemcpyHostToDevice));
+  }
   return SB2_OK;
 }
 
@@ -700,86 +503,24 @@ static int ilu0_factor(const sb2_csr* A, int modified, std::vector<int>& ptr,
   return st;
 }
 
-static GatherSubPacked sweep_op(const GatherSweep& S, const double* pre, const double* post,
-                                double* x) {
-  return GatherSubPacked{S.lv.d_rows, S.d_ptr, S.d_ind, S.d_val, pre, post, x};
-}
-
 // IlutPreconditioning::Solve / TransSolve (IlutPreconditioning.cxx:329-374):
-// the launches.
-static int ilut_launch(const sb2_precond* M, bool trans, const double* r, double* z,
-                       cudaStream_t s) {
-  const int n = M->n_ilu;
-  double* t = M->d_t;
-  const int g = std::min((n + 255) / 256, num_sms(current_device()) * 8);
-  if (M->ilu_sym) {
-    perm_scatter_kernel<<<g, 256, 0, s>>>(n, M->d_prow, r, t);
-    SB2_TRY(run_levels_pos(M->s_lf.lv, n, sweep_op(M->s_lf, nullptr, nullptr, t), s));
-    SB2_TRY(run_levels_pos(M->s_ub.lv, n, sweep_op(M->s_ub, M->d_dinv, nullptr, t), s));
-    perm_gather_kernel<<<g, 256, 0, s>>>(n, M->d_prow, t, z);
-  } else if (!trans) {
-    perm_scatter_kernel<<<g, 256, 0, s>>>(n, M->d_prow, r, t);
-    SB2_TRY(run_levels_pos(M->s_lf.lv, n, sweep_op(M->s_lf, nullptr, nullptr, t), s));
-    SB2_TRY(run_levels_pos(M->s_ub.lv, n, sweep_op(M->s_ub, nullptr, M->d_dinv, t), s));
-    perm_scatter_kernel<<<g, 256, 0, s>>>(n, M->d_pcol, t, z);
-  } else {
-    perm_gather_kernel<<<g, 256, 0, s>>>(n, M->d_pcol, r, t);
-    SB2_TRY(run_levels_pos(M->s_utf.lv, n, sweep_op(M->s_utf, nullptr, M->d_dinv, t), s));
-    SB2_TRY(run_levels_pos(M->s_ltb.lv, n, sweep_op(M->s_ltb, nullptr, nullptr, t), s));
-    perm_gather_kernel<<<g, 256, 0, s>>>(n, M->d_prow, t, z);
-  }
-  SB2_CUDA_TRY(cudaGetLastError());
-  return SB2_OK;
-}
-
-constexpr int kIluGraphs = 8;  // recorded applies kept per preconditioner
-
-// Applies of large systems launch once per level: they are recorded once per
-// (r, z, direction) as a CUDA graph and replayed, so the launches cost the
-// device's dependency resolution only, not a host call each.  `launch`
-// enqueues the apply on the stream it is given.
-template <class Launch>
-static int replay_recorded(sb2_precond* M, bool trans, const double* r, double* z,
-                           cudaStream_t s, const Launch& launch) {
-  std::lock_guard<std::mutex> g(M->mu);
-  for (const auto& e : M->graphs)
-    if (e.r == r && e.z == z && e.trans == trans) {
-      SB2_CUDA_TRY(cudaGraphLaunch(e.exec, s));
-      return SB2_OK;
-    }
-  if (!M->cap_stream)
-    SB2_CUDA_TRY(cudaStreamCreateWithFlags(&M->cap_stream, cudaStreamNonBlocking));
-  SB2_CUDA_TRY(cudaStreamBeginCapture(M->cap_stream, cudaStreamCaptureModeThreadLocal));
-  int st = launch(M->cap_stream);
-  cudaGraph_t graph = nullptr;
-  cudaError_t e = cudaStreamEndCapture(M->cap_stream, &graph);
-  if (st != SB2_OK) {
-    if (graph) cudaGraphDestroy(graph);
-    return st;
-  }
-  SB2_CUDA_TRY(e);
-  cudaGraphExec_t exec = nullptr;
-  e = cudaGraphInstantiate(&exec, graph, 0);
-  cudaGraphDestroy(graph);
-  SB2_CUDA_TRY(e);
-  if ((int)M->graphs.size() >= kIluGraphs) {
-    // the oldest recording goes once the stream has no launch of it pending
-    cudaStreamSynchronize(s);
-    cudaGraphExecDestroy(M->graphs.front().exec);
-    M->graphs.erase(M->graphs.begin());
-  }
-  M->graphs.push_back({r, z, trans, exec});
-  SB2_CUDA_TRY(cudaGraphLaunch(exec, s));
-  return SB2_OK;
-}
-
-// Small systems run every level in one CTA (one launch); larger ones replay
-// a recorded graph of the per-level launches.
+// both sweeps and both permutations in one launch.  Seldon's t[prow[i]] = r[i]
+// and z[i] = t[prow[i]] are t[j] = r[iprow[j]] and z[iprow[j]] = t[j] for the
+// thread that owns row j.
 static int ilut_apply(sb2_precond* M, bool trans, const double* r, double* z, cudaStream_t s) {
-  if (M->n_ilu <= kSorSingleCtaMaxN) return ilut_launch(M, trans, r, z, s);
-  return replay_recorded(M, trans, r, z, s, [&](cudaStream_t cs) {
-    return ilut_launch(M, trans, r, z, cs);
-  });
+  const bool sym = M->ilu_sym != 0;
+  const GatherSweep& first = !sym && trans ? M->s_utf : M->s_lf;
+  const GatherSweep& second = !sym && trans ? M->s_ltb : M->s_ub;
+  const double* d = M->d_dinv;
+  FactorSolve op{{first.d_ind, second.d_ind},
+                 {first.d_val, second.d_val},
+                 {nullptr, sym ? d : nullptr},
+                 {!sym && trans ? d : nullptr, !sym && !trans ? d : nullptr},
+                 r, !sym && trans ? M->d_pcol : M->d_iprow,
+                 z, !sym && !trans ? M->d_pcol : M->d_iprow};
+  const SweepPlan* const plan[2] = {&first.plan, &second.plan};
+  const bool fwd[2] = {true, false};
+  return launch_sweeps(M->grid, plan, fwd, M->grid.d_new[0], M->grid.d_new[1], op, s);
 }
 
 int precond_kind(const sb2_precond* M) { return M->kind; }
@@ -805,15 +546,19 @@ int precond_apply(const sb2_precond* cM, bool trans, const double* r, double* z,
   }
   // SorPreconditioner::Solve / TransSolve (Precond_Ssor.cxx:62-90)
   const int type = M->symmetric ? 0 : (trans ? 3 : 2);
-  SB2_TRY(plan_sor(M));
-  if (!M->A->sym) SB2_TRY(ensure_diag(M->A));
-  auto launch = [&](cudaStream_t cs) -> int {
-    SB2_CUDA_TRY(cudaMemsetAsync(z, 0, sizeof(double) * n, cs));
-    return sor_run(M, z, r, M->omega, M->nb_iter, type, cs);
-  };
-  if (n <= kSorSingleCtaMaxN) return launch(s);
-  // the symmetric sweeps' trans flag does not change the launches
-  return replay_recorded(M, M->symmetric ? false : trans, r, z, s, launch);
+  return sor_apply(M, nullptr, z, r, M->omega, M->nb_iter, type, s);
+}
+
+// Whether a wait of the preconditioner's sweeps ran out since the last call
+// (synchronizes the stream).
+int precond_check(const sb2_precond* M, cudaStream_t s) {
+  if (!M || !M->grid.d_state) return SB2_OK;
+  unsigned late = 0;
+  SB2_CUDA_TRY(cudaMemcpyAsync(&late, M->grid.d_state + 1, sizeof(late), cudaMemcpyDeviceToHost, s));
+  SB2_CUDA_TRY(cudaStreamSynchronize(s));
+  if (!late) return SB2_OK;
+  SB2_CUDA_TRY(cudaMemsetAsync(M->grid.d_state + 1, 0, sizeof(late), s));
+  return SB2_ERR_TIMEOUT;
 }
 
 }  // namespace sb2
@@ -881,17 +626,15 @@ int sb2_precond_create_ilu0(const sb2_csr* A, int modified, void* stream, sb2_pr
 
 int sb2_precond_destroy(sb2_precond* M) try {
   if (!M) return SB2_OK;
-  if (!M->graphs.empty()) cudaDeviceSynchronize();  // no replay may be in flight
-  for (auto& e : M->graphs) cudaGraphExecDestroy(e.exec);
-  if (M->cap_stream) cudaStreamDestroy(M->cap_stream);
+  M->grid.release();
   M->fwd.release();
   M->bwd.release();
-  cudaFree(M->d_t);
+  cudaFree(M->d_sdiag);
   M->s_lf.release();
   M->s_ub.release();
   M->s_utf.release();
   M->s_ltb.release();
-  cudaFree(M->d_prow);
+  cudaFree(M->d_iprow);
   cudaFree(M->d_pcol);
   cudaFree(M->d_dinv);
   delete M;
@@ -919,13 +662,16 @@ int sb2_sor(const sb2_csr* A, double* x, const double* b, double omega, int iter
   sb2_precond tmp;
   tmp.A = A;
   tmp.kind = SB2_PRECOND_SOR;
-  int st = sor_apply(&tmp, x, b, omega, iter, type_ssor, (cudaStream_t)stream);
+  int st = sor_apply(&tmp, x, x, b, omega, iter, type_ssor, (cudaStream_t)stream);
   // the plan is released after the stream has consumed it
+  const int late = precond_check(&tmp, (cudaStream_t)stream);
   cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);
+  tmp.grid.release();
   tmp.fwd.release();
   tmp.bwd.release();
-  cudaFree(tmp.d_t);
+  cudaFree(tmp.d_sdiag);
   if (st == SB2_OK && e != cudaSuccess) st = map_cuda_error(e);
+  if (st == SB2_OK) st = late;
   return st;
 } SB2_CATCH
 

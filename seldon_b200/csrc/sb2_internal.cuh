@@ -189,7 +189,7 @@ int launch_spmv(const CsrArrays& a, double alpha, const double* x, double beta,
                 double* y, bool overwrite, cudaStream_t s);
 
 // Limit of the persistent solvers' bounded grid-barrier waits, microseconds.
-extern std::atomic<long long> g_wait_limit_us;
+inline std::atomic<long long> g_wait_limit_us{2000000};
 inline unsigned long long barrier_wait_ns() { return (unsigned long long)g_wait_limit_us.load() * 1000ull; }
 // The TMA product's ring waits (bulk copies in flight) never use less than 1 s.
 inline unsigned long long ring_wait_ns() {

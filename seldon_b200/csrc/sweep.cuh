@@ -1,0 +1,693 @@
+// Sequential sweeps (Gauss-Seidel, triangular solves) as one persistent launch
+// whose rows wait for the values they read, not for levels.
+//
+// The rows are cut into one contiguous block per CTA.  Inside a block they
+// are ordered by dependency level and dealt to the warps in items of up to 32
+// rows of one level; a warp takes its items in order, one row per lane.
+//  - Values of the CTA's own block live in its shared memory.  The items of
+//    one level form a step with an mbarrier, and an item waits for the step
+//    before its own, suspended by the hardware.
+//  - Values of other blocks come through global memory.  The vector a sweep
+//    writes was filled with a reserved NaN, so a value announces itself: the
+//    row polls the entries it needs until they differ from the fill.  No
+//    flag, fence or grid barrier stands between a value and its use.
+// Each row repeats the reference's operations in the reference's order, so
+// the result does not depend on the timing.
+//
+// What bounds it is the chain of dependent rows.  Inside a block a level costs
+// what one row does between its turn and its barrier (430 cycles for three
+// entries, measured with clock64); the loads and everything that reads only
+// old values come before, while the warp's predecessors still work.  From one
+// CTA to the next a value takes 2-3 us.  Two sweeps on a 7-point grid, against
+// a graph of one launch per level before: ILU(0) apply 96^3 651 us (2070), 128^3
+// 1066 us (2970); SSOR of symmetric storage, 64^3 395 us (2700).
+// 384 threads: with 256 the small grids lose a fifth (ILU(0) 16^3 54 us
+// against 45), with 768 and more the registers spill on the chain (83 us).
+//
+// Progress: all CTAs are resident (cooperative launch), a warp's items are in
+// level order and a row reads rows of smaller levels only.  Every wait is
+// bounded: when no CTA has made progress for the wait limit, the waiting warp
+// sets the status word and the grid leaves; rows not reached keep the fill
+// (a NaN).
+#pragma once
+
+#include <algorithm>
+#include <vector>
+
+#include "sb2_internal.cuh"
+
+namespace sb2 {
+
+constexpr int kSweepMaxCtas = 148;
+constexpr int kSweepStep = 32;   // items of one step at most
+constexpr int kSweepRing = 64;   // step barriers (more than the warps of a CTA)
+constexpr int kSweepSmem = 224 * 1024;  // most shared memory a CTA takes for its values
+// The fill: a signalling NaN, which no arithmetic produces.  A value that
+// was copied from the caller with these very bits is stored as the quiet NaN.
+constexpr unsigned long long kSweepFill = 0x7ff4b2005e1d0001ull;
+
+// The rows of one sweep in the order they are taken.
+struct SweepPlan {
+  int* d_rows = nullptr;      // [n] row of each position
+  int4* d_span = nullptr;     // [n] entry ranges of each position's row
+  int4* d_item = nullptr;     // [items] first position, rows, step, arrivals (below)
+  int* d_cta_item = nullptr;  // [ctas + 1] first item of each CTA
+  int* d_steps = nullptr;     // [ctas] steps of each CTA
+  void release() {
+    cudaFree(d_rows);
+    cudaFree(d_span);
+    cudaFree(d_item);
+    cudaFree(d_cta_item);
+    cudaFree(d_steps);
+    d_rows = d_cta_item = d_steps = nullptr;
+    d_span = nullptr;
+    d_item = nullptr;
+  }
+};
+
+// The row blocks shared by all sweeps of one preconditioner, and the vectors
+// the sweeps write.
+struct SweepGrid {
+  int n = 0, ctas = 0, max_rows = 0;
+  std::vector<int> h_blk;     // [ctas + 1] first row of each block
+  int* d_blk = nullptr;
+  double* d_new[2] = {nullptr, nullptr};
+  unsigned* d_state = nullptr;  // [0] leave, [1] some wait ran out, [2 + c] progress of CTA c
+  void release() {
+    cudaFree(d_blk);
+    cudaFree(d_new[0]);
+    cudaFree(d_new[1]);
+    cudaFree(d_state);
+    d_blk = nullptr;
+    d_new[0] = d_new[1] = nullptr;
+    d_state = nullptr;
+  }
+};
+
+struct SweepPhase {
+  const int* rows;
+  const int4* span;
+  const int4* item;
+  const int* cta_item;
+  const int* steps;
+  int forward;     // new values are those of smaller rows
+  double* out;     // values of this phase (filled before the launch)
+};
+
+struct SweepArgs {
+  const int* blk;
+  int max_rows;
+  int nph;          // 1 or 2 sweeps in this launch
+  SweepPhase ph[2];
+  unsigned* state;
+  unsigned long long wait_ns;
+};
+
+// ------------------------------------------------------------------ planning
+
+// Cuts n rows into blocks of about 2048, one CTA each, and larger ones where
+// the SMs run out.  SSOR on 7-point grids, 2048 / 4096 / 8192 rows a block:
+// 20^3 123 / 177 / 238 us, 40^3 244 / 273 / 423, 64^3 395 / 413 / 499; smaller
+// blocks add CTAs for a chain of rows to cross (1024: 433 us at 64^3).
+inline int make_sweep_grid(int n, SweepGrid* G) {
+  G->n = n;
+  const int most = std::min(kSweepMaxCtas, num_sms(current_device()));
+  G->ctas = std::max(1, std::min(most, (n + 2047) / 2048));
+  const int per = (n + G->ctas - 1) / G->ctas;
+  G->max_rows = per;
+  G->h_blk.resize(G->ctas + 1);
+  for (int c = 0; c <= G->ctas; c++) G->h_blk[c] = (int)std::min<long long>((long long)c * per, n);
+  SB2_CUDA_TRY(cudaMalloc(&G->d_blk, sizeof(int) * (G->ctas + 1)));
+  SB2_CUDA_TRY(cudaMemcpy(G->d_blk, G->h_blk.data(), sizeof(int) * (G->ctas + 1), cudaMemcpyHostToDevice));
+  for (int k = 0; k < 2; k++) SB2_CUDA_TRY(cudaMalloc(&G->d_new[k], sizeof(double) * std::max(n, 1)));
+  SB2_CUDA_TRY(cudaMalloc(&G->d_state, sizeof(unsigned) * (2 + kSweepMaxCtas)));
+  SB2_CUDA_TRY(cudaMemset(G->d_state, 0, sizeof(unsigned) * (2 + kSweepMaxCtas)));
+  return SB2_OK;
+}
+
+// Positions, items and spans of one sweep from the rows' levels.  span(i, j)
+// gives the entry ranges of row j at position i; `order` returns the rows.
+template <class Span>
+int make_sweep_plan(const SweepGrid& G, const std::vector<int>& level, SweepPlan* P,
+                    std::vector<int>& order, const Span& span) {
+  const int n = G.n;
+  int nlev = 0;
+  for (int i = 0; i < n; i++) nlev = std::max(nlev, level[i] + 1);
+  std::vector<int> first(nlev + 1, 0), by_level(std::max(n, 1));
+  for (int i = 0; i < n; i++) first[level[i] + 1]++;
+  for (int l = 0; l < nlev; l++) first[l + 1] += first[l];
+  for (int i = 0; i < n; i++) by_level[first[level[i]]++] = i;
+  // dealt to the blocks in level order
+  const int per = std::max(1, G.max_rows);
+  std::vector<int> at(G.h_blk.begin(), G.h_blk.end());
+  order.assign(std::max(n, 1), 0);
+  for (int q = 0; q < n; q++) order[at[by_level[q] / per]++] = by_level[q];
+  std::vector<int4> item;
+  std::vector<int> cta_item(G.ctas + 1, 0), steps(G.ctas, 0);
+  std::vector<int4> sp(std::max(n, 1));
+  for (int c = 0; c < G.ctas; c++) {
+    cta_item[c] = (int)item.size();
+    for (int i = G.h_blk[c]; i < G.h_blk[c + 1];) {
+      // a step: up to kSweepStep items of one level; its last item makes up
+      // the barrier's count
+      const int lev = level[order[i]];
+      int q = 0;
+      for (; q < kSweepStep && i < G.h_blk[c + 1] && level[order[i]] == lev; q++) {
+        const int s = i;
+        while (i < G.h_blk[c + 1] && i - s < 32 && level[order[i]] == lev) i++;
+        item.push_back(make_int4(s, i - s, steps[c], 1));
+      }
+      item.back().w = kSweepStep - (q - 1);
+      steps[c]++;
+    }
+  }
+  cta_item[G.ctas] = (int)item.size();
+  for (int i = 0; i < n; i++) sp[i] = span(i, order[i]);
+  SB2_CUDA_TRY(cudaMalloc(&P->d_rows, sizeof(int) * std::max(n, 1)));
+  SB2_CUDA_TRY(cudaMalloc(&P->d_span, sizeof(int4) * std::max(n, 1)));
+  SB2_CUDA_TRY(cudaMalloc(&P->d_item, sizeof(int4) * std::max<size_t>(item.size(), 1)));
+  SB2_CUDA_TRY(cudaMalloc(&P->d_cta_item, sizeof(int) * cta_item.size()));
+  SB2_CUDA_TRY(cudaMemcpy(P->d_rows, order.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
+  SB2_CUDA_TRY(cudaMemcpy(P->d_span, sp.data(), sizeof(int4) * n, cudaMemcpyHostToDevice));
+  SB2_CUDA_TRY(cudaMemcpy(P->d_item, item.data(), sizeof(int4) * item.size(), cudaMemcpyHostToDevice));
+  SB2_CUDA_TRY(cudaMalloc(&P->d_steps, sizeof(int) * G.ctas));
+  SB2_CUDA_TRY(cudaMemcpy(P->d_steps, steps.data(), sizeof(int) * G.ctas, cudaMemcpyHostToDevice));
+  SB2_CUDA_TRY(cudaMemcpy(P->d_cta_item, cta_item.data(), sizeof(int) * cta_item.size(), cudaMemcpyHostToDevice));
+  return SB2_OK;
+}
+
+#ifdef __CUDACC__
+
+// ------------------------------------------------------------------ waiting
+
+__device__ __forceinline__ bool is_fill(double v) {
+  return (unsigned long long)__double_as_longlong(v) == kSweepFill;
+}
+
+// A value made by copying, never the fill.
+__device__ __forceinline__ double not_fill(double v) {
+  return is_fill(v) ? __longlong_as_double((long long)(kSweepFill | 0x0008000000000000ull)) : v;
+}
+
+__device__ __forceinline__ double ld_shared(unsigned at) {
+  double v;
+  asm volatile("ld.volatile.shared.f64 %0, [%1];" : "=d"(v) : "r"(at) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_shared(unsigned at, double v) {
+  asm volatile("st.volatile.shared.f64 [%0], %1;" ::"r"(at), "d"(v) : "memory");
+}
+__device__ __forceinline__ double ld_volatile(const double* p) {
+  return *reinterpret_cast<const volatile double*>(p);
+}
+
+// Step barriers: mbarriers of this CTA.  A waiting warp is suspended by the
+// hardware, where polling loops would take issue slots from the warp that the
+// others wait for.
+__device__ __forceinline__ unsigned smem_u32(const void* p) {
+  return (unsigned)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ void mbar_init(unsigned long long* b, unsigned count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned long long* b, unsigned count) {
+  asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(count)
+               : "memory");
+}
+// whether the phase of this parity is complete, suspended until it is or a
+// system-defined time has passed; the second form does not wait
+__device__ __forceinline__ bool mbar_try_wait(unsigned long long* b, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n .reg .pred p;\n"
+      " mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n"
+      " selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(ok)
+      : "r"(smem_u32(b)), "r"(parity)
+      : "memory");
+  return ok != 0u;
+}
+__device__ __forceinline__ bool mbar_test_wait(unsigned long long* b, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n .reg .pred p;\n"
+      " mbarrier.test_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n"
+      " selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(ok)
+      : "r"(smem_u32(b)), "r"(parity)
+      : "memory");
+  return ok != 0u;
+}
+
+// State of a warp's waits: gives up when the grid was told to leave, or when
+// no CTA has finished an item for wait_ns.
+struct SweepWait {
+  unsigned* state;
+  int ctas;
+  unsigned long long wait_ns;
+  __device__ __forceinline__ unsigned progress() const {
+    unsigned s = 0;
+    for (int c = 0; c < ctas; c++) s = s * 31u + *((volatile unsigned*)state + 2 + c);
+    return s;
+  }
+  // called now and then by a waiting warp; false: leave.  (The progress words
+  // are read only when the limit has passed: reading them takes microseconds.)
+  __device__ __noinline__ bool go_on(unsigned long long& t0, unsigned& seen) const {
+    if (*((volatile unsigned*)state) != 0u) return false;
+    const unsigned long long t = global_timer_ns();
+    if (t0 == 0ull) t0 = t;
+    if (t - t0 <= wait_ns) return true;
+    const unsigned p = progress() | 1u;
+    if (p != seen) {
+      seen = p;
+      t0 = t;
+      return true;
+    }
+    atomicExch(state, 1u);
+    atomicExch(state + 1, 1u);
+    return false;
+  }
+};
+
+// The values of one vector: those of the CTA's own rows in its shared memory
+// at `own`, all of them in global memory.
+struct SweepSource {
+  const double* g;
+  unsigned own;
+};
+
+// ------------------------------------------------------------------ row operations
+// An operation describes one row's new value as a sequence of entries (column,
+// coefficient) to be taken in order:
+//   Row r = op.load(ph, fwd, j, span)     what does not depend on other rows
+//   op.entry(r, k, c, a)                  entry k of r.len
+//   op.is_new(r, k, c)                    it reads this sweep's value of c
+//   op.first(r, s, xj)                    xj: the row's value before the sweep
+//   op.take(r, s, k, c, a, x)             entry k with the value x of column c
+//   op.lead(r, s, k)                      entries 0..k-1 are taken, none new
+//   op.last(r, s)                         the new value
+
+// Division by a divisor known ahead: y = RN(1 / b) is made before the row's
+// turn, and two of Markstein's correction steps (IBM J. Res. Dev. 34, 1990:
+// q' = q + y (a - b q), the remainder exact by fma) give RN(a / b) where no
+// intermediate leaves the normal range.  The full division, several hundred
+// cycles of one warp, stays for the operands outside it.
+struct Divisor {
+  double b, y;  // y = 0: use the full division
+  __device__ __forceinline__ explicit Divisor(double v) : b(v), y(0.0) {
+    const double m = fabs(v);
+    if (m > 0x1p-400 && m < 0x1p400) y = __drcp_rn(v);
+  }
+  __device__ __forceinline__ Divisor() : b(1.0), y(0.0) {}
+  __device__ __forceinline__ double divide(double a) const {
+    const double m = fabs(a);
+    if (y != 0.0 && m > 0x1p-500 && m < 0x1p500) {
+      double q = __dmul_rn(a, y);
+      q = __fma_rn(__fma_rn(-b, q, a), y, q);
+      return __fma_rn(__fma_rn(-b, q, a), y, q);
+    }
+    return __ddiv_rn(a, b);
+  }
+};
+
+// RowSparse sweep (Relaxation_MatVect.cxx:69-77 / :83-91).  span.x..y: row j.
+struct GeneralSor {
+  static constexpr int kAhead = 8, kThreads = 384;
+  const int* ind; const double* val; const double* diag;
+  const double* b; const double* x0; double omega, rest;  // rest = 1 - omega
+  struct Row { int j, k0, len; bool fwd; double bj; Divisor ajj; };
+  struct Sum { double temp, xj; };
+  __device__ __forceinline__ Row load(int, bool fwd, int j, const int4& sp) const {
+    return Row{j, sp.x, sp.y - sp.x, fwd, __ldg(b + j), Divisor(__ldg(diag + j))};
+  }
+  __device__ __forceinline__ void entry(const Row& r, int k, int& c, double& a) const {
+    c = __ldg(ind + r.k0 + k);
+    a = __ldg(val + r.k0 + k);
+  }
+  __device__ __forceinline__ bool is_new(const Row& r, int, int c) const {
+    return r.fwd ? c < r.j : c > r.j;
+  }
+  __device__ __forceinline__ void first(const Row&, Sum& s, double xj) const {
+    s.temp = 0.0;
+    s.xj = xj;
+  }
+  __device__ __forceinline__ void take(const Row&, Sum& s, int, int, double a, double x) const {
+    s.temp = add_rn(s.temp, mul_rn(a, x));
+  }
+  __device__ __forceinline__ void lead(const Row&, Sum&, int) const {}
+  __device__ __forceinline__ double last(const Row& r, const Sum& s) const {
+    const double temp = add_rn(__dsub_rn(r.bj, s.temp), mul_rn(r.ajj.b, s.xj));
+    return add_rn(mul_rn(rest, s.xj), r.ajj.divide(mul_rn(omega, temp)));
+  }
+  __device__ __forceinline__ void store(const Row&, double) const {}
+};
+
+// RowSymSparse sweeps.  span.x..y: the stored (upper) row j; span.z..w: the
+// mirrored entries of row j (columns < j, increasing) in the full pattern;
+// diag: the sum of the row's diagonal entries.
+// Forward (Relaxation_MatVect.cxx:214-249): t = ((1-w)/w * ajj) * x_j +
+// (b_j - sum_{p != j} a_jp x_p), x read old, then x_j = (t - sum a_kj x_k) *
+// (w / ajj), the x_k new and k increasing: the stored entries, then the
+// mirrored ones.  Backward (:257-294): y = sum a_kj x_k, old; t =
+// (((1-w)/w * ajj) * x_j + b_j) - y; x_j = ((t - sum_{p != j} a_jp x_p) * w) /
+// ajj, the x_p new: the mirrored entries, then the stored ones.
+struct SymmetricSor {
+  static constexpr int kAhead = 8, kThreads = 384;
+  const int* uind; const double* uval; const int* find; const double* fval;
+  const double* diag; const double* b; const double* x0;
+  double omega, ratio;  // ratio = (1 - omega) / omega
+  struct Row { int j, u0, f0, nu, len; bool fwd; double bj, scale; Divisor ajj; };
+  struct Sum { double temp, t, xj; bool started; };
+  __device__ __forceinline__ Row load(int, bool fwd, int j, const int4& sp) const {
+    const Divisor d(__ldg(diag + j));
+    return Row{j, sp.x, sp.z, sp.y - sp.x, sp.y - sp.x + sp.w - sp.z, fwd, __ldg(b + j),
+               fwd ? __ddiv_rn(omega, d.b) : 0.0, d};
+  }
+  __device__ __forceinline__ bool stored(const Row& r, int k) const {
+    return r.fwd ? k < r.nu : k >= r.len - r.nu;
+  }
+  __device__ __forceinline__ void entry(const Row& r, int k, int& c, double& a) const {
+    const bool st = stored(r, k);
+    const int q = st ? r.u0 + (r.fwd ? k : k - (r.len - r.nu)) : r.f0 + (r.fwd ? k - r.nu : k);
+    c = __ldg((st ? uind : find) + q);
+    a = __ldg((st ? uval : fval) + q);
+  }
+  __device__ __forceinline__ bool is_new(const Row& r, int k, int c) const {
+    return r.fwd ? k >= r.nu : stored(r, k) && c != r.j;
+  }
+  __device__ __forceinline__ void first(const Row&, Sum& s, double xj) const {
+    s.temp = s.t = 0.0;
+    s.xj = xj;
+    s.started = false;
+  }
+  // t before the entries that read new values
+  __device__ __forceinline__ void start(const Row& r, Sum& s) const {
+    const double q = mul_rn(mul_rn(ratio, r.ajj.b), s.xj);
+    s.t = r.fwd ? add_rn(q, __dsub_rn(r.bj, s.temp)) : __dsub_rn(add_rn(q, r.bj), s.t);
+    s.started = true;
+  }
+  __device__ __forceinline__ int olds(const Row& r) const { return r.fwd ? r.nu : r.len - r.nu; }
+  __device__ __forceinline__ void take(const Row& r, Sum& s, int k, int c, double a, double x) const {
+    if (!s.started && k >= olds(r)) start(r, s);
+    if (stored(r, k)) {
+      if (c != r.j) s.temp = add_rn(s.temp, mul_rn(a, x));
+    } else if (r.fwd) {
+      s.t = __dsub_rn(s.t, mul_rn(a, x));
+    } else {
+      s.t = add_rn(s.t, mul_rn(a, x));
+    }
+  }
+  __device__ __forceinline__ void lead(const Row& r, Sum& s, int k) const {
+    if (!s.started && k >= olds(r)) start(r, s);
+  }
+  __device__ __forceinline__ double last(const Row& r, Sum& s) const {
+    if (!s.started) start(r, s);
+    return r.fwd ? mul_rn(s.t, r.scale) : r.ajj.divide(mul_rn(__dsub_rn(s.t, s.temp), omega));
+  }
+  __device__ __forceinline__ void store(const Row&, double) const {}
+};
+
+// The two sweeps of an ILUT apply in gather form: x_j = (x_j * pre_j - v_1
+// x_{c1} - v_2 x_{c2} - ...) * post_j, the subtractions in the listed order
+// (pre and post may be null).  The first sweep starts from r through the
+// input permutation, the second from the first's values; its results also go
+// to z through the output permutation.  span.x..y: the row's update list.
+struct FactorSolve {
+  static constexpr int kAhead = 4, kThreads = 384;
+  const int* ind[2]; const double* val[2];
+  const double* pre[2]; const double* post[2];
+  const double* r; const int* in_at;
+  double* z; const int* out_at;
+  struct Row { int ph, k0, len, out; double in, pre, post; bool has_pre, has_post; };
+  struct Sum { double t; };
+  __device__ __forceinline__ Row load(int ph, bool, int j, const int4& sp) const {
+    const double* pr = ph ? pre[1] : pre[0];
+    const double* po = ph ? post[1] : post[0];
+    return Row{ph, sp.x, sp.y - sp.x, ph ? __ldg(out_at + j) : 0,
+               ph ? 0.0 : __ldg(r + __ldg(in_at + j)),
+               pr ? __ldg(pr + j) : 0.0, po ? __ldg(po + j) : 0.0, pr != nullptr, po != nullptr};
+  }
+  __device__ __forceinline__ void entry(const Row& r, int k, int& c, double& a) const {
+    c = __ldg((r.ph ? ind[1] : ind[0]) + r.k0 + k);
+    a = __ldg((r.ph ? val[1] : val[0]) + r.k0 + k);
+  }
+  __device__ __forceinline__ bool is_new(const Row&, int, int) const { return true; }
+  __device__ __forceinline__ void first(const Row& r, Sum& s, double xj) const {
+    s.t = r.ph ? xj : r.in;
+    if (r.has_pre) s.t = mul_rn(s.t, r.pre);
+  }
+  __device__ __forceinline__ void take(const Row&, Sum& s, int, int, double a, double x) const {
+    s.t = __dsub_rn(s.t, mul_rn(a, x));
+  }
+  __device__ __forceinline__ void lead(const Row&, Sum&, int) const {}
+  __device__ __forceinline__ double last(const Row& r, const Sum& s) const {
+    return r.has_post ? mul_rn(s.t, r.post) : s.t;
+  }
+  __device__ __forceinline__ void store(const Row& r, double v) const {
+    if (r.ph == 1) z[r.out] = v;
+  }
+};
+
+// x0 of an operation that reads values from before the first sweep
+template <class Op>
+__device__ __forceinline__ const double* sweep_start(const Op& op) { return op.x0; }
+__device__ __forceinline__ const double* sweep_start(const FactorSolve&) { return nullptr; }
+
+// ------------------------------------------------------------------ the kernel
+
+template <class Op, bool OWN>
+__global__ void __launch_bounds__(Op::kThreads, 1) sweep_kernel(SweepArgs a, Op op) {
+  extern __shared__ double s_own[];
+  __shared__ unsigned long long s_bar[kSweepRing];  // step s completes s_bar[s % ring]
+  constexpr int U = Op::kAhead, W = Op::kThreads / 32;
+  static_assert(W + 2 < kSweepRing, "a warp may be W items ahead of the oldest unfinished step");
+  const int c0 = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int r0 = __ldg(a.blk + c0), rows = __ldg(a.blk + c0 + 1) - r0;
+  if (threadIdx.x < kSweepRing) mbar_init(&s_bar[threadIdx.x], kSweepStep);
+  const SweepWait w{a.state, (int)gridDim.x, a.wait_ns};
+  const double* x0 = sweep_start(op);
+  SweepSource old{nullptr, 0u};
+  int base = 0;  // this CTA's steps of the sweeps before
+  bool ok = true;
+  for (int ph = 0; ph < a.nph; ph++) {
+    // every value of the CTA's rows from the sweep before is in place
+    if (__syncthreads_or(!ok)) return;
+    const SweepPhase P = ph ? a.ph[1] : a.ph[0];
+    const SweepSource fresh{P.out, OWN ? smem_u32(s_own + (size_t)ph * a.max_rows) : 0u};
+    const bool fwd = P.forward != 0;
+    const int it0 = __ldg(P.cta_item + c0), it1 = __ldg(P.cta_item + c0 + 1);
+    // the next item's row and entry ranges are loaded an item ahead
+    int4 item = make_int4(0, 0, 0, 0);
+    int j = -1;
+    int4 span = make_int4(0, 0, 0, 0);
+    auto fetch = [&](int q) {
+      j = -1;
+      if (q >= it1) return;
+      item = __ldg(P.item + q);
+      if (lane < item.y) {
+        j = __ldg(P.rows + item.x + lane);
+        span = __ldg(P.span + item.x + lane);
+      }
+    };
+    fetch(it0 + warp);
+    for (int it = it0 + warp; it < it1 && ok; it += W) {
+      const bool live = j >= 0;
+      const int row = j;
+      // this item's step, and what it adds to the step's barrier; the step
+      // before must be complete (it waited for the one before it, and so on)
+      const int step = base + item.z, arrivals = item.w;
+      typename Op::Row R = {};
+      typename Op::Sum s;
+      int c[U];
+      double f[U], x[U];
+      unsigned isnew = 0u, far = 0u, near = 0u;  // far: awaited in L2, near: in shared memory
+      double xj = 0.0;
+      if (live) {
+        R = op.load(ph, fwd, row, span);
+        if (ph == 0 && x0) xj = __ldcg(x0 + row);
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          c[u] = 0;
+          f[u] = 0.0;
+          if (u < R.len) op.entry(R, u, c[u], f[u]);
+        }
+      }
+      const int len = live ? R.len : 0;
+      fetch(it + W);
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        x[u] = 0.0;
+        if (u < len) {
+          const bool nw = op.is_new(R, u, c[u]);
+          if (nw) isnew |= 1u << u;
+          if (nw || ph == 1) {
+            if (OWN && (unsigned)(c[u] - r0) < (unsigned)rows) near |= 1u << u;
+            else far |= 1u << u;
+          } else if (x0) {
+            x[u] = __ldcg(x0 + c[u]);
+          }
+        }
+      }
+      // looks once at the values that other CTAs have yet to give
+      auto look = [&]() {
+        double y[U];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if (far >> u & 1u) y[u] = ld_volatile((isnew >> u & 1u ? fresh.g : old.g) + c[u]);
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if ((far >> u & 1u) && !is_fill(y[u])) {
+            x[u] = y[u];
+            far &= ~(1u << u);
+          }
+      };
+      unsigned long long t0 = 0ull;
+      unsigned seen = 0u, spin = 0u;
+      auto poll = [&](unsigned mask) -> bool {  // whether some lane still awaits an entry of `mask`
+        if (far) look();
+        if ((++spin & 1023u) == 0u && __any_sync(0xffffffffu, !w.go_on(t0, seen))) ok = false;
+        return __any_sync(0xffffffffu, (far & mask) != 0u);
+      };
+      // the values of the sweep before, and the entries that lead the row
+      // up to the first new one
+      const int lead = isnew ? min(__ffs(isnew) - 1, len) : min(len, U);
+      if (ph == 1) {
+        while (poll(~isnew) && ok) {}
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if ((near & ~isnew) >> u & 1u) x[u] = ld_shared(old.own + 8u * (unsigned)(c[u] - r0));
+        if (live) {
+          xj = OWN ? ld_shared(old.own + 8u * (unsigned)(row - r0)) : ld_volatile(old.g + row);
+        }
+      }
+      if (live) {
+        op.first(R, s, xj);
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if (u < lead) op.take(R, s, u, c[u], f[u], x[u]);
+        op.lead(R, s, lead);
+      }
+      near &= isnew;
+      // wait for the other CTAs' new values and for this CTA's earlier steps
+      while (ok) {
+        const bool more = poll(~0u);
+        unsigned long long* bar = &s_bar[(step - 1) & (kSweepRing - 1)];
+        const unsigned parity = (unsigned)((step - 1) / kSweepRing) & 1u;
+        const bool turn = step == 0 || (more ? mbar_test_wait(bar, parity) : mbar_try_wait(bar, parity));
+        if (__all_sync(0xffffffffu, !more && turn)) break;
+      }
+      if (live && ok) {
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if (near >> u & 1u) x[u] = ld_shared(fresh.own + 8u * (unsigned)(c[u] - r0));
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if (u >= lead && u < len) op.take(R, s, u, c[u], f[u], x[u]);
+        // rows longer than the entries held in registers
+        for (int k = U; k < len && ok; k++) {
+          int cc;
+          double ff, y = 0.0;
+          op.entry(R, k, cc, ff);
+          const bool nw = op.is_new(R, k, cc);
+          if (nw || ph == 1) {
+            const SweepSource& S = nw ? fresh : old;
+            const bool here = OWN && (unsigned)(cc - r0) < (unsigned)rows;
+            y = here ? ld_shared(S.own + 8u * (unsigned)(cc - r0)) : ld_volatile(S.g + cc);
+            for (unsigned n = 1; !here && is_fill(y); n++) {
+              if ((n & 255u) == 0u && !w.go_on(t0, seen)) {
+                ok = false;
+                break;
+              }
+              y = ld_volatile(S.g + cc);
+            }
+          } else if (x0) {
+            y = __ldcg(x0 + cc);
+          }
+          op.take(R, s, k, cc, ff, y);
+        }
+        if (ok) {
+          const double v = not_fill(op.last(R, s));
+          if (OWN) st_shared(fresh.own + 8u * (unsigned)(row - r0), v);
+          *((volatile double*)P.out + row) = v;
+          op.store(R, v);
+        }
+      }
+      ok = __all_sync(0xffffffffu, ok) != 0;
+      if (lane == 0 && ok) {
+        mbar_arrive(&s_bar[step & (kSweepRing - 1)], arrivals);
+        *((volatile unsigned*)a.state + 2 + c0) = (unsigned)step + 1u;
+      }
+    }
+    base += __ldg(P.steps + c0);
+    old = fresh;
+  }
+}
+
+// Sum of the diagonal entries of each stored row, in stored order (the
+// reference's ajj, Relaxation_MatVect.cxx:214-294).
+__global__ void sym_diag_kernel(int n, const int* __restrict__ ptr, const int* __restrict__ ind,
+                                const double* __restrict__ val, double* __restrict__ d) {
+  for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < n;
+       j += (long long)gridDim.x * blockDim.x) {
+    double ajj = 0.0;
+    for (int k = ptr[j]; k < ptr[j + 1]; k++)
+      if (ind[k] == j) ajj = add_rn(ajj, val[k]);
+    d[j] = ajj;
+  }
+}
+
+__global__ void __launch_bounds__(256) sweep_fill_kernel(int n, double* x, double* y,
+                                                         unsigned* state) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *state = 0u;
+  const double f = __longlong_as_double((long long)kSweepFill);
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x) {
+    x[i] = f;
+    if (y) y[i] = f;
+  }
+}
+
+// One launch of one or two sweeps; out1 null: one.
+template <class Op>
+int launch_sweeps(const SweepGrid& G, const SweepPlan* const (&plan)[2], const bool (&forward)[2],
+                  double* out0, double* out1, const Op& op, cudaStream_t s) {
+  const int n = G.n;
+  if (n == 0) return SB2_OK;
+  SweepArgs a;
+  a.blk = G.d_blk;
+  a.max_rows = G.max_rows;
+  a.nph = out1 ? 2 : 1;
+  double* out[2] = {out0, out1};
+  for (int k = 0; k < 2; k++) {
+    const SweepPlan& P = *plan[out1 ? k : 0];
+    a.ph[k] = SweepPhase{P.d_rows, P.d_span, P.d_item, P.d_cta_item, P.d_steps, forward[out1 ? k : 0] ? 1 : 0, out[k]};
+  }
+  a.state = G.d_state;
+  a.wait_ns = ring_wait_ns();
+  // values of the CTA's own rows stay in shared memory when both sweeps' fit
+  const size_t smem = sizeof(double) * (size_t)a.nph * G.max_rows;
+  const bool own = smem <= (size_t)kSweepSmem;
+  const int g = std::min((n + 255) / 256, num_sms(current_device()) * 8);
+  sweep_fill_kernel<<<g, 256, 0, s>>>(n, out0, out1, G.d_state);
+  SB2_CUDA_TRY(cudaGetLastError());
+  const void* kern = own ? (const void*)sweep_kernel<Op, true> : (const void*)sweep_kernel<Op, false>;
+  if (own && smem > 48 * 1024)
+    SB2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(G.ctas);
+  cfg.blockDim = dim3(Op::kThreads);
+  cfg.dynamicSmemBytes = own ? smem : 0;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;  // the CTAs wait for one another
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  void* args[2] = {(void*)&a, (void*)const_cast<Op*>(&op)};
+  SB2_CUDA_TRY(cudaLaunchKernelExC(&cfg, kern, args));
+  return SB2_OK;
+}
+
+#endif  // __CUDACC__
+
+}  // namespace sb2

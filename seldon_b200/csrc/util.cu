@@ -7,7 +7,6 @@
 
 namespace sb2 {
 
-std::atomic<long long> g_wait_limit_us{2000000};
 
 int map_cuda_error(cudaError_t e) {
   if (e == cudaSuccess) return SB2_OK;
