@@ -37,7 +37,8 @@ int precond_apply(const sb2_precond* M, bool trans, const double* r, double* z,
                   cudaStream_t s);
 int precond_check(const sb2_precond* M, cudaStream_t s);
 
-constexpr int NT = kSpmvThreads;
+// One CTA per SM: the grid barrier costs more with the number of CTAs.
+constexpr int NT = 1024;
 
 // ----------------------------------------------------------------- common
 
@@ -215,7 +216,7 @@ struct CgVecs {
   double *x, *r, *p, *q;
 };
 
-__global__ void __launch_bounds__(NT, 4) cg_fused_kernel(OpArgs A, CgVecs v, IterArgs it,
+__global__ void __launch_bounds__(NT, 1) cg_fused_kernel(OpArgs A, CgVecs v, IterArgs it,
                                                       Persist P, History H, SolveOut* out) {
   SB2_SHARED_DECL;
   const int tid = threadIdx.x;
@@ -374,7 +375,7 @@ struct EpiStoreDot2 {
   }
 };
 
-__global__ void __launch_bounds__(NT, 4) bicgstab_fused_kernel(OpArgs A, BicgVecs v, IterArgs it,
+__global__ void __launch_bounds__(NT, 1) bicgstab_fused_kernel(OpArgs A, BicgVecs v, IterArgs it,
                                                             Persist P, History H,
                                                             SolveOut* out) {
   SB2_SHARED_DECL;
@@ -594,7 +595,7 @@ struct EpiResidUpdate {
 
 // Cgs (Cgs.cxx:45-132): four grid barriers per loop, two products; the
 // second product is fused with the residual update and both reductions.
-__global__ void __launch_bounds__(NT, 4) cgs_fused_kernel(OpArgs A, CgsVecs v, IterArgs it,
+__global__ void __launch_bounds__(NT, 1) cgs_fused_kernel(OpArgs A, CgsVecs v, IterArgs it,
                                                        Persist P, History H, SolveOut* out) {
   SB2_SHARED_DECL;
   const int tid = threadIdx.x;
@@ -876,7 +877,7 @@ struct EpiTfqmrNextV {
 // TfQmr (TfQmr.cxx:44-243), left preconditioned: four grid barriers and two
 // products per loop of two half steps.  The vector work of each half step
 // rides in the epilogue of the product that follows it.
-__global__ void __launch_bounds__(NT, 4) tfqmr_fused_kernel(OpArgs A, TfqmrVecs v, IterArgs it,
+__global__ void __launch_bounds__(NT, 1) tfqmr_fused_kernel(OpArgs A, TfqmrVecs v, IterArgs it,
                                                          Persist P, History H, SolveOut* out) {
   SB2_SHARED_DECL;
   const int tid = threadIdx.x;
@@ -1049,7 +1050,7 @@ struct MinresVecs {
 // rotations of the buffers: every thread swaps the same register pointers.  The
 // scalar recurrences are rounded step by step (mul_rn / add_rn), as the
 // reference's separately rounded products and sums.
-__global__ void __launch_bounds__(NT, 4) minres_fused_kernel(OpArgs A, MinresVecs v, IterArgs it,
+__global__ void __launch_bounds__(NT, 1) minres_fused_kernel(OpArgs A, MinresVecs v, IterArgs it,
                                                           Persist P, History H, SolveOut* out) {
   SB2_SHARED_DECL;
   const int tid = threadIdx.x;
@@ -1313,7 +1314,7 @@ struct EpiGcrQ {
 // the reference's two Finished() calls are.  Where the reference never
 // returns -- a cycle whose inner loop takes no step, which every later cycle
 // then repeats -- the solve stops after that cycle.
-__global__ void __launch_bounds__(NT, 4) gcr_fused_kernel(OpArgs A, GcrVecs v, IterArgs it,
+__global__ void __launch_bounds__(NT, 1) gcr_fused_kernel(OpArgs A, GcrVecs v, IterArgs it,
                                                        Persist P, History H, SolveOut* out) {
   SB2_SHARED_DECL;
   __shared__ double s_beta[kGcrMaxRestart + 1];
@@ -1511,7 +1512,7 @@ struct EpiBiclInit {
 // as in the reference; tau and the gammas carry over between cycles.  x is
 // mapped back by M^{-1} at the end.  Where the reference can repeat a cycle
 // for ever (one that counts no iteration) the solve stops after it.
-__global__ void __launch_bounds__(NT, 4) bicgstabl_fused_kernel(OpArgs A, BicglVecs v,
+__global__ void __launch_bounds__(NT, 1) bicgstabl_fused_kernel(OpArgs A, BicglVecs v,
                                                              IterArgs it, Persist P, History H,
                                                              SolveOut* out) {
   SB2_SHARED_DECL;
@@ -1822,7 +1823,7 @@ struct EpiQcgsFit {
 // new u = r_qcgs - r and four projections; the smoothing pass with
 // ||r_qcgs||^2 and the next (rtilde, r).  x becomes M^{-1} x_qcgs at the
 // end, breakdown or not, as in the reference.
-__global__ void __launch_bounds__(NT, 4) qcgs_fused_kernel(OpArgs A, QcgsVecs v, IterArgs it,
+__global__ void __launch_bounds__(NT, 1) qcgs_fused_kernel(OpArgs A, QcgsVecs v, IterArgs it,
                                                         Persist P, History H, SolveOut* out) {
   SB2_SHARED_DECL;
   const int tid = threadIdx.x;
@@ -2040,7 +2041,7 @@ struct EpiStore {
 // Seldon's Mlt(SeldonTrans, ...) sums row i of the transpose in increasing
 // index order (Functions_MatVect.cxx:1279-1317), which is what the product
 // over the explicit transpose (or the expanded symmetric pattern) does.
-__global__ void __launch_bounds__(NT, 4) bicg_fused_kernel(OpArgs A, BcgVecs v, IterArgs it,
+__global__ void __launch_bounds__(NT, 1) bicg_fused_kernel(OpArgs A, BcgVecs v, IterArgs it,
                                                         Persist P, History H, SolveOut* out) {
   SB2_SHARED_DECL;
   const int tid = threadIdx.x;
@@ -2222,7 +2223,7 @@ struct EpiStoreNorm {
 // update pass with ||r||^2 and the next rho = (r, M^{-1} M^{-T} r).  The
 // first test is on ||A^T b|| even from an initial guess, as in the
 // reference.
-__global__ void __launch_bounds__(NT, 4) cgne_fused_kernel(OpArgs A, CgneVecs v, IterArgs it,
+__global__ void __launch_bounds__(NT, 1) cgne_fused_kernel(OpArgs A, CgneVecs v, IterArgs it,
                                                         Persist P, History H, SolveOut* out) {
   SB2_SHARED_DECL;
   const int tid = threadIdx.x;
@@ -2364,7 +2365,7 @@ struct SymmlqVecs {
 // r -= alpha v + beta v_old, z -= alpha u + beta u_old with (r, z).  The
 // first test is on ||b|| even from an initial guess; x takes
 // ceta_bar * w_bar after the loop, as in the reference.
-__global__ void __launch_bounds__(NT, 4) symmlq_fused_kernel(OpArgs A, SymmlqVecs v, IterArgs it,
+__global__ void __launch_bounds__(NT, 1) symmlq_fused_kernel(OpArgs A, SymmlqVecs v, IterArgs it,
                                                           Persist P, History H, SolveOut* out) {
   SB2_SHARED_DECL;
   const int tid = threadIdx.x;
@@ -2566,7 +2567,7 @@ struct QmrsVecs {
 // delta = (v, y) (the reference scales them at the top of its next step,
 // after the test, which reads neither).  Fail codes 1, 3, 4, 5, 6 as in the
 // reference.
-__global__ void __launch_bounds__(NT, 4) qmrsym_fused_kernel(OpArgs A, QmrsVecs v, IterArgs it,
+__global__ void __launch_bounds__(NT, 1) qmrsym_fused_kernel(OpArgs A, QmrsVecs v, IterArgs it,
                                                           Persist P, History H, SolveOut* out) {
   SB2_SHARED_DECL;
   const int tid = threadIdx.x;
@@ -2791,7 +2792,7 @@ struct EpiAxpyNorm {
 // loop (two counted iterations): u1 = A v - alpha u with ||u1||^2; u1 /=
 // beta; v1 = A^T u1 - beta v with ||v1||^2; the pass that scales v1 and
 // updates x and w.  u, u1 and v, v1 swap by pointer.
-__global__ void __launch_bounds__(NT, 4) lsqr_fused_kernel(OpArgs A, LsqrVecs v, IterArgs it,
+__global__ void __launch_bounds__(NT, 1) lsqr_fused_kernel(OpArgs A, LsqrVecs v, IterArgs it,
                                                         Persist P, History H, SolveOut* out) {
   SB2_SHARED_DECL;
   const int tid = threadIdx.x;
@@ -2957,7 +2958,7 @@ struct EpiBcrA {
 // the p, a, w pass with ||v||^2 and the next step's rho = (w, v) and
 // mu = (w, a).  The count starts at 1: the reference counts the first
 // product a = A p before its first test.
-__global__ void __launch_bounds__(NT, 4) bicgcr_fused_kernel(OpArgs A, BcrVecs v, IterArgs it,
+__global__ void __launch_bounds__(NT, 1) bicgcr_fused_kernel(OpArgs A, BcrVecs v, IterArgs it,
                                                           Persist P, History H, SolveOut* out) {
   SB2_SHARED_DECL;
   const int tid = threadIdx.x;
@@ -3125,7 +3126,7 @@ struct EpiPrecDot {
   }
 };
 
-__global__ void __launch_bounds__(NT, 4) gmres_fused_kernel(OpArgs A, GmresVecs v, IterArgs it,
+__global__ void __launch_bounds__(NT, 1) gmres_fused_kernel(OpArgs A, GmresVecs v, IterArgs it,
                                                          Persist P, History H, SolveOut* out) {
   SB2_SHARED_DECL;
   extern __shared__ double s_dyn[];
@@ -3333,7 +3334,7 @@ static int alloc_scratch(cudaStream_t s, int n, int nvec, int grid, int hist_cap
   SB2_CUDA_TRY(pool_malloc((void**)&S->vecs.p, vbytes, s));
   S->vec = (double*)S->vecs.p;
   S->hist_cap = std::max(hist_cap, 1);
-  const size_t sync_b = 256, part_b = sizeof(double) * kMaxRed * grid, out_b = 256;
+  const size_t sync_b = 256, part_b = sizeof(double) * 2 * kMaxRed * grid, out_b = 256;
   const size_t hist_b = sizeof(double) * S->hist_cap, hit_b = sizeof(int) * S->hist_cap;
   const size_t total = sync_b + ((part_b + 255) / 256) * 256 + out_b + ((hist_b + 255) / 256) * 256 + hit_b;
   SB2_CUDA_TRY(pool_malloc((void**)&S->state.p, total, s));
@@ -3357,10 +3358,9 @@ static int coop_grid(const void* kernel, size_t smem, const sb2_csr* A) {
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, NT, smem) != cudaSuccess ||
       per_sm < 1)
     return 0;
-  const int cap = per_sm * num_sms(dev);
-  const int n = A->m;
+  const int cap = std::min(kPersistMaxCtas, num_sms(dev));
   // enough CTAs to cover the work, no more: a small grid makes the barriers cheap
-  const int want = std::max((n + NT * 4 - 1) / (NT * 4), (A->full.part.nblk + 1) / 2);
+  const int want = (A->m + NT - 1) / NT;
   return std::max(1, std::min(cap, want));
 }
 
@@ -5136,9 +5136,8 @@ namespace sb2 {
 // loads this library (about 3.2 MB each) until the process exits, and every
 // call on a GPU reuses the same array.
 constexpr int kNoAllocMaxN = 131072;
-constexpr int kNoAllocMaxGrid = 2048;
 constexpr size_t kNoAllocVec = 3 * (size_t)kNoAllocMaxN;
-constexpr size_t kNoAllocPart = (size_t)kMaxRed * kNoAllocMaxGrid;
+constexpr size_t kNoAllocPart = 2 * (size_t)kMaxRed * kPersistMaxCtas;
 constexpr size_t kNoAllocDoubles = kNoAllocVec + kNoAllocPart + 64 + 64 + 16;
 static __device__ __align__(256) double g_cg_noalloc_scratch[kNoAllocDoubles];
 
@@ -5170,7 +5169,6 @@ static int cg_noalloc(const sb2_csr* A, double* x, const double* b, const sb2_it
   if (A->m <= 0) return SB2_OK;
   const int grid = coop_grid((const void*)cg_fused_kernel, 0, A);
   if (grid < 1) return SB2_ERR_CUDA;
-  if (grid > kNoAllocMaxGrid) return SB2_ERR_NOT_SUPPORTED;
   double* base = nullptr;
   SB2_TRY(cg_noalloc_scratch(&base));
   const size_t n = (size_t)A->m;

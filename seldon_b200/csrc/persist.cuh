@@ -13,12 +13,13 @@ namespace sb2 {
 
 constexpr int kMaxRed = 8;  // scalars reduced by one barrier at most
 
+constexpr int kPersistMaxCtas = 160;  // one CTA per SM
+
 struct GridSync {
-  unsigned count;  // arrivals at the current barrier
-  unsigned gen;    // barrier generation
+  unsigned count;  // arrivals (grid_sync: since the launch; grid_sync_wide: at this barrier)
+  unsigned gen;    // generation (grid_sync_wide)
   int status;      // 0 ok, 1 a wait ran out
   int pad;
-  double res[kMaxRed];
 };
 
 struct SolveOut {
@@ -32,7 +33,7 @@ struct SolveOut {
 
 struct Persist {
   GridSync* sync;
-  double* partials;  // [kMaxRed * gridDim.x]
+  double* partials;  // deposits (grid_sync: [2 * kMaxRed * gridDim.x])
   unsigned long long wait_ns;
 };
 
@@ -45,66 +46,68 @@ struct History {
 
 #ifdef __CUDACC__
 
-// Grid barrier.  Thread 0 of each CTA deposits K block sums (s_vals[0..K)),
-// the last CTA to arrive sums the deposits in CTA order (the same tree on
-// every run), publishes them and releases the grid; on return s_vals holds
-// the K grid sums in every CTA.  Returns false when a wait ran out or another
-// CTA reported so.
+// Grid barrier.  Each CTA deposits K block sums (s_vals[0..K), written by
+// thread 0) and adds one to a counter; when all have, every CTA adds the
+// deposits in CTA order (the same tree on every run and in every CTA).  On
+// return s_vals holds the K grid sums.  False when a wait ran out; the other
+// CTAs then run out of theirs.
+// It costs one red.release and the polling load that sees it, and with K > 0
+// one more trip for the deposits: 1.4 us and 2.2 us at 148 CTAs.  The form it
+// replaced (the last CTA to arrive sums and releases the others, 592 CTAs of
+// 256 threads) took 2.8 us; deposits that carry their own tags, polled by
+// every CTA, 3.7 us: a line that 148 SMs poll is slow to write.
+// The counter only grows; deposits alternate between two sets, since a CTA
+// can be one barrier ahead of another, never two.
 template <int NT>
 __device__ __forceinline__ bool grid_sync(const Persist& P, unsigned& epoch, int K,
                                           double* s_vals, double* s_red) {
-  __shared__ int s_last, s_ok;  // separate: a lagging warp may still read s_last
-  const int tid = threadIdx.x;
-  const unsigned G = gridDim.x;
-  if (tid == 0)
-    for (int k = 0; k < K; k++) P.partials[k * G + blockIdx.x] = s_vals[k];
+  static_assert(NT / 32 >= kMaxRed, "one warp sums one value");
+  __shared__ int s_late;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int G = gridDim.x;
+  double* part = P.partials + (size_t)(epoch & 1u) * kMaxRed * G;
+  const unsigned target = ++epoch * (unsigned)G;
   __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    const unsigned prev = atomicAdd(&P.sync->count, 1u);
-    s_last = (prev == G - 1) ? 1 : 0;
-  }
-  __syncthreads();
-  if (s_last) {
-    __threadfence();
-    for (int k = 0; k < K; k++) {
-      const double* pv = P.partials + k * G;
-      double v0 = 0.0, v1 = 0.0;
-      unsigned i = tid;
-      for (; i + NT < G; i += 2 * NT) {
-        v0 = add_rn(v0, __ldcg(pv + i));
-        v1 = add_rn(v1, __ldcg(pv + i + NT));
+  if (warp == 0) {
+    if (lane < K) __stcg(part + (size_t)lane * G + blockIdx.x, s_vals[lane]);
+    __syncwarp();
+    if (lane == 0) {
+      red_release_u32(&P.sync->count, 1u);
+      const unsigned long long t0 = global_timer_ns();
+      int late = 0;
+      while ((int)(ld_acquire_u32(&P.sync->count) - target) < 0) {
+        if (global_timer_ns() - t0 > P.wait_ns) {
+          atomicExch(&P.sync->status, 1);
+          late = 1;
+          break;
+        }
       }
-      if (i < G) v0 = add_rn(v0, __ldcg(pv + i));
-      const double v = block_sum<NT>(add_rn(v0, v1), s_red);
-      if (tid == 0) P.sync->res[k] = v;
+      // a gpu-scope fence after the wait, as cooperative groups' grid.sync
+      // takes: with the CTA barrier below, the L1-cached gathers of the next
+      // phase (XLoadCa) see every write made before the barrier
+      asm volatile("fence.acq_rel.gpu;" ::: "memory");
+      s_late = late;
     }
-    if (tid == 0) {
-      P.sync->count = 0u;
-      __threadfence();
-      st_release_u32(&P.sync->gen, epoch + 1u);
-    }
-  } else if (tid == 0) {
-    const unsigned long long t0 = global_timer_ns();
-    while (ld_acquire_u32(&P.sync->gen) == epoch) {
-      if (global_timer_ns() - t0 > P.wait_ns) {
-        atomicExch(&P.sync->status, 1);
-        break;
-      }
-      __nanosleep(32);
-    }
-    // a gpu-scope fence after the wait, as cooperative groups' grid.sync
-    // takes: with the CTA barrier below, the L1-cached gathers of the next
-    // phase (XLoadCa) see every write made before the barrier
-    __threadfence();
-  }
-  if (tid == 0) {
-    for (int k = 0; k < K; k++) s_vals[k] = __ldcg(P.sync->res + k);
-    s_ok = (*((volatile int*)&P.sync->status) == 0) ? 1 : 0;
   }
   __syncthreads();
-  epoch++;
-  return s_ok != 0;
+  if (s_late) return false;
+  if (K) {
+    if (warp < K) {
+      double v = 0.0;
+      double in[(kPersistMaxCtas + 31) / 32];
+#pragma unroll
+      for (int q = 0; q < (kPersistMaxCtas + 31) / 32; q++) {
+        const int c = lane + 32 * q;
+        in[q] = c < G ? __ldcg(part + (size_t)warp * G + c) : 0.0;
+      }
+#pragma unroll
+      for (int q = 0; q < (kPersistMaxCtas + 31) / 32; q++) v = add_rn(v, in[q]);
+      v = warp_sum(v);
+      if (lane == 0) s_vals[warp] = v;
+    }
+    __syncthreads();
+  }
+  return true;
 }
 
 // Gathers of the product's operand inside a persistent kernel: cached in L1

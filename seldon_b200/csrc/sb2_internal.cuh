@@ -248,6 +248,10 @@ __device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+__device__ __forceinline__ void red_release_u32(unsigned* p, unsigned v) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
 __device__ __forceinline__ unsigned atom_add_acqrel_u32(unsigned* p, unsigned v) {
   unsigned old;
   asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;"
