@@ -229,6 +229,7 @@ int build_sell_host(const int* ptr, const int* ind, const double* val, int rows,
   out->ncta = (int)cr.size();
   SB2_CUDA_TRY(cudaMalloc(&out->d_sptr, sizeof(long long) * (ns + 1)));
   SB2_CUDA_TRY(cudaMemcpy(out->d_sptr, sptr.data(), sizeof(long long) * (ns + 1), cudaMemcpyHostToDevice));
+  out->h_sptr = sptr;
   SB2_CUDA_TRY(cudaMalloc(&out->d_qinfo, sizeof(uint2) * std::max<size_t>(qinfo.size(), 1)));
   if (!qinfo.empty())
     SB2_CUDA_TRY(cudaMemcpy(out->d_qinfo, qinfo.data(), sizeof(uint2) * qinfo.size(), cudaMemcpyHostToDevice));

@@ -22,6 +22,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <climits>
 #include <type_traits>
 #include <cmath>
 #include <vector>
@@ -39,6 +40,9 @@ int precond_check(const sb2_precond* M, cudaStream_t s);
 
 // One CTA per SM: the grid barrier costs more with the number of CTAs.
 constexpr int NT = 1024;
+
+// Rows sb2_cg_noalloc has scratch for.
+constexpr int kNoAllocMaxN = 131072;
 
 // ----------------------------------------------------------------- common
 
@@ -3296,6 +3300,12 @@ __global__ void __launch_bounds__(NT, 1) gmres_fused_kernel(OpArgs A, GmresVecs 
   if (lead) write_out(out, nb_iter, it.max_iter, 0, facteur, reste, hlen);
 }
 
+}  // namespace sb2
+
+#include "resident.cuh"
+
+namespace sb2 {
+
 // ----------------------------------------------------------------- launch glue
 
 struct DeviceBuf {
@@ -3327,10 +3337,11 @@ size_t vector_stride(int n, size_t elem_bytes) {
   return bytes / elem_bytes;
 }
 
+// nvec work vectors for n rows, then `extra` doubles, and the solve's state.
 static int alloc_scratch(cudaStream_t s, int n, int nvec, int grid, int hist_cap,
-                         SolveScratch* S) {
+                         SolveScratch* S, size_t extra = 0) {
   S->vecs.s = S->state.s = s;
-  const size_t vbytes = sizeof(double) * vector_stride(n, sizeof(double)) * nvec;
+  const size_t vbytes = sizeof(double) * (vector_stride(n, sizeof(double)) * nvec + extra);
   SB2_CUDA_TRY(pool_malloc((void**)&S->vecs.p, vbytes, s));
   S->vec = (double*)S->vecs.p;
   S->hist_cap = std::max(hist_cap, 1);
@@ -3531,6 +3542,74 @@ static int fused_solve(int which, const sb2_csr* A, const double* diag, double* 
   }
   SB2_CUDA_TRY(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(NT), args, smem, s));
   return finish_solve(S, s, res, hist, hist_it, hcap - 1 > 0 ? hcap - 1 : 0, prm->max_iter);
+}
+
+// ----------------------------------------------------------------- vectors on chip
+
+// 512 threads with the matrix on chip, where a phase is short and its barriers
+// matter; 1024 where the matrix streams and more loads in flight do.  (Two
+// quads a thread of 512 are more rows than fit with their part of the matrix.)
+static const void* gmres_resident(bool ms, int quads, int* threads) {
+  *threads = ms ? 512 : 1024;
+  const int qr = (quads + *threads - 1) / *threads;
+  if (ms) return qr <= 1 ? (const void*)gmres_resident_kernel<512, 1, true>
+                 : qr <= 2 ? (const void*)gmres_resident_kernel<512, 2, true> : nullptr;
+  return qr <= 1   ? (const void*)gmres_resident_kernel<1024, 1, false>
+         : qr <= 2 ? (const void*)gmres_resident_kernel<1024, 2, false>
+         : qr <= 4 ? (const void*)gmres_resident_kernel<1024, 4, false> : nullptr;
+}
+
+// Cg, BiCgStab or Gmres with the vectors in shared memory (resident.cuh), or
+// SB2_ERR_NOT_SUPPORTED where the operator has long or reordered rows or the
+// vectors of n rows do not fit the GPU's shared memory.
+static int resident_solve(int which, const sb2_csr* A, const double* diag, double* x,
+                          const double* b, const sb2_iter_params* prm, sb2_iter_result* res,
+                          double* hist, int* hist_it, int hist_cap, cudaStream_t s) {
+  const SellArrays& S = A->full.sell;
+  const int n = A->m, m = std::max(prm->restart, 1);
+  if (S.nslice <= 0 || S.sorted || S.nwarp || S.ncta || (int)S.h_sptr.size() != S.nslice + 1)
+    return SB2_ERR_NOT_SUPPORTED;
+  const bool jac = diag != nullptr;
+  const int sms = std::min(kPersistMaxCtas, num_sms(current_device()));
+  const int per = (S.nslice + sms - 1) / sms;
+  const int grid = (S.nslice + per - 1) / per;
+  const int nvec = which == kCg ? res_cg_vecs(jac) : which == kBicg ? res_bicg_vecs(jac) : 2;
+  size_t smem = sizeof(double) * (size_t)nvec * per * kQuadRows;
+  if (which == kGmres) smem += sizeof(double) * 4 * (size_t)((m + 4) / 4 * 4);
+  if (smem > (size_t)kResSmem) return SB2_ERR_NOT_SUPPORTED;
+  // the matrix too where it fits: 12 bytes an entry
+  long long groups = 0;
+  for (int c = 0; c < grid; c++)
+    groups = std::max(groups, S.h_sptr[std::min(S.nslice, (c + 1) * per)] - S.h_sptr[c * per]);
+  const bool ms = smem + 48 * (size_t)groups <= (size_t)kResSmem;
+  if (ms) smem += 48 * (size_t)groups;
+  // Cg and BiCgStab gain only with the matrix on chip
+  if (!ms && which != kGmres) return SB2_ERR_NOT_SUPPORTED;
+  int threads = 512;
+  const void* kern = which == kCg     ? (const void*)cg_resident_kernel<512, true>
+                     : which == kBicg ? (const void*)bicgstab_resident_kernel<512, true>
+                                      : gmres_resident(ms, per * 32, &threads);
+  if (!kern) return SB2_ERR_NOT_SUPPORTED;
+  SB2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // padded to whole quads of the last slice
+  const size_t nn = vector_stride(S.nslice * kQuadRows, sizeof(double));
+  const size_t hm = which == kGmres ? (size_t)grid * (m + 1) * (m + 1) : 0;
+  const int gvec = which == kGmres ? m + 1 : 3;
+  SolveScratch sc;
+  const int hcap = std::max(hist_cap, 0) + 1;
+  SB2_TRY(alloc_scratch(s, (int)std::min<size_t>(nn, INT_MAX), gvec, grid, hcap, &sc, hm));
+  Persist P{sc.sync, sc.partials, barrier_wait_ns()};
+  History H{sc.hist, sc.hist_it, hcap};
+  IterArgs it{prm->tol, prm->max_iter, m, prm->init_guess_null};
+  ResOp op{S.d_sptr, S.d_qinfo, S.d_scol, S.d_sval, diag, S.nslice, n, per, ms ? (int)groups : 0};
+  double* V = sc.vec;
+  CgResVecs cv{b, x, V, {V + nn, V + 2 * nn}};
+  BicgResVecs bv{b, x, V, V + nn, V + 2 * nn};
+  GmresResVecs gv{b, x, V, V + (size_t)gvec * nn, (long long)nn};
+  void* args[6] = {&op, which == kCg ? (void*)&cv : which == kBicg ? (void*)&bv : (void*)&gv, &it, &P, &H,
+                   &sc.out};
+  SB2_CUDA_TRY(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(threads), args, smem, s));
+  return finish_solve(sc, s, res, hist, hist_it, hcap - 1 > 0 ? hcap - 1 : 0, prm->max_iter);
 }
 
 // ----------------------------------------------------------------- host-driven drivers (SOR)
@@ -4958,6 +5037,11 @@ static int solve_entry(int which, const sb2_csr* A, const sb2_precond* M, double
     const int st = cluster_cg_solve(A, diag, x, b, prm, res, hist, hist_it, hist_cap, s);
     if (st != SB2_ERR_NOT_SUPPORTED) return st;
   }
+  // with its cluster form off, Cg keeps to the kernel that sb2_cg_noalloc runs
+  if ((which == kCg && (g_cluster_cg || A->m > kNoAllocMaxN)) || which == kBicg || which == kGmres) {
+    const int st = resident_solve(which, A, diag, x, b, prm, res, hist, hist_it, hist_cap, s);
+    if (st != SB2_ERR_NOT_SUPPORTED) return st;
+  }
   return fused_solve(which, A, diag, x, b, prm, res, hist, hist_it, hist_cap, s);
 }
 
@@ -5135,7 +5219,6 @@ namespace sb2 {
 // rows.  It is a file-scope device array, so it exists on every GPU that
 // loads this library (about 3.2 MB each) until the process exits, and every
 // call on a GPU reuses the same array.
-constexpr int kNoAllocMaxN = 131072;
 constexpr size_t kNoAllocVec = 3 * (size_t)kNoAllocMaxN;
 constexpr size_t kNoAllocPart = 2 * (size_t)kMaxRed * kPersistMaxCtas;
 constexpr size_t kNoAllocDoubles = kNoAllocVec + kNoAllocPart + 64 + 64 + 16;

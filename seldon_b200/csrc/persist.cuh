@@ -58,36 +58,48 @@ struct History {
 // every CTA, 3.7 us: a line that 148 SMs poll is slow to write.
 // The counter only grows; deposits alternate between two sets, since a CTA
 // can be one barrier ahead of another, never two.
+// grid_arrive and grid_wait are its halves: work between them overlaps the
+// trip.  Asynchronous copies belong there (a release waits for those its
+// thread has in flight), and then `fence` is false: without it grid_wait
+// orders only the sums, not other data of other CTAs.
 template <int NT>
-__device__ __forceinline__ bool grid_sync(const Persist& P, unsigned& epoch, int K,
-                                          double* s_vals, double* s_red) {
+__device__ __forceinline__ void grid_arrive(const Persist& P, unsigned& epoch, int K,
+                                            const double* s_vals) {
   static_assert(NT / 32 >= kMaxRed, "one warp sums one value");
+  const int lane = threadIdx.x & 31, G = gridDim.x;
+  double* part = P.partials + (size_t)(epoch & 1u) * kMaxRed * G;
+  epoch++;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    if (lane < K) __stcg(part + (size_t)lane * G + blockIdx.x, s_vals[lane]);
+    __syncwarp();
+    if (lane == 0) red_release_u32(&P.sync->count, 1u);
+  }
+}
+
+template <int NT>
+__device__ __forceinline__ bool grid_wait(const Persist& P, unsigned epoch, int K, double* s_vals,
+                                          bool fence) {
   __shared__ int s_late;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int G = gridDim.x;
-  double* part = P.partials + (size_t)(epoch & 1u) * kMaxRed * G;
-  const unsigned target = ++epoch * (unsigned)G;
-  __syncthreads();
-  if (warp == 0) {
-    if (lane < K) __stcg(part + (size_t)lane * G + blockIdx.x, s_vals[lane]);
-    __syncwarp();
-    if (lane == 0) {
-      red_release_u32(&P.sync->count, 1u);
-      const unsigned long long t0 = global_timer_ns();
-      int late = 0;
-      while ((int)(ld_acquire_u32(&P.sync->count) - target) < 0) {
-        if (global_timer_ns() - t0 > P.wait_ns) {
-          atomicExch(&P.sync->status, 1);
-          late = 1;
-          break;
-        }
+  const double* part = P.partials + (size_t)((epoch - 1u) & 1u) * kMaxRed * G;
+  const unsigned target = epoch * (unsigned)G;
+  if (tid == 0) {
+    const unsigned long long t0 = global_timer_ns();
+    int late = 0;
+    while ((int)(ld_acquire_u32(&P.sync->count) - target) < 0) {
+      if (global_timer_ns() - t0 > P.wait_ns) {
+        atomicExch(&P.sync->status, 1);
+        late = 1;
+        break;
       }
-      // a gpu-scope fence after the wait, as cooperative groups' grid.sync
-      // takes: with the CTA barrier below, the L1-cached gathers of the next
-      // phase (XLoadCa) see every write made before the barrier
-      asm volatile("fence.acq_rel.gpu;" ::: "memory");
-      s_late = late;
     }
+    // a gpu-scope fence after the wait, as cooperative groups' grid.sync
+    // takes: with the CTA barrier below, the L1-cached gathers of the next
+    // phase (XLoadCa) see every write made before the barrier
+    if (fence) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    s_late = late;
   }
   __syncthreads();
   if (s_late) return false;
@@ -108,6 +120,13 @@ __device__ __forceinline__ bool grid_sync(const Persist& P, unsigned& epoch, int
     __syncthreads();
   }
   return true;
+}
+
+template <int NT>
+__device__ __forceinline__ bool grid_sync(const Persist& P, unsigned& epoch, int K,
+                                          double* s_vals, double*) {
+  grid_arrive<NT>(P, epoch, K, s_vals);
+  return grid_wait<NT>(P, epoch, K, s_vals, true);
 }
 
 // Gathers of the product's operand inside a persistent kernel: cached in L1

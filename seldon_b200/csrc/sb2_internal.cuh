@@ -101,6 +101,7 @@ struct SellArrays {
   int* d_crows = nullptr;
   long long padded = 0;       // stored entries incl. padding
   bool sorted = false;
+  std::vector<long long> h_sptr;  // host copy of d_sptr
   long long* d_pos = nullptr; // SELL position of each CSR entry of the thread
                               // bin, -1 for entries of the warp/CTA bins
 };
