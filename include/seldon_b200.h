@@ -702,7 +702,10 @@ int sb2_batch_solve(const sb2_batch* B, double* x, const double* b,
                     const sb2_batch_params* params, int* d_iters, double* d_relres,
                     sb2_batch_result* result, void* stream);
 
-/* The solve's plan, chosen per size class of the systems:
+/* Until a plan is set or tuned, one CTA solves each system with its vectors
+ * (and its part of the matrix, where that fits) in shared memory; its size
+ * follows the largest system.  A plan keeps the vectors in L2 instead and is
+ * chosen per size class of the systems:
  *   threads   CTA size (128, 256 or 512) of the systems a whole CTA solves
  *   warp_max  systems of at most this many rows are solved by one warp each
  *             (a CTA holds several of them), with shuffle reductions and no
@@ -710,8 +713,8 @@ int sb2_batch_solve(const sb2_batch* B, double* x, const double* b,
  * The queue hands systems out largest first, so a CTA that takes a system of
  * at most warp_max rows turns to warps for the rest of the launch.
  * Autotuner: times the solve of this batch (x is overwritten) under each
- * candidate plan (threads 128, 256, 512 by warp_max 0, 256, 1024) and keeps
- * the fastest for later solves.  The choice is cached per (histogram of the
+ * candidate plan (threads 128, 256, 512 by warp_max 0, 256, 1024, clusters,
+ * and the vectors in shared memory) and keeps the fastest for later solves.  The choice is cached per (histogram of the
  * systems' sizes in power-of-two classes, mode): a later batch with the same
  * histogram takes it without timing. */
 int sb2_batch_autotune(sb2_batch* B, double* x, const double* b,

@@ -5,9 +5,10 @@
 // systems.  CTAs of a persistent grid take systems from an atomic queue,
 // largest first (the order is fixed when the batch is created), and run a
 // whole solve per system: all reductions are CTA-wide (__syncthreads), so no
-// CTA ever waits for another one.  Each system keeps its working set (its
-// rows of the operator in FP32 and FP64 and its vectors) warm in L2 while the
-// CTA iterates on it.
+// CTA ever waits for another one.  By default a system's vectors stay in the
+// CTA's shared memory while it iterates (the on-chip form); the plans that a
+// caller sets, and the other candidates of the autotuner, keep the working set
+// (the rows of the operator in FP32 and FP64 and the vectors) warm in L2.
 //
 // Solver per system (identity preconditioner):
 //   mode 0 -- FP32 conjugate gradients with reliable updates: the FP32
@@ -51,6 +52,7 @@ struct sb2_batch {
   int warp_max = 0;
   int cluster = 0;       // CTAs of a cluster plan (0: none)
   int cluster_min = 0;   // systems of more rows are solved by a whole cluster
+  bool onchip = true;    // vectors in shared memory (until a plan is set or tuned)
   int max_rows = 0;
   unsigned long long histo_key = 0;  // size histogram, for the tuned-plan cache
 };
@@ -492,6 +494,337 @@ __global__ void __launch_bounds__(NT, 1536 / NT) batch_kernel(BatchArgs a) {
   }
 }
 
+// ---------------------------------------------------------------- on-chip form
+//
+// One CTA per system with the vectors of its iteration in shared memory: p and
+// r always, then q, then the correction d (mixed mode) or the solution (FP64
+// mode), then the matrix, each where it still fits.  What does not fit is read
+// through L2, two rows a thread at a time.  The forms above keep everything in
+// L2 and wait for it with three CTAs per SM: 0.56 of the copy bandwidth in DRAM
+// traffic, long-scoreboard stalls 39 of 46 cycles.  Here a row moves at most 30
+// bytes of matrix an iteration, and none up to 4,500 rows of five entries.
+// 512 shifted 2D Laplacians of sides 8 to 140, mixed, to 1e-13: 10.0 ms, against
+// 62.5 ms with one 256-thread CTA per system and 19.3 ms with the best plan of
+// the forms above (4-CTA clusters); in FP64 26-29 ms against 30.2.  Systems of
+// more than about 28,000 rows (14,000 in FP64) do not fit and are solved by
+// the same CTAs through L2.
+
+// The CTA's threads, sums by a shuffle tree over the warps' partials.
+template <int NT>
+struct ChipGroup {
+  template <typename T>
+  static __device__ __forceinline__ T ld(const T* p) { return *p; }
+  double* red;  // shared: 2 buffers x 2 values x NT/32 warps
+  int ph;
+  static constexpr int kSize = NT;
+  __device__ __forceinline__ int rank() const { return threadIdx.x; }
+  __device__ __forceinline__ int stride() const { return NT; }
+  __device__ __forceinline__ void sync() const { __syncthreads(); }
+  template <int K, typename T>
+  __device__ __forceinline__ void sums(T (&v)[K]) {
+    constexpr int W = NT / 32;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double* buf = red + ph * 2 * W;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const T t = warp_sum(v[k]);
+      if (lane == 0) buf[k * W + w] = (double)t;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const T t = lane < W ? (T)buf[k * W + lane] : T(0);
+      v[k] = __shfl_sync(0xffffffffu, warp_sum(t), 0);
+    }
+    ph ^= 1;
+  }
+  template <typename T>
+  __device__ __forceinline__ T sum(T v) {
+    T o[1] = {v};
+    sums<1>(o);
+    return o[0];
+  }
+};
+
+// One system's rows: row pointers and entries in shared or global memory
+// (`base`: position of the first row's first entry in ptr's counting).
+template <typename IT, typename VT>
+struct ChipRows {
+  const int* ptr;
+  const IT* ind;
+  const VT* val;
+  int base;
+};
+
+// q = A p (entries in stored order) with (p, q): two rows of a thread in
+// flight, each in chunks of four entries.
+template <class G, typename IT, typename T>
+__device__ __forceinline__ T chip_product(G& g, const ChipRows<IT, T>& A, int n, const T* p, T* q) {
+  constexpr int R = 2, U = 5;
+  T pq = T(0);
+  for (int i0 = g.rank(); i0 < n; i0 += R * g.stride()) {
+    int k[R], e[R];
+    T t[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      const int i = i0 + r * g.stride();
+      k[r] = i < n ? A.ptr[i] - A.base : 0;
+      e[r] = i < n ? A.ptr[i + 1] - A.base : 0;
+      t[r] = T(0);
+    }
+    while (k[0] < e[0] || k[1] < e[1]) {
+      int c[R][U];
+      T v[R][U];
+#pragma unroll
+      for (int r = 0; r < R; r++)
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          const bool in = k[r] + u < e[r];
+          c[r][u] = in ? (int)A.ind[k[r] + u] : 0;
+          v[r][u] = in ? A.val[k[r] + u] : T(0);
+        }
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if (k[r] + u < e[r]) t[r] = add_rn(t[r], mul_rn(v[r][u], p[c[r][u]]));
+        k[r] += U;
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      const int i = i0 + r * g.stride();
+      if (i < n) {
+        q[i] = t[r];
+        pq = add_rn(pq, mul_rn(p[i], t[r]));
+      }
+    }
+  }
+  return g.sum(pq);
+}
+
+// Where a system's arrays go: the vectors and the matrix in `room` bytes of
+// shared memory, in the order above.  False: not even p and r fit.
+template <typename IT, typename T>
+__device__ __forceinline__ bool chip_layout(const BatchArgs& a, const T* val, char* smem, int room,
+                                            int r0, int n, T*& p, T*& r, T*& q, T*& d,
+                                            ChipRows<IT, T>& A) {
+  const size_t vec = ((size_t)n * sizeof(T) + 15) / 16 * 16;
+  if (2 * vec > (size_t)room) return false;
+  p = reinterpret_cast<T*>(smem);
+  r = reinterpret_cast<T*>(smem + vec);
+  size_t at = 2 * vec;
+  T** more[2] = {&q, &d};
+  for (int k = 0; k < 2; k++)
+    if (at + vec <= (size_t)room) {
+      *more[k] = reinterpret_cast<T*>(smem + at);
+      at += vec;
+    }
+  const int k0 = __ldg(a.ptr + r0), nnz = __ldg(a.ptr + r0 + n) - k0;
+  const IT* ind = static_cast<const IT*>(a.ind);
+  const size_t bv = ((size_t)nnz * sizeof(T) + 15) / 16 * 16, bp = ((size_t)(n + 1) * 4 + 15) / 16 * 16,
+               bi = (size_t)nnz * sizeof(IT);
+  if (at + bv + bp + bi <= (size_t)room) {
+    T* sv = reinterpret_cast<T*>(smem + at);
+    int* sp = reinterpret_cast<int*>(smem + at + bv);
+    IT* si = reinterpret_cast<IT*>(smem + at + bv + bp);
+    for (int k = threadIdx.x; k < nnz; k += blockDim.x) {
+      sv[k] = __ldg(val + k0 + k);
+      si[k] = __ldg(ind + k0 + k);
+    }
+    for (int i = threadIdx.x; i <= n; i += blockDim.x) sp[i] = __ldg(a.ptr + r0 + i);
+    __syncthreads();
+    A = ChipRows<IT, T>{sp, si, sv, k0};
+  } else {
+    A = ChipRows<IT, T>{a.ptr + r0, ind, val, 0};
+  }
+  return true;
+}
+
+// Plain FP64 CG, as solve_fp64.
+template <class G, typename IT>
+__device__ bool chip_fp64(G& g, const BatchArgs& a, int s, int r0, int n, double nb, char* smem,
+                          int room) {
+  double *p, *r, *q = reinterpret_cast<double*>(a.w32) + r0, *x = a.x + r0;
+  ChipRows<IT, double> A;
+  if (!chip_layout(a, a.val, smem, room, r0, n, p, r, q, x, A)) return false;
+  double rr;
+  if (a.init_guess_null) {
+    double acc = 0.0;
+    for (int i = g.rank(); i < n; i += g.stride()) {
+      x[i] = 0.0;
+      const double bi = __ldg(a.b + r0 + i);
+      r[i] = bi;
+      acc = add_rn(acc, mul_rn(bi, bi));
+    }
+    rr = g.sum(acc);
+  } else {
+    rr = fp64_residual<G, IT>(g, a, r0, n, a.x + r0);
+    for (int i = g.rank(); i < n; i += g.stride()) {
+      r[i] = a.r64[r0 + i];
+      if (x != a.x + r0) x[i] = a.x[r0 + i];
+    }
+  }
+  const double facteur = 1.0 / nb;
+  double rho = rr, rho_1 = 1.0, res = facteur * sqrt(rr), beta = 0.0;
+  int it = 0;
+  while (!(res < a.tol) && it < a.max_iter) {
+    if (rho == 0.0) break;
+    direction(g, n, r, p, it == 0, beta, 1.0);
+    g.sync();
+    const double delta = chip_product(g, A, n, p, q);
+    if (delta == 0.0) break;
+    const double alpha = rho / delta;
+    double acc = 0.0;
+    for (int i = g.rank(); i < n; i += g.stride()) {
+      x[i] = add_rn(x[i], mul_rn(alpha, p[i]));
+      const double ri = add_rn(r[i], mul_rn(-alpha, q[i]));
+      r[i] = ri;
+      acc = add_rn(acc, mul_rn(ri, ri));
+    }
+    rr = g.sum(acc);
+    rho_1 = rho;
+    rho = rr;
+    beta = rho / rho_1;
+    res = facteur * sqrt(rr);
+    it++;
+  }
+  if (x != a.x + r0)
+    for (int i = g.rank(); i < n; i += g.stride()) a.x[r0 + i] = x[i];
+  if (g.rank() == 0) {
+    if (a.iters) a.iters[s] = it;
+    if (a.relres) a.relres[s] = res;
+  }
+  return true;
+}
+
+// FP32 CG with FP64 reliable updates, as solve_mixed.
+template <class G, typename IT>
+__device__ bool chip_mixed(G& g, const BatchArgs& a, int s, int r0, int n, double nb, char* smem,
+                           int room) {
+  double* x = a.x + r0;
+  float *p, *r, *q = a.w32 + 3 * (size_t)a.m + r0, *d = a.w32 + 4 * (size_t)a.m + r0;
+  ChipRows<IT, float> A;
+  if (!chip_layout(a, a.val32, smem, room, r0, n, p, r, q, d, A)) return false;
+  if (a.init_guess_null)
+    for (int i = g.rank(); i < n; i += g.stride()) x[i] = 0.0;
+  g.sync();
+  double rr64 = fp64_residual<G, IT>(g, a, r0, n, x);
+  double res = sqrt(rr64) / nb;
+  int it = 0;
+  if (!(res < a.tol)) {
+    const float fnb = (float)nb;
+    float acc = 0.0f;
+    for (int i = g.rank(); i < n; i += g.stride()) {
+      const float ri = (float)a.r64[r0 + i];
+      r[i] = ri;
+      d[i] = 0.0f;
+      acc = add_rn(acc, mul_rn(ri, ri));
+    }
+    float rho = g.sum(acc), rho_1 = 1.0f, zc = 1.0f, beta = 0.0f;
+    float rmax = sqrtf(rho);
+    bool first = true;
+    for (;;) {
+      direction(g, n, r, p, first, beta, zc);
+      g.sync();
+      const float delta = chip_product(g, A, n, p, q);
+      first = false;
+      zc = 1.0f;
+      if (delta == 0.0f) break;
+      const float alpha = rho / delta;
+      acc = 0.0f;
+      for (int i = g.rank(); i < n; i += g.stride()) {
+        d[i] = add_rn(d[i], mul_rn(alpha, p[i]));
+        const float ri = add_rn(r[i], mul_rn(-alpha, q[i]));
+        r[i] = ri;
+        acc = add_rn(acc, mul_rn(ri, ri));
+      }
+      const float rr = g.sum(acc);
+      it++;
+      const float rn = sqrtf(rr);
+      const bool correct = (rn / fnb < (float)a.tol) || (rn < (float)a.ratio * rmax) ||
+                           it >= a.max_iter;
+      if (!correct) {
+        rho_1 = rho;
+        rho = rr;
+        beta = rho / rho_1;
+        continue;
+      }
+      // FP64 correction: x += d, d = 0, r64 = b - A x
+      for (int i = g.rank(); i < n; i += g.stride()) {
+        x[i] = add_rn(x[i], (double)d[i]);
+        d[i] = 0.0f;
+      }
+      g.sync();
+      rr64 = fp64_residual<G, IT>(g, a, r0, n, x);
+      res = sqrt(rr64) / nb;
+      if (res < a.tol || it >= a.max_iter) break;
+      // replace the FP32 residual; keep the direction, minus its component
+      // along the new residual
+      float v2[2] = {0.0f, 0.0f};
+      for (int i = g.rank(); i < n; i += g.stride()) {
+        const float ri = (float)a.r64[r0 + i];
+        r[i] = ri;
+        v2[0] = add_rn(v2[0], mul_rn(ri, ri));
+        v2[1] = add_rn(v2[1], mul_rn(ri, p[i]));
+      }
+      g.sums(v2);
+      rmax = sqrtf(v2[0]);
+      rho_1 = rho;
+      rho = v2[0];
+      if (rho == 0.0f) break;
+      beta = rho / rho_1;
+      zc = 1.0f - beta * (v2[1] / rho);
+    }
+  }
+  if (g.rank() == 0) {
+    if (a.iters) a.iters[s] = it;
+    if (a.relres) a.relres[s] = res;
+  }
+  return true;
+}
+
+template <int NT, typename IT>
+__global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 2) batch_chip_kernel(BatchArgs a, int room) {
+  extern __shared__ __align__(16) char s_chip[];
+  __shared__ int s_sys;
+  __shared__ double s_red[2 * 2 * (NT / 32)];
+  ChipGroup<NT> g{s_red, 0};
+  for (;;) {
+    if (threadIdx.x == 0) {
+      const unsigned k = atomicAdd(a.queue, 1u);
+      s_sys = (k < (unsigned)a.nsys) ? __ldg(a.order + k) : -1;
+    }
+    __syncthreads();
+    const int s = s_sys;
+    __syncthreads();
+    if (s < 0) return;
+    const int r0 = __ldg(a.sys_row + s), n = __ldg(a.sys_row + s + 1) - r0;
+    double acc = 0.0;
+    for (int i = g.rank(); i < n; i += NT) {
+      const double bi = __ldg(a.b + r0 + i);
+      acc = add_rn(acc, mul_rn(bi, bi));
+    }
+    const double nb = sqrt(g.sum(acc));
+    if (nb == 0.0) {  // zero right-hand side: x untouched (Iterative.cxx:240-241)
+      if (g.rank() == 0) {
+        if (a.iters) a.iters[s] = 0;
+        if (a.relres) a.relres[s] = 0.0;
+      }
+      continue;
+    }
+    // a system whose p and r do not fit keeps its vectors in L2
+    if (a.mode == 1) {
+      if (!chip_fp64<ChipGroup<NT>, IT>(g, a, s, r0, n, nb, s_chip, room))
+        solve_fp64<ChipGroup<NT>, IT>(g, a, s, r0, n, nb);
+    } else {
+      if (!chip_mixed<ChipGroup<NT>, IT>(g, a, s, r0, n, nb, s_chip, room))
+        solve_mixed<ChipGroup<NT>, IT>(g, a, s, r0, n, nb);
+    }
+    __syncthreads();
+  }
+}
+
 // Clusters of `cluster` CTAs that one GPU holds at once for this kernel
 // (0: the launch cannot be scheduled).
 template <int NT, typename IT, bool WARPS>
@@ -566,14 +899,46 @@ static int launch_batch_t(const BatchArgs& a, int threads, int cluster, cudaStre
                         : launch_batch_w<IT, false>(a, threads, cluster, s);
 }
 
+constexpr int kChipRoom = 224 * 1024;
+
+template <int NT, typename IT>
+static int launch_chip(const BatchArgs& a, int room, cudaStream_t s) {
+  auto* k = batch_chip_kernel<NT, IT>;
+  if (room > 48 * 1024)
+    SB2_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, NT, room) != cudaSuccess || per_sm < 1)
+    return SB2_ERR_NOT_SUPPORTED;
+  const int grid = std::min(a.nsys, per_sm * num_sms(current_device()));
+  k<<<std::max(grid, 1), NT, room, s>>>(a, room);
+  SB2_CUDA_TRY(cudaGetLastError());
+  return SB2_OK;
+}
+
+// CTA size by the largest system: enough threads for its rows, and small CTAs
+// side by side on an SM where all systems are small.
+template <typename IT>
+static int launch_onchip(const BatchArgs& a, int max_rows, long long nnz, cudaStream_t s) {
+  // room for the largest system with its matrix (mean entries a row), if it fits
+  const size_t t = a.mode == 1 ? 8 : 4;
+  const double per_row = 4.0 * t + 4.0 + (t + sizeof(IT)) * (double)nnz / std::max(a.m, 1);
+  const int room = (int)std::min<double>(kChipRoom, 1.05 * per_row * max_rows + 512);
+  if (max_rows <= 512) return launch_chip<128, IT>(a, room, s);
+  if (max_rows <= 2048) return launch_chip<256, IT>(a, room, s);
+  return launch_chip<1024, IT>(a, room, s);
+}
+
 static int batch_run(const sb2_batch* B, double* x, const double* b, const sb2_batch_params* prm,
                      int* iters, double* relres, int threads, int warp_max, int cluster,
-                     int cluster_min, cudaStream_t s) {
+                     int cluster_min, bool onchip, cudaStream_t s) {
   BatchArgs a{B->nsys, B->d_sys_row, B->d_order, B->d_ptr, B->d_ind, B->d_val, B->d_val32,
               b, x, B->d_r64, B->d_w32, B->m, B->d_queue, prm->tol, prm->update_ratio,
               prm->max_iter, prm->mode, prm->init_guess_null, warp_max, cluster_min, iters,
               relres};
   SB2_CUDA_TRY(cudaMemsetAsync(B->d_queue, 0, sizeof(unsigned), s));
+  if (onchip)
+    return B->ind16 ? launch_onchip<unsigned short>(a, B->max_rows, B->nnz, s)
+                    : launch_onchip<int>(a, B->max_rows, B->nnz, s);
   return B->ind16 ? launch_batch_t<unsigned short>(a, threads, cluster, s)
                   : launch_batch_t<int>(a, threads, cluster, s);
 }
@@ -613,6 +978,7 @@ static unsigned long long size_histogram_key(int nsys, const int* sys_row) {
 
 struct BatchPlan {
   int threads, warp_max, cluster, cluster_min;
+  bool onchip;
 };
 // Plans chosen by sb2_batch_autotune, per (size histogram, mode): a later
 // batch with the same histogram takes its plan without timing.
@@ -731,7 +1097,7 @@ int sb2_batch_solve(const sb2_batch* B, double* x, const double* b, const sb2_ba
     return SB2_OK;
   }
   SB2_TRY(batch_run(B, x, b, prm, d_iters, d_relres, B->threads, B->warp_max, B->cluster,
-                    B->cluster_min, s));
+                    B->cluster_min, B->onchip, s));
   if (!result) return SB2_OK;
   // host summary (synchronizes): per-system counts and residuals
   std::vector<int> it(B->nsys);
@@ -756,6 +1122,7 @@ int sb2_batch_solve(const sb2_batch* B, double* x, const double* b, const sb2_ba
 int sb2_batch_set_threads(sb2_batch* B, int threads) try {
   if (!B || (threads != 128 && threads != 256 && threads != 512)) return SB2_ERR_INVALID_VALUE;
   B->threads = threads;
+  B->onchip = false;
   return SB2_OK;
 } SB2_CATCH
 
@@ -768,6 +1135,7 @@ int sb2_batch_set_plan(sb2_batch* B, int threads, int warp_max) try {
   B->warp_max = warp_max;
   B->cluster = 0;
   B->cluster_min = 0;
+  B->onchip = false;
   return SB2_OK;
 } SB2_CATCH
 
@@ -777,6 +1145,7 @@ int sb2_batch_set_cluster_plan(sb2_batch* B, int cluster, int cluster_min) try {
     return SB2_ERR_INVALID_VALUE;
   B->cluster = cluster;
   B->cluster_min = cluster ? cluster_min : 0;
+  B->onchip = false;
   return SB2_OK;
 } SB2_CATCH
 
@@ -809,6 +1178,7 @@ extern "C" int sb2_batch_autotune(sb2_batch* B, double* x, const double* b,
       B->warp_max = it->second.warp_max;
       B->cluster = it->second.cluster;
       B->cluster_min = it->second.cluster_min;
+      B->onchip = it->second.onchip;
       return SB2_OK;
     }
   }
@@ -817,18 +1187,18 @@ extern "C" int sb2_batch_autotune(sb2_batch* B, double* x, const double* b,
   SB2_CUDA_TRY(cudaEventCreate(&e0));
   SB2_CUDA_TRY(cudaEventCreate(&e1));
   float best = 1e30f;
-  sb2::BatchPlan bp{B->threads, B->warp_max, B->cluster, B->cluster_min};
+  sb2::BatchPlan bp{B->threads, B->warp_max, B->cluster, B->cluster_min, B->onchip};
   int st = SB2_OK;
   // one untimed run, one timed run of the same solve; a cluster plan the
   // GPU cannot schedule is skipped
   auto trial = [&](const sb2::BatchPlan& p) {
     int r = sb2::batch_run(B, x, b, prm, nullptr, nullptr, p.threads, p.warp_max, p.cluster,
-                           p.cluster_min, s);
+                           p.cluster_min, p.onchip, s);
     if (r == SB2_ERR_NOT_SUPPORTED) return SB2_OK;
     if (r != SB2_OK) return r;
     cudaEventRecord(e0, s);
     r = sb2::batch_run(B, x, b, prm, nullptr, nullptr, p.threads, p.warp_max, p.cluster,
-                       p.cluster_min, s);
+                       p.cluster_min, p.onchip, s);
     cudaEventRecord(e1, s);
     if (cudaEventSynchronize(e1) != cudaSuccess) r = SB2_ERR_CUDA;
     float ms = 0.0f;
@@ -845,7 +1215,7 @@ extern "C" int sb2_batch_autotune(sb2_batch* B, double* x, const double* b,
   for (int ci = 0; ci < 9 && st == SB2_OK; ci++) {
     const int t = cand_t[ci / 3], w = cand_w[ci % 3];
     if (w > 0 && ci % 3 > 0 && cand_w[ci % 3 - 1] >= B->max_rows) continue;  // same plan as a smaller w
-    st = trial(sb2::BatchPlan{t, w, 0, 0});
+    st = trial(sb2::BatchPlan{t, w, 0, 0, false});
   }
   // then clusters of 4 or 16 CTAs for the systems above half or an eighth of
   // the largest, on the best plan's CTA size and warp systems
@@ -853,7 +1223,9 @@ extern "C" int sb2_batch_autotune(sb2_batch* B, double* x, const double* b,
   const int cand_c[2] = {4, 16};
   const int cand_m[2] = {B->max_rows / 2, B->max_rows / 8};
   for (int ci = 0; ci < 4 && st == SB2_OK; ci++)
-    st = trial(sb2::BatchPlan{base.threads, base.warp_max, cand_c[ci / 2], cand_m[ci % 2]});
+    st = trial(sb2::BatchPlan{base.threads, base.warp_max, cand_c[ci / 2], cand_m[ci % 2], false});
+  // and the on-chip form
+  if (st == SB2_OK) st = trial(sb2::BatchPlan{base.threads, base.warp_max, 0, 0, true});
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (st == SB2_OK) {
@@ -861,6 +1233,7 @@ extern "C" int sb2_batch_autotune(sb2_batch* B, double* x, const double* b,
     B->warp_max = bp.warp_max;
     B->cluster = bp.cluster;
     B->cluster_min = bp.cluster_min;
+    B->onchip = bp.onchip;
     std::lock_guard<std::mutex> g(sb2::g_plan_mu);
     sb2::g_plans[key] = bp;
   }
