@@ -7,7 +7,11 @@
 // equal keys in input order.  The result is the triplets in stable
 // (row, column) order, duplicates kept as separate entries.  Here:
 //
-//   k_coo_stats       sizes: largest row and column, bad indices, kept count
+//   k_coo_stats       sizes: largest row and column, bad indices, kept count,
+//                     and whether the triplets come in order already
+//   k_coo_sorted      triplets in order: copies, and ptr from the row changes
+//   k_bkt_*           the rest, where buckets of rows fit a CTA (see there)
+//   otherwise:
 //   k_row_count       entries per row (warp-aggregated atomics), scanned
 //                     into ptr
 //   k_row_scatter     each entry's key (column << ib | input position) to a
@@ -20,6 +24,10 @@
 //                     in shared memory
 //   longer rows       the stable LSD radix sort below, on the row's keys
 //   (the sorted keys give ind directly and val through the position)
+//
+// The whole call, from Python: 14.6M shuffled triplets of the 128^3 operator
+// 615 us (1030 with the last form), the same in order 206 us (483), 13.7M in
+// order of power-law rows 195 us (1274).
 //
 // All of it is integer and byte movement bound by HBM bandwidth and L2
 // atomics; the matrix comes out deterministic whatever order the atomics
@@ -44,32 +52,93 @@ struct CooStats {
   int col_max;
   int bad;      // some index - index < 0 or too large
   int kept;     // entries with row <= col
+  int unsorted; // the triplets are not in (row, column) order
 };
 
+// Also whether the triplets come in (row, column) order already: each is
+// compared with the next.
 __global__ void __launch_bounds__(kAsmThreads)
 k_coo_stats(const int* __restrict__ row, const int* __restrict__ col, long long nnz, int index,
             CooStats* st) {
-  int rmax = 0, cmax = 0, bad = 0, kept = 0;
+  constexpr int U = 4;
+  int rmax = 0, cmax = 0, bad = 0, kept = 0, unsorted = 0;
   const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += stride) {
-    const long long r = (long long)row[i] - index, c = (long long)col[i] - index;
-    if (r < 0 || c < 0 || r >= INT_MAX || c >= INT_MAX) {
-      bad = 1;
-      continue;
+  const int lane = threadIdx.x & 31;
+  for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < nnz;
+       i0 += U * stride) {
+    int rv[U], cv[U], rn[U], cn[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const long long i = i0 + u * stride + lane;
+      rv[u] = i < nnz ? __ldg(row + i) : index;
+      cv[u] = i < nnz ? __ldg(col + i) : index;
+      // the next triplet comes from the next lane, the last lane's from memory
+      const bool edge = lane == 31 && i + 1 < nnz;
+      rn[u] = edge ? __ldg(row + i + 1) : INT_MAX;
+      cn[u] = edge ? __ldg(col + i + 1) : INT_MAX;
     }
-    rmax = max(rmax, (int)r);
-    cmax = max(cmax, (int)c);
-    kept += (r <= c);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const long long i = i0 + u * stride + lane;
+      const long long r = (long long)rv[u] - index, c = (long long)cv[u] - index;
+      const int r2 = __shfl_down_sync(0xffffffffu, rv[u], 1), c2 = __shfl_down_sync(0xffffffffu, cv[u], 1);
+      if (lane < 31) {
+        rn[u] = r2;
+        cn[u] = c2;
+      }
+      if (i + 1 < nnz) unsorted |= rn[u] < rv[u] || (rn[u] == rv[u] && cn[u] < cv[u]);
+      const bool out = r < 0 || c < 0 || r >= INT_MAX || c >= INT_MAX;
+      bad |= out;
+      if (!out && i < nnz) {
+        rmax = max(rmax, (int)r);
+        cmax = max(cmax, (int)c);
+        kept += (r <= c);
+      }
+    }
   }
   rmax = __reduce_max_sync(0xffffffffu, rmax);
   cmax = __reduce_max_sync(0xffffffffu, cmax);
   bad = __reduce_or_sync(0xffffffffu, bad);
   kept = __reduce_add_sync(0xffffffffu, kept);
-  if ((threadIdx.x & 31) == 0) {
+  unsorted = __reduce_or_sync(0xffffffffu, unsorted);
+  // one set of atomics per CTA: with one per warp they took longer than the reads
+  __shared__ int s_st[kAsmWarps][5];
+  if (lane == 0) {
+    int* w = s_st[threadIdx.x >> 5];
+    w[0] = rmax; w[1] = cmax; w[2] = bad; w[3] = kept; w[4] = unsorted;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kAsmWarps; w++) {
+      rmax = max(rmax, s_st[w][0]);
+      cmax = max(cmax, s_st[w][1]);
+      bad |= s_st[w][2];
+      kept += s_st[w][3];
+      unsorted |= s_st[w][4];
+    }
     atomicMax(&st->row_max, rmax);
     atomicMax(&st->col_max, cmax);
     if (bad) atomicOr(&st->bad, 1);
     atomicAdd(&st->kept, kept);
+    if (unsorted) atomicOr(&st->unsorted, 1);
+  }
+}
+
+// Triplets that are in order: ind and val are copies, and ptr[r] is the place
+// of the first triplet of row r or beyond.
+__global__ void __launch_bounds__(kAsmThreads)
+k_coo_sorted(const int* __restrict__ row, const int* __restrict__ col,
+             const double* __restrict__ val, long long nnz, int index, int m,
+             int* __restrict__ ptr, int* __restrict__ ind, double* __restrict__ vout) {
+  const long long stride = (long long)gridDim.x * blockDim.x;
+#pragma unroll 4
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += stride) {
+    const int r = __ldg(row + i) - index, before = i ? __ldg(row + i - 1) - index : -1;
+    ind[i] = __ldcs(col + i) - index;
+    vout[i] = __ldcs(val + i);
+    for (int q = before + 1; q <= r; q++) ptr[q] = (int)i;
+    if (i == nnz - 1)
+      for (int q = r + 1; q <= m; q++) ptr[q] = (int)nnz;
   }
 }
 
@@ -276,6 +345,7 @@ k_row_sort_short(const int* __restrict__ ptr, int m, const unsigned long long* _
     const int b = ptr[r], e = ptr[r + 1];
     if (e - b > kShortRow) {
       long_rows[atomicAdd(nlong, 1)] = r;
+      if (e - b > kCtaRow) atomicAdd(nlong + 1, 1);
       continue;
     }
     for (int a = b; a < e; ++a) {
@@ -326,6 +396,309 @@ k_emit_segment(const unsigned long long* __restrict__ key, long long b, long lon
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < L; i += stride)
     emit(key[b + i], b + i, ib, val, ind, vout);
+}
+
+// ---------------------------------------------------------------- two-pass form
+//
+// The triplets' keys are first dealt to buckets of consecutive rows, then
+// every bucket is sorted in shared memory and written out.  A tile of keys is
+// grouped by bucket in shared memory before it goes to global memory, then its
+// values through the same shared memory, so that a bucket's part of a tile is
+// written as one run and no access of either pass is a lone 8-byte one.  (With
+// the values gathered by the second pass, a 32-byte sector each, that pass
+// alone took 458 us for 14.6M triplets of 7 a row, against 161 us.)  The form after it scatters one
+// key at a time to its row and gathers one value at a time; it stays for what
+// does not fit here: more than kBktMax buckets, buckets beyond a CTA's shared
+// memory (rows of very uneven length), keys beyond 64 bits.
+//   k_bkt_count  entries per bucket
+//   k_bkt_scan   first entry of each bucket; whether one is too large
+//   k_bkt_deal   tiles of keys (row in the bucket, column, input position) and
+//                values grouped by bucket
+//   k_bkt_sort   one CTA per bucket: entries placed by row (shared-memory
+//                counters), then an entry's place in a row of up to kBktRank
+//                entries is the number of smaller keys there, and longer rows
+//                take a bitonic sort; ptr, ind and val written
+
+constexpr int kBktMax = 4096;      // buckets
+constexpr int kBktThreads = 1024;
+constexpr int kDealThreads = 512;
+constexpr int kBktTile = 16 * kDealThreads;
+constexpr int kSortThreads = 512;
+constexpr int kBktCap = 5376;      // entries of a bucket at most: two CTAs an SM
+constexpr int kBktRows = 4096;     // rows of a bucket at most
+constexpr int kBktRank = 48;
+constexpr int kBktLong = 256;      // longer rows of one bucket, at most
+
+struct BktArgs {
+  const int* row;
+  const int* col;
+  const double* val;
+  long long nnz, nout;
+  int index, sym, m;
+  int lb, cb, ib;  // bits of a row in its bucket, of a column, of an input position
+  int nb;          // buckets
+  int* count;      // [nb + 1] entries, then first entry, of each bucket
+  int* cursor;     // [nb] next free entry
+  int* over;       // a bucket is too large
+  unsigned long long* key;
+  double* kval;
+  int* ptr;
+  int* ind;
+  double* vout;
+};
+
+__global__ void __launch_bounds__(kBktThreads) k_bkt_count(BktArgs a) {
+  __shared__ int h[kBktMax];
+  for (int b = threadIdx.x; b < a.nb; b += kBktThreads) h[b] = 0;
+  __syncthreads();
+  const long long stride = (long long)gridDim.x * kBktThreads;
+#pragma unroll 4
+  for (long long i = (long long)blockIdx.x * kBktThreads + threadIdx.x; i < a.nnz; i += stride) {
+    const int r = __ldg(a.row + i);
+    if (!a.sym || r <= __ldg(a.col + i)) atomicAdd(&h[(r - a.index) >> a.lb], 1);
+  }
+  __syncthreads();
+  for (int b = threadIdx.x; b < a.nb; b += kBktThreads)
+    if (h[b]) atomicAdd(&a.count[b], h[b]);
+}
+
+// Exclusive scan of v over W warps.
+template <int W>
+__device__ __forceinline__ int block_scan(int v, int* s_warp) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (lane == 31) s_warp[warp] = incl;
+  __syncthreads();
+  if (warp == 0) {
+    int w = lane < W ? s_warp[lane] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += t;
+    }
+    if (lane < W) s_warp[lane] = w;
+  }
+  __syncthreads();
+  const int base = warp ? s_warp[warp - 1] : 0;
+  __syncthreads();
+  return base + incl - v;
+}
+
+__global__ void __launch_bounds__(kBktThreads) k_bkt_scan(BktArgs a) {
+  __shared__ int s_warp[32];
+  constexpr int P = kBktMax / kBktThreads;
+  int c[P], sum = 0, most = 0;
+#pragma unroll
+  for (int j = 0; j < P; j++) {
+    const int b = threadIdx.x * P + j;
+    c[j] = b < a.nb ? a.count[b] : 0;
+    sum += c[j];
+    most = max(most, c[j]);
+  }
+  int at = block_scan<kBktThreads / 32>(sum, s_warp);
+#pragma unroll
+  for (int j = 0; j < P; j++) {
+    const int b = threadIdx.x * P + j;
+    if (b < a.nb) {
+      a.count[b] = at;
+      a.cursor[b] = at;
+    }
+    at += c[j];
+  }
+  if (most > kBktCap) *a.over = 1;
+  if (threadIdx.x == 0) {
+    a.count[a.nb] = (int)a.nout;
+    a.ptr[a.m] = (int)a.nout;
+  }
+}
+
+// shared memory of k_bkt_deal: keys and buckets of a tile, and per bucket the
+// tile's first place and the distance to its place in global memory
+constexpr size_t kDealSmem = kBktTile * (8 + 2) + (2 * kBktMax + 4) * 4;
+
+__global__ void __launch_bounds__(kDealThreads, 2) k_bkt_deal(BktArgs a) {
+  extern __shared__ __align__(16) unsigned char s_deal[];
+  __shared__ int s_warp[32];
+  unsigned long long* skey = reinterpret_cast<unsigned long long*>(s_deal);
+  int* loc = reinterpret_cast<int*>(skey + kBktTile);  // [kBktMax + 1]
+  int* delta = loc + kBktMax + 4;
+  unsigned short* sb = reinterpret_cast<unsigned short*>(delta + kBktMax);
+  constexpr int E = kBktTile / kDealThreads, P = kBktMax / kDealThreads;
+  const int tid = threadIdx.x;
+  if (*a.over) return;
+  const long long tiles = (a.nnz + kBktTile - 1) / kBktTile;
+  for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const long long t0 = tile * kBktTile;
+    for (int b = tid; b < kBktMax; b += kDealThreads) loc[b] = 0;
+    __syncthreads();
+    int br[E];  // bucket << 16 | place among the tile's entries of the bucket, or -1
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      const long long i = t0 + e * kDealThreads + tid;
+      br[e] = -1;
+      if (i < a.nnz) {
+        const int r = __ldg(a.row + i);
+        if (!a.sym || r <= __ldg(a.col + i)) br[e] = (r - a.index) >> a.lb;
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < E; e++)
+      if (br[e] >= 0) br[e] = (br[e] << 16) | atomicAdd(&loc[br[e]], 1);
+    __syncthreads();
+    int c[P], sum = 0;
+#pragma unroll
+    for (int j = 0; j < P; j++) {
+      c[j] = loc[tid * P + j];
+      sum += c[j];
+    }
+    int at = block_scan<kDealThreads / 32>(sum, s_warp);
+#pragma unroll
+    for (int j = 0; j < P; j++) {
+      loc[tid * P + j] = at;
+      at += c[j];
+    }
+    if (tid == kDealThreads - 1) loc[kBktMax] = at;
+    __syncthreads();
+    // consecutive threads take consecutive cursors, in every CTA the same way:
+    // runs of a bucket that follow one another then meet in L2 while their
+    // sector is still open (from a place that differs by CTA: 338 us, not 279)
+#pragma unroll
+    for (int j = 0; j < P; j++) {
+      const int b = j * kDealThreads + tid;
+      const int l = loc[b], n = loc[b + 1] - l;
+      if (n) delta[b] = atomicAdd(&a.cursor[b], n) - l;
+    }
+#pragma unroll
+    for (int e = 0; e < E; e++)
+      if (br[e] >= 0) {
+        const long long i = t0 + e * kDealThreads + tid;
+        const int r = __ldg(a.row + i) - a.index, cc = __ldg(a.col + i) - a.index;
+        const int b = br[e] >> 16, q = loc[b] + (br[e] & 0xffff);
+        skey[q] = ((unsigned long long)(r & ((1 << a.lb) - 1)) << (a.cb + a.ib)) |
+                  ((unsigned long long)(unsigned)cc << a.ib) | (unsigned long long)i;
+        sb[q] = (unsigned short)b;
+      }
+    __syncthreads();
+    const int kept = loc[kBktMax];
+#pragma unroll 4
+    for (int q = tid; q < kept; q += kDealThreads) a.key[delta[sb[q]] + q] = skey[q];
+    __syncthreads();
+    double* sval = reinterpret_cast<double*>(skey);
+#pragma unroll
+    for (int e = 0; e < E; e++)
+      if (br[e] >= 0)
+        sval[loc[br[e] >> 16] + (br[e] & 0xffff)] = __ldcs(a.val + t0 + e * kDealThreads + tid);
+    __syncthreads();
+#pragma unroll 4
+    for (int q = tid; q < kept; q += kDealThreads) a.kval[delta[sb[q]] + q] = sval[q];
+    __syncthreads();
+  }
+}
+
+constexpr size_t kSortSmem = (size_t)kBktCap * (8 + 8 + 2) + (kBktRows + 4) * 4 + kBktLong * 4;
+
+// Two CTAs per SM: while one waits for its keys or values the other works.
+__global__ void __launch_bounds__(kSortThreads, 2) k_bkt_sort(BktArgs a) {
+  extern __shared__ __align__(16) unsigned char s_sort[];
+  __shared__ int s_warp[32];
+  __shared__ int s_nlong;
+  unsigned long long* skey = reinterpret_cast<unsigned long long*>(s_sort);
+  double* sval = reinterpret_cast<double*>(skey + kBktCap);
+  int* off = reinterpret_cast<int*>(sval + kBktCap);  // [rows + 1]
+  int* lrow = off + kBktRows + 4;
+  unsigned short* place = reinterpret_cast<unsigned short*>(lrow + kBktLong);
+  constexpr int NS = kSortThreads, P = kBktRows / NS;
+  if (*a.over) return;
+  const int tid = threadIdx.x, b = blockIdx.x;
+  const int rb = 1 << a.lb, row0 = b << a.lb, rows = min(rb, a.m - row0);
+  const int start = __ldg(a.count + b), n = __ldg(a.count + b + 1) - start;
+  const int rs = a.cb + a.ib;
+  for (int r = tid; r <= rows; r += NS) off[r] = 0;
+  if (tid == 0) s_nlong = 0;
+  __syncthreads();
+#pragma unroll 4
+  for (int q = tid; q < n; q += NS)
+    place[q] = (unsigned short)atomicAdd(&off[(int)(__ldg(a.key + start + q) >> rs)], 1);
+  __syncthreads();
+  int c[P], sum = 0;
+#pragma unroll
+  for (int j = 0; j < P; j++) {
+    const int r = tid * P + j;
+    c[j] = r < rows ? off[r] : 0;
+    sum += c[j];
+  }
+  int at = block_scan<NS / 32>(sum, s_warp);
+#pragma unroll
+  for (int j = 0; j < P; j++) {
+    const int r = tid * P + j;
+    if (r < rows) {
+      off[r] = at;
+      if (c[j] > kBktRank) {
+        const int k = atomicAdd(&s_nlong, 1);
+        if (k < kBktLong) lrow[k] = r;
+      }
+    }
+    at += c[j];
+  }
+  if (tid == NS - 1) off[rows] = n;
+  __syncthreads();
+  for (int r = tid; r < rows; r += NS) a.ptr[row0 + r] = start + off[r];
+#pragma unroll 4
+  for (int q = tid; q < n; q += NS) {
+    const unsigned long long k = __ldg(a.key + start + q);
+    const double v = __ldcs(a.kval + start + q);
+    const int p = off[(int)(k >> rs)] + place[q];
+    skey[p] = k;
+    sval[p] = v;
+  }
+  __syncthreads();
+  const unsigned long long cmask = (1ull << a.cb) - 1ull;
+#pragma unroll 4
+  for (int q = tid; q < n; q += NS) {
+    const unsigned long long k = skey[q];
+    const int r = (int)(k >> rs), r0 = off[r], r1 = off[r + 1];
+    if (r1 - r0 > kBktRank) continue;
+    int f = r0;
+    for (int x = r0; x < r1; x++) f += skey[x] < k;
+    a.ind[start + f] = (int)((k >> a.ib) & cmask);
+    a.vout[start + f] = sval[q];
+  }
+  // (a bucket holds at most kBktCap / (kBktRank + 1) longer rows)
+  static_assert(kBktCap / (kBktRank + 1) < kBktLong, "the list holds every longer row");
+  for (int l = 0; l < s_nlong; l++) {
+    const int r0 = off[lrow[l]], L = off[lrow[l] + 1] - r0;
+    int S = 1;
+    while (S < L) S <<= 1;
+    // the places past the row hold keys larger than any: with the first step
+    // of a merge mirrored, every exchange is ascending and leaves them there
+    for (int k = 2; k <= S; k <<= 1)
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        __syncthreads();
+        for (int i = tid; i < S; i += NS) {
+          const int y = j == (k >> 1) ? (i ^ (k - 1)) : (i ^ j);
+          if (y > i && y < L) {
+            const unsigned long long u = skey[r0 + i], w = skey[r0 + y];
+            if (u > w) {
+              skey[r0 + i] = w;
+              skey[r0 + y] = u;
+              const double t = sval[r0 + i];
+              sval[r0 + i] = sval[r0 + y];
+              sval[r0 + y] = t;
+            }
+          }
+        }
+      }
+    __syncthreads();
+    for (int i = tid; i < L; i += NS) {
+      a.ind[start + r0 + i] = (int)((skey[r0 + i] >> a.ib) & cmask);
+      a.vout[start + r0 + i] = sval[r0 + i];
+    }
+  }
 }
 
 int bits_for(long long v) {  // bits needed to store 0..v
@@ -387,6 +760,68 @@ int radix_sort(K* key, int* pos, long long nnz, int bits, cudaStream_t s) {
   return st;
 }
 
+// Shared memory of the two-pass kernels, taken once per device.
+cudaError_t bkt_shared_memory() {
+  static std::atomic<unsigned long long> taken{0};
+  const int dev = current_device();
+  const unsigned long long bit = dev >= 0 && dev < 64 ? 1ull << dev : 0ull;
+  if (bit && (taken.load() & bit)) return cudaSuccess;
+  cudaError_t e = cudaFuncSetAttribute(k_bkt_deal, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDealSmem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_bkt_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSortSmem);
+  if (e == cudaSuccess) taken.fetch_or(bit);
+  return e;
+}
+
+// The two-pass form.  *done false: the triplets do not suit it (the outputs
+// are then unwritten).  Synchronizes the stream.
+int assemble_buckets(long long nnz, const int* row, const int* col, const double* val, int index,
+                     int m, int cb, int sym, long long nout, int* ptr, int* ind, double* vout,
+                     cudaStream_t s, bool* done) {
+  *done = false;
+  if (nout == 0) return SB2_OK;
+  const int sms = num_sms(current_device());
+  const int ib = bits_for(nnz - 1);
+  const double target = std::max(256.0, std::min(4800.0, (double)nout / (2.0 * sms)));
+  int lb = 0;
+  while (lb < 12 && (2.0 * nout / m) * (double)(1 << lb) <= target) lb++;
+  while (lb < 12 && ((long long)m + (1 << lb) - 1) >> lb > kBktMax) lb++;
+  const long long nb = ((long long)m + (1 << lb) - 1) >> lb;
+  if (nb > kBktMax || (double)nout / m * (1 << lb) > 0.9 * kBktCap || lb + cb + ib > 64)
+    return SB2_OK;
+  BktArgs a{row, col, val, nnz, nout, index, sym, m, lb, cb, ib, (int)nb};
+  a.ptr = ptr;
+  a.ind = ind;
+  a.vout = vout;
+  char* buf = nullptr;
+  const size_t ints = 2 * (size_t)kBktMax + 64;
+  SB2_CUDA_TRY(pool_malloc((void**)&buf, 16 * (size_t)nout + sizeof(int) * ints, s));
+  a.key = reinterpret_cast<unsigned long long*>(buf);
+  a.kval = reinterpret_cast<double*>(buf + 8 * (size_t)nout);
+  a.count = reinterpret_cast<int*>(buf + 16 * (size_t)nout);
+  a.cursor = a.count + kBktMax + 1;
+  a.over = a.cursor + kBktMax;
+  cudaError_t e = cudaMemsetAsync(a.count, 0, sizeof(int) * ints, s);
+  if (e == cudaSuccess) e = bkt_shared_memory();
+  int over = 0;
+  if (e == cudaSuccess) {
+    const long long tiles = (nnz + kBktTile - 1) / kBktTile;
+    const int grid = (int)std::min<long long>(tiles, 2LL * sms);
+    const int cgrid = (int)std::min<long long>((nnz + kBktThreads - 1) / kBktThreads, 2LL * sms);
+    k_bkt_count<<<cgrid, kBktThreads, 0, s>>>(a);
+    k_bkt_scan<<<1, kBktThreads, 0, s>>>(a);
+    k_bkt_deal<<<grid, kDealThreads, kDealSmem, s>>>(a);
+    k_bkt_sort<<<(int)nb, kSortThreads, kSortSmem, s>>>(a);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&over, a.over, sizeof(int), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  cudaFreeAsync(buf, s);
+  SB2_CUDA_TRY(e);
+  *done = over == 0;
+  return SB2_OK;
+}
+
 int assemble(long long nnz, const int* row, const int* col, const double* val, int index, int m,
              int cb, int sym, long long nout, int* ptr, int* ind, double* vout, cudaStream_t s) {
   const int grid = num_sms(current_device()) * 8;
@@ -399,10 +834,10 @@ int assemble(long long nnz, const int* row, const int* col, const double* val, i
   cudaError_t e = pool_malloc((void**)&key, sizeof(unsigned long long) * nout, s);
   if (e == cudaSuccess) e = pool_malloc((void**)&fill, sizeof(int) * ((size_t)m + 1), s);
   if (e == cudaSuccess) e = pool_malloc((void**)&long_rows, sizeof(int) * ((size_t)m + 1), s);
-  if (e == cudaSuccess) e = pool_malloc((void**)&nlong, sizeof(int), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(nlong, 0, sizeof(int), s);
+  if (e == cudaSuccess) e = pool_malloc((void**)&nlong, 2 * sizeof(int), s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(nlong, 0, 2 * sizeof(int), s);
   int st = map_cuda_error(e);
-  int h_nlong = 0;
+  int h_nlong = 0, h_long[2] = {0, 0};  // rows past kShortRow, and past kCtaRow
   std::vector<int> hrows, hptr;
   if (st == SB2_OK) {
     k_row_count<<<grid, kAsmThreads, 0, s>>>(row, col, nnz, index, sym, ptr);
@@ -416,12 +851,16 @@ int assemble(long long nnz, const int* row, const int* col, const double* val, i
                                                     nlong);
       e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&h_nlong, nlong, sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h_long, nlong, sizeof(h_long), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     st = map_cuda_error(e);
+    h_nlong = h_long[0];
   }
   if (st == SB2_OK && h_nlong > 0) {
     k_row_sort_cta<<<h_nlong, kAsmThreads, 0, s>>>(ptr, long_rows, key, ib, val, ind, vout);
+    st = map_cuda_error(cudaGetLastError());
+  }
+  if (st == SB2_OK && h_long[1] > 0) {
     // rows past the CTA sort: each sorted on its own
     hrows.resize(h_nlong);
     hptr.resize((size_t)m + 1);
@@ -470,7 +909,7 @@ int sb2_coo_to_csr(int nnz, const int* row, const int* col, const double* val, i
   *val_out = nullptr;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 
-  CooStats h = {0, 0, 0, 0};
+  CooStats h = {0, 0, 0, 0, 0};
   if (nnz > 0) {
     CooStats* d = nullptr;
     SB2_CUDA_TRY(pool_malloc((void**)&d, sizeof(CooStats), s));
@@ -511,9 +950,23 @@ int sb2_coo_to_csr(int nnz, const int* row, const int* col, const double* val, i
   if (e == cudaSuccess && nout > 0) e = pool_malloc_owned((void**)&di, sizeof(int) * nout, s);
   if (e == cudaSuccess && nout > 0) e = pool_malloc_owned((void**)&dv, sizeof(double) * nout, s);
   int st = map_cuda_error(e);
-  if (st == SB2_OK)
+  bool done = false;
+  // (a run of empty rows is filled by one thread: the buckets take those)
+  if (st == SB2_OK && nnz > 0 && !h.unsorted && nout == nnz && m <= 4LL * nnz) {
+    const int grid = (int)std::min<long long>((nnz + kAsmThreads - 1) / kAsmThreads,
+                                              num_sms(current_device()) * 8LL);
+    k_coo_sorted<<<grid, kAsmThreads, 0, s>>>(row, col, val, nnz, index, (int)m, dp, di, dv);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    st = map_cuda_error(e);
+    done = true;
+  }
+  if (st == SB2_OK && !done)
+    st = assemble_buckets(nnz, row, col, val, index, (int)m, cb, symmetric_upper, nout, dp, di, dv, s,
+                          &done);
+  if (st == SB2_OK && !done)
     st = assemble(nnz, row, col, val, index, (int)m, cb, symmetric_upper, nout, dp, di, dv, s);
-  if (st == SB2_OK) st = map_cuda_error(cudaStreamSynchronize(s));
+  if (st == SB2_OK && !done) st = map_cuda_error(cudaStreamSynchronize(s));
   if (st != SB2_OK) {
     sb2_device_free(dp);
     sb2_device_free(di);
