@@ -21,22 +21,44 @@ from ._lib import IrParams, IrResult, IterParams, IterResult, check
 _L = _lib.load()
 
 
+def _find_raw_stream():
+    """The raw handle of torch's current stream without its Stream object,
+    which costs 3.5 us a call (a whole product of a small matrix takes 6)."""
+    import torch
+    raw, dev = (getattr(torch._C, n, None)
+                for n in ("_cuda_getCurrentRawStream", "_cuda_getDevice"))
+    if raw is None or dev is None:
+        return lambda: torch.cuda.current_stream().cuda_stream
+    torch.cuda.current_stream()  # CUDA is initialized from here on
+    return lambda: raw(dev())
+
+
+_raw_stream = None
+
+
 def _stream(stream=None):
     if stream is not None:
-        return ctypes.c_void_p(int(stream))
-    import torch
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        return int(stream)
+    global _raw_stream
+    if _raw_stream is None:
+        _raw_stream = _find_raw_stream()
+    return _raw_stream()
+
+
+_torch = None
 
 
 def _dev_ptr(t, n=None, name="vector"):
-    import torch
-    if not isinstance(t, torch.Tensor) or not t.is_cuda or t.dtype != torch.float64:
+    global _torch
+    if _torch is None:
+        import torch as _torch
+    if not isinstance(t, _torch.Tensor) or not t.is_cuda or t.dtype != _torch.float64:
         raise TypeError(f"{name}: expected a CUDA float64 tensor")
     if not t.is_contiguous():
         raise ValueError(f"{name}: expected a contiguous tensor")
     if n is not None and t.numel() != n:
         raise ValueError(f"{name}: length {t.numel()} != {n} (WrongDim)")
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def _np_ptr(a):

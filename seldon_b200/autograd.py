@@ -27,8 +27,7 @@ def _vp(t):
     return ctypes.c_void_p(t.data_ptr())
 
 
-def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+_stream = api._stream
 
 
 class SparsePattern:
