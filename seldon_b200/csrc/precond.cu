@@ -188,6 +188,7 @@ struct sb2_precond {
   int symmetric = 1;
   sb2::SweepGrid grid;      // row blocks and work vectors of the sweeps
   sb2::SweepPlan fwd, bwd;  // SOR
+  double* d_tmp = nullptr;    // SOR, several launches: their other target
   double* d_sdiag = nullptr;  // SOR, symmetric storage: diagonal of each stored row
   std::mutex mu;
   bool planned = false;
@@ -228,12 +229,12 @@ static int plan_sor(sb2_precond* M) {
     const int stored = uptr[j + 1] - uptr[j];
     return make_int4(uptr[j], uptr[j + 1], ptr[j], ptr[j + 1] - stored);
   };
-  std::vector<int> level, order;
+  std::vector<int> level, order, pos;
   tri_levels(n, ptr.data(), ind.data(), true, level);
-  SB2_TRY(make_sweep_plan(M->grid, level, &M->fwd, order, span));
+  SB2_TRY(make_sweep_plan(M->grid, level, &M->fwd, order, pos, span));
   if (A->sym) tri_levels(n, uptr.data(), uind.data(), false, level);
   else tri_levels(n, ptr.data(), ind.data(), false, level);
-  SB2_TRY(make_sweep_plan(M->grid, level, &M->bwd, order, span));
+  SB2_TRY(make_sweep_plan(M->grid, level, &M->bwd, order, pos, span));
   if (A->sym) {
     // values of symmetric storage never change (sb2_csr_set_values)
     const CsrArrays& u = A->upper;
@@ -260,25 +261,27 @@ static int sor_apply(sb2_precond* M, const double* x0, double* x, const double* 
   const int nf = type_ssor % 2 == 0 ? std::max(iter, 0) : 0;
   const int total = nf + (type_ssor % 3 == 0 ? std::max(iter, 0) : 0);
   const int launches = (total + 1) / 2;
+  // targets alternate between x and a work vector, so that none is the
+  // vector its launch starts from; from zero the last one is x
+  if (launches > (x0 ? 0 : 1) && !M->d_tmp) {
+    std::lock_guard<std::mutex> g(M->mu);
+    if (!M->d_tmp) SB2_CUDA_TRY(cudaMalloc(&M->d_tmp, sizeof(double) * std::max(n, 1)));
+  }
   const double* cur = x0;
   for (int l = 0, done = 0; l < launches; l++, done += 2) {
-    const bool two = done + 1 < total;
+    const int sweeps = done + 1 < total ? 2 : 1;
     const bool fwd[2] = {done < nf, done + 1 < nf};
     const SweepPlan* const plan[2] = {fwd[0] ? &M->fwd : &M->bwd, fwd[1] ? &M->fwd : &M->bwd};
-    // targets alternate between x and a work vector, so that none is the
-    // vector its launch starts from; from zero the last one is x
     const bool into_x = x0 ? l % 2 == 1 : (launches - 1 - l) % 2 == 0;
-    double* last = into_x ? x : G.d_new[1];
-    double* out0 = two ? G.d_new[0] : last;
-    double* out1 = two ? last : nullptr;
+    double* last = into_x ? x : M->d_tmp;
     if (A->sym) {
       const CsrArrays &u = A->upper, &f = A->full;
-      SB2_TRY(launch_sweeps(G, plan, fwd, out0, out1,
+      SB2_TRY(launch_sweeps(G, sweeps, plan, fwd, last,
                             SymmetricSor{u.d_ind, u.d_val, f.d_ind, f.d_val, M->d_sdiag, b, cur, omega,
                                          (1.0 - omega) / omega}, s));
     } else {
       const CsrArrays& f = A->full;
-      SB2_TRY(launch_sweeps(G, plan, fwd, out0, out1,
+      SB2_TRY(launch_sweeps(G, sweeps, plan, fwd, last,
                             GeneralSor{f.d_ind, f.d_val, A->d_diag, b, cur, omega, 1.0 - omega}, s));
     }
     cur = last;
@@ -306,16 +309,16 @@ static void gather_levels(int n, const std::vector<int>& ptr, const std::vector<
 static int upload_sweep(const SweepGrid& G, const std::vector<int>& ptr,
                         const std::vector<int>& ind, const std::vector<double>& val,
                         bool ascending, GatherSweep* S) {
-  std::vector<int> level, order;
+  std::vector<int> level, order, pos;
   gather_levels(G.n, ptr, ind, ascending, level);
-  // the lists in the order the rows are taken
+  // the lists in the order the rows are taken, columns as positions
   std::vector<int> pind;
   std::vector<double> pval;
   pind.reserve(ind.size());
   pval.reserve(val.size());
-  SB2_TRY(make_sweep_plan(G, level, &S->plan, order, [&](int, int j) {
+  SB2_TRY(make_sweep_plan(G, level, &S->plan, order, pos, [&](int, int j) {
     const int k0 = (int)pind.size();
-    pind.insert(pind.end(), ind.begin() + ptr[j], ind.begin() + ptr[j + 1]);
+    for (int k = ptr[j]; k < ptr[j + 1]; k++) pind.push_back(pos[ind[k]]);
     pval.insert(pval.end(), val.begin() + ptr[j], val.begin() + ptr[j + 1]);
     return make_int4(k0, (int)pind.size(), 0, 0);
   }));
@@ -520,7 +523,7 @@ static int ilut_apply(sb2_precond* M, bool trans, const double* r, double* z, cu
                  z, !sym && !trans ? M->d_pcol : M->d_iprow};
   const SweepPlan* const plan[2] = {&first.plan, &second.plan};
   const bool fwd[2] = {true, false};
-  return launch_sweeps(M->grid, plan, fwd, M->grid.d_new[0], M->grid.d_new[1], op, s);
+  return launch_sweeps(M->grid, 2, plan, fwd, nullptr, op, s);
 }
 
 int precond_kind(const sb2_precond* M) { return M->kind; }
@@ -630,6 +633,7 @@ int sb2_precond_destroy(sb2_precond* M) try {
   M->fwd.release();
   M->bwd.release();
   cudaFree(M->d_sdiag);
+  cudaFree(M->d_tmp);
   M->s_lf.release();
   M->s_ub.release();
   M->s_utf.release();
@@ -670,6 +674,7 @@ int sb2_sor(const sb2_csr* A, double* x, const double* b, double omega, int iter
   tmp.fwd.release();
   tmp.bwd.release();
   cudaFree(tmp.d_sdiag);
+  cudaFree(tmp.d_tmp);
   if (st == SB2_OK && e != cudaSuccess) st = map_cuda_error(e);
   if (st == SB2_OK) st = late;
   return st;

@@ -10,19 +10,24 @@
 //  - Values of other blocks come through global memory.  The vector a sweep
 //    writes was filled with a reserved NaN, so a value announces itself: the
 //    row polls the entries it needs until they differ from the fill.  No
-//    flag, fence or grid barrier stands between a value and its use.
+//    flag, fence or grid barrier stands between a value and its use.  The
+//    vector is in the order the rows are taken: an item's values are one run
+//    that is written once.  (By row, a line held values of 16 levels, and a
+//    line that other SMs poll is slow to write: 3 us from CTA to CTA.)
 // Each row repeats the reference's operations in the reference's order, so
 // the result does not depend on the timing.
 //
 // What bounds it is the chain of dependent rows.  Inside a block a level costs
 // what one row does between its turn and its barrier (430 cycles for three
-// entries, measured with clock64); the loads and everything that reads only
-// old values come before, while the warp's predecessors still work.  From one
-// CTA to the next a value takes 2-3 us.  Two sweeps on a 7-point grid, against
-// a graph of one launch per level before: ILU(0) apply 96^3 651 us (2070), 128^3
-// 1066 us (2970); SSOR of symmetric storage, 64^3 395 us (2700).
-// 384 threads: with 256 the small grids lose a fifth (ILU(0) 16^3 54 us
-// against 45), with 768 and more the registers spill on the chain (83 us).
+// entries, measured with clock64): its loads, products, sums and exact
+// division; everything that reads only old values comes before, while the
+// warp's predecessors still work.  From one CTA to the next a value takes about
+// a microsecond.  Two sweeps on a 7-point grid, against a graph of one launch
+// per level before: ILU(0) apply 96^3 424 us (2070), 128^3 694 us (2970); SSOR on
+// 64^3 with symmetric storage 289 us (1446), with general storage 271 us (1547).
+// 384 threads for three-entry and symmetric rows: with 256 the small grids lose
+// (ILU(0) 16^3 54 us against 45), with 768 and more the registers spill on the
+// chain (83 us); general rows hold more and spill at 384 already (64^3 307 us).
 //
 // Progress: all CTAs are resident (cooperative launch), a warp's items are in
 // level order and a row reads rows of smaller levels only.  Every wait is
@@ -53,13 +58,15 @@ struct SweepPlan {
   int4* d_item = nullptr;     // [items] first position, rows, step, arrivals (below)
   int* d_cta_item = nullptr;  // [ctas + 1] first item of each CTA
   int* d_steps = nullptr;     // [ctas] steps of each CTA
+  int* d_pos = nullptr;       // [n] position of each row
   void release() {
     cudaFree(d_rows);
     cudaFree(d_span);
     cudaFree(d_item);
     cudaFree(d_cta_item);
     cudaFree(d_steps);
-    d_rows = d_cta_item = d_steps = nullptr;
+    cudaFree(d_pos);
+    d_rows = d_cta_item = d_steps = d_pos = nullptr;
     d_span = nullptr;
     d_item = nullptr;
   }
@@ -90,14 +97,17 @@ struct SweepPhase {
   const int4* item;
   const int* cta_item;
   const int* steps;
+  const int* pos;       // position of each row here
+  const int* pos_prev;  // and in the sweep before (of the same launch)
   int forward;     // new values are those of smaller rows
-  double* out;     // values of this phase (filled before the launch)
+  double* out;     // values of this phase by position (filled before the launch)
 };
 
 struct SweepArgs {
   const int* blk;
   int max_rows;
   int nph;          // 1 or 2 sweeps in this launch
+  double* result;   // the last sweep's values by row (may be null)
   SweepPhase ph[2];
   unsigned* state;
   unsigned long long wait_ns;
@@ -106,9 +116,10 @@ struct SweepArgs {
 // ------------------------------------------------------------------ planning
 
 // Cuts n rows into blocks of about 2048, one CTA each, and larger ones where
-// the SMs run out.  SSOR on 7-point grids, 2048 / 4096 / 8192 rows a block:
-// 20^3 123 / 177 / 238 us, 40^3 244 / 273 / 423, 64^3 395 / 413 / 499; smaller
-// blocks add CTAs for a chain of rows to cross (1024: 433 us at 64^3).
+// the SMs run out.  SSOR on 7-point grids with a first form of the kernel, 2048
+// / 4096 / 8192 rows a block: 20^3 123 / 177 / 238 us, 40^3 244 / 273 / 423,
+// 64^3 395 / 413 / 499; smaller blocks add CTAs for a chain of rows to cross
+// (1024: 433 us at 64^3).
 inline int make_sweep_grid(int n, SweepGrid* G) {
   G->n = n;
   const int most = std::min(kSweepMaxCtas, num_sms(current_device()));
@@ -126,10 +137,11 @@ inline int make_sweep_grid(int n, SweepGrid* G) {
 }
 
 // Positions, items and spans of one sweep from the rows' levels.  span(i, j)
-// gives the entry ranges of row j at position i; `order` returns the rows.
+// gives the entry ranges of row j at position i, once `order` (the row of each
+// position) and `pos` (the position of each row) are complete.
 template <class Span>
 int make_sweep_plan(const SweepGrid& G, const std::vector<int>& level, SweepPlan* P,
-                    std::vector<int>& order, const Span& span) {
+                    std::vector<int>& order, std::vector<int>& pos, const Span& span) {
   const int n = G.n;
   int nlev = 0;
   for (int i = 0; i < n; i++) nlev = std::max(nlev, level[i] + 1);
@@ -142,6 +154,8 @@ int make_sweep_plan(const SweepGrid& G, const std::vector<int>& level, SweepPlan
   std::vector<int> at(G.h_blk.begin(), G.h_blk.end());
   order.assign(std::max(n, 1), 0);
   for (int q = 0; q < n; q++) order[at[by_level[q] / per]++] = by_level[q];
+  pos.assign(std::max(n, 1), 0);
+  for (int i = 0; i < n; i++) pos[order[i]] = i;
   std::vector<int4> item;
   std::vector<int> cta_item(G.ctas + 1, 0), steps(G.ctas, 0);
   std::vector<int4> sp(std::max(n, 1));
@@ -170,6 +184,8 @@ int make_sweep_plan(const SweepGrid& G, const std::vector<int>& level, SweepPlan
   SB2_CUDA_TRY(cudaMemcpy(P->d_rows, order.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
   SB2_CUDA_TRY(cudaMemcpy(P->d_span, sp.data(), sizeof(int4) * n, cudaMemcpyHostToDevice));
   SB2_CUDA_TRY(cudaMemcpy(P->d_item, item.data(), sizeof(int4) * item.size(), cudaMemcpyHostToDevice));
+  SB2_CUDA_TRY(cudaMalloc(&P->d_pos, sizeof(int) * std::max(n, 1)));
+  SB2_CUDA_TRY(cudaMemcpy(P->d_pos, pos.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
   SB2_CUDA_TRY(cudaMalloc(&P->d_steps, sizeof(int) * G.ctas));
   SB2_CUDA_TRY(cudaMemcpy(P->d_steps, steps.data(), sizeof(int) * G.ctas, cudaMemcpyHostToDevice));
   SB2_CUDA_TRY(cudaMemcpy(P->d_cta_item, cta_item.data(), sizeof(int) * cta_item.size(), cudaMemcpyHostToDevice));
@@ -280,30 +296,40 @@ struct SweepSource {
 // An operation describes one row's new value as a sequence of entries (column,
 // coefficient) to be taken in order:
 //   Row r = op.load(ph, fwd, j, span)     what does not depend on other rows
-//   op.entry(r, k, c, a)                  entry k of r.len
+//   op.entry(r, k, c, a)                  entry k of r.len; c is its column, or with
+//                                         Op::kPositions the column's position
 //   op.is_new(r, k, c)                    it reads this sweep's value of c
 //   op.first(r, s, xj)                    xj: the row's value before the sweep
 //   op.take(r, s, k, c, a, x)             entry k with the value x of column c
 //   op.lead(r, s, k)                      entries 0..k-1 are taken, none new
 //   op.last(r, s)                         the new value
+// The entries after the lead that are held in registers only add products to
+// one number, so that nothing but loads, products and sums follows the row's
+// turn:
+//   op.skips(r, c)                        such an entry adds nothing
+//   op.signed_value(r, a)                 what multiplies x
+//   op.running(r, s), op.run_to(r, s, v)  that number, and what became of it
 
-// Division by a divisor known ahead: y = RN(1 / b) is made before the row's
-// turn, and two of Markstein's correction steps (IBM J. Res. Dev. 34, 1990:
-// q' = q + y (a - b q), the remainder exact by fma) give RN(a / b) where no
-// intermediate leaves the normal range.  The full division, several hundred
-// cycles of one warp, stays for the operands outside it.
+// Division by a divisor known ahead: y + z = 1 / b to twice the precision is
+// made before the row's turn; then q = a y + a z is within an ulp of a / b, and
+// one of Markstein's correction steps (IBM J. Res. Dev. 34, 1990: q' = q + y
+// (a - b q), the remainder exact by fma) gives RN(a / b) where no intermediate
+// leaves the normal range.  The full division, several hundred cycles of one
+// warp, stays for the operands outside it.
 struct Divisor {
-  double b, y;  // y = 0: use the full division
-  __device__ __forceinline__ explicit Divisor(double v) : b(v), y(0.0) {
+  double b, y, z;  // y = 0: use the full division
+  __device__ __forceinline__ explicit Divisor(double v) : b(v), y(0.0), z(0.0) {
     const double m = fabs(v);
-    if (m > 0x1p-400 && m < 0x1p400) y = __drcp_rn(v);
+    if (m > 0x1p-400 && m < 0x1p400) {
+      y = __drcp_rn(v);
+      z = __dmul_rn(__fma_rn(-v, y, 1.0), y);
+    }
   }
-  __device__ __forceinline__ Divisor() : b(1.0), y(0.0) {}
+  __device__ __forceinline__ Divisor() : b(1.0), y(0.0), z(0.0) {}
   __device__ __forceinline__ double divide(double a) const {
     const double m = fabs(a);
-    if (y != 0.0 && m > 0x1p-500 && m < 0x1p500) {
-      double q = __dmul_rn(a, y);
-      q = __fma_rn(__fma_rn(-b, q, a), y, q);
+    if (y != 0.0 && m > 0x1p-400 && m < 0x1p400) {
+      const double q = __fma_rn(a, y, __dmul_rn(a, z));
       return __fma_rn(__fma_rn(-b, q, a), y, q);
     }
     return __ddiv_rn(a, b);
@@ -312,7 +338,8 @@ struct Divisor {
 
 // RowSparse sweep (Relaxation_MatVect.cxx:69-77 / :83-91).  span.x..y: row j.
 struct GeneralSor {
-  static constexpr int kAhead = 8, kThreads = 384;
+  static constexpr int kAhead = 8, kThreads = 256;
+  static constexpr bool kPositions = false;
   const int* ind; const double* val; const double* diag;
   const double* b; const double* x0; double omega, rest;  // rest = 1 - omega
   struct Row { int j, k0, len; bool fwd; double bj; Divisor ajj; };
@@ -335,6 +362,10 @@ struct GeneralSor {
     s.temp = add_rn(s.temp, mul_rn(a, x));
   }
   __device__ __forceinline__ void lead(const Row&, Sum&, int) const {}
+  __device__ __forceinline__ bool skips(const Row&, int) const { return false; }
+  __device__ __forceinline__ double signed_value(const Row&, double a) const { return a; }
+  __device__ __forceinline__ double running(const Row&, const Sum& s) const { return s.temp; }
+  __device__ __forceinline__ void run_to(const Row&, Sum& s, double v) const { s.temp = v; }
   __device__ __forceinline__ double last(const Row& r, const Sum& s) const {
     const double temp = add_rn(__dsub_rn(r.bj, s.temp), mul_rn(r.ajj.b, s.xj));
     return add_rn(mul_rn(rest, s.xj), r.ajj.divide(mul_rn(omega, temp)));
@@ -353,6 +384,7 @@ struct GeneralSor {
 // ajj, the x_p new: the mirrored entries, then the stored ones.
 struct SymmetricSor {
   static constexpr int kAhead = 8, kThreads = 384;
+  static constexpr bool kPositions = false;
   const int* uind; const double* uval; const int* find; const double* fval;
   const double* diag; const double* b; const double* x0;
   double omega, ratio;  // ratio = (1 - omega) / omega
@@ -400,6 +432,14 @@ struct SymmetricSor {
   __device__ __forceinline__ void lead(const Row& r, Sum& s, int k) const {
     if (!s.started && k >= olds(r)) start(r, s);
   }
+  __device__ __forceinline__ bool skips(const Row& r, int c) const { return c == r.j; }
+  __device__ __forceinline__ double signed_value(const Row& r, double a) const { return r.fwd ? -a : a; }
+  // (an entry held in registers comes after the lead only once t is started)
+  __device__ __forceinline__ double running(const Row& r, const Sum& s) const { return r.fwd ? s.t : s.temp; }
+  __device__ __forceinline__ void run_to(const Row& r, Sum& s, double v) const {
+    if (r.fwd) s.t = v;
+    else s.temp = v;
+  }
   __device__ __forceinline__ double last(const Row& r, Sum& s) const {
     if (!s.started) start(r, s);
     return r.fwd ? mul_rn(s.t, r.scale) : r.ajj.divide(mul_rn(__dsub_rn(s.t, s.temp), omega));
@@ -414,6 +454,7 @@ struct SymmetricSor {
 // to z through the output permutation.  span.x..y: the row's update list.
 struct FactorSolve {
   static constexpr int kAhead = 4, kThreads = 384;
+  static constexpr bool kPositions = true;
   const int* ind[2]; const double* val[2];
   const double* pre[2]; const double* post[2];
   const double* r; const int* in_at;
@@ -440,6 +481,10 @@ struct FactorSolve {
     s.t = __dsub_rn(s.t, mul_rn(a, x));
   }
   __device__ __forceinline__ void lead(const Row&, Sum&, int) const {}
+  __device__ __forceinline__ bool skips(const Row&, int) const { return false; }
+  __device__ __forceinline__ double signed_value(const Row&, double a) const { return -a; }
+  __device__ __forceinline__ double running(const Row&, const Sum& s) const { return s.t; }
+  __device__ __forceinline__ void run_to(const Row&, Sum& s, double v) const { s.t = v; }
   __device__ __forceinline__ double last(const Row& r, const Sum& s) const {
     return r.has_post ? mul_rn(s.t, r.post) : s.t;
   }
@@ -489,22 +534,29 @@ __global__ void __launch_bounds__(Op::kThreads, 1) sweep_kernel(SweepArgs a, Op 
         span = __ldg(P.span + item.x + lane);
       }
     };
+    // where the value of column c is: its position in this sweep, or in the
+    // one before, or the row itself in the vector given
+    auto place = [&](int c, bool nw) {
+      return Op::kPositions ? c : nw ? __ldg(P.pos + c) : ph == 1 ? __ldg(P.pos_prev + c) : c;
+    };
     fetch(it0 + warp);
     for (int it = it0 + warp; it < it1 && ok; it += W) {
       const bool live = j >= 0;
-      const int row = j;
+      const int row = j, slot = item.x + lane;
       // this item's step, and what it adds to the step's barrier; the step
       // before must be complete (it waited for the one before it, and so on)
       const int step = base + item.z, arrivals = item.w;
       typename Op::Row R = {};
       typename Op::Sum s;
-      int c[U];
+      int c[U], at[U];
       double f[U], x[U];
       unsigned isnew = 0u, far = 0u, near = 0u;  // far: awaited in L2, near: in shared memory
       double xj = 0.0;
+      int before = 0;  // this row's position in the sweep before
       if (live) {
         R = op.load(ph, fwd, row, span);
         if (ph == 0 && x0) xj = __ldcg(x0 + row);
+        if (ph == 1) before = __ldg(P.pos_prev + row);
 #pragma unroll
         for (int u = 0; u < U; u++) {
           c[u] = 0;
@@ -516,15 +568,22 @@ __global__ void __launch_bounds__(Op::kThreads, 1) sweep_kernel(SweepArgs a, Op 
       fetch(it + W);
 #pragma unroll
       for (int u = 0; u < U; u++) {
-        x[u] = 0.0;
+        at[u] = 0;
         if (u < len) {
           const bool nw = op.is_new(R, u, c[u]);
           if (nw) isnew |= 1u << u;
-          if (nw || ph == 1) {
-            if (OWN && (unsigned)(c[u] - r0) < (unsigned)rows) near |= 1u << u;
+          at[u] = place(c[u], nw);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        x[u] = 0.0;
+        if (u < len) {
+          if ((isnew >> u & 1u) || ph == 1) {
+            if (OWN && (unsigned)(at[u] - r0) < (unsigned)rows) near |= 1u << u;
             else far |= 1u << u;
           } else if (x0) {
-            x[u] = __ldcg(x0 + c[u]);
+            x[u] = __ldcg(x0 + at[u]);
           }
         }
       }
@@ -533,7 +592,7 @@ __global__ void __launch_bounds__(Op::kThreads, 1) sweep_kernel(SweepArgs a, Op 
         double y[U];
 #pragma unroll
         for (int u = 0; u < U; u++)
-          if (far >> u & 1u) y[u] = ld_volatile((isnew >> u & 1u ? fresh.g : old.g) + c[u]);
+          if (far >> u & 1u) y[u] = ld_volatile((isnew >> u & 1u ? fresh.g : old.g) + at[u]);
 #pragma unroll
         for (int u = 0; u < U; u++)
           if ((far >> u & 1u) && !is_fill(y[u])) {
@@ -555,9 +614,9 @@ __global__ void __launch_bounds__(Op::kThreads, 1) sweep_kernel(SweepArgs a, Op 
         while (poll(~isnew) && ok) {}
 #pragma unroll
         for (int u = 0; u < U; u++)
-          if ((near & ~isnew) >> u & 1u) x[u] = ld_shared(old.own + 8u * (unsigned)(c[u] - r0));
+          if ((near & ~isnew) >> u & 1u) x[u] = ld_shared(old.own + 8u * (unsigned)(at[u] - r0));
         if (live) {
-          xj = OWN ? ld_shared(old.own + 8u * (unsigned)(row - r0)) : ld_volatile(old.g + row);
+          xj = OWN ? ld_shared(old.own + 8u * (unsigned)(before - r0)) : ld_volatile(old.g + before);
         }
       }
       if (live) {
@@ -568,6 +627,15 @@ __global__ void __launch_bounds__(Op::kThreads, 1) sweep_kernel(SweepArgs a, Op 
         op.lead(R, s, lead);
       }
       near &= isnew;
+      // the entries after the lead: which add, with what, and from where
+      unsigned adds = 0u, from[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        if (u >= lead && u < len && !op.skips(R, c[u])) adds |= 1u << u;
+        if (u >= lead) f[u] = op.signed_value(R, f[u]);
+        from[u] = fresh.own + ((near >> u & 1u) ? 8u * (unsigned)(at[u] - r0) : 0u);
+      }
+      double sum = live ? op.running(R, s) : 0.0;
       // wait for the other CTAs' new values and for this CTA's earlier steps
       while (ok) {
         const bool more = poll(~0u);
@@ -577,12 +645,19 @@ __global__ void __launch_bounds__(Op::kThreads, 1) sweep_kernel(SweepArgs a, Op 
         if (__all_sync(0xffffffffu, !more && turn)) break;
       }
       if (live && ok) {
+        if (OWN) {
+          double y[U];
+#pragma unroll
+          for (int u = 0; u < U; u++) y[u] = ld_shared(from[u]);
+#pragma unroll
+          for (int u = 0; u < U; u++) x[u] = (near >> u & 1u) ? y[u] : x[u];
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) x[u] = mul_rn(f[u], x[u]);
 #pragma unroll
         for (int u = 0; u < U; u++)
-          if (near >> u & 1u) x[u] = ld_shared(fresh.own + 8u * (unsigned)(c[u] - r0));
-#pragma unroll
-        for (int u = 0; u < U; u++)
-          if (u >= lead && u < len) op.take(R, s, u, c[u], f[u], x[u]);
+          if (adds >> u & 1u) sum = add_rn(sum, x[u]);
+        if (adds) op.run_to(R, s, sum);
         // rows longer than the entries held in registers
         for (int k = U; k < len && ok; k++) {
           int cc;
@@ -591,14 +666,15 @@ __global__ void __launch_bounds__(Op::kThreads, 1) sweep_kernel(SweepArgs a, Op 
           const bool nw = op.is_new(R, k, cc);
           if (nw || ph == 1) {
             const SweepSource& S = nw ? fresh : old;
-            const bool here = OWN && (unsigned)(cc - r0) < (unsigned)rows;
-            y = here ? ld_shared(S.own + 8u * (unsigned)(cc - r0)) : ld_volatile(S.g + cc);
+            const int q = place(cc, nw);
+            const bool here = OWN && (unsigned)(q - r0) < (unsigned)rows;
+            y = here ? ld_shared(S.own + 8u * (unsigned)(q - r0)) : ld_volatile(S.g + q);
             for (unsigned n = 1; !here && is_fill(y); n++) {
               if ((n & 255u) == 0u && !w.go_on(t0, seen)) {
                 ok = false;
                 break;
               }
-              y = ld_volatile(S.g + cc);
+              y = ld_volatile(S.g + q);
             }
           } else if (x0) {
             y = __ldcg(x0 + cc);
@@ -607,8 +683,9 @@ __global__ void __launch_bounds__(Op::kThreads, 1) sweep_kernel(SweepArgs a, Op 
         }
         if (ok) {
           const double v = not_fill(op.last(R, s));
-          if (OWN) st_shared(fresh.own + 8u * (unsigned)(row - r0), v);
-          *((volatile double*)P.out + row) = v;
+          if (OWN) st_shared(fresh.own + 8u * (unsigned)(slot - r0), v);
+          *((volatile double*)P.out + slot) = v;
+          if (a.result && ph == a.nph - 1) a.result[row] = v;
           op.store(R, v);
         }
       }
@@ -647,20 +724,23 @@ __global__ void __launch_bounds__(256) sweep_fill_kernel(int n, double* x, doubl
   }
 }
 
-// One launch of one or two sweeps; out1 null: one.
+// One launch of `sweeps` (1 or 2) sweeps; the last one's values go to `result`
+// (may be null) by row.
 template <class Op>
-int launch_sweeps(const SweepGrid& G, const SweepPlan* const (&plan)[2], const bool (&forward)[2],
-                  double* out0, double* out1, const Op& op, cudaStream_t s) {
+int launch_sweeps(const SweepGrid& G, int sweeps, const SweepPlan* const (&plan)[2],
+                  const bool (&forward)[2], double* result, const Op& op, cudaStream_t s) {
   const int n = G.n;
   if (n == 0) return SB2_OK;
   SweepArgs a;
   a.blk = G.d_blk;
   a.max_rows = G.max_rows;
-  a.nph = out1 ? 2 : 1;
-  double* out[2] = {out0, out1};
+  a.nph = sweeps;
+  a.result = result;
   for (int k = 0; k < 2; k++) {
-    const SweepPlan& P = *plan[out1 ? k : 0];
-    a.ph[k] = SweepPhase{P.d_rows, P.d_span, P.d_item, P.d_cta_item, P.d_steps, forward[out1 ? k : 0] ? 1 : 0, out[k]};
+    const int q = k < sweeps ? k : 0;
+    const SweepPlan& P = *plan[q];
+    a.ph[k] = SweepPhase{P.d_rows, P.d_span, P.d_item, P.d_cta_item, P.d_steps, P.d_pos,
+                         plan[0]->d_pos, forward[q] ? 1 : 0, G.d_new[k]};
   }
   a.state = G.d_state;
   a.wait_ns = ring_wait_ns();
@@ -668,7 +748,7 @@ int launch_sweeps(const SweepGrid& G, const SweepPlan* const (&plan)[2], const b
   const size_t smem = sizeof(double) * (size_t)a.nph * G.max_rows;
   const bool own = smem <= (size_t)kSweepSmem;
   const int g = std::min((n + 255) / 256, num_sms(current_device()) * 8);
-  sweep_fill_kernel<<<g, 256, 0, s>>>(n, out0, out1, G.d_state);
+  sweep_fill_kernel<<<g, 256, 0, s>>>(n, G.d_new[0], sweeps > 1 ? G.d_new[1] : nullptr, G.d_state);
   SB2_CUDA_TRY(cudaGetLastError());
   const void* kern = own ? (const void*)sweep_kernel<Op, true> : (const void*)sweep_kernel<Op, false>;
   if (own && smem > 48 * 1024)
