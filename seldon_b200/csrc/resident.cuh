@@ -20,8 +20,8 @@
 // operation; only the grouping of the reductions differs.
 //
 // Measured against the fused kernels on the same barrier (us per iteration,
-// 7- or 5-point operators): Cg 512^2 16.4 -> 9.4, 64^3 18.8 -> 11.5;
-// BiCgStab with Jacobi 32^3 17.0 -> 10.0; Gmres(30) with Jacobi 32^3 65.9 ->
+// 7- or 5-point operators): Cg 512^2 16.4 -> 8.4, 64^3 18.8 -> 10.8;
+// BiCgStab with Jacobi 32^3 17.0 -> 9.0; Gmres(30) with Jacobi 32^3 65.9 ->
 // 49.5, 64^3 74.9 -> 56.7, and with the matrix streamed 96^3 119 -> 91, 128^3
 // 190 -> 174.  Cg and BiCgStab with the matrix streamed gained nothing (80^3
 // 20.8 -> 21.4, 90^3 32 -> 33): there the product sets the pace, and with the
@@ -272,7 +272,7 @@ __device__ __noinline__ void res_product(const ResOp& A, int s0, int s1, const i
 
 #define SB2_RES_DECL                                   \
   extern __shared__ __align__(16) double s_res[];      \
-  __shared__ double s_red[NTR / 32];                   \
+  __shared__ double s_red[2 * (NTR / 32)];             \
   __shared__ double s_vals[kMaxRed];                   \
   const int tid = threadIdx.x;                         \
   const ResCta C = res_cta(A);                         \
@@ -283,16 +283,14 @@ __device__ __noinline__ void res_product(const ResOp& A, int s0, int s1, const i
   constexpr std::integral_constant<int, NTR == 512 ? (MS ? 4 : 3) : (MS ? 2 : 1)> kRound; \
   unsigned epoch = 0;                                  \
   int hlen = 0;                                        \
-  auto reduce1 = [&](double a) {                       \
-    a = block_sum<NTR>(a, s_red);                      \
-    if (tid == 0) s_vals[0] = a;                       \
-    return grid_sync<NTR>(P, epoch, 1, s_vals, s_red); \
+  /* fence: another CTA's vector is read before the next barrier */ \
+  auto reduce1 = [&](double a, bool fence = true) {    \
+    grid_arrive_sums<NTR, 1>(P, epoch, {a}, s_red);    \
+    return grid_wait<NTR, kPollerSums>(P, epoch, 1, s_vals, fence); \
   };                                                   \
-  auto reduce2 = [&](double a, double b) {             \
-    a = block_sum<NTR>(a, s_red);                      \
-    b = block_sum<NTR>(b, s_red);                      \
-    if (tid == 0) { s_vals[0] = a; s_vals[1] = b; }    \
-    return grid_sync<NTR>(P, epoch, 2, s_vals, s_red); \
+  auto reduce2 = [&](double a, double b, bool fence = true) { \
+    grid_arrive_sums<NTR, 2>(P, epoch, {a, b}, s_red); \
+    return grid_wait<NTR, kPollerSums>(P, epoch, 2, s_vals, fence); \
   };                                                   \
   /* t = A v, t and v in shared memory planes */ \
   auto product = [&](auto uc, const auto& g, const ResVec& t, const double* diag = nullptr) { \
@@ -320,6 +318,7 @@ constexpr int res_cg_vecs(bool jac) { return jac ? 6 : 4; }
 template <int NTR, bool MS>
 __global__ void __launch_bounds__(NTR, 1) cg_resident_kernel(ResOp A, CgResVecs v, IterArgs it,
                                                              Persist P, History H, SolveOut* out) {
+  constexpr bool kPollerSums = true;
   SB2_RES_DECL;
   const size_t plane = 4 * (size_t)C.NQ;
   const ResVec xs{s_res, C.NQ}, rs{s_res + plane, C.NQ}, ps{s_res + 2 * plane, C.NQ},
@@ -409,7 +408,7 @@ __global__ void __launch_bounds__(NTR, 1) cg_resident_kernel(ResOp A, CgResVecs 
           for (int j = 0; j < 4; j++)
             if (live(q, j)) d = add_rn(d, mul_rn(ps.at(q, j), t[j]));
         });
-    if (!reduce1(d)) return;
+    if (!reduce1(d, false)) return;
     const double delta = s_vals[0];
     if (delta == 0.0) { fail = 2; break; }
     const double alpha = rho / delta;
@@ -468,6 +467,7 @@ template <int NTR, bool MS>
 __global__ void __launch_bounds__(NTR, 1) bicgstab_resident_kernel(ResOp A, BicgResVecs v,
                                                                    IterArgs it, Persist P,
                                                                    History H, SolveOut* out) {
+  constexpr bool kPollerSums = true;
   SB2_RES_DECL;
   const size_t plane = 4 * (size_t)C.NQ;
   const ResVec ps{s_res, C.NQ}, rs{s_res + plane, C.NQ}, vs{s_res + 2 * plane, C.NQ},
@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(NTR, 1) bicgstab_resident_kernel(ResOp A, Bicg
       for (int j = 0; j < 4; j++)
         if (live(q, j)) d = add_rn(d, mul_rn(wv[j], vs.at(q, j)));
     });
-    if (!reduce1(d)) return;
+    if (!reduce1(d, false)) return;
     const double sigma = s_vals[0];
     if (sigma == 0.0) { fail = 3; break; }
     alpha = rho_1 / sigma;
@@ -615,7 +615,7 @@ __global__ void __launch_bounds__(NTR, 1) bicgstab_resident_kernel(ResOp A, Bicg
         t1 = add_rn(t1, mul_rn(t, t));
       }
     });
-    if (!reduce2(t0, t1)) return;
+    if (!reduce2(t0, t1, false)) return;
     omega = s_vals[0] / s_vals[1];
     // Add(alpha, phat, x); Add(omega, shat, x); Copy(s, r); Add(-omega, t, r)
     rr = 0.0;
@@ -640,7 +640,7 @@ __global__ void __launch_bounds__(NTR, 1) bicgstab_resident_kernel(ResOp A, Bicg
       res_store(v.x, row, A.n, xv);
       rs.set(q, rv);
     });
-    if (!reduce2(rr, rtr)) return;
+    if (!reduce2(rr, rtr, false)) return;
     rr = s_vals[0];
     rho_2 = rho_1;
     rho_1 = s_vals[1];
@@ -667,6 +667,7 @@ struct GmresResVecs {
 template <int NTR, int QR, bool MS>
 __global__ void __launch_bounds__(NTR, 1) gmres_resident_kernel(ResOp A, GmresResVecs v, IterArgs it,
                                                                 Persist P, History H, SolveOut* out) {
+  constexpr bool kPollerSums = false;
   SB2_RES_DECL;
   const int m = it.restart, ld = m + 1;
   const size_t plane = 4 * (size_t)C.NQ;
@@ -720,21 +721,7 @@ __global__ void __launch_bounds__(NTR, 1) gmres_resident_kernel(ResOp A, GmresRe
   };
   const int pairs = 2 * C.nq;
   auto live2 = [&](int e, int j) { return C.r0 + 2 * e + j < A.n; };
-  // arrival with one sum: warp 0 adds the warps' and deposits the CTA's
-  auto arrive1 = [&](double a) {
-    a = warp_sum(a);
-    if ((tid & 31) == 0) s_red[tid >> 5] = a;
-    __syncthreads();
-    double* part = P.partials + (size_t)(epoch & 1u) * kMaxRed * gridDim.x;
-    epoch++;
-    if (tid < 32) {
-      a = warp_sum(tid < NTR / 32 ? s_red[tid] : 0.0);
-      if (tid == 0) {
-        __stcg(part + blockIdx.x, a);
-        red_release_u32(&P.sync->count, 1u);
-      }
-    }
-  };
+  auto arrive1 = [&](double a) { grid_arrive_sums<NTR, 1>(P, epoch, {a}, s_red); };
 
   // w = b (- A x); r = M^{-1} w; beta = ||r|| (Gmres.cxx:82-90)
   double rr = 0.0;
