@@ -69,6 +69,10 @@ struct IterArgs {
   __shared__ double s_prod[kNnzCap];        \
   __shared__ double s_red[NT / 32];         \
   __shared__ double s_vals[kMaxRed]
+// ... and the arrivals' own warp sums (grid_sums, up to 4 values)
+#define SB2_SUMS_DECL                       \
+  SB2_SHARED_DECL;                          \
+  __shared__ double s_arr[4 * (NT / 32)]
 
 __device__ __forceinline__ double precond_val(const double* diag, int i, double r) {
   return diag ? __ddiv_rn(r, diag[i]) : r;  // Jacobi z_i = r_i / A(i,i)
@@ -220,6 +224,9 @@ struct CgVecs {
   double *x, *r, *p, *q;
 };
 
+// Its sums stay block_sum's with grid_sync: grid_sums, 3 % faster in BiCgStab
+// (20.8 to 20.3 us an iteration on 80^3), Cgs and Minres, loses 2 % here (35.1
+// to 35.8 on 100^3).
 __global__ void __launch_bounds__(NT, 1) cg_fused_kernel(OpArgs A, CgVecs v, IterArgs it,
                                                       Persist P, History H, SolveOut* out) {
   SB2_SHARED_DECL;
@@ -382,7 +389,7 @@ struct EpiStoreDot2 {
 __global__ void __launch_bounds__(NT, 1) bicgstab_fused_kernel(OpArgs A, BicgVecs v, IterArgs it,
                                                             Persist P, History H,
                                                             SolveOut* out) {
-  SB2_SHARED_DECL;
+  SB2_SUMS_DECL;
   const int tid = threadIdx.x;
   const long long gt = (long long)blockIdx.x * NT + tid, gs = (long long)gridDim.x * NT;
   const int n = A.n;
@@ -395,9 +402,7 @@ __global__ void __launch_bounds__(NT, 1) bicgstab_fused_kernel(OpArgs A, BicgVec
     const double bi = __ldg(v.b + i);
     acc = add_rn(acc, mul_rn(bi, bi));
   }
-  acc = block_sum<NT>(acc, s_red);
-  if (tid == 0) s_vals[0] = acc;
-  if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+  if (!grid_sums<NT, 1>(P, epoch, {acc}, s_vals, s_arr)) return;
   const double normb = sqrt(s_vals[0]);
   if (normb == 0.0) {
     if (lead) { out->init_failed = 1; out->hist_len = 0; }
@@ -422,9 +427,7 @@ __global__ void __launch_bounds__(NT, 1) bicgstab_fused_kernel(OpArgs A, BicgVec
     if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
     for (long long i = gt; i < n; i += gs) v.rt[i] = __ldcg(v.r + i);
   }
-  rr = block_sum<NT>(rr, s_red);
-  if (tid == 0) { s_vals[0] = rr; s_vals[1] = rr; }
-  if (!grid_sync<NT>(P, epoch, 2, s_vals, s_red)) return;
+  if (!grid_sums<NT, 2>(P, epoch, {rr, rr}, s_vals, s_arr)) return;
   rr = s_vals[0];
   double rho_1 = s_vals[1];  // (rtilde, r) with rtilde = r
   double rho_2 = 0.0, alpha = 0.0, omega = 0.0;
@@ -468,9 +471,7 @@ __global__ void __launch_bounds__(NT, 1) bicgstab_fused_kernel(OpArgs A, BicgVec
     // v = A phat, sigma = (rtilde, v)
     EpiStoreDot2 e1{v.v, v.rt, false, 0.0, 0.0};
     spmv_phase(A, ph, e1, s_prod, s_red);
-    double d = block_sum<NT>(e1.acc0, s_red);
-    if (tid == 0) s_vals[0] = d;
-    if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+    if (!grid_sums<NT, 1>(P, epoch, {e1.acc0}, s_vals, s_arr)) return;
     const double sigma = s_vals[0];
     if (sigma == 0.0) { fail = 3; break; }
     alpha = rho_1 / sigma;
@@ -489,9 +490,7 @@ __global__ void __launch_bounds__(NT, 1) bicgstab_fused_kernel(OpArgs A, BicgVec
 #pragma unroll
       for (int j = 0; j < W; j++) ss = add_rn(ss, mul_rn(si.v[j], si.v[j]));
     });
-    ss = block_sum<NT>(ss, s_red);
-    if (tid == 0) s_vals[0] = ss;
-    if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+    if (!grid_sums<NT, 1>(P, epoch, {ss}, s_vals, s_arr)) return;
     nb_iter++;
     reste = facteur * sqrt(s_vals[0]);
     if (lead) hist_push(H, &hlen, nb_iter, reste);
@@ -505,10 +504,7 @@ __global__ void __launch_bounds__(NT, 1) bicgstab_fused_kernel(OpArgs A, BicgVec
     // t = A shat; omega = (t, s) / (t, t)
     EpiStoreDot2 e2{v.t, v.s, true, 0.0, 0.0};
     spmv_phase(A, sh, e2, s_prod, s_red);
-    const double ts = block_sum<NT>(e2.acc0, s_red);
-    const double tt = block_sum<NT>(e2.acc1, s_red);
-    if (tid == 0) { s_vals[0] = ts; s_vals[1] = tt; }
-    if (!grid_sync<NT>(P, epoch, 2, s_vals, s_red)) return;
+    if (!grid_sums<NT, 2>(P, epoch, {e2.acc0, e2.acc1}, s_vals, s_arr)) return;
     omega = s_vals[0] / s_vals[1];
     // Add(alpha, phat, x); Add(omega, shat, x); Copy(s, r); Add(-omega, t, r)
     rr = 0.0;
@@ -541,10 +537,7 @@ __global__ void __launch_bounds__(NT, 1) bicgstab_fused_kernel(OpArgs A, BicgVec
         rtr = add_rn(rtr, mul_rn(rti.v[j], ri.v[j]));
       }
     });
-    rr = block_sum<NT>(rr, s_red);
-    rtr = block_sum<NT>(rtr, s_red);
-    if (tid == 0) { s_vals[0] = rr; s_vals[1] = rtr; }
-    if (!grid_sync<NT>(P, epoch, 2, s_vals, s_red)) return;
+    if (!grid_sums<NT, 2>(P, epoch, {rr, rtr}, s_vals, s_arr)) return;
     rr = s_vals[0];
     rho_2 = rho_1;
     rho_1 = s_vals[1];
@@ -601,7 +594,7 @@ struct EpiResidUpdate {
 // second product is fused with the residual update and both reductions.
 __global__ void __launch_bounds__(NT, 1) cgs_fused_kernel(OpArgs A, CgsVecs v, IterArgs it,
                                                        Persist P, History H, SolveOut* out) {
-  SB2_SHARED_DECL;
+  SB2_SUMS_DECL;
   const int tid = threadIdx.x;
   const long long gt = (long long)blockIdx.x * NT + tid, gs = (long long)gridDim.x * NT;
   const int n = A.n;
@@ -614,9 +607,7 @@ __global__ void __launch_bounds__(NT, 1) cgs_fused_kernel(OpArgs A, CgsVecs v, I
     const double bi = __ldg(v.b + i);
     acc = add_rn(acc, mul_rn(bi, bi));
   }
-  acc = block_sum<NT>(acc, s_red);
-  if (tid == 0) s_vals[0] = acc;
-  if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+  if (!grid_sums<NT, 1>(P, epoch, {acc}, s_vals, s_arr)) return;
   const double normb = sqrt(s_vals[0]);
   if (normb == 0.0) {
     if (lead) { out->init_failed = 1; out->hist_len = 0; }
@@ -641,9 +632,7 @@ __global__ void __launch_bounds__(NT, 1) cgs_fused_kernel(OpArgs A, CgsVecs v, I
     if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
     for (long long i = gt; i < n; i += gs) v.rt[i] = __ldcg(v.r + i);
   }
-  rr = block_sum<NT>(rr, s_red);
-  if (tid == 0) s_vals[0] = rr;
-  if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+  if (!grid_sums<NT, 1>(P, epoch, {rr}, s_vals, s_arr)) return;
   rr = s_vals[0];
   double rho_1 = rr, rho_2 = 0.0;
   const bool jac = (A.diag != nullptr);
@@ -688,9 +677,7 @@ __global__ void __launch_bounds__(NT, 1) cgs_fused_kernel(OpArgs A, CgsVecs v, I
     // vhat = A phat fused with delta = (rtilde, vhat)
     EpiStoreDot e1{v.vh, v.rt, 0.0};
     spmv_phase(A, ph, e1, s_prod, s_red);
-    const double d = block_sum<NT>(e1.acc, s_red);
-    if (tid == 0) s_vals[0] = d;
-    if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+    if (!grid_sums<NT, 1>(P, epoch, {e1.acc}, s_vals, s_arr)) return;
     nb_iter++;
     const double delta = s_vals[0];
     if (delta == 0.0) { fail = 2; break; }
@@ -720,10 +707,7 @@ __global__ void __launch_bounds__(NT, 1) cgs_fused_kernel(OpArgs A, CgsVecs v, I
     // qhat = A uhat fused with Add(-alpha, qhat, r), ||r||^2 and (rtilde, r)
     EpiResidUpdate e2{v.r, v.rt, -alpha, 0.0, 0.0};
     spmv_phase(A, uh, e2, s_prod, s_red);
-    rr = block_sum<NT>(e2.rr, s_red);
-    const double rtr = block_sum<NT>(e2.rtr, s_red);
-    if (tid == 0) { s_vals[0] = rr; s_vals[1] = rtr; }
-    if (!grid_sync<NT>(P, epoch, 2, s_vals, s_red)) return;
+    if (!grid_sums<NT, 2>(P, epoch, {e2.rr, e2.rtr}, s_vals, s_arr)) return;
     rr = s_vals[0];
     rho_2 = rho_1;
     rho_1 = s_vals[1];
@@ -883,7 +867,7 @@ struct EpiTfqmrNextV {
 // rides in the epilogue of the product that follows it.
 __global__ void __launch_bounds__(NT, 1) tfqmr_fused_kernel(OpArgs A, TfqmrVecs v, IterArgs it,
                                                          Persist P, History H, SolveOut* out) {
-  SB2_SHARED_DECL;
+  SB2_SUMS_DECL;
   const int tid = threadIdx.x;
   const long long gt = (long long)blockIdx.x * NT + tid, gs = (long long)gridDim.x * NT;
   const int n = A.n;
@@ -908,9 +892,7 @@ __global__ void __launch_bounds__(NT, 1) tfqmr_fused_kernel(OpArgs A, TfqmrVecs 
     spmv_phase(A, v.x, epi, s_prod, s_red);
     rr = epi.rr;
   }
-  rr = block_sum<NT>(rr, s_red);
-  if (tid == 0) s_vals[0] = rr;
-  if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+  if (!grid_sums<NT, 1>(P, epoch, {rr}, s_vals, s_arr)) return;
   // iter.Init(r0); tau = Norm2(r0); rho = (rtilde, r0) with rtilde = r0
   const double tau0 = sqrt(s_vals[0]);
   if (tau0 == 0.0) {
@@ -923,9 +905,7 @@ __global__ void __launch_bounds__(NT, 1) tfqmr_fused_kernel(OpArgs A, TfqmrVecs 
   {
     EpiTfqmrFirstV epi{A.diag, v.rt, v.v, v.g, 0.0};
     spmv_phase(A, v.y1, epi, s_prod, s_red);
-    const double sg = block_sum<NT>(epi.sigma, s_red);
-    if (tid == 0) s_vals[0] = sg;
-    if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+    if (!grid_sums<NT, 1>(P, epoch, {epi.sigma}, s_vals, s_arr)) return;
   }
   double sigma = s_vals[0];
 
@@ -958,9 +938,7 @@ __global__ void __launch_bounds__(NT, 1) tfqmr_fused_kernel(OpArgs A, TfqmrVecs 
         stw<W>(v.w, i, wi);
         stw<W>(v.d, i, di);
       });
-      ww = block_sum<NT>(ww, s_red);
-      if (tid == 0) s_vals[0] = ww;
-      if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+      if (!grid_sums<NT, 1>(P, epoch, {ww}, s_vals, s_arr)) return;
     }
     // 14.-21. theta, c, tau, eta; x += eta d; Finished(kappa)
     theta = sqrt(s_vals[0]) / tau;
@@ -983,10 +961,7 @@ __global__ void __launch_bounds__(NT, 1) tfqmr_fused_kernel(OpArgs A, TfqmrVecs 
       EpiTfqmrHalf epi{A.diag, v.rt, v.y0, v.h, v.x, v.w, v.d,
                         eta, -alpha, theta * theta * eta / alpha, 0.0, 0.0};
       spmv_phase(A, v.y0, epi, s_prod, s_red);
-      const double ww = block_sum<NT>(epi.ww, s_red);
-      const double rtw = block_sum<NT>(epi.rtw, s_red);
-      if (tid == 0) { s_vals[0] = ww; s_vals[1] = rtw; }
-      if (!grid_sync<NT>(P, epoch, 2, s_vals, s_red)) return;
+      if (!grid_sums<NT, 2>(P, epoch, {epi.ww, epi.rtw}, s_vals, s_arr)) return;
     }
     if (tau == 0.0) { fail = 4; break; }
     theta = sqrt(s_vals[0]) / tau;
@@ -1029,9 +1004,7 @@ __global__ void __launch_bounds__(NT, 1) tfqmr_fused_kernel(OpArgs A, TfqmrVecs 
     {
       EpiTfqmrNextV epi{A.diag, v.rt, v.h, v.g, v.v, beta, beta * beta, 0.0};
       spmv_phase(A, v.y1, epi, s_prod, s_red);
-      const double sg = block_sum<NT>(epi.sigma, s_red);
-      if (tid == 0) s_vals[0] = sg;
-      if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+      if (!grid_sums<NT, 1>(P, epoch, {epi.sigma}, s_vals, s_arr)) return;
     }
     sigma = s_vals[0];
     nb_iter++;
@@ -1056,7 +1029,7 @@ struct MinresVecs {
 // reference's separately rounded products and sums.
 __global__ void __launch_bounds__(NT, 1) minres_fused_kernel(OpArgs A, MinresVecs v, IterArgs it,
                                                           Persist P, History H, SolveOut* out) {
-  SB2_SHARED_DECL;
+  SB2_SUMS_DECL;
   const int tid = threadIdx.x;
   const long long gt = (long long)blockIdx.x * NT + tid, gs = (long long)gridDim.x * NT;
   const int n = A.n;
@@ -1070,9 +1043,7 @@ __global__ void __launch_bounds__(NT, 1) minres_fused_kernel(OpArgs A, MinresVec
     const double bi = __ldg(v.b + i);
     acc = add_rn(acc, mul_rn(bi, bi));
   }
-  acc = block_sum<NT>(acc, s_red);
-  if (tid == 0) s_vals[0] = acc;
-  if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+  if (!grid_sums<NT, 1>(P, epoch, {acc}, s_vals, s_arr)) return;
   const double normb = sqrt(s_vals[0]);
   if (normb == 0.0) {
     if (lead) { out->init_failed = 1; out->hist_len = 0; }
@@ -1094,9 +1065,7 @@ __global__ void __launch_bounds__(NT, 1) minres_fused_kernel(OpArgs A, MinresVec
     spmv_phase(A, v.x, epi, s_prod, s_red);
     dp = epi.rz;
   }
-  dp = block_sum<NT>(dp, s_red);
-  if (tid == 0) s_vals[0] = dp;
-  if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+  if (!grid_sums<NT, 1>(P, epoch, {dp}, s_vals, s_arr)) return;
   double beta = sqrt(s_vals[0]);
   double eta = beta;
   {
@@ -1139,9 +1108,7 @@ __global__ void __launch_bounds__(NT, 1) minres_fused_kernel(OpArgs A, MinresVec
     {
       EpiStoreDot epi{v.r, u, 0.0};
       spmv_phase(A, u, epi, s_prod, s_red);
-      const double a = block_sum<NT>(epi.acc, s_red);
-      if (tid == 0) s_vals[0] = a;
-      if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+      if (!grid_sums<NT, 1>(P, epoch, {epi.acc}, s_vals, s_arr)) return;
     }
     const double alpha = s_vals[0];
     // z = M^{-1} r; Add(-alpha, v, r); Add(-alpha, u, z); Add(-beta, v_old, r);
@@ -1173,9 +1140,7 @@ __global__ void __launch_bounds__(NT, 1) minres_fused_kernel(OpArgs A, MinresVec
 #pragma unroll
         for (int j = 0; j < W; j++) d = add_rn(d, mul_rn(ri.v[j], zi.v[j]));
       });
-      d = block_sum<NT>(d, s_red);
-      if (tid == 0) s_vals[0] = d;
-      if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+      if (!grid_sums<NT, 1>(P, epoch, {d}, s_vals, s_arr)) return;
     }
     const double beta_old = beta;
     beta = sqrt(s_vals[0]);
@@ -1320,7 +1285,7 @@ struct EpiGcrQ {
 // then repeats -- the solve stops after that cycle.
 __global__ void __launch_bounds__(NT, 1) gcr_fused_kernel(OpArgs A, GcrVecs v, IterArgs it,
                                                        Persist P, History H, SolveOut* out) {
-  SB2_SHARED_DECL;
+  SB2_SUMS_DECL;
   __shared__ double s_beta[kGcrMaxRestart + 1];
   __shared__ double s_delta[kMaxRed];
   const int tid = threadIdx.x;
@@ -1338,9 +1303,7 @@ __global__ void __launch_bounds__(NT, 1) gcr_fused_kernel(OpArgs A, GcrVecs v, I
     const double bi = __ldg(v.b + i);
     acc = add_rn(acc, mul_rn(bi, bi));
   }
-  acc = block_sum<NT>(acc, s_red);
-  if (tid == 0) s_vals[0] = acc;
-  if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+  if (!grid_sums<NT, 1>(P, epoch, {acc}, s_vals, s_arr)) return;
   const double normb = sqrt(s_vals[0]);
   if (normb == 0.0) {
     if (lead) { out->init_failed = 1; out->hist_len = 0; }
@@ -1362,9 +1325,7 @@ __global__ void __launch_bounds__(NT, 1) gcr_fused_kernel(OpArgs A, GcrVecs v, I
     spmv_phase(A, v.x, epi, s_prod, s_red);
     rr = epi.rr;
   }
-  rr = block_sum<NT>(rr, s_red);
-  if (tid == 0) s_vals[0] = rr;
-  if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+  if (!grid_sums<NT, 1>(P, epoch, {rr}, s_vals, s_arr)) return;
   rr = s_vals[0];
   double normr = sqrt(rr);
 
@@ -1400,10 +1361,7 @@ __global__ void __launch_bounds__(NT, 1) gcr_fused_kernel(OpArgs A, GcrVecs v, I
       {
         EpiGcrW epi{wj, v.r, A.diag, 0.0, 0.0};
         spmv_phase(A, pj, epi, s_prod, s_red);
-        const double ww = block_sum<NT>(epi.ww, s_red);
-        const double wr = block_sum<NT>(epi.wr, s_red);
-        if (tid == 0) { s_vals[0] = ww; s_vals[1] = wr; }
-        if (!grid_sync<NT>(P, epoch, 2, s_vals, s_red)) return;
+        if (!grid_sums<NT, 2>(P, epoch, {epi.ww, epi.wr}, s_vals, s_arr)) return;
       }
       const double beta_j = s_vals[0];
       if (beta_j == 0.0) { fail = 1; break; }
@@ -1431,9 +1389,7 @@ __global__ void __launch_bounds__(NT, 1) gcr_fused_kernel(OpArgs A, GcrVecs v, I
 #pragma unroll
           for (int k = 0; k < Wd; k++) a = add_rn(a, mul_rn(ri.v[k], ri.v[k]));
         });
-        a = block_sum<NT>(a, s_red);
-        if (tid == 0) s_vals[0] = a;
-        if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+        if (!grid_sums<NT, 1>(P, epoch, {a}, s_vals, s_arr)) return;
         rr = s_vals[0];
       }
       nb_iter++;
@@ -1519,7 +1475,7 @@ struct EpiBiclInit {
 __global__ void __launch_bounds__(NT, 1) bicgstabl_fused_kernel(OpArgs A, BicglVecs v,
                                                              IterArgs it, Persist P, History H,
                                                              SolveOut* out) {
-  SB2_SHARED_DECL;
+  SB2_SUMS_DECL;
   __shared__ double s_tau[(kBicglMax + 1) * (kBicglMax + 1)];
   __shared__ double s_g[kBicglMax + 1], s_gp[kBicglMax + 1], s_gt[kBicglMax + 1];
   const int tid = threadIdx.x;
@@ -1548,9 +1504,7 @@ __global__ void __launch_bounds__(NT, 1) bicgstabl_fused_kernel(OpArgs A, BicglV
       Uv(k)[i] = 0.0;
     }
   }
-  acc = block_sum<NT>(acc, s_red);
-  if (tid == 0) s_vals[0] = acc;
-  if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+  if (!grid_sums<NT, 1>(P, epoch, {acc}, s_vals, s_arr)) return;
   // iter.Init(b) comes after r_0 in the reference; r_0 is not observable
   // when it fails, x (zeroed for a null guess) is
   const double normb = sqrt(s_vals[0]);
@@ -1573,9 +1527,7 @@ __global__ void __launch_bounds__(NT, 1) bicgstabl_fused_kernel(OpArgs A, BicglV
     spmv_phase(A, v.x, epi, s_prod, s_red);
     rr = epi.rr;
   }
-  rr = block_sum<NT>(rr, s_red);
-  if (tid == 0) s_vals[0] = rr;
-  if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+  if (!grid_sums<NT, 1>(P, epoch, {rr}, s_vals, s_arr)) return;
   rr = s_vals[0];
   double rho_next = rr;  // (r_0, r0) with r0 = r_0
   double rho_0 = 1.0, alpha = 0.0, omega = 1.0;
@@ -1612,9 +1564,7 @@ __global__ void __launch_bounds__(NT, 1) bicgstabl_fused_kernel(OpArgs A, BicglV
       {
         EpiStoreDot epi{Uv(j + 1), v.rt, 0.0};
         spmv_phase(A, jac ? v.q : Uv(j), epi, s_prod, s_red);
-        const double d = block_sum<NT>(epi.acc, s_red);
-        if (tid == 0) s_vals[0] = d;
-        if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+        if (!grid_sums<NT, 1>(P, epoch, {epi.acc}, s_vals, s_arr)) return;
       }
       nb_iter++;
       const double sigma = s_vals[0];
@@ -1646,9 +1596,7 @@ __global__ void __launch_bounds__(NT, 1) bicgstabl_fused_kernel(OpArgs A, BicglV
       {
         EpiStoreDot epi{Rv(j + 1), v.rt, 0.0};
         spmv_phase(A, jac ? v.q : Rv(j), epi, s_prod, s_red);
-        const double d = block_sum<NT>(epi.acc, s_red);
-        if (tid == 0) s_vals[0] = d;
-        if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+        if (!grid_sums<NT, 1>(P, epoch, {epi.acc}, s_vals, s_arr)) return;
       }
       rho_next = s_vals[0];
       nb_iter++;
@@ -1686,10 +1634,9 @@ __global__ void __launch_bounds__(NT, 1) bicgstabl_fused_kernel(OpArgs A, BicglV
             }
           }
         });
-        d0 = block_sum<NT>(d0, s_red);
-        if (last) d1 = block_sum<NT>(d1, s_red);
-        if (tid == 0) { s_vals[0] = d0; s_vals[1] = d1; }
-        if (!grid_sync<NT>(P, epoch, last ? 2 : 1, s_vals, s_red)) return;
+        if (!(last ? grid_sums<NT, 2>(P, epoch, {d0, d1}, s_vals, s_arr)
+                   : grid_sums<NT, 1>(P, epoch, {d0}, s_vals, s_arr)))
+          return;
         if (!last) {
           ptau = s_vals[0] / s_g[i];
           if (tid == 0) s_tau[i * L1 + j] = ptau;
@@ -1773,10 +1720,7 @@ __global__ void __launch_bounds__(NT, 1) bicgstabl_fused_kernel(OpArgs A, BicglV
           a1 = add_rn(a1, mul_rn(r0e.v[k], rte.v[k]));
         }
       });
-      a0 = block_sum<NT>(a0, s_red);
-      a1 = block_sum<NT>(a1, s_red);
-      if (tid == 0) { s_vals[0] = a0; s_vals[1] = a1; }
-      if (!grid_sync<NT>(P, epoch, 2, s_vals, s_red)) return;
+      if (!grid_sums<NT, 2>(P, epoch, {a0, a1}, s_vals, s_arr)) return;
       rr = s_vals[0];
       rho_next = s_vals[1];
     }
@@ -1829,7 +1773,7 @@ struct EpiQcgsFit {
 // end, breakdown or not, as in the reference.
 __global__ void __launch_bounds__(NT, 1) qcgs_fused_kernel(OpArgs A, QcgsVecs v, IterArgs it,
                                                         Persist P, History H, SolveOut* out) {
-  SB2_SHARED_DECL;
+  SB2_SUMS_DECL;
   const int tid = threadIdx.x;
   const long long gt = (long long)blockIdx.x * NT + tid, gs = (long long)gridDim.x * NT;
   const int n = A.n;
@@ -1844,9 +1788,7 @@ __global__ void __launch_bounds__(NT, 1) qcgs_fused_kernel(OpArgs A, QcgsVecs v,
     const double bi = __ldg(v.b + i);
     acc = add_rn(acc, mul_rn(bi, bi));
   }
-  acc = block_sum<NT>(acc, s_red);
-  if (tid == 0) s_vals[0] = acc;
-  if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+  if (!grid_sums<NT, 1>(P, epoch, {acc}, s_vals, s_arr)) return;
   const double normb = sqrt(s_vals[0]);
   if (normb == 0.0) {
     if (lead) { out->init_failed = 1; out->hist_len = 0; }
@@ -1876,9 +1818,7 @@ __global__ void __launch_bounds__(NT, 1) qcgs_fused_kernel(OpArgs A, QcgsVecs v,
     v.p[i] = 0.0;
     rr = add_rn(rr, mul_rn(ri, ri));
   }
-  rr = block_sum<NT>(rr, s_red);
-  if (tid == 0) s_vals[0] = rr;
-  if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+  if (!grid_sums<NT, 1>(P, epoch, {rr}, s_vals, s_arr)) return;
   double rqq = s_vals[0], rho_2 = s_vals[0], rho_1 = 1.0;
 
   int nb_iter = 0, fail = 0;
@@ -1909,10 +1849,7 @@ __global__ void __launch_bounds__(NT, 1) qcgs_fused_kernel(OpArgs A, QcgsVecs v,
     {
       EpiStoreDot2 epi{v.v, v.rt, true, 0.0, 0.0};
       spmv_phase(A, ph, epi, s_prod, s_red);
-      const double sg = block_sum<NT>(epi.acc0, s_red);
-      const double vv = block_sum<NT>(epi.acc1, s_red);
-      if (tid == 0) { s_vals[0] = sg; s_vals[1] = vv; }
-      if (!grid_sync<NT>(P, epoch, 2, s_vals, s_red)) return;
+      if (!grid_sums<NT, 2>(P, epoch, {epi.acc0, epi.acc1}, s_vals, s_arr)) return;
     }
     nb_iter++;
     const double sigma = s_vals[0];
@@ -1946,12 +1883,7 @@ __global__ void __launch_bounds__(NT, 1) qcgs_fused_kernel(OpArgs A, QcgsVecs v,
     {
       EpiQcgsFit epi{v.r, v.uf, v.rq, v.v, -alpha, 0.0, 0.0, 0.0, 0.0};
       spmv_phase(A, jac ? v.ph : v.u, epi, s_prod, s_red);
-      const double uu = block_sum<NT>(epi.uu, s_red);
-      const double uv = block_sum<NT>(epi.uv, s_red);
-      const double ur = block_sum<NT>(epi.ur, s_red);
-      const double vr = block_sum<NT>(epi.vr, s_red);
-      if (tid == 0) { s_vals[0] = uu; s_vals[1] = uv; s_vals[2] = ur; s_vals[3] = vr; }
-      if (!grid_sync<NT>(P, epoch, 4, s_vals, s_red)) return;
+      if (!grid_sums<NT, 4>(P, epoch, {epi.uu, epi.uv, epi.ur, epi.vr}, s_vals, s_arr)) return;
     }
     const double b00 = s_vals[0], b10 = s_vals[1];
     // the symmetric 2 x 2 inverse (b(0,1) is b(1,0))
@@ -2000,10 +1932,7 @@ __global__ void __launch_bounds__(NT, 1) qcgs_fused_kernel(OpArgs A, QcgsVecs v,
           a1 = add_rn(a1, mul_rn(rti.v[j], ri.v[j]));
         }
       });
-      a0 = block_sum<NT>(a0, s_red);
-      a1 = block_sum<NT>(a1, s_red);
-      if (tid == 0) { s_vals[0] = a0; s_vals[1] = a1; }
-      if (!grid_sync<NT>(P, epoch, 2, s_vals, s_red)) return;
+      if (!grid_sums<NT, 2>(P, epoch, {a0, a1}, s_vals, s_arr)) return;
       rqq = s_vals[0];
       rho_1 = rho_2;
       rho_2 = s_vals[1];
@@ -2047,7 +1976,7 @@ struct EpiStore {
 // over the explicit transpose (or the expanded symmetric pattern) does.
 __global__ void __launch_bounds__(NT, 1) bicg_fused_kernel(OpArgs A, BcgVecs v, IterArgs it,
                                                         Persist P, History H, SolveOut* out) {
-  SB2_SHARED_DECL;
+  SB2_SUMS_DECL;
   const int tid = threadIdx.x;
   const long long gt = (long long)blockIdx.x * NT + tid, gs = (long long)gridDim.x * NT;
   const int n = A.n;
@@ -2060,9 +1989,7 @@ __global__ void __launch_bounds__(NT, 1) bicg_fused_kernel(OpArgs A, BcgVecs v, 
     const double bi = __ldg(v.b + i);
     acc = add_rn(acc, mul_rn(bi, bi));
   }
-  acc = block_sum<NT>(acc, s_red);
-  if (tid == 0) s_vals[0] = acc;
-  if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+  if (!grid_sums<NT, 1>(P, epoch, {acc}, s_vals, s_arr)) return;
   const double normb = sqrt(s_vals[0]);
   if (normb == 0.0) {
     if (lead) { out->init_failed = 1; out->hist_len = 0; }
@@ -2089,10 +2016,7 @@ __global__ void __launch_bounds__(NT, 1) bicg_fused_kernel(OpArgs A, BcgVecs v, 
     rr = add_rn(rr, mul_rn(ri, ri));
     rz = add_rn(rz, mul_rn(precond_val(A.diag, (int)i, ri), ri));
   }
-  rr = block_sum<NT>(rr, s_red);
-  rz = block_sum<NT>(rz, s_red);
-  if (tid == 0) { s_vals[0] = rr; s_vals[1] = rz; }
-  if (!grid_sync<NT>(P, epoch, 2, s_vals, s_red)) return;
+  if (!grid_sums<NT, 2>(P, epoch, {rr, rz}, s_vals, s_arr)) return;
   rr = s_vals[0];
   double rho_1 = s_vals[1], rho_2 = 0.0;
 
@@ -2133,9 +2057,7 @@ __global__ void __launch_bounds__(NT, 1) bicg_fused_kernel(OpArgs A, BcgVecs v, 
       spmv_phase(A, v.p, e1, s_prod, s_red);
       EpiStore e2{v.qt};
       spmv_phase(v.AT, v.pt, e2, s_prod, s_red);
-      const double d = block_sum<NT>(e1.acc, s_red);
-      if (tid == 0) s_vals[0] = d;
-      if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+      if (!grid_sums<NT, 1>(P, epoch, {e1.acc}, s_vals, s_arr)) return;
     }
     nb_iter++;
     const double delta = s_vals[0];
@@ -2172,10 +2094,7 @@ __global__ void __launch_bounds__(NT, 1) bicg_fused_kernel(OpArgs A, BcgVecs v, 
           a1 = add_rn(a1, mul_rn(zi.v[j], rti.v[j]));
         }
       });
-      a0 = block_sum<NT>(a0, s_red);
-      a1 = block_sum<NT>(a1, s_red);
-      if (tid == 0) { s_vals[0] = a0; s_vals[1] = a1; }
-      if (!grid_sync<NT>(P, epoch, 2, s_vals, s_red)) return;
+      if (!grid_sums<NT, 2>(P, epoch, {a0, a1}, s_vals, s_arr)) return;
       rr = s_vals[0];
       rho_2 = rho_1;
       rho_1 = s_vals[1];
@@ -2229,7 +2148,7 @@ struct EpiStoreNorm {
 // reference.
 __global__ void __launch_bounds__(NT, 1) cgne_fused_kernel(OpArgs A, CgneVecs v, IterArgs it,
                                                         Persist P, History H, SolveOut* out) {
-  SB2_SHARED_DECL;
+  SB2_SUMS_DECL;
   const int tid = threadIdx.x;
   const long long gt = (long long)blockIdx.x * NT + tid, gs = (long long)gridDim.x * NT;
   const int n = A.n;
@@ -2241,9 +2160,7 @@ __global__ void __launch_bounds__(NT, 1) cgne_fused_kernel(OpArgs A, CgneVecs v,
   {
     EpiStoreNorm epi{v.q, 0.0};
     spmv_phase(v.AT, v.b, epi, s_prod, s_red);
-    const double a = block_sum<NT>(epi.acc, s_red);
-    if (tid == 0) s_vals[0] = a;
-    if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+    if (!grid_sums<NT, 1>(P, epoch, {epi.acc}, s_vals, s_arr)) return;
   }
   const double dq = sqrt(s_vals[0]);
   if (dq == 0.0) {
@@ -2268,9 +2185,7 @@ __global__ void __launch_bounds__(NT, 1) cgne_fused_kernel(OpArgs A, CgneVecs v,
     spmv_phase(v.AT, v.p, e2, s_prod, s_red);
     rz = e2.rz;
   }
-  rz = block_sum<NT>(rz, s_red);
-  if (tid == 0) s_vals[0] = rz;
-  if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+  if (!grid_sums<NT, 1>(P, epoch, {rz}, s_vals, s_arr)) return;
   double rho = s_vals[0], rho_1 = 0.0;
   double dp = dq;  // Norm2(q)
 
@@ -2309,9 +2224,7 @@ __global__ void __launch_bounds__(NT, 1) cgne_fused_kernel(OpArgs A, CgneVecs v,
     {
       EpiStoreDot e{v.z, v.p, 0.0};
       spmv_phase(v.AT, v.q, e, s_prod, s_red);
-      const double d = block_sum<NT>(e.acc, s_red);
-      if (tid == 0) s_vals[0] = d;
-      if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+      if (!grid_sums<NT, 1>(P, epoch, {e.acc}, s_vals, s_arr)) return;
     }
     const double delta = s_vals[0];
     if (delta == 0.0) { fail = 2; break; }
@@ -2342,10 +2255,7 @@ __global__ void __launch_bounds__(NT, 1) cgne_fused_kernel(OpArgs A, CgneVecs v,
           a1 = add_rn(a1, mul_rn(ri.v[j], zn.v[j]));
         }
       });
-      a0 = block_sum<NT>(a0, s_red);
-      a1 = block_sum<NT>(a1, s_red);
-      if (tid == 0) { s_vals[0] = a0; s_vals[1] = a1; }
-      if (!grid_sync<NT>(P, epoch, 2, s_vals, s_red)) return;
+      if (!grid_sums<NT, 2>(P, epoch, {a0, a1}, s_vals, s_arr)) return;
       rho_1 = rho;
       rho = s_vals[1];
       dp = sqrt(s_vals[0]);
@@ -2371,7 +2281,7 @@ struct SymmlqVecs {
 // ceta_bar * w_bar after the loop, as in the reference.
 __global__ void __launch_bounds__(NT, 1) symmlq_fused_kernel(OpArgs A, SymmlqVecs v, IterArgs it,
                                                           Persist P, History H, SolveOut* out) {
-  SB2_SHARED_DECL;
+  SB2_SUMS_DECL;
   const int tid = threadIdx.x;
   const long long gt = (long long)blockIdx.x * NT + tid, gs = (long long)gridDim.x * NT;
   const int n = A.n;
@@ -2384,9 +2294,7 @@ __global__ void __launch_bounds__(NT, 1) symmlq_fused_kernel(OpArgs A, SymmlqVec
     const double bi = __ldg(v.b + i);
     acc = add_rn(acc, mul_rn(bi, bi));
   }
-  acc = block_sum<NT>(acc, s_red);
-  if (tid == 0) s_vals[0] = acc;
-  if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+  if (!grid_sums<NT, 1>(P, epoch, {acc}, s_vals, s_arr)) return;
   const double normb = sqrt(s_vals[0]);
   if (normb == 0.0) {
     if (lead) { out->init_failed = 1; out->hist_len = 0; }
@@ -2414,9 +2322,7 @@ __global__ void __launch_bounds__(NT, 1) symmlq_fused_kernel(OpArgs A, SymmlqVec
       v.z[i] = zi;
       a0 = add_rn(a0, mul_rn(ri, zi));
     }
-    a0 = block_sum<NT>(a0, s_red);
-    if (tid == 0) s_vals[0] = a0;
-    if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+    if (!grid_sums<NT, 1>(P, epoch, {a0}, s_vals, s_arr)) return;
   }
   double beta = sqrt(s_vals[0]);
   const double beta1 = beta;
@@ -2483,9 +2389,7 @@ __global__ void __launch_bounds__(NT, 1) symmlq_fused_kernel(OpArgs A, SymmlqVec
     {
       EpiStoreDot e{v.r, u, 0.0};
       spmv_phase(A, u, e, s_prod, s_red);
-      const double a = block_sum<NT>(e.acc, s_red);
-      if (tid == 0) s_vals[0] = a;
-      if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+      if (!grid_sums<NT, 1>(P, epoch, {e.acc}, s_vals, s_arr)) return;
     }
     const double alpha = s_vals[0];
     // z = M^{-1} r; Add(-alpha, v, r); Add(-alpha, u, z); Add(-beta, v_old, r);
@@ -2518,9 +2422,7 @@ __global__ void __launch_bounds__(NT, 1) symmlq_fused_kernel(OpArgs A, SymmlqVec
 #pragma unroll
         for (int j = 0; j < W; j++) a0 = add_rn(a0, mul_rn(ri.v[j], zi.v[j]));
       });
-      a0 = block_sum<NT>(a0, s_red);
-      if (tid == 0) s_vals[0] = a0;
-      if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+      if (!grid_sums<NT, 1>(P, epoch, {a0}, s_vals, s_arr)) return;
     }
     const double beta_old = beta;
     beta = sqrt(s_vals[0]);
@@ -2573,7 +2475,7 @@ struct QmrsVecs {
 // reference.
 __global__ void __launch_bounds__(NT, 1) qmrsym_fused_kernel(OpArgs A, QmrsVecs v, IterArgs it,
                                                           Persist P, History H, SolveOut* out) {
-  SB2_SHARED_DECL;
+  SB2_SUMS_DECL;
   const int tid = threadIdx.x;
   const long long gt = (long long)blockIdx.x * NT + tid, gs = (long long)gridDim.x * NT;
   const int n = A.n;
@@ -2586,9 +2488,7 @@ __global__ void __launch_bounds__(NT, 1) qmrsym_fused_kernel(OpArgs A, QmrsVecs 
     const double bi = __ldg(v.b + i);
     acc = add_rn(acc, mul_rn(bi, bi));
   }
-  acc = block_sum<NT>(acc, s_red);
-  if (tid == 0) s_vals[0] = acc;
-  if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+  if (!grid_sums<NT, 1>(P, epoch, {acc}, s_vals, s_arr)) return;
   const double normb = sqrt(s_vals[0]);
   if (normb == 0.0) {
     if (lead) { out->init_failed = 1; out->hist_len = 0; }
@@ -2619,10 +2519,7 @@ __global__ void __launch_bounds__(NT, 1) qmrsym_fused_kernel(OpArgs A, QmrsVecs 
       a0 = add_rn(a0, mul_rn(yi, yi));
       a1 = add_rn(a1, mul_rn(ri, ri));
     }
-    a0 = block_sum<NT>(a0, s_red);
-    a1 = block_sum<NT>(a1, s_red);
-    if (tid == 0) { s_vals[0] = a0; s_vals[1] = a1; }
-    if (!grid_sync<NT>(P, epoch, 2, s_vals, s_red)) return;
+    if (!grid_sums<NT, 2>(P, epoch, {a0, a1}, s_vals, s_arr)) return;
     rho = sqrt(s_vals[0]);
     rr = s_vals[1];
   }
@@ -2637,9 +2534,7 @@ __global__ void __launch_bounds__(NT, 1) qmrsym_fused_kernel(OpArgs A, QmrsVecs 
       v.y[i] = yi;
       a0 = add_rn(a0, mul_rn(vi, yi));
     }
-    a0 = block_sum<NT>(a0, s_red);
-    if (tid == 0) s_vals[0] = a0;
-    if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+    if (!grid_sums<NT, 1>(P, epoch, {a0}, s_vals, s_arr)) return;
     delta = s_vals[0];
   }
   double ep = 0.0, theta = 0.0, gamma = 1.0, eta = -1.0;
@@ -2674,9 +2569,7 @@ __global__ void __launch_bounds__(NT, 1) qmrsym_fused_kernel(OpArgs A, QmrsVecs 
     {
       EpiStoreDot e{v.pt, v.p, 0.0};
       spmv_phase(A, v.p, e, s_prod, s_red);
-      const double a = block_sum<NT>(e.acc, s_red);
-      if (tid == 0) s_vals[0] = a;
-      if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+      if (!grid_sums<NT, 1>(P, epoch, {e.acc}, s_vals, s_arr)) return;
     }
     ep = s_vals[0];
     if (ep == 0.0) { fail = 4; break; }
@@ -2697,9 +2590,7 @@ __global__ void __launch_bounds__(NT, 1) qmrsym_fused_kernel(OpArgs A, QmrsVecs 
 #pragma unroll
         for (int j = 0; j < W; j++) a0 = add_rn(a0, mul_rn(yi.v[j], yi.v[j]));
       });
-      a0 = block_sum<NT>(a0, s_red);
-      if (tid == 0) s_vals[0] = a0;
-      if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+      if (!grid_sums<NT, 1>(P, epoch, {a0}, s_vals, s_arr)) return;
     }
     const double rho_1 = rho;
     rho = sqrt(s_vals[0]);
@@ -2756,10 +2647,7 @@ __global__ void __launch_bounds__(NT, 1) qmrsym_fused_kernel(OpArgs A, QmrsVecs 
         stw<W>(v.v, i, vi);
         stw<W>(v.y, i, yi);
       });
-      a0 = block_sum<NT>(a0, s_red);
-      a1 = block_sum<NT>(a1, s_red);
-      if (tid == 0) { s_vals[0] = a0; s_vals[1] = a1; }
-      if (!grid_sync<NT>(P, epoch, 2, s_vals, s_red)) return;
+      if (!grid_sums<NT, 2>(P, epoch, {a0, a1}, s_vals, s_arr)) return;
       rr = s_vals[0];
       delta = s_vals[1];
     }
@@ -2798,7 +2686,7 @@ struct EpiAxpyNorm {
 // updates x and w.  u, u1 and v, v1 swap by pointer.
 __global__ void __launch_bounds__(NT, 1) lsqr_fused_kernel(OpArgs A, LsqrVecs v, IterArgs it,
                                                         Persist P, History H, SolveOut* out) {
-  SB2_SHARED_DECL;
+  SB2_SUMS_DECL;
   const int tid = threadIdx.x;
   const long long gt = (long long)blockIdx.x * NT + tid, gs = (long long)gridDim.x * NT;
   const int n = A.n;
@@ -2811,9 +2699,7 @@ __global__ void __launch_bounds__(NT, 1) lsqr_fused_kernel(OpArgs A, LsqrVecs v,
     const double bi = __ldg(v.b + i);
     acc = add_rn(acc, mul_rn(bi, bi));
   }
-  acc = block_sum<NT>(acc, s_red);
-  if (tid == 0) s_vals[0] = acc;
-  if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+  if (!grid_sums<NT, 1>(P, epoch, {acc}, s_vals, s_arr)) return;
   const double normb = sqrt(s_vals[0]);
   if (normb == 0.0) {
     if (lead) { out->init_failed = 1; out->hist_len = 0; }
@@ -2825,9 +2711,7 @@ __global__ void __launch_bounds__(NT, 1) lsqr_fused_kernel(OpArgs A, LsqrVecs v,
   if (!it.init_guess_null) {
     EpiResidual epi{v.b, v.u, nullptr, 0.0, 0.0};
     spmv_phase(A, v.x, epi, s_prod, s_red);
-    const double r2 = block_sum<NT>(epi.rr, s_red);
-    if (tid == 0) s_vals[0] = r2;
-    if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+    if (!grid_sums<NT, 1>(P, epoch, {epi.rr}, s_vals, s_arr)) return;
     rnorm = sqrt(s_vals[0]);
   }
   // u = b / ||b||; x = 0
@@ -2844,9 +2728,7 @@ __global__ void __launch_bounds__(NT, 1) lsqr_fused_kernel(OpArgs A, LsqrVecs v,
   {
     EpiStoreNorm e{v.v, 0.0};
     spmv_phase(v.AT, v.u, e, s_prod, s_red);
-    const double a = block_sum<NT>(e.acc, s_red);
-    if (tid == 0) s_vals[0] = a;
-    if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+    if (!grid_sums<NT, 1>(P, epoch, {e.acc}, s_vals, s_arr)) return;
     alpha = sqrt(s_vals[0]);
     const double ta = 1.0 / alpha;
     for (long long i = gt; i < n; i += gs) {
@@ -2869,9 +2751,7 @@ __global__ void __launch_bounds__(NT, 1) lsqr_fused_kernel(OpArgs A, LsqrVecs v,
     {
       EpiAxpyNorm e{u1, u, -alpha, 0.0};
       spmv_phase(A, vv, e, s_prod, s_red);
-      const double a = block_sum<NT>(e.acc, s_red);
-      if (tid == 0) s_vals[0] = a;
-      if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+      if (!grid_sums<NT, 1>(P, epoch, {e.acc}, s_vals, s_arr)) return;
     }
     const double beta = sqrt(s_vals[0]);
     if (beta == 0.0) { fail = 1; break; }
@@ -2891,9 +2771,7 @@ __global__ void __launch_bounds__(NT, 1) lsqr_fused_kernel(OpArgs A, LsqrVecs v,
     {
       EpiAxpyNorm e{v1, vv, -beta, 0.0};
       spmv_phase(v.AT, u1, e, s_prod, s_red);
-      const double a = block_sum<NT>(e.acc, s_red);
-      if (tid == 0) s_vals[0] = a;
-      if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+      if (!grid_sums<NT, 1>(P, epoch, {e.acc}, s_vals, s_arr)) return;
     }
     alpha = sqrt(s_vals[0]);
     if (alpha == 0.0) { fail = 2; break; }
@@ -2964,7 +2842,7 @@ struct EpiBcrA {
 // product a = A p before its first test.
 __global__ void __launch_bounds__(NT, 1) bicgcr_fused_kernel(OpArgs A, BcrVecs v, IterArgs it,
                                                           Persist P, History H, SolveOut* out) {
-  SB2_SHARED_DECL;
+  SB2_SUMS_DECL;
   const int tid = threadIdx.x;
   const long long gt = (long long)blockIdx.x * NT + tid, gs = (long long)gridDim.x * NT;
   const int n = A.n;
@@ -2977,9 +2855,7 @@ __global__ void __launch_bounds__(NT, 1) bicgcr_fused_kernel(OpArgs A, BcrVecs v
     const double bi = __ldg(v.b + i);
     acc = add_rn(acc, mul_rn(bi, bi));
   }
-  acc = block_sum<NT>(acc, s_red);
-  if (tid == 0) s_vals[0] = acc;
-  if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+  if (!grid_sums<NT, 1>(P, epoch, {acc}, s_vals, s_arr)) return;
   const double normb = sqrt(s_vals[0]);
   if (normb == 0.0) {
     if (lead) { out->init_failed = 1; out->hist_len = 0; }
@@ -3010,11 +2886,7 @@ __global__ void __launch_bounds__(NT, 1) bicgcr_fused_kernel(OpArgs A, BcrVecs v
   {
     EpiBcrA e{v.a, v.w, v.v, A.diag, 0.0, 0.0, 0.0};
     spmv_phase(A, v.p, e, s_prod, s_red);
-    vv = block_sum<NT>(e.vv, s_red);
-    wv = block_sum<NT>(e.wv, s_red);
-    wa = block_sum<NT>(e.wa, s_red);
-    if (tid == 0) { s_vals[0] = vv; s_vals[1] = wv; s_vals[2] = wa; }
-    if (!grid_sync<NT>(P, epoch, 3, s_vals, s_red)) return;
+    if (!grid_sums<NT, 3>(P, epoch, {e.vv, e.wv, e.wa}, s_vals, s_arr)) return;
     vv = s_vals[0]; wv = s_vals[1]; wa = s_vals[2];
   }
 
@@ -3049,9 +2921,7 @@ __global__ void __launch_bounds__(NT, 1) bicgcr_fused_kernel(OpArgs A, BcrVecs v
     {
       EpiStoreDot e{v.z, v.w, 0.0};
       spmv_phase(A, v.s, e, s_prod, s_red);
-      const double d = block_sum<NT>(e.acc, s_red);
-      if (tid == 0) s_vals[0] = d;
-      if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+      if (!grid_sums<NT, 1>(P, epoch, {e.acc}, s_vals, s_arr)) return;
     }
     const double tau = s_vals[0];
     if (tau == 0.0) { fail = 2; break; }
@@ -3080,11 +2950,7 @@ __global__ void __launch_bounds__(NT, 1) bicgcr_fused_kernel(OpArgs A, BcrVecs v
           a2 = add_rn(a2, mul_rn(wi.v[j], ai.v[j]));
         }
       });
-      a0 = block_sum<NT>(a0, s_red);
-      a1 = block_sum<NT>(a1, s_red);
-      a2 = block_sum<NT>(a2, s_red);
-      if (tid == 0) { s_vals[0] = a0; s_vals[1] = a1; s_vals[2] = a2; }
-      if (!grid_sync<NT>(P, epoch, 3, s_vals, s_red)) return;
+      if (!grid_sums<NT, 3>(P, epoch, {a0, a1, a2}, s_vals, s_arr)) return;
       vv = s_vals[0]; wv = s_vals[1]; wa = s_vals[2];
     }
     nb_iter++;
@@ -3132,7 +2998,7 @@ struct EpiPrecDot {
 
 __global__ void __launch_bounds__(NT, 1) gmres_fused_kernel(OpArgs A, GmresVecs v, IterArgs it,
                                                          Persist P, History H, SolveOut* out) {
-  SB2_SHARED_DECL;
+  SB2_SUMS_DECL;
   extern __shared__ double s_dyn[];
   const int m = it.restart;
   const int ld = m + 1;
@@ -3170,9 +3036,7 @@ __global__ void __launch_bounds__(NT, 1) gmres_fused_kernel(OpArgs A, GmresVecs 
       rr = add_rn(rr, mul_rn(ri, ri));
     }
   }
-  rr = block_sum<NT>(rr, s_red);
-  if (tid == 0) s_vals[0] = rr;
-  if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+  if (!grid_sums<NT, 1>(P, epoch, {rr}, s_vals, s_arr)) return;
   double beta = sqrt(s_vals[0]);
   // outer.Init(r)
   if (beta == 0.0) {
@@ -3203,9 +3067,7 @@ __global__ void __launch_bounds__(NT, 1) gmres_fused_kernel(OpArgs A, GmresVecs 
       // u = A V_i; w = M^{-1} u; h_{0,i} = (V_0, w)
       EpiPrecDot epi{v.w, v.V, A.diag, 0.0};
       spmv_phase(A, Vi, epi, s_prod, s_red);
-      double d = block_sum<NT>(epi.acc, s_red);
-      if (tid == 0) s_vals[0] = d;
-      if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+      if (!grid_sums<NT, 1>(P, epoch, {epi.acc}, s_vals, s_arr)) return;
       // modified Gram-Schmidt: H(k,i) = (V_k, w); Add(-H(k,i), V_k, w)
       for (int k = 0; k <= i; k++) {
         const double h = s_vals[0];
@@ -3228,9 +3090,7 @@ __global__ void __launch_bounds__(NT, 1) gmres_fused_kernel(OpArgs A, GmresVecs 
 #pragma unroll
           for (int j = 0; j < W; j++) acc = add_rn(acc, mul_rn(vne.v[j], we.v[j]));
         });
-        acc = block_sum<NT>(acc, s_red);
-        if (tid == 0) s_vals[0] = acc;
-        if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+        if (!grid_sums<NT, 1>(P, epoch, {acc}, s_vals, s_arr)) return;
       }
       // h_{i+1,i} = ||w||; V_{i+1} = w / h
       double hi_ip1 = sqrt(s_vals[0]);
@@ -3292,9 +3152,7 @@ __global__ void __launch_bounds__(NT, 1) gmres_fused_kernel(OpArgs A, GmresVecs 
       v.r[e] = re;
       rr = add_rn(rr, mul_rn(re, re));
     }
-    rr = block_sum<NT>(rr, s_red);
-    if (tid == 0) s_vals[0] = rr;
-    if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+    if (!grid_sums<NT, 1>(P, epoch, {rr}, s_vals, s_arr)) return;
     beta = sqrt(s_vals[0]);
   }
   if (lead) write_out(out, nb_iter, it.max_iter, 0, facteur, reste, hlen);

@@ -173,6 +173,15 @@ __device__ __forceinline__ bool grid_sync(const Persist& P, unsigned& epoch, int
   return grid_wait<NT>(P, epoch, K, s_vals, true);
 }
 
+// K sums over the grid and the barrier (s_red: K * NT / 32, the caller's own:
+// no block sum may be using it).
+template <int NT, int K>
+__device__ __forceinline__ bool grid_sums(const Persist& P, unsigned& epoch, const double (&a)[K],
+                                          double* s_vals, double* s_red) {
+  grid_arrive_sums<NT, K>(P, epoch, a, s_red);
+  return grid_wait<NT, (K <= 2)>(P, epoch, K, s_vals, true);
+}
+
 // Gathers of the product's operand inside a persistent kernel: cached in L1
 // (ld.ca), where a stencil's neighbouring columns hit.  The operand must have
 // been written in an EARLIER phase, never in the phase that gathers it: every
