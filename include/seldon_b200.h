@@ -271,7 +271,7 @@ int sb2_precond_destroy(sb2_precond* M);
  *                           the apply reads, and the solvers then accept it
  *                           for any matrix of order n
  * Solve / TransSolve (IlutPreconditioning.cxx:329-374) then run on the
- * device as level-scheduled sweeps with the reference's own operation order:
+ * device, a launch per sweep, with the reference's own operation order:
  * z is the reference's z bit for bit.  The arrays are copied.  A factor
  * whose rows break the layout above gives SB2_ERR_INVALID_CSR, a
  * permutation that is not one SB2_ERR_INVALID_VALUE.  The Krylov drivers
@@ -359,7 +359,7 @@ int sb2_precond_trans_solve(const sb2_precond* M, const double* r, double* z,
 
 /* In-place relaxation on x: SOR(A, X, B, omega, iter, type_ssor) with
  * type_ssor 2 (forward), 3 (backward) or 0 (both), reproducing the
- * sequential sweep order exactly by level scheduling.
+ * sequential sweep order exactly.
  * Relaxation_MatVect.cxx:41-95 (RowSparse), :176-298 (RowSymSparse). */
 int sb2_sor(const sb2_csr* A, double* x, const double* b, double omega,
             int iter, int type_ssor, void* stream);

@@ -8,8 +8,11 @@
 // vector updates with the next residual norm; grid-wide reductions are
 // deterministic (fixed CTA order).
 //
-// SOR and ILUT preconditioning (level-scheduled sweeps, many dependent
-// launches) of Cg, BiCgStab and Gmres run as device-resident chains around the
+// Cg, BiCgStab and Gmres on systems whose vectors fit the chip's shared memory
+// run there (resident.cuh), the smallest in one cluster.
+//
+// SOR and ILUT preconditioning (sweeps with a launch of their own, sweep.cuh)
+// of Cg, BiCgStab and Gmres run as device-resident chains around the
 // sweeps (chain.cu); the other drivers with them, and every driver when those
 // chains are switched off, go through a host-driven driver over the same
 // device kernels, one operation at a time, in the reference's order.

@@ -1,4 +1,4 @@
-// Preconditioners: identity, Jacobi, level-scheduled SOR and the ILUT apply.
+// Preconditioners: identity, Jacobi, SOR and the ILUT apply.
 //
 // SOR reproduces the reference's strictly sequential sweeps
 // (Relaxation_MatVect.cxx:41-95 RowSparse, :176-298 RowSymSparse) bit for
