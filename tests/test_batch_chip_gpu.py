@@ -76,3 +76,19 @@ def test_chip_irregular_rows(cuda, oracle):
         for k, (s, b) in enumerate(zip(systems, rhs)):
             xk = x[B.sys_row[k]:B.sys_row[k + 1]]
             assert np.linalg.norm(b - matgen.matvec(*s, xk)) <= 2e-11 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("tuned_mixed", [True, False])
+def test_tuned_mode_leaves_the_other_its_plan(cuda, tuned_mixed):
+    """A batch tuned in one mode runs the other with its plan, bit for bit."""
+    from seldon_b200 import api
+    sides = [9, 30, 31, 64, 90]
+    systems = [matgen.lap2d(g, shift=0.01) for g in sides]
+    b = to_dev(np.random.default_rng(8).uniform(-1, 1, sum(g * g for g in sides)))
+    x = [to_dev(np.zeros(b.numel())) for _ in range(2)]
+    A, B = api.Batch(systems), api.Batch(systems)
+    A.autotune(x[0], b, tol=1e-9, mixed=tuned_mixed)
+    B.set_plan(*A.plan(), *A.cluster_plan())
+    for v, M in zip(x, (A, B)):
+        assert M.solve(v, b, tol=1e-9, mixed=not tuned_mixed).converged == len(sides)
+    assert np.array_equal(to_host(x[0]), to_host(x[1]))
