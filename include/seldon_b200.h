@@ -713,10 +713,12 @@ int sb2_batch_solve(const sb2_batch* B, double* x, const double* b,
  * The queue hands systems out largest first, so a CTA that takes a system of
  * at most warp_max rows turns to warps for the rest of the launch.
  * Autotuner: times the solve of this batch (x is overwritten) under each
- * candidate plan (threads 128, 256, 512 by warp_max 0, 256, 1024, clusters,
- * and the vectors in shared memory) and keeps the fastest for later solves.  The choice is cached per (histogram of the
- * systems' sizes in power-of-two classes, mode): a later batch with the same
- * histogram takes it without timing. */
+ * candidate plan (threads 128, 256, 512 by warp_max 0, 256, 1024, clusters)
+ * and with the vectors in shared memory, and keeps the best plan and, for
+ * this mode, whether shared memory was faster still; the other mode runs the
+ * plan unless it was tuned itself.  The choice is cached per (histogram of
+ * the systems' sizes in power-of-two classes, mode): a later batch with the
+ * same histogram takes it without timing. */
 int sb2_batch_autotune(sb2_batch* B, double* x, const double* b,
                        const sb2_batch_params* params, void* stream);
 int sb2_batch_set_threads(sb2_batch* B, int threads);
