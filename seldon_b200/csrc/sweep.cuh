@@ -690,6 +690,9 @@ __global__ void __launch_bounds__(Op::kThreads, 1) sweep_kernel(SweepArgs a, Op 
         }
       }
       ok = __all_sync(0xffffffffu, ok) != 0;
+      // every lane's value is ordered before lane 0's arrival, which publishes
+      // them all (a vote orders no memory)
+      __syncwarp();
       if (lane == 0 && ok) {
         mbar_arrive(&s_bar[step & (kSweepRing - 1)], arrivals);
         *((volatile unsigned*)a.state + 2 + c0) = (unsigned)step + 1u;
