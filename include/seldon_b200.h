@@ -19,8 +19,11 @@
  *     inside it SB2_ERR_HOST.  Solver convergence/breakdown is
  *     NOT a status: it is reported in sb2_iter_result.error_code exactly as
  *     Seldon's Iteration::ErrorCode() (Iterative.cxx:344-354).
- *   - Device-side waits (grid barriers of the fused solvers) are bounded; a
- *     wait that runs out ends the kernel and the call returns SB2_ERR_TIMEOUT.
+ *   - Device-side waits (grid barriers of the fused solvers, values awaited by
+ *     the sweeps of SOR and ILUT) are bounded; a wait that runs out ends the
+ *     kernel and the call returns SB2_ERR_TIMEOUT.  Calls that return before
+ *     their kernels run have a status call instead (sb2_precond_status,
+ *     sb2_spmv_status).
  *   - Threads: calls from several host threads, each on its own stream, may
  *     share a matrix handle.  Its lazily built members (transpose, diagonal,
  *     FP32 copy, cluster plan) are built under the handle's lock and
@@ -356,6 +359,14 @@ int sb2_precond_solve(const sb2_precond* M, const double* r, double* z,
                       void* stream);
 int sb2_precond_trans_solve(const sb2_precond* M, const double* r, double* z,
                             void* stream);
+
+/* Device-side condition of the applies queued by the two calls above (which
+ * return before their sweeps run, and can be captured): *status receives 0
+ * (none) or 1 (since the last call a bounded wait of a SOR or ILUT sweep ran
+ * out; the entries of z that were not reached are NaN), and the word is
+ * cleared.  Waits for the stream.  The solvers and sb2_sor look for
+ * themselves and return SB2_ERR_TIMEOUT.  No counterpart in the reference. */
+int sb2_precond_status(const sb2_precond* M, void* stream, int* status);
 
 /* In-place relaxation on x: SOR(A, X, B, omega, iter, type_ssor) with
  * type_ssor 2 (forward), 3 (backward) or 0 (both), reproducing the
@@ -785,8 +796,8 @@ int sb2_set_wait_limit_ms(int ms);
  * CTA may wait for the slowest at a grid barrier makes the fused solvers end
  * with SB2_ERR_TIMEOUT: every CTA leaves the kernel, the context stays
  * usable, and the next call with a longer limit solves normally.  The TMA
- * product's ring waits keep a floor of 1 s whatever this limit is.  No
- * counterpart in the reference. */
+ * product's ring waits and the sweeps' waits keep a floor of 1 s whatever this
+ * limit is.  No counterpart in the reference. */
 int sb2_set_wait_limit_us(int us);
 
 #ifdef __cplusplus

@@ -195,6 +195,7 @@ _PROTOS = [
     ("sb2_precond_destroy", ctypes.c_int, [c_void_p]),
     ("sb2_precond_solve", ctypes.c_int, [c_void_p, c_void_p, c_void_p, c_void_p]),
     ("sb2_precond_trans_solve", ctypes.c_int, [c_void_p, c_void_p, c_void_p, c_void_p]),
+    ("sb2_precond_status", ctypes.c_int, [c_void_p, c_void_p, c_int_p]),
     ("sb2_sor", ctypes.c_int,
      [c_void_p, c_void_p, c_void_p, ctypes.c_double, ctypes.c_int, ctypes.c_int, c_void_p]),
 ]

@@ -39,6 +39,7 @@ namespace sb2 {
 
 int precond_apply(const sb2_precond* M, bool trans, const double* r, double* z,
                   cudaStream_t s);
+int precond_begin(const sb2_precond* M, cudaStream_t s);
 int precond_check(const sb2_precond* M, cudaStream_t s);
 
 // One CTA per SM: the grid barrier costs more with the number of CTAs.
@@ -4419,6 +4420,7 @@ static int host_solve(int which, const sb2_csr* A, const sb2_precond* M, double*
   it.max_iter = prm->max_iter;
   int init_failed = 0;
   double* V = (double*)buf.p;
+  SB2_TRY(precond_begin(M, s));
   if (which == kCg) SB2_TRY(host_cg(o, x, b, prm, it, V, &init_failed));
   else if (which == kBicg) SB2_TRY(host_bicgstab(o, x, b, prm, it, V, &init_failed));
   else if (which == kCgs) SB2_TRY(host_cgs(o, x, b, prm, it, V, &init_failed));
@@ -4825,6 +4827,7 @@ static int pcg_solve(const sb2_csr* A, const sb2_precond* M, double* x, const do
   double* dh = (double*)(c + vb + sb + pb);
   int* dhi = (int*)(c + vb + sb + pb + hb);
   ChainState<double> o;
+  SB2_TRY(precond_begin(M, s));
   if (which == kGmres) {
     double* hb = work + (size_t)ldv * (m + 4);
     GmresChainExtra* ex = reinterpret_cast<GmresChainExtra*>(

@@ -252,7 +252,7 @@ static int plan_sor(sb2_precond* M) {
 // SOR(A, X, B, omega, iter, type_ssor) on the device: the sweeps from x0
 // (null: zero) into x, two a launch.  x0 is null or x itself.
 static int sor_apply(sb2_precond* M, const double* x0, double* x, const double* b, double omega,
-                     int iter, int type_ssor, cudaStream_t s) {
+                     int iter, int type_ssor, int late, cudaStream_t s) {
   SB2_TRY(plan_sor(M));
   const sb2_csr* A = M->A;
   const int n = A->m;
@@ -278,11 +278,11 @@ static int sor_apply(sb2_precond* M, const double* x0, double* x, const double* 
       const CsrArrays &u = A->upper, &f = A->full;
       SB2_TRY(launch_sweeps(G, sweeps, plan, fwd, last,
                             SymmetricSor{u.d_ind, u.d_val, f.d_ind, f.d_val, M->d_sdiag, b, cur, omega,
-                                         (1.0 - omega) / omega}, s));
+                                         (1.0 - omega) / omega}, late, s));
     } else {
       const CsrArrays& f = A->full;
       SB2_TRY(launch_sweeps(G, sweeps, plan, fwd, last,
-                            GeneralSor{f.d_ind, f.d_val, A->d_diag, b, cur, omega, 1.0 - omega}, s));
+                            GeneralSor{f.d_ind, f.d_val, A->d_diag, b, cur, omega, 1.0 - omega}, late, s));
     }
     cur = last;
   }
@@ -510,7 +510,8 @@ static int ilu0_factor(const sb2_csr* A, int modified, std::vector<int>& ptr,
 // both sweeps and both permutations in one launch.  Seldon's t[prow[i]] = r[i]
 // and z[i] = t[prow[i]] are t[j] = r[iprow[j]] and z[iprow[j]] = t[j] for the
 // thread that owns row j.
-static int ilut_apply(sb2_precond* M, bool trans, const double* r, double* z, cudaStream_t s) {
+static int ilut_apply(sb2_precond* M, bool trans, const double* r, double* z, int late,
+                      cudaStream_t s) {
   const bool sym = M->ilu_sym != 0;
   const GatherSweep& first = !sym && trans ? M->s_utf : M->s_lf;
   const GatherSweep& second = !sym && trans ? M->s_ltb : M->s_ub;
@@ -523,17 +524,17 @@ static int ilut_apply(sb2_precond* M, bool trans, const double* r, double* z, cu
                  z, !sym && !trans ? M->d_pcol : M->d_iprow};
   const SweepPlan* const plan[2] = {&first.plan, &second.plan};
   const bool fwd[2] = {true, false};
-  return launch_sweeps(M->grid, 2, plan, fwd, nullptr, op, s);
+  return launch_sweeps(M->grid, 2, plan, fwd, nullptr, op, late, s);
 }
 
 int precond_kind(const sb2_precond* M) { return M->kind; }
 int precond_n(const sb2_precond* M) { return M->kind == SB2_PRECOND_ILUT ? M->n_ilu : M->A->m; }
 const sb2_csr* precond_matrix(const sb2_precond* M) { return M->A; }
 
-int precond_apply(const sb2_precond* cM, bool trans, const double* r, double* z,
-                  cudaStream_t s) {
+static int apply(const sb2_precond* cM, bool trans, const double* r, double* z, int late,
+                 cudaStream_t s) {
   sb2_precond* M = const_cast<sb2_precond*>(cM);
-  if (M->kind == SB2_PRECOND_ILUT) return M->n_ilu ? ilut_apply(M, trans, r, z, s) : SB2_OK;
+  if (M->kind == SB2_PRECOND_ILUT) return M->n_ilu ? ilut_apply(M, trans, r, z, late, s) : SB2_OK;
   const int n = M->A->m;
   if (n == 0) return SB2_OK;
   if (M->kind == SB2_PRECOND_IDENTITY) {
@@ -549,19 +550,39 @@ int precond_apply(const sb2_precond* cM, bool trans, const double* r, double* z,
   }
   // SorPreconditioner::Solve / TransSolve (Precond_Ssor.cxx:62-90)
   const int type = M->symmetric ? 0 : (trans ? 3 : 2);
-  return sor_apply(M, nullptr, z, r, M->omega, M->nb_iter, type, s);
+  return sor_apply(M, nullptr, z, r, M->omega, M->nb_iter, type, late, s);
 }
 
-// Whether a wait of the preconditioner's sweeps ran out since the last call
-// (synchronizes the stream).
-int precond_check(const sb2_precond* M, cudaStream_t s) {
-  if (!M || !M->grid.d_state) return SB2_OK;
-  unsigned late = 0;
-  SB2_CUDA_TRY(cudaMemcpyAsync(&late, M->grid.d_state + 1, sizeof(late), cudaMemcpyDeviceToHost, s));
+// An apply inside a solver.
+int precond_apply(const sb2_precond* M, bool trans, const double* r, double* z, cudaStream_t s) {
+  return apply(M, trans, r, z, kStLateSolve, s);
+}
+
+// Whether a wait of the preconditioner's sweeps ran out since the word was
+// last read, which clears it (synchronizes the stream).
+static int read_late(const sb2_precond* M, int word, unsigned* late, cudaStream_t s) {
+  *late = 0;
+  if (!M->grid.d_state) return SB2_OK;
+  unsigned* d = M->grid.d_state + word;
+  SB2_CUDA_TRY(cudaMemcpyAsync(late, d, sizeof(*late), cudaMemcpyDeviceToHost, s));
   SB2_CUDA_TRY(cudaStreamSynchronize(s));
-  if (!late) return SB2_OK;
-  SB2_CUDA_TRY(cudaMemsetAsync(M->grid.d_state + 1, 0, sizeof(late), s));
-  return SB2_ERR_TIMEOUT;
+  if (*late) SB2_CUDA_TRY(cudaMemsetAsync(d, 0, sizeof(*late), s));
+  return SB2_OK;
+}
+
+// A solver with M starts: what an earlier one that ended with an error left in
+// its word is not this one's.
+int precond_begin(const sb2_precond* M, cudaStream_t s) {
+  if (!M || !M->grid.d_state) return SB2_OK;
+  SB2_CUDA_TRY(cudaMemsetAsync(M->grid.d_state + kStLateSolve, 0, sizeof(unsigned), s));
+  return SB2_OK;
+}
+
+// A solver with M ends: whether a wait ran out in it.
+int precond_check(const sb2_precond* M, cudaStream_t s) {
+  unsigned late = 0;
+  if (M) SB2_TRY(read_late(M, kStLateSolve, &late, s));
+  return late ? SB2_ERR_TIMEOUT : SB2_OK;
 }
 
 }  // namespace sb2
@@ -649,14 +670,23 @@ int sb2_precond_solve(const sb2_precond* M, const double* r, double* z, void* st
   SB2_TRACE("sb2_precond_solve");
   if (!M || (precond_n(M) > 0 && (!r || !z)) || (r == z && precond_n(M) > 0))
     return SB2_ERR_INVALID_VALUE;
-  return precond_apply(M, false, r, z, (cudaStream_t)stream);
+  return apply(M, false, r, z, kStLateApply, (cudaStream_t)stream);
 } SB2_CATCH
 
 int sb2_precond_trans_solve(const sb2_precond* M, const double* r, double* z, void* stream) try {
   SB2_TRACE("sb2_precond_trans_solve");
   if (!M || (precond_n(M) > 0 && (!r || !z)) || (r == z && precond_n(M) > 0))
     return SB2_ERR_INVALID_VALUE;
-  return precond_apply(M, true, r, z, (cudaStream_t)stream);
+  return apply(M, true, r, z, kStLateApply, (cudaStream_t)stream);
+} SB2_CATCH
+
+int sb2_precond_status(const sb2_precond* M, void* stream, int* status) try {
+  if (!M || !status) return SB2_ERR_INVALID_VALUE;
+  unsigned late = 0;
+  SB2_TRY(read_late(M, kStLateApply, &late, (cudaStream_t)stream));
+  if (!M->grid.d_state) SB2_CUDA_TRY(cudaStreamSynchronize((cudaStream_t)stream));
+  *status = late ? 1 : 0;
+  return SB2_OK;
 } SB2_CATCH
 
 int sb2_sor(const sb2_csr* A, double* x, const double* b, double omega, int iter,
@@ -666,7 +696,7 @@ int sb2_sor(const sb2_csr* A, double* x, const double* b, double omega, int iter
   sb2_precond tmp;
   tmp.A = A;
   tmp.kind = SB2_PRECOND_SOR;
-  int st = sor_apply(&tmp, x, x, b, omega, iter, type_ssor, (cudaStream_t)stream);
+  int st = sor_apply(&tmp, x, x, b, omega, iter, type_ssor, kStLateSolve, (cudaStream_t)stream);
   // the plan is released after the stream has consumed it
   const int late = precond_check(&tmp, (cudaStream_t)stream);
   cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);

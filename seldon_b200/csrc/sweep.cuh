@@ -31,9 +31,9 @@
 //
 // Progress: all CTAs are resident (cooperative launch), a warp's items are in
 // level order and a row reads rows of smaller levels only.  Every wait is
-// bounded: when no CTA has made progress for the wait limit, the waiting warp
-// sets the status word and the grid leaves; rows not reached keep the fill
-// (a NaN).
+// bounded: when no CTA has made progress for the wait limit (a long row that is
+// being summed is progress), the waiting warp sets the status words and the
+// grid leaves; the rows it did not finish come out as NaN.
 #pragma once
 
 #include <algorithm>
@@ -47,6 +47,11 @@ constexpr int kSweepMaxCtas = 148;
 constexpr int kSweepStep = 32;   // items of one step at most
 constexpr int kSweepRing = 64;   // step barriers (more than the warps of a CTA)
 constexpr int kSweepSmem = 224 * 1024;  // most shared memory a CTA takes for its values
+constexpr int kSweepNote = 4096;  // entries of a long row between two notes of progress
+// Words of SweepGrid::d_state: the grid leaves; a wait ran out since the word
+// was last read, in a solver's apply and in a caller's own; then one word a
+// CTA that changes as it gets on.
+constexpr int kStLeave = 0, kStLateSolve = 1, kStLateApply = 2, kStProgress = 3;
 // The fill: a signalling NaN, which no arithmetic produces.  A value that
 // was copied from the caller with these very bits is stored as the quiet NaN.
 constexpr unsigned long long kSweepFill = 0x7ff4b2005e1d0001ull;
@@ -79,7 +84,7 @@ struct SweepGrid {
   std::vector<int> h_blk;     // [ctas + 1] first row of each block
   int* d_blk = nullptr;
   double* d_new[2] = {nullptr, nullptr};
-  unsigned* d_state = nullptr;  // [0] leave, [1] some wait ran out, [2 + c] progress of CTA c
+  unsigned* d_state = nullptr;  // [kStProgress + kSweepMaxCtas]
   void release() {
     cudaFree(d_blk);
     cudaFree(d_new[0]);
@@ -110,6 +115,7 @@ struct SweepArgs {
   double* result;   // the last sweep's values by row (may be null)
   SweepPhase ph[2];
   unsigned* state;
+  int late;         // the word of state that tells of a wait that ran out
   unsigned long long wait_ns;
 };
 
@@ -131,8 +137,8 @@ inline int make_sweep_grid(int n, SweepGrid* G) {
   SB2_CUDA_TRY(cudaMalloc(&G->d_blk, sizeof(int) * (G->ctas + 1)));
   SB2_CUDA_TRY(cudaMemcpy(G->d_blk, G->h_blk.data(), sizeof(int) * (G->ctas + 1), cudaMemcpyHostToDevice));
   for (int k = 0; k < 2; k++) SB2_CUDA_TRY(cudaMalloc(&G->d_new[k], sizeof(double) * std::max(n, 1)));
-  SB2_CUDA_TRY(cudaMalloc(&G->d_state, sizeof(unsigned) * (2 + kSweepMaxCtas)));
-  SB2_CUDA_TRY(cudaMemset(G->d_state, 0, sizeof(unsigned) * (2 + kSweepMaxCtas)));
+  SB2_CUDA_TRY(cudaMalloc(&G->d_state, sizeof(unsigned) * (kStProgress + kSweepMaxCtas)));
+  SB2_CUDA_TRY(cudaMemset(G->d_state, 0, sizeof(unsigned) * (kStProgress + kSweepMaxCtas)));
   return SB2_OK;
 }
 
@@ -259,28 +265,28 @@ __device__ __forceinline__ bool mbar_test_wait(unsigned long long* b, unsigned p
 // no CTA has finished an item for wait_ns.
 struct SweepWait {
   unsigned* state;
-  int ctas;
+  int late, ctas;
   unsigned long long wait_ns;
   __device__ __forceinline__ unsigned progress() const {
     unsigned s = 0;
-    for (int c = 0; c < ctas; c++) s = s * 31u + *((volatile unsigned*)state + 2 + c);
+    for (int c = 0; c < ctas; c++) s = s * 31u + *((volatile unsigned*)state + kStProgress + c);
     return s;
   }
   // called now and then by a waiting warp; false: leave.  (The progress words
   // are read only when the limit has passed: reading them takes microseconds.)
   __device__ __noinline__ bool go_on(unsigned long long& t0, unsigned& seen) const {
-    if (*((volatile unsigned*)state) != 0u) return false;
+    if (*((volatile unsigned*)state + kStLeave) != 0u) return false;
     const unsigned long long t = global_timer_ns();
     if (t0 == 0ull) t0 = t;
     if (t - t0 <= wait_ns) return true;
-    const unsigned p = progress() | 1u;
+    const unsigned p = progress() * 2u + 1u;  // never 0
     if (p != seen) {
       seen = p;
       t0 = t;
       return true;
     }
-    atomicExch(state, 1u);
-    atomicExch(state + 1, 1u);
+    atomicExch(state + kStLeave, 1u);
+    atomicExch(state + late, 1u);
     return false;
   }
 };
@@ -303,6 +309,7 @@ struct SweepSource {
 //   op.take(r, s, k, c, a, x)             entry k with the value x of column c
 //   op.lead(r, s, k)                      entries 0..k-1 are taken, none new
 //   op.last(r, s)                         the new value
+//   op.store(r, v)                        where it goes beside
 // The entries after the lead that are held in registers only add products to
 // one number, so that nothing but loads, products and sums follows the row's
 // turn:
@@ -497,6 +504,30 @@ struct FactorSolve {
 template <class Op>
 __device__ __forceinline__ const double* sweep_start(const Op& op) { return op.x0; }
 __device__ __forceinline__ const double* sweep_start(const FactorSolve&) { return nullptr; }
+// and where the last sweep's values go
+template <class Op>
+__device__ __forceinline__ double* sweep_out(const Op&, double* result, const int** at) {
+  *at = nullptr;
+  return result;
+}
+__device__ __forceinline__ double* sweep_out(const FactorSolve& op, double*, const int** at) {
+  *at = op.out_at;
+  return op.z;
+}
+
+// The rows of the last sweep that this warp did not finish, from item q of its
+// own on, come out as NaN: out[at[row]], or out[row] with no `at`.
+static __device__ __noinline__ void sweep_mark(const int4* items, const int* rows, int q, int q1,
+                                               int step, double* out, const int* at) {
+  const int lane = threadIdx.x & 31;
+  for (; q < q1; q += step) {
+    const int4 item = __ldg(items + q);
+    if (lane < item.y) {
+      const int j = __ldg(rows + item.x + lane);
+      out[at ? __ldg(at + j) : j] = __longlong_as_double(0x7ff8000000000000ll);
+    }
+  }
+}
 
 // ------------------------------------------------------------------ the kernel
 
@@ -509,14 +540,24 @@ __global__ void __launch_bounds__(Op::kThreads, 1) sweep_kernel(SweepArgs a, Op 
   const int c0 = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int r0 = __ldg(a.blk + c0), rows = __ldg(a.blk + c0 + 1) - r0;
   if (threadIdx.x < kSweepRing) mbar_init(&s_bar[threadIdx.x], kSweepStep);
-  const SweepWait w{a.state, (int)gridDim.x, a.wait_ns};
+  const SweepWait w{a.state, a.late, (int)gridDim.x, a.wait_ns};
   const double* x0 = sweep_start(op);
   SweepSource old{nullptr, 0u};
   int base = 0;  // this CTA's steps of the sweeps before
   bool ok = true;
+  // this warp leaves: its items of the last sweep from the given one on
+  auto mark = [&](int from) {
+    const SweepPhase& P = a.nph > 1 ? a.ph[1] : a.ph[0];
+    const int* at;
+    double* out = sweep_out(op, a.result, &at);
+    sweep_mark(P.item, P.rows, from, __ldg(P.cta_item + c0 + 1), W, out, at);
+  };
   for (int ph = 0; ph < a.nph; ph++) {
     // every value of the CTA's rows from the sweep before is in place
-    if (__syncthreads_or(!ok)) return;
+    if (__syncthreads_or(!ok)) {
+      mark(__ldg((a.nph > 1 ? a.ph[1] : a.ph[0]).cta_item + c0) + warp);
+      return;
+    }
     const SweepPhase P = ph ? a.ph[1] : a.ph[0];
     const SweepSource fresh{P.out, OWN ? smem_u32(s_own + (size_t)ph * a.max_rows) : 0u};
     const bool fwd = P.forward != 0;
@@ -540,7 +581,8 @@ __global__ void __launch_bounds__(Op::kThreads, 1) sweep_kernel(SweepArgs a, Op 
       return Op::kPositions ? c : nw ? __ldg(P.pos + c) : ph == 1 ? __ldg(P.pos_prev + c) : c;
     };
     fetch(it0 + warp);
-    for (int it = it0 + warp; it < it1 && ok; it += W) {
+    int it = it0 + warp;
+    for (; it < it1 && ok; it += W) {
       const bool live = j >= 0;
       const int row = j, slot = item.x + lane;
       // this item's step, and what it adds to the step's barrier; the step
@@ -660,6 +702,7 @@ __global__ void __launch_bounds__(Op::kThreads, 1) sweep_kernel(SweepArgs a, Op 
         if (adds) op.run_to(R, s, sum);
         // rows longer than the entries held in registers
         for (int k = U; k < len && ok; k++) {
+          if (k % kSweepNote == 0) *((volatile unsigned*)a.state + kStProgress + c0) = ~(unsigned)k;
           int cc;
           double ff, y = 0.0;
           op.entry(R, k, cc, ff);
@@ -695,9 +738,10 @@ __global__ void __launch_bounds__(Op::kThreads, 1) sweep_kernel(SweepArgs a, Op 
       __syncwarp();
       if (lane == 0 && ok) {
         mbar_arrive(&s_bar[step & (kSweepRing - 1)], arrivals);
-        *((volatile unsigned*)a.state + 2 + c0) = (unsigned)step + 1u;
+        *((volatile unsigned*)a.state + kStProgress + c0) = (unsigned)step + 1u;
       }
     }
+    if (!ok && ph == a.nph - 1) mark(it - W);
     base += __ldg(P.steps + c0);
     old = fresh;
   }
@@ -717,8 +761,9 @@ __global__ void sym_diag_kernel(int n, const int* __restrict__ ptr, const int* _
 }
 
 __global__ void __launch_bounds__(256) sweep_fill_kernel(int n, double* x, double* y,
-                                                         unsigned* state) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) *state = 0u;
+                                                         unsigned* state, int late) {
+  // a solver's applies after one whose wait ran out leave at once: the solve is lost
+  if (blockIdx.x == 0 && threadIdx.x == 0) state[kStLeave] = late == kStLateSolve ? state[late] : 0u;
   const double f = __longlong_as_double((long long)kSweepFill);
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
@@ -728,10 +773,10 @@ __global__ void __launch_bounds__(256) sweep_fill_kernel(int n, double* x, doubl
 }
 
 // One launch of `sweeps` (1 or 2) sweeps; the last one's values go to `result`
-// (may be null) by row.
+// by row (null: the operation stores them).  late: kStLateSolve or kStLateApply.
 template <class Op>
 int launch_sweeps(const SweepGrid& G, int sweeps, const SweepPlan* const (&plan)[2],
-                  const bool (&forward)[2], double* result, const Op& op, cudaStream_t s) {
+                  const bool (&forward)[2], double* result, const Op& op, int late, cudaStream_t s) {
   const int n = G.n;
   if (n == 0) return SB2_OK;
   SweepArgs a;
@@ -746,12 +791,14 @@ int launch_sweeps(const SweepGrid& G, int sweeps, const SweepPlan* const (&plan)
                          plan[0]->d_pos, forward[q] ? 1 : 0, G.d_new[k]};
   }
   a.state = G.d_state;
+  a.late = late;
   a.wait_ns = ring_wait_ns();
   // values of the CTA's own rows stay in shared memory when both sweeps' fit
   const size_t smem = sizeof(double) * (size_t)a.nph * G.max_rows;
   const bool own = smem <= (size_t)kSweepSmem;
   const int g = std::min((n + 255) / 256, num_sms(current_device()) * 8);
-  sweep_fill_kernel<<<g, 256, 0, s>>>(n, G.d_new[0], sweeps > 1 ? G.d_new[1] : nullptr, G.d_state);
+  sweep_fill_kernel<<<g, 256, 0, s>>>(n, G.d_new[0], sweeps > 1 ? G.d_new[1] : nullptr, G.d_state,
+                                   late);
   SB2_CUDA_TRY(cudaGetLastError());
   const void* kern = own ? (const void*)sweep_kernel<Op, true> : (const void*)sweep_kernel<Op, false>;
   if (own && smem > 48 * 1024)
