@@ -907,8 +907,7 @@ constexpr int kChipRoom = 224 * 1024;
 template <int NT, typename IT>
 static int launch_chip(const BatchArgs& a, int room, cudaStream_t s) {
   auto* k = batch_chip_kernel<NT, IT>;
-  if (room > 48 * 1024)
-    SB2_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
+  if (room > 48 * 1024) SB2_CUDA_TRY(allow_shared((const void*)k, kChipRoom));
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, NT, room) != cudaSuccess || per_sm < 1)
     return SB2_ERR_NOT_SUPPORTED;

@@ -683,9 +683,9 @@ static int cgs2_solve(const sb2_csr* A, const SellOp<VT>& Ain, const double* dia
                       Cgs2Out* o, double* hist, int* hist_it, int hist_cap, cudaStream_t s) {
   const int n = A->m;
   // the Hessenberg matrix rotated and as built, s and the rotations
-  const size_t smem = sizeof(double) * (2 * (size_t)(m + 1) * (m + 1) + 3 * (size_t)(m + 1));
-  SB2_CUDA_TRY(cudaFuncSetAttribute(gmres_cgs2_kernel<VT>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  auto bytes = [](size_t k) { return sizeof(double) * (2 * (k + 1) * (k + 1) + 3 * (k + 1)); };
+  const size_t smem = bytes(m);
+  SB2_CUDA_TRY(allow_shared((const void*)gmres_cgs2_kernel<VT>, bytes(kCgs2MaxK)));
   const int grid = cgs2_grid<VT>(smem, Ain, n);
   if (grid < 1) return SB2_ERR_CUDA;
   const long long ldv = (long long)vector_stride(n, sizeof(VT));

@@ -3273,6 +3273,9 @@ enum Solver {
   kSymm = 14                                     // Symmlq
 };
 
+// Most shared memory of the fused Gmres's Hessenberg matrix and rotations.
+constexpr size_t kGmresSmem = 160 * 1024;
+
 static int fused_solve(int which, const sb2_csr* A, const double* diag, double* x,
                        const double* b, const sb2_iter_params* prm, sb2_iter_result* res,
                        double* hist, int* hist_it, int hist_cap, cudaStream_t s) {
@@ -3303,9 +3306,8 @@ static int fused_solve(int which, const sb2_csr* A, const double* diag, double* 
     kern = (const void*)gmres_fused_kernel;
     nvec = 2 + (m + 1);
     smem = sizeof(double) * ((size_t)(m + 1) * (m + 1) + 3 * (m + 1));
-    if (smem > 160 * 1024) return SB2_ERR_NOT_SUPPORTED;
-    SB2_CUDA_TRY(cudaFuncSetAttribute(gmres_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+    if (smem > kGmresSmem) return SB2_ERR_NOT_SUPPORTED;
+    SB2_CUDA_TRY(allow_shared(kern, kGmresSmem));
   }
   const int grid = coop_grid(kern, smem, A);
   if (grid < 1) return SB2_ERR_CUDA;
@@ -3452,7 +3454,7 @@ static int resident_solve(int which, const sb2_csr* A, const double* diag, doubl
                      : which == kBicg ? (const void*)bicgstab_resident_kernel<512, true>
                                       : gmres_resident(ms, per * 32, &threads);
   if (!kern) return SB2_ERR_NOT_SUPPORTED;
-  SB2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  SB2_CUDA_TRY(allow_shared(kern, kResSmem));
   // padded to whole quads of the last slice
   const size_t nn = vector_stride(S.nslice * kQuadRows, sizeof(double));
   const size_t hm = which == kGmres ? (size_t)grid * (m + 1) * (m + 1) : 0;
@@ -4660,6 +4662,8 @@ __global__ void __launch_bounds__(NTC, 1) cg_cluster_kernel(ClusterCgArgs a) {
   cl.sync();  // no CTA leaves while another may still read its shared memory
 }
 
+constexpr size_t kClusterSmem = 226 * 1024;  // most shared memory a CTA takes
+
 // Shared memory of one CTA for `rpc` rows and a largest slice of `nnz_max`.
 static size_t cluster_smem(int rpc, int nnz_max) {
   return sizeof(double) * ((size_t)nnz_max + 5 * (size_t)rpc + 4) +
@@ -4681,7 +4685,8 @@ static int cluster_plan(const sb2_csr* A, int* ranks, int* rpc, int* nnz_max) {
       SB2_CUDA_TRY(cudaMemcpy(ptr.data(), A->full.d_ptr, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost));
       int dev_smem = 0;
       cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, current_device());
-      const size_t limit = (size_t)std::max(dev_smem - 1024, 0);  // static shared memory
+      // (less what is static)
+      const size_t limit = std::min(kClusterSmem, (size_t)std::max(dev_smem - 1024, 0));
       for (int c = std::min(kClusterMaxRanks, cap); c >= 2; c /= 2) {
         const int r = (n + c - 1) / c;
         int mx = 0;
@@ -4713,8 +4718,7 @@ static int cluster_cg_solve(const sb2_csr* A, const double* diag, double* x, con
   if (C < 2) return SB2_ERR_NOT_SUPPORTED;
   const size_t smem = cluster_smem(rpc, nnz_max);
   SB2_CUDA_TRY(cudaFuncSetAttribute(cg_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  SB2_CUDA_TRY(cudaFuncSetAttribute(cg_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
+  SB2_CUDA_TRY(allow_shared((const void*)cg_cluster_kernel, kClusterSmem));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(C);
   cfg.blockDim = dim3(NTC);

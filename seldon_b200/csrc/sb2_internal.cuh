@@ -177,6 +177,13 @@ int get_red_scratch(cudaStream_t s, RedScratch** out);
 
 int current_device();
 int num_sms(int device);
+// Lets a kernel be launched with dynamic shared memory of up to `most` bytes:
+// the most that any of its launches takes, not what this one does.  The
+// attribute belongs to the kernel, and a smaller value that another thread
+// sets between this call and the launch would make the launch fail.
+inline cudaError_t allow_shared(const void* kern, size_t most) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
 // Stream-ordered workspace allocation from the library's own memory pool
 // (freed with cudaFreeAsync).
 cudaError_t pool_malloc(void** p, size_t bytes, cudaStream_t s);

@@ -801,8 +801,7 @@ int launch_sweeps(const SweepGrid& G, int sweeps, const SweepPlan* const (&plan)
                                    late);
   SB2_CUDA_TRY(cudaGetLastError());
   const void* kern = own ? (const void*)sweep_kernel<Op, true> : (const void*)sweep_kernel<Op, false>;
-  if (own && smem > 48 * 1024)
-    SB2_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (own && smem > 48 * 1024) SB2_CUDA_TRY(allow_shared(kern, kSweepSmem));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(G.ctas);
   cfg.blockDim = dim3(Op::kThreads);
