@@ -410,6 +410,8 @@ int sb2_bicgstab(const sb2_csr* A, const sb2_precond* M, double* x,
                  const double* b, const sb2_iter_params* params,
                  sb2_iter_result* result, double* hist, int* hist_it,
                  int hist_cap, void* stream);
+/* Gmres(params->restart).  With the identity or Jacobi a restart of more than
+ * 140 gives SB2_ERR_NOT_SUPPORTED. */
 int sb2_gmres(const sb2_csr* A, const sb2_precond* M, double* x,
               const double* b, const sb2_iter_params* params,
               sb2_iter_result* result, double* hist, int* hist_it,

@@ -3273,7 +3273,11 @@ enum Solver {
   kSymm = 14                                     // Symmlq
 };
 
-// Most shared memory of the fused Gmres's Hessenberg matrix and rotations.
+// Shared memory of the fused Gmres's Hessenberg matrix and rotations, and the
+// most of it: Gmres takes restarts up to 140, whatever form it runs in.
+static size_t gmres_smem(int m) {
+  return sizeof(double) * ((size_t)(m + 1) * (m + 1) + 3 * (size_t)(m + 1));
+}
 constexpr size_t kGmresSmem = 160 * 1024;
 
 static int fused_solve(int which, const sb2_csr* A, const double* diag, double* x,
@@ -3305,7 +3309,7 @@ static int fused_solve(int which, const sb2_csr* A, const double* diag, double* 
   if (which == kGmres) {
     kern = (const void*)gmres_fused_kernel;
     nvec = 2 + (m + 1);
-    smem = sizeof(double) * ((size_t)(m + 1) * (m + 1) + 3 * (m + 1));
+    smem = gmres_smem(m);
     if (smem > kGmresSmem) return SB2_ERR_NOT_SUPPORTED;
     SB2_CUDA_TRY(allow_shared(kern, kGmresSmem));
   }
@@ -3433,6 +3437,7 @@ static int resident_solve(int which, const sb2_csr* A, const double* diag, doubl
   const int n = A->m, m = std::max(prm->restart, 1);
   if (S.nslice <= 0 || S.sorted || S.nwarp || S.ncta || (int)S.h_sptr.size() != S.nslice + 1)
     return SB2_ERR_NOT_SUPPORTED;
+  if (which == kGmres && gmres_smem(m) > kGmresSmem) return SB2_ERR_NOT_SUPPORTED;
   const bool jac = diag != nullptr;
   const int sms = std::min(kPersistMaxCtas, num_sms(current_device()));
   const int per = (S.nslice + sms - 1) / sms;
@@ -3461,7 +3466,9 @@ static int resident_solve(int which, const sb2_csr* A, const double* diag, doubl
   const int gvec = which == kGmres ? m + 1 : 3;
   SolveScratch sc;
   const int hcap = std::max(hist_cap, 0) + 1;
-  SB2_TRY(alloc_scratch(s, (int)std::min<size_t>(nn, INT_MAX), gvec, grid, hcap, &sc, hm));
+  const int st = alloc_scratch(s, (int)std::min<size_t>(nn, INT_MAX), gvec, grid, hcap, &sc, hm);
+  if (st == SB2_ERR_NO_MEMORY) return SB2_ERR_NOT_SUPPORTED;  // the fused form may need less
+  SB2_TRY(st);
   Persist P{sc.sync, sc.partials, barrier_wait_ns()};
   History H{sc.hist, sc.hist_it, hcap};
   IterArgs it{prm->tol, prm->max_iter, m, prm->init_guess_null};

@@ -97,3 +97,36 @@ def test_resident_vs_oracle(api, oracle, which, name, n, restart, most, jacobi, 
     ro = b - matgen.matvec(ptr, ind, val, xo)
     if co == 0:
         assert np.linalg.norm(r) <= 2e-10 * np.linalg.norm(b) + 2 * np.linalg.norm(ro)
+
+
+@pytest.mark.parametrize("long_row", [False, True])
+@pytest.mark.parametrize("restart,taken", [(140, True), (141, False), (200, False), (1000, False)])
+def test_restarts_taken(api, long_row, restart, taken):
+    """Gmres takes the same restarts whichever of its kernels a matrix runs on
+    (a row of more than 32 entries keeps it off the chip)."""
+    import torch
+    from seldon_b200 import _lib
+    n = 3000
+    ptr, ind, val = _ragged(n, 5, False)
+    if long_row:
+        k = ptr[1]
+        cols = np.union1d(ind[:k], np.arange(0, 400, 8)).astype(np.int32)
+        row0 = np.full(cols.size, 1e-3)
+        row0[0] = 2.0
+        ind = np.concatenate([cols, ind[k:]])
+        val = np.concatenate([row0, val[k:]])
+        ptr = np.concatenate([[0], ptr[1:] + cols.size - k]).astype(np.int32)
+    A = api.RowSparse(n, n, ptr, ind, val)
+    b = to_dev(np.random.default_rng(6).standard_normal(n))
+    x = torch.zeros_like(b)
+    it = api.Iteration(2, 1e-10)
+    it.SetRestart(restart)
+    it.HideMessages()
+    if taken:
+        api.Gmres(A, x, b, api.Preconditioner_Base(), it)
+        # (a cycle runs to its restart or the tolerance, whatever max_iter is)
+        assert 2 <= it.GetNumberIteration() <= restart
+    else:
+        with pytest.raises(_lib.SeldonB200Error) as err:
+            api.Gmres(A, x, b, api.Preconditioner_Base(), it)
+        assert err.value.status == _lib.SB2_ERR_NOT_SUPPORTED
