@@ -213,7 +213,7 @@ __device__ __forceinline__ void spmv_phase(const OpArgs& A, const double* x, Epi
                                            double* s_prod, double* s_red) {
   XLoadCa<double> xl{x};
   if (A.sell.nslice >= 0) {
-    sell_spmv<NT, double, double>(A.sell, xl, epi, s_red, blockIdx.x, gridDim.x);
+    sell_spmv_wide<NT, double, double>(A.sell, xl, epi, s_red);
     return;
   }
   for (int b = blockIdx.x; b < A.nblk; b += gridDim.x)
@@ -3231,10 +3231,7 @@ static int coop_grid(const void* kernel, size_t smem, const sb2_csr* A) {
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, NT, smem) != cudaSuccess ||
       per_sm < 1)
     return 0;
-  const int cap = std::min(kPersistMaxCtas, num_sms(dev));
-  // enough CTAs to cover the work, no more: a small grid makes the barriers cheap
-  const int want = (A->m + NT - 1) / NT;
-  return std::max(1, std::min(cap, want));
+  return persist_ctas(A->m, A->full.part.nblk, std::min(kPersistMaxCtas, num_sms(dev)));
 }
 
 static int finish_solve(SolveScratch& S, cudaStream_t s, sb2_iter_result* res, double* hist,

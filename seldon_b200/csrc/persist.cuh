@@ -7,6 +7,8 @@
 // never hang the GPU.
 #pragma once
 
+#include <algorithm>
+
 #include "spmv_core.cuh"
 
 namespace sb2 {
@@ -43,6 +45,19 @@ struct History {
   int* it;
   int cap;
 };
+
+// CTAs of 1024 threads for a solver on `rows` rows in `blocks` row blocks (of up
+// to 2048 entries): a row a thread, and no more than four blocks a CTA.  No
+// more than that, since a small grid makes the barriers cheap; no less, since a
+// product by few CTAs leaves the other SMs' loads unused.  Cg, us an iteration,
+// by rows alone against this: 8192 rows of 301 entries 94 -> 19, 4096 of 1001 194
+// -> 20, 20,000 of 81 63 -> 21, 27,000 of 27 34 -> 25; Lsqr 98 -> 15, 210 -> 17, 60
+// -> 17, 31 -> 26.  Two blocks a CTA: the same where rows are wide, Lsqr on the
+// 27,000 rows 29.
+inline int persist_ctas(int rows, int blocks, int most) {
+  const int want = std::max((rows + 1023) / 1024, (blocks + 3) / 4);
+  return std::max(1, std::min(most, want));
+}
 
 #ifdef __CUDACC__
 
