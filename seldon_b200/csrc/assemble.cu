@@ -10,6 +10,7 @@
 //   k_coo_stats       sizes: largest row and column, bad indices, kept count,
 //                     and whether the triplets come in order already
 //   k_coo_sorted      triplets in order: copies, and ptr from the row changes
+//   k_coo_rows        or, across long runs of empty rows, from a search a row
 //   k_bkt_*           the rest, where buckets of rows fit a CTA (see there)
 //   otherwise:
 //   k_row_count       entries per row (warp-aggregated atomics), scanned
@@ -53,6 +54,7 @@ struct CooStats {
   int bad;      // some index - index < 0 or too large
   int kept;     // entries with row <= col
   int unsorted; // the triplets are not in (row, column) order
+  int gap;      // most rows between a triplet and the next (of the first: from -1)
 };
 
 // Also whether the triplets come in (row, column) order already: each is
@@ -61,7 +63,7 @@ __global__ void __launch_bounds__(kAsmThreads)
 k_coo_stats(const int* __restrict__ row, const int* __restrict__ col, long long nnz, int index,
             CooStats* st) {
   constexpr int U = 4;
-  int rmax = 0, cmax = 0, bad = 0, kept = 0, unsorted = 0;
+  int rmax = 0, cmax = 0, bad = 0, kept = 0, unsorted = 0, gap = 0;
   const long long stride = (long long)gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31;
   for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < nnz;
@@ -86,13 +88,17 @@ k_coo_stats(const int* __restrict__ row, const int* __restrict__ col, long long 
         rn[u] = r2;
         cn[u] = c2;
       }
-      if (i + 1 < nnz) unsorted |= rn[u] < rv[u] || (rn[u] == rv[u] && cn[u] < cv[u]);
+      if (i + 1 < nnz) {
+        unsorted |= rn[u] < rv[u] || (rn[u] == rv[u] && cn[u] < cv[u]);
+        if (rn[u] > rv[u]) gap = max(gap, (int)((unsigned)rn[u] - (unsigned)rv[u]));
+      }
       const bool out = r < 0 || c < 0 || r >= INT_MAX || c >= INT_MAX;
       bad |= out;
       if (!out && i < nnz) {
         rmax = max(rmax, (int)r);
         cmax = max(cmax, (int)c);
         kept += (r <= c);
+        if (i == 0) gap = max(gap, (int)r + 1);
       }
     }
   }
@@ -101,11 +107,12 @@ k_coo_stats(const int* __restrict__ row, const int* __restrict__ col, long long 
   bad = __reduce_or_sync(0xffffffffu, bad);
   kept = __reduce_add_sync(0xffffffffu, kept);
   unsorted = __reduce_or_sync(0xffffffffu, unsorted);
+  gap = __reduce_max_sync(0xffffffffu, gap);
   // one set of atomics per CTA: with one per warp they took longer than the reads
-  __shared__ int s_st[kAsmWarps][5];
+  __shared__ int s_st[kAsmWarps][6];
   if (lane == 0) {
     int* w = s_st[threadIdx.x >> 5];
-    w[0] = rmax; w[1] = cmax; w[2] = bad; w[3] = kept; w[4] = unsorted;
+    w[0] = rmax; w[1] = cmax; w[2] = bad; w[3] = kept; w[4] = unsorted; w[5] = gap;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -115,17 +122,27 @@ k_coo_stats(const int* __restrict__ row, const int* __restrict__ col, long long 
       bad |= s_st[w][2];
       kept += s_st[w][3];
       unsorted |= s_st[w][4];
+      gap = max(gap, s_st[w][5]);
     }
     atomicMax(&st->row_max, rmax);
     atomicMax(&st->col_max, cmax);
     if (bad) atomicOr(&st->bad, 1);
     atomicAdd(&st->kept, kept);
     if (unsorted) atomicOr(&st->unsorted, 1);
+    atomicMax(&st->gap, gap);
   }
 }
 
+// Rows that one thread of k_coo_sorted fills ptr for at most.  1M triplets, gaps
+// of 1024 rows: 132 us a call so, 175 with the searches; of 4096: 179 and 173; one
+// gap of 16M rows: 56 ms and 0.44.
+constexpr int kGapRows = 2048;
+
 // Triplets that are in order: ind and val are copies, and ptr[r] is the place
-// of the first triplet of row r or beyond.
+// of the first triplet of row r or beyond: the triplet's thread fills ptr from
+// the row of the one before.  Where that may be many rows (GAPS) k_coo_rows
+// fills it instead.
+template <bool GAPS>
 __global__ void __launch_bounds__(kAsmThreads)
 k_coo_sorted(const int* __restrict__ row, const int* __restrict__ col,
              const double* __restrict__ val, long long nnz, int index, int m,
@@ -136,9 +153,26 @@ k_coo_sorted(const int* __restrict__ row, const int* __restrict__ col,
     const int r = __ldg(row + i) - index, before = i ? __ldg(row + i - 1) - index : -1;
     ind[i] = __ldcs(col + i) - index;
     vout[i] = __ldcs(val + i);
-    for (int q = before + 1; q <= r; q++) ptr[q] = (int)i;
-    if (i == nnz - 1)
-      for (int q = r + 1; q <= m; q++) ptr[q] = (int)nnz;
+    if (!GAPS) {
+      for (int q = before + 1; q <= r; q++) ptr[q] = (int)i;
+      if (i == nnz - 1)
+        for (int q = r + 1; q <= m; q++) ptr[q] = (int)nnz;
+    }
+  }
+}
+
+// ptr of triplets in order by a search for each row.
+__global__ void __launch_bounds__(kAsmThreads)
+k_coo_rows(const int* __restrict__ row, long long nnz, int index, int m, int* __restrict__ ptr) {
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r <= m; r += stride) {
+    long long lo = 0, hi = nnz;  // the first triplet of row r or beyond lies in [lo, hi]
+    while (lo < hi) {
+      const long long mid = (lo + hi) >> 1;
+      if ((long long)__ldg(row + mid) - index < r) lo = mid + 1;
+      else hi = mid;
+    }
+    ptr[r] = (int)lo;
   }
 }
 
@@ -909,7 +943,7 @@ int sb2_coo_to_csr(int nnz, const int* row, const int* col, const double* val, i
   *val_out = nullptr;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 
-  CooStats h = {0, 0, 0, 0, 0};
+  CooStats h = {};
   if (nnz > 0) {
     CooStats* d = nullptr;
     SB2_CUDA_TRY(pool_malloc((void**)&d, sizeof(CooStats), s));
@@ -951,11 +985,17 @@ int sb2_coo_to_csr(int nnz, const int* row, const int* col, const double* val, i
   if (e == cudaSuccess && nout > 0) e = pool_malloc_owned((void**)&dv, sizeof(double) * nout, s);
   int st = map_cuda_error(e);
   bool done = false;
-  // (a run of empty rows is filled by one thread: the buckets take those)
-  if (st == SB2_OK && nnz > 0 && !h.unsorted && nout == nnz && m <= 4LL * nnz) {
+  if (st == SB2_OK && nnz > 0 && !h.unsorted && nout == nnz) {
     const int grid = (int)std::min<long long>((nnz + kAsmThreads - 1) / kAsmThreads,
                                               num_sms(current_device()) * 8LL);
-    k_coo_sorted<<<grid, kAsmThreads, 0, s>>>(row, col, val, nnz, index, (int)m, dp, di, dv);
+    if (std::max<long long>(h.gap, m - h.row_max) > kGapRows) {
+      k_coo_sorted<true><<<grid, kAsmThreads, 0, s>>>(row, col, val, nnz, index, (int)m, dp, di, dv);
+      const int rgrid =
+          (int)std::min<long long>((m + kAsmThreads) / kAsmThreads, num_sms(current_device()) * 8LL);
+      k_coo_rows<<<rgrid, kAsmThreads, 0, s>>>(row, nnz, index, (int)m, dp);
+    } else {
+      k_coo_sorted<false><<<grid, kAsmThreads, 0, s>>>(row, col, val, nnz, index, (int)m, dp, di, dv);
+    }
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     st = map_cuda_error(e);
