@@ -460,8 +460,13 @@ constexpr int kBktTile = 16 * kDealThreads;
 constexpr int kSortThreads = 512;
 constexpr int kBktCap = 5376;      // entries of a bucket at most: two CTAs an SM
 constexpr int kBktRows = 4096;     // rows of a bucket at most
-constexpr int kBktRank = 48;
-constexpr int kBktLong = 256;      // longer rows of one bucket, at most
+// Longest row that is ranked.  A row of the bitonic sort has the CTA to itself,
+// 28 CTA barriers for 80 entries and half its threads idle up to 512; a rank
+// reads the row once an entry, all lanes of a row the same key.  4M triplets,
+// exactly 49 / 81 / 125 / 257 a row: 235 / 272 / 284 / 387 us a call, 1289 / 1071 / 793 /
+// 752 with rows past 48 sorted; at 400 the two meet (502 and 610).
+constexpr int kBktRank = 448;
+constexpr int kBktLong = 16;       // longer rows of one bucket, at most
 
 struct BktArgs {
   const int* row;
@@ -821,6 +826,11 @@ int assemble_buckets(long long nnz, const int* row, const int* col, const double
   while (lb < 12 && (2.0 * nout / m) * (double)(1 << lb) <= target) lb++;
   while (lb < 12 && ((long long)m + (1 << lb) - 1) >> lb > kBktMax) lb++;
   const long long nb = ((long long)m + (1 << lb) - 1) >> lb;
+  // rows that are mostly too long to be ranked and too short for the bitonic
+  // sort: 8M triplets of 500 / 700 / 1000 a row 1119 / 1170 / 1130 us here, 925 / 995 /
+  // 1090 row by row; 2M of 500 382 and 421, 8M of 2000 1175 and 1325
+  const double mean = (double)nout / m;
+  if (mean > kBktRank - 32 && mean < 1024.0 && nout >= 4000000) return SB2_OK;
   if (nb > kBktMax || (double)nout / m * (1 << lb) > 0.9 * kBktCap || lb + cb + ib > 64)
     return SB2_OK;
   BktArgs a{row, col, val, nnz, nout, index, sym, m, lb, cb, ib, (int)nb};

@@ -1,6 +1,7 @@
 """The COO assembly (csrc/assemble.cu) where rows are missing: triplets in order
 with runs of empty rows before, between and behind them, around the length that
-one thread fills."""
+one thread fills; and where rows are long, around the lengths that buckets rank,
+sort and leave to the row form."""
 import numpy as np
 import pytest
 
@@ -47,3 +48,30 @@ def test_one_long_run_takes_no_longer_than_a_search(cuda):
         best = min(best, a.elapsed_time(b))
     assert m == 16_000_000 and int(ptr[-1]) == nnz and int(ptr[-2]) == nnz - 1 and int(ptr[1001]) == nnz - 1
     assert best < 10.0
+
+
+@pytest.mark.parametrize("length", [47, 49, 65, 81, 447, 448, 449, 513, 900])
+@pytest.mark.parametrize("sym", [False, True])
+def test_rows_of_a_length(cuda, length, sym):
+    """Rows of this many entries and one of each neighbouring length, shuffled."""
+    rng = np.random.default_rng(length)
+    m = 300
+    lens = np.full(m, length)
+    lens[[3, 100]] = length - 1
+    lens[[7, 200]] = length + 1
+    lens[50] = 0
+    r = np.repeat(np.arange(m), lens)
+    c = rng.integers(0, 40 if length % 2 else 100000, r.size)
+    if sym:
+        c = c % m
+    at = rng.permutation(r.size)
+    _check(r[at], c[at], rng.standard_normal(r.size), 0, m, sym)
+
+
+@pytest.mark.parametrize("mean", [400, 430, 1100])
+def test_many_triplets_in_long_rows(cuda, mean):
+    """4M triplets and more, where the mean row decides the form."""
+    rng = np.random.default_rng(mean)
+    nnz = 4_100_000
+    m = nnz // mean
+    _check(rng.integers(0, m, nnz), rng.integers(0, m, nnz), rng.standard_normal(nnz), 0, m, False)
