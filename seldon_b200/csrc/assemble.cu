@@ -812,8 +812,9 @@ cudaError_t bkt_shared_memory() {
   return e;
 }
 
-// The two-pass form.  *done false: the triplets do not suit it (the outputs
-// are then unwritten).  Synchronizes the stream.
+// The two-pass form.  *done false: the triplets do not suit it, or its scratch
+// of 16 bytes a triplet is not to be had (the form after it takes 8); the outputs
+// are then unfinished.  Synchronizes the stream.
 int assemble_buckets(long long nnz, const int* row, const int* col, const double* val, int index,
                      int m, int cb, int sym, long long nout, int* ptr, int* ind, double* vout,
                      cudaStream_t s, bool* done) {
@@ -839,13 +840,18 @@ int assemble_buckets(long long nnz, const int* row, const int* col, const double
   a.vout = vout;
   char* buf = nullptr;
   const size_t ints = 2 * (size_t)kBktMax + 64;
-  SB2_CUDA_TRY(pool_malloc((void**)&buf, 16 * (size_t)nout + sizeof(int) * ints, s));
+  cudaError_t e = pool_malloc((void**)&buf, 16 * (size_t)nout + sizeof(int) * ints, s);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return SB2_OK;
+  }
+  SB2_CUDA_TRY(e);
   a.key = reinterpret_cast<unsigned long long*>(buf);
   a.kval = reinterpret_cast<double*>(buf + 8 * (size_t)nout);
   a.count = reinterpret_cast<int*>(buf + 16 * (size_t)nout);
   a.cursor = a.count + kBktMax + 1;
   a.over = a.cursor + kBktMax;
-  cudaError_t e = cudaMemsetAsync(a.count, 0, sizeof(int) * ints, s);
+  e = cudaMemsetAsync(a.count, 0, sizeof(int) * ints, s);
   if (e == cudaSuccess) e = bkt_shared_memory();
   int over = 0;
   if (e == cudaSuccess) {

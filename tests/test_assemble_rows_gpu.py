@@ -75,3 +75,47 @@ def test_many_triplets_in_long_rows(cuda, mean):
     nnz = 4_100_000
     m = nnz // mean
     _check(rng.integers(0, m, nnz), rng.integers(0, m, nnz), rng.standard_normal(nnz), 0, m, False)
+
+
+def _starved():
+    import torch
+    from seldon_b200 import api
+    nnz, m = 18 << 20, 1 << 22  # 4096 buckets of 4608 entries
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    row = torch.randint(0, m, (nnz,), device="cuda", dtype=torch.int32, generator=gen)
+    col = torch.randint(0, 1000, (nnz,), device="cuda", dtype=torch.int32, generator=gen)
+    val = torch.ones(nnz, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    # outputs of 12 bytes a triplet and a row's 4 (232 MB), then 288 MB of scratch
+    # or 144 MB and two arrays of a row's 4 (176 MB)
+    free = torch.cuda.mem_get_info()[0]
+    spare = (232 + 232) << 20
+    assert free > spare
+    full = torch.empty(free - spare, dtype=torch.uint8, device="cuda")
+    try:
+        M, N, ptr, ind, v = api.ConvertMatrix_from_Coordinates(row, col, val, 0, m, 0, False)
+    finally:
+        del full
+        torch.cuda.empty_cache()
+    count = torch.bincount(row, minlength=m)
+    assert M == m and torch.equal(torch.diff(ptr).long(), count)
+    assert int(ind.long().sum()) == int(col.long().sum()) and bool((v == 1.0).all())
+    # columns in order within each row
+    same = torch.ones(nnz - 1, dtype=torch.bool, device="cuda")
+    ends = ptr[1:-1].long()
+    same[ends[(ends > 0) & (ends < nnz)] - 1] = False
+    assert bool((ind[1:] >= ind[:-1])[same].all())
+
+
+def test_scratch_that_does_not_fit(cuda):
+    """The bucket form's scratch is 16 bytes a triplet, the row form's 8: with
+    room for the second only the call still succeeds.  (A process of its own: no
+    memory that earlier calls left in the library's pool.)"""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    run = "from tests.test_assemble_rows_gpu import _starved; _starved(); print('starved: done')"
+    p = subprocess.run([sys.executable, "-c", run], cwd=root, capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0 and "starved: done" in p.stdout, p.stderr[-3000:]
