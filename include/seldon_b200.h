@@ -705,8 +705,9 @@ int sb2_batch_create(int nsys, const int* sys_row, const int* ptr, const int* in
                      const double* val, sb2_batch** out);
 int sb2_batch_destroy(sb2_batch* B);
 
-/* Solve every system in ONE persistent launch (CTAs take systems from a
- * queue, largest first).  x, b: device vectors of all rows.  d_iters /
+/* Solve every system, in ONE persistent launch (CTAs take systems from a
+ * queue, largest first) or one for each of up to three size classes, which
+ * overlap.  x, b: device vectors of all rows.  d_iters /
  * d_relres (device, may be NULL): per-system iteration count and final
  * relative residual.  With result == NULL the call only enqueues work on
  * `stream` (no host synchronization, so it can be captured in a CUDA graph);
@@ -716,8 +717,8 @@ int sb2_batch_solve(const sb2_batch* B, double* x, const double* b,
                     sb2_batch_result* result, void* stream);
 
 /* Until a plan is set or tuned, one CTA solves each system with its vectors
- * (and its part of the matrix, where that fits) in shared memory; its size
- * follows the largest system.  A plan keeps the vectors in L2 instead and is
+ * (and its part of the matrix, where that fits) in shared memory: 128 threads
+ * for systems of up to 512 rows, 256 up to 2048, else 1024.  A plan keeps the vectors in L2 instead and is
  * chosen per size class of the systems:
  *   threads   CTA size (128, 256 or 512) of the systems a whole CTA solves
  *   warp_max  systems of at most this many rows are solved by one warp each

@@ -56,6 +56,8 @@ struct sb2_batch {
   // autotuner found it faster in that mode
   bool onchip[2] = {true, true};
   bool tuned[2] = {false, false};
+  int chip_count[3] = {0, 0, 0};  // systems of each class of the on-chip form
+  int chip_rows[3] = {0, 0, 0};   // rows of its largest
   int max_rows = 0;
   unsigned long long histo_key = 0;  // size histogram, for the tuned-plan cache
 };
@@ -505,7 +507,9 @@ __global__ void __launch_bounds__(NT, 1536 / NT) batch_kernel(BatchArgs a) {
 // through L2, two rows a thread at a time.  The forms above keep everything in
 // L2 and wait for it with three CTAs per SM: 0.56 of the copy bandwidth in DRAM
 // traffic, long-scoreboard stalls 39 of 46 cycles.  Here a row moves at most 30
-// bytes of matrix an iteration, and none up to 4,500 rows of five entries.
+// bytes of matrix an iteration, and none up to 4,500 rows of five entries.  CTAs
+// of 128 and 256 threads come six and three to an SM: with half of that, 4096
+// systems of 24^2 rows took 2.8 ms, 2.3 as now and with a plan.
 // 512 shifted 2D Laplacians of sides 8 to 140, mixed, to 1e-13: 10.0 ms, against
 // 62.5 ms with one 256-thread CTA per system and 19.3 ms with the best plan of
 // the forms above (4-CTA clusters); in FP64 26-29 ms against 30.2.  Systems of
@@ -788,11 +792,12 @@ __device__ bool chip_mixed(G& g, const BatchArgs& a, int s, int r0, int n, doubl
 }
 
 template <int NT, typename IT>
-__global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 2) batch_chip_kernel(BatchArgs a, int room) {
+__global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 768 / NT) batch_chip_kernel(BatchArgs a, int room) {
   extern __shared__ __align__(16) char s_chip[];
   __shared__ int s_sys;
   __shared__ double s_red[2 * 2 * (NT / 32)];
   ChipGroup<NT> g{s_red, 0};
+  pdl_release();  // the next class takes the SMs this one leaves idle at its end
   for (;;) {
     if (threadIdx.x == 0) {
       const unsigned k = atomicAdd(a.queue, 1u);
@@ -801,7 +806,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 2) batch_chip_kernel(Batc
     __syncthreads();
     const int s = s_sys;
     __syncthreads();
-    if (s < 0) return;
+    if (s < 0) break;
     const int r0 = __ldg(a.sys_row + s), n = __ldg(a.sys_row + s + 1) - r0;
     double acc = 0.0;
     for (int i = g.rank(); i < n; i += NT) {
@@ -826,6 +831,9 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 2) batch_chip_kernel(Batc
     }
     __syncthreads();
   }
+  // one CTA stays until the class before is done, so that what follows on the
+  // stream follows every class
+  if (blockIdx.x == 0) pdl_wait();
 }
 
 // Clusters of `cluster` CTAs that one GPU holds at once for this kernel
@@ -905,29 +913,55 @@ static int launch_batch_t(const BatchArgs& a, int threads, int cluster, cudaStre
 constexpr int kChipRoom = 224 * 1024;
 
 template <int NT, typename IT>
-static int launch_chip(const BatchArgs& a, int room, cudaStream_t s) {
+static int launch_chip(const BatchArgs& a, int room, bool overlap, cudaStream_t s) {
   auto* k = batch_chip_kernel<NT, IT>;
   if (room > 48 * 1024) SB2_CUDA_TRY(allow_shared((const void*)k, kChipRoom));
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, NT, room) != cudaSuccess || per_sm < 1)
     return SB2_ERR_NOT_SUPPORTED;
-  const int grid = std::min(a.nsys, per_sm * num_sms(current_device()));
-  k<<<std::max(grid, 1), NT, room, s>>>(a, room);
-  SB2_CUDA_TRY(cudaGetLastError());
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(std::min(a.nsys, per_sm * num_sms(current_device())));
+  cfg.blockDim = dim3(NT);
+  cfg.dynamicSmemBytes = room;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  SB2_CUDA_TRY(cudaLaunchKernelEx(&cfg, k, a, room));
   return SB2_OK;
 }
 
-// CTA size by the largest system: enough threads for its rows, and small CTAs
-// side by side on an SM where all systems are small.
+// Rows up to which a system is solved by 128 and by 256 threads, else by 1024.
+constexpr int kChipRows[2] = {512, 2048};
+
+// One launch per class of sizes, the largest systems first: enough threads for
+// a system's rows, and small CTAs side by side on an SM for small systems.  The
+// launches overlap: the systems are independent, and a class only starts once
+// every CTA of the one before runs.  (One launch sized for the largest system:
+// 20,000 systems of 10^2 rows and one of 60^2 took 10.3 ms, 3.2 with a CTA of 256
+// threads each through L2.)
 template <typename IT>
-static int launch_onchip(const BatchArgs& a, int max_rows, long long nnz, cudaStream_t s) {
-  // room for the largest system with its matrix (mean entries a row), if it fits
-  const size_t t = a.mode == 1 ? 8 : 4;
-  const double per_row = 4.0 * t + 4.0 + (t + sizeof(IT)) * (double)nnz / std::max(a.m, 1);
-  const int room = (int)std::min<double>(kChipRoom, 1.05 * per_row * max_rows + 512);
-  if (max_rows <= 512) return launch_chip<128, IT>(a, room, s);
-  if (max_rows <= 2048) return launch_chip<256, IT>(a, room, s);
-  return launch_chip<1024, IT>(a, room, s);
+static int launch_onchip(const sb2_batch* B, const BatchArgs& all, cudaStream_t s) {
+  // room for a class's largest system with its matrix (mean entries a row), if it fits
+  const size_t t = all.mode == 1 ? 8 : 4;
+  const double per_row = 4.0 * t + 4.0 + (t + sizeof(IT)) * (double)B->nnz / std::max(all.m, 1);
+  int first = 0;
+  for (int c = 0; c < 3; c++) {
+    const int count = B->chip_count[c];
+    if (!count) continue;
+    BatchArgs a = all;
+    a.nsys = count;
+    a.order += first;
+    a.queue += c;
+    const int room = (int)std::min<double>(kChipRoom, 1.05 * per_row * B->chip_rows[c] + 512);
+    if (c == 0) SB2_TRY((launch_chip<1024, IT>(a, room, first > 0, s)));
+    else if (c == 1) SB2_TRY((launch_chip<256, IT>(a, room, first > 0, s)));
+    else SB2_TRY((launch_chip<128, IT>(a, room, first > 0, s)));
+    first += count;
+  }
+  return SB2_OK;
 }
 
 static int batch_run(const sb2_batch* B, double* x, const double* b, const sb2_batch_params* prm,
@@ -937,10 +971,8 @@ static int batch_run(const sb2_batch* B, double* x, const double* b, const sb2_b
               b, x, B->d_r64, B->d_w32, B->m, B->d_queue, prm->tol, prm->update_ratio,
               prm->max_iter, prm->mode, prm->init_guess_null, warp_max, cluster_min, iters,
               relres};
-  SB2_CUDA_TRY(cudaMemsetAsync(B->d_queue, 0, sizeof(unsigned), s));
-  if (onchip)
-    return B->ind16 ? launch_onchip<unsigned short>(a, B->max_rows, B->nnz, s)
-                    : launch_onchip<int>(a, B->max_rows, B->nnz, s);
+  SB2_CUDA_TRY(cudaMemsetAsync(B->d_queue, 0, sizeof(unsigned) * 3, s));
+  if (onchip) return B->ind16 ? launch_onchip<unsigned short>(B, a, s) : launch_onchip<int>(B, a, s);
   return B->ind16 ? launch_batch_t<unsigned short>(a, threads, cluster, s)
                   : launch_batch_t<int>(a, threads, cluster, s);
 }
@@ -1032,6 +1064,12 @@ int sb2_batch_create(int nsys, const int* sys_row, const int* ptr, const int* in
   B->m = m;
   B->nnz = nnz;
   B->max_rows = maxrows;
+  for (int s = nsys - 1; s >= 0; s--) {
+    const int rows = sys_row[order[s] + 1] - sys_row[order[s]];
+    const int c = rows > kChipRows[1] ? 0 : rows > kChipRows[0] ? 1 : 2;
+    B->chip_count[c]++;
+    B->chip_rows[c] = rows;  // (from the smallest up)
+  }
   B->histo_key = size_histogram_key(nsys, sys_row);
   cudaError_t e = cudaMalloc(&B->d_sys_row, sizeof(int) * (nsys + 1));
   if (e == cudaSuccess) e = cudaMalloc(&B->d_order, sizeof(int) * std::max(nsys, 1));
