@@ -718,7 +718,9 @@ int sb2_batch_solve(const sb2_batch* B, double* x, const double* b,
 
 /* Until a plan is set or tuned, one CTA solves each system with its vectors
  * (and its part of the matrix, where that fits) in shared memory: 128 threads
- * for systems of up to 512 rows, 256 up to 2048, else 1024.  A plan keeps the vectors in L2 instead and is
+ * for systems of up to 512 rows, 256 up to 2048, else 1024.  (A batch with
+ * four or more systems per SM too large for that, above some 28,000 rows or
+ * 14,000 in mode 1, runs the plan below from the start.)  A plan keeps the vectors in L2 instead and is
  * chosen per size class of the systems:
  *   threads   CTA size (128, 256 or 512) of the systems a whole CTA solves
  *   warp_max  systems of at most this many rows are solved by one warp each

@@ -52,8 +52,8 @@ struct sb2_batch {
   int warp_max = 0;
   int cluster = 0;       // CTAs of a cluster plan (0: none)
   int cluster_min = 0;   // systems of more rows are solved by a whole cluster
-  // vectors in shared memory, per mode: until a plan is set, and where the
-  // autotuner found it faster in that mode
+  // vectors in shared memory, per mode: until a plan is set, unless too many
+  // systems do not fit (kChipOver), and where the autotuner found it faster
   bool onchip[2] = {true, true};
   bool tuned[2] = {false, false};
   int chip_count[3] = {0, 0, 0};  // systems of each class of the on-chip form
@@ -514,7 +514,7 @@ __global__ void __launch_bounds__(NT, 1536 / NT) batch_kernel(BatchArgs a) {
 // 62.5 ms with one 256-thread CTA per system and 19.3 ms with the best plan of
 // the forms above (4-CTA clusters); in FP64 26-29 ms against 30.2.  Systems of
 // more than about 28,000 rows (14,000 in FP64) do not fit and are solved by
-// the same CTAs through L2.
+// the same CTAs through L2 (but see kChipOver).
 
 // The CTA's threads, sums by a shuffle tree over the warps' partials.
 template <int NT>
@@ -610,13 +610,18 @@ __device__ __forceinline__ T chip_product(G& g, const ChipRows<IT, T>& A, int n,
   return g.sum(pq);
 }
 
+// Bytes of a vector in shared memory.
+__host__ __device__ __forceinline__ size_t chip_vector(int n, size_t size) {
+  return ((size_t)n * size + 15) / 16 * 16;
+}
+
 // Where a system's arrays go: the vectors and the matrix in `room` bytes of
 // shared memory, in the order above.  False: not even p and r fit.
 template <typename IT, typename T>
 __device__ __forceinline__ bool chip_layout(const BatchArgs& a, const T* val, char* smem, int room,
                                             int r0, int n, T*& p, T*& r, T*& q, T*& d,
                                             ChipRows<IT, T>& A) {
-  const size_t vec = ((size_t)n * sizeof(T) + 15) / 16 * 16;
+  const size_t vec = chip_vector(n, sizeof(T));
   if (2 * vec > (size_t)room) return false;
   p = reinterpret_cast<T*>(smem);
   r = reinterpret_cast<T*>(smem + vec);
@@ -933,6 +938,13 @@ static int launch_chip(const BatchArgs& a, int room, bool overlap, cudaStream_t 
   return SB2_OK;
 }
 
+// Systems per SM whose p and r do not fit that make an untuned batch take the
+// default plan (a CTA of 256 threads each, six to an SM, through L2).  One CTA of
+// 1024 threads to an SM solves fewer of them sooner and more of them later: 148 /
+// 444 / 592 / 888 systems of 200^2 rows, mixed, 32 / 95 / 126 / 189 ms, with the plan
+// 102 / 116 / 121 / 132; the same ratios from 170^2 to 300^2, and in FP64 from 120^2.
+constexpr int kChipOver = 4;
+
 // Rows up to which a system is solved by 128 and by 256 threads, else by 1024.
 constexpr int kChipRows[2] = {512, 2048};
 
@@ -1064,12 +1076,15 @@ int sb2_batch_create(int nsys, const int* sys_row, const int* ptr, const int* in
   B->m = m;
   B->nnz = nnz;
   B->max_rows = maxrows;
+  int over[2] = {0, 0};  // systems whose p and r do not fit, per mode
   for (int s = nsys - 1; s >= 0; s--) {
     const int rows = sys_row[order[s] + 1] - sys_row[order[s]];
+    for (int mode = 0; mode < 2; mode++) over[mode] += 2 * chip_vector(rows, mode ? 8 : 4) > (size_t)kChipRoom;
     const int c = rows > kChipRows[1] ? 0 : rows > kChipRows[0] ? 1 : 2;
     B->chip_count[c]++;
     B->chip_rows[c] = rows;  // (from the smallest up)
   }
+  for (int mode = 0; mode < 2; mode++) B->onchip[mode] = over[mode] < kChipOver * num_sms(B->device);
   B->histo_key = size_histogram_key(nsys, sys_row);
   cudaError_t e = cudaMalloc(&B->d_sys_row, sizeof(int) * (nsys + 1));
   if (e == cudaSuccess) e = cudaMalloc(&B->d_order, sizeof(int) * std::max(nsys, 1));

@@ -64,3 +64,33 @@ def test_classes(cuda, name, mixed):
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(x, y) and torch.equal(it, n)
+
+
+@pytest.mark.parametrize("mixed", [True, False])
+@pytest.mark.parametrize("per_sm,planned", [(3, False), (4, True)])
+def test_systems_that_do_not_fit(cuda, mixed, per_sm, planned):
+    """With four systems an SM too large for shared memory an untuned batch runs
+    the default plan (the same bits), with fewer it does not."""
+    import torch
+
+    from seldon_b200 import api
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = 28673 if mixed else 14337  # one row more than 224 KB hold twice
+    assert 2 * n * (4 if mixed else 8) > 224 * 1024
+    rng = np.random.default_rng(per_sm)
+    big, fits = _chain(n), _chain(n - 1)
+    systems = [big] * (per_sm * sms) + [fits] * 5
+    xs = []
+    b = to_dev(rng.uniform(-1, 1, per_sm * sms * n + 5 * (n - 1)))
+    for plan in (False, True):
+        B = api.Batch(systems)
+        if plan:
+            B.set_plan(256, 0)
+        x = to_dev(np.zeros(B.m))
+        it = torch.zeros(B.nsys, dtype=torch.int32, device="cuda")
+        rr = torch.zeros(B.nsys, dtype=torch.float64, device="cuda")
+        B.solve(x, b, it, rr, summary=False, tol=1e-30, max_iter=20, mixed=mixed)
+        xs.append(x)
+        B.close()
+    assert torch.equal(*xs) == planned
+    assert float((xs[0] - xs[1]).norm()) <= 1e-5 * float(xs[1].norm())
