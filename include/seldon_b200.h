@@ -733,8 +733,8 @@ int sb2_batch_solve(const sb2_batch* B, double* x, const double* b,
  * and with the vectors in shared memory, and keeps the best plan and, for
  * this mode, whether shared memory was faster still; the other mode runs the
  * plan unless it was tuned itself.  The choice is cached per (histogram of
- * the systems' sizes in power-of-two classes, mode): a later batch with the
- * same histogram takes it without timing. */
+ * the systems' sizes in power-of-two classes, mean entries of a row, mode): a
+ * later batch with the same of these takes it without timing. */
 int sb2_batch_autotune(sb2_batch* B, double* x, const double* b,
                        const sb2_batch_params* params, void* stream);
 int sb2_batch_set_threads(sb2_batch* B, int threads);

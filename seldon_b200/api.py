@@ -1139,7 +1139,7 @@ class Batch:
 
     def autotune(self, x, b, stream=None, **kw):
         """Times the candidate plans on this batch (x is overwritten) and keeps
-        the fastest; a batch with the same size histogram reuses the cached
+        the fastest; a batch of the same sizes and mean row reuses the cached
         choice.  Returns the CTA size (see plan())."""
         prm = self.params(**kw)
         check(_L.sb2_batch_autotune(self._h, _dev_ptr(x, self.m, "x"), _dev_ptr(b, self.m, "b"),

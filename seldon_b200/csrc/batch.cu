@@ -59,7 +59,7 @@ struct sb2_batch {
   int chip_count[3] = {0, 0, 0};  // systems of each class of the on-chip form
   int chip_rows[3] = {0, 0, 0};   // rows of its largest
   int max_rows = 0;
-  unsigned long long histo_key = 0;  // size histogram, for the tuned-plan cache
+  unsigned long long plan_key = 0;  // for the tuned-plan cache
 };
 
 namespace sb2 {
@@ -1002,8 +1002,12 @@ __global__ void batch_to_float(long long n, const double* __restrict__ a, float*
 }
 
 // Key of the tuned-plan cache: the count of systems in each power-of-two
-// row-count class (and the number of systems), hashed.
-static unsigned long long size_histogram_key(int nsys, const int* sys_row) {
+// row-count class (and the number of systems), and what else decides whether
+// vectors and matrix fit on chip: the mean entries of a row, the width of a
+// column index, `fits` (whether the untuned batch runs there, a bit per mode);
+// and the device.  Hashed.
+static unsigned long long plan_key(int nsys, const int* sys_row, int entries, bool ind16, int fits,
+                                   int device) {
   int cnt[33] = {0};
   for (int s = 0; s < nsys; s++) {
     unsigned v = (unsigned)(sys_row[s + 1] - sys_row[s]);
@@ -1015,10 +1019,12 @@ static unsigned long long size_histogram_key(int nsys, const int* sys_row) {
     cnt[c]++;
   }
   unsigned long long h = 1469598103934665603ull ^ (unsigned long long)nsys;
-  for (int c = 0; c < 33; c++) {
-    h ^= (unsigned long long)cnt[c] + 0x9e3779b97f4a7c15ull + (h << 6) + (h >> 2);
+  auto fold = [&](int v) {
+    h ^= (unsigned long long)v + 0x9e3779b97f4a7c15ull + (h << 6) + (h >> 2);
     h *= 1099511628211ull;
-  }
+  };
+  for (int c = 0; c < 33; c++) fold(cnt[c]);
+  for (int v : {entries, (int)ind16, fits, device}) fold(v);
   return h;
 }
 
@@ -1026,8 +1032,8 @@ struct BatchPlan {
   int threads, warp_max, cluster, cluster_min;
   bool onchip;
 };
-// Plans chosen by sb2_batch_autotune, per (size histogram, mode): a later
-// batch with the same histogram takes its plan without timing.
+// Plans chosen by sb2_batch_autotune, per (plan key, mode): a later batch with
+// the same key takes its plan without timing.
 static std::mutex g_plan_mu;
 static std::map<std::pair<unsigned long long, int>, BatchPlan> g_plans;
 
@@ -1085,11 +1091,12 @@ int sb2_batch_create(int nsys, const int* sys_row, const int* ptr, const int* in
     B->chip_rows[c] = rows;  // (from the smallest up)
   }
   for (int mode = 0; mode < 2; mode++) B->onchip[mode] = over[mode] < kChipOver * num_sms(B->device);
-  B->histo_key = size_histogram_key(nsys, sys_row);
   cudaError_t e = cudaMalloc(&B->d_sys_row, sizeof(int) * (nsys + 1));
   if (e == cudaSuccess) e = cudaMalloc(&B->d_order, sizeof(int) * std::max(nsys, 1));
   if (e == cudaSuccess) e = cudaMalloc(&B->d_ptr, sizeof(int) * (m + 1));
   B->ind16 = (maxrows <= 65536);
+  B->plan_key = plan_key(nsys, sys_row, (int)((double)nnz / std::max(m, 1) + 0.5), B->ind16,
+                         B->onchip[0] + 2 * B->onchip[1], B->device);
   if (e == cudaSuccess) e = cudaMalloc(&B->d_ind, (B->ind16 ? sizeof(unsigned short) : sizeof(int)) *
                                                       std::max<long long>(nnz, 1));
   if (e == cudaSuccess) e = cudaMalloc(&B->d_val, sizeof(double) * std::max<long long>(nnz, 1));
@@ -1238,7 +1245,7 @@ extern "C" int sb2_batch_autotune(sb2_batch* B, double* x, const double* b,
                                   const sb2_batch_params* prm, void* stream) try {
   if (!B || !prm) return SB2_ERR_INVALID_VALUE;
   if (B->nsys == 0) return SB2_OK;
-  const std::pair<unsigned long long, int> key{B->histo_key, prm->mode};
+  const std::pair<unsigned long long, int> key{B->plan_key, prm->mode};
   {
     std::lock_guard<std::mutex> g(sb2::g_plan_mu);
     auto it = sb2::g_plans.find(key);

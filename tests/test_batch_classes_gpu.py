@@ -94,3 +94,30 @@ def test_systems_that_do_not_fit(cuda, mixed, per_sm, planned):
         B.close()
     assert torch.equal(*xs) == planned
     assert float((xs[0] - xs[1]).norm()) <= 1e-5 * float(xs[1].norm())
+
+
+def test_tuning_is_kept_by_what_fits(cuda):
+    """A batch with the sizes of a tuned one and other rows is timed itself; one
+    with the same rows takes the tuned plan without timing."""
+    from seldon_b200 import api
+    rng = np.random.default_rng(3)
+    n = 1500
+
+    def banded(k):
+        i = np.repeat(np.arange(n), 2 * k + 1)
+        j = i + np.tile(np.arange(-k, k + 1), n)
+        ok = (j >= 0) & (j < n)
+        i, j = i[ok], j[ok]
+        ptr = np.concatenate([[0], np.cumsum(np.bincount(i, minlength=n))]).astype(np.int32)
+        return ptr, j.astype(np.int32), np.where(i == j, 4.0 * k, -1.0)
+
+    b = to_dev(rng.uniform(-1, 1, 40 * n))
+
+    def timed(k):
+        B = api.Batch([banded(k)] * 40)
+        x = to_dev(np.full(B.m, 7.0))
+        B.autotune(x, b, tol=1e-6)
+        return bool((x != 7.0).any())
+
+    assert timed(2) and not timed(2)
+    assert timed(13) and not timed(13)
