@@ -3451,6 +3451,12 @@ static int resident_solve(int which, const sb2_csr* A, const double* diag, doubl
   if (ms) smem += 48 * (size_t)groups;
   // Cg and BiCgStab gain only with the matrix on chip
   if (!ms && which != kGmres) return SB2_ERR_NOT_SUPPORTED;
+  // Gmres with the matrix streamed loses time in the product (the L1 is taken)
+  // and gains it in every Gram-Schmidt pass, so short restarts stay with the
+  // fused kernel.  us a step here / there: 104^3 rows (up to 8192 a CTA) at restart
+  // 1, 2, 4, 7, 30: 76 / 73, 60 / 58, 55 / 54, 57 / 59, 101 / 128; 128^3 at 7, 14, 18, 30:
+  // 108 / 99, 127 / 122, 139 / 139, 182 / 189; 1400^2: 92 / 86, 112 / 111, 122 / 127, 161 / 177
+  if (!ms && m < (per * kQuadRows > 8192 ? 18 : 4)) return SB2_ERR_NOT_SUPPORTED;
   int threads = 512;
   const void* kern = which == kCg     ? (const void*)cg_resident_kernel<512, true>
                      : which == kBicg ? (const void*)bicgstab_resident_kernel<512, true>

@@ -130,3 +130,11 @@ def test_restarts_taken(api, long_row, restart, taken):
         with pytest.raises(_lib.SeldonB200Error) as err:
             api.Gmres(A, x, b, api.Preconditioner_Base(), it)
         assert err.value.status == _lib.SB2_ERR_NOT_SUPPORTED
+
+
+@pytest.mark.parametrize("n", [148 * 8192, 148 * 8192 + 1])
+@pytest.mark.parametrize("restart", [3, 4, 17, 18])
+def test_gmres_where_the_forms_change(api, oracle, n, restart):
+    """Up to 8192 rows a CTA and one more, at the restarts where the fused kernel
+    hands over."""
+    test_resident_vs_oracle(api, oracle, "gmres", "ragged", n, restart, 20, True, False)
