@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(NT, 1) cg_fused_kernel(OpArgs A, CgVecs v, Ite
   }
   acc = block_sum<NT>(acc, s_red);
   if (tid == 0) s_vals[0] = acc;
-  if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+  if (!grid_sync<NT>(P, epoch, 1, s_vals)) return;
   const double normb = sqrt(s_vals[0]);
   if (normb == 0.0) {
     if (lead) { out->init_failed = 1; out->hist_len = 0; }
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(NT, 1) cg_fused_kernel(OpArgs A, CgVecs v, Ite
   rr = block_sum<NT>(rr, s_red);
   rz = block_sum<NT>(rz, s_red);
   if (tid == 0) { s_vals[0] = rr; s_vals[1] = rz; }
-  if (!grid_sync<NT>(P, epoch, 2, s_vals, s_red)) return;
+  if (!grid_sync<NT>(P, epoch, 2, s_vals)) return;
   rr = s_vals[0];
   double rho = s_vals[1], rho_1 = 1.0;
 
@@ -307,13 +307,13 @@ __global__ void __launch_bounds__(NT, 1) cg_fused_kernel(OpArgs A, CgVecs v, Ite
         }
       });
     }
-    if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     // q = A p fused with delta = (p, q)
     EpiStoreDot epi{v.q, v.p, 0.0};
     spmv_phase(A, v.p, epi, s_prod, s_red);
     double d = block_sum<NT>(epi.acc, s_red);
     if (tid == 0) s_vals[0] = d;
-    if (!grid_sync<NT>(P, epoch, 1, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 1, s_vals)) return;
     const double delta = s_vals[0];
     if (delta == 0.0) { fail = 2; break; }
     const double alpha = rho / delta;
@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(NT, 1) cg_fused_kernel(OpArgs A, CgVecs v, Ite
     rr = block_sum<NT>(rr, s_red);
     rz = block_sum<NT>(rz, s_red);
     if (tid == 0) { s_vals[0] = rr; s_vals[1] = rz; }
-    if (!grid_sync<NT>(P, epoch, 2, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 2, s_vals)) return;
     rr = s_vals[0];
     rho_1 = rho;
     rho = s_vals[1];
@@ -428,7 +428,7 @@ __global__ void __launch_bounds__(NT, 1) bicgstab_fused_kernel(OpArgs A, BicgVec
     EpiResidual epi{v.b, v.r, nullptr, 0.0, 0.0};
     spmv_phase(A, v.x, epi, s_prod, s_red);
     rr = epi.rr;
-    if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     for (long long i = gt; i < n; i += gs) v.rt[i] = __ldcg(v.r + i);
   }
   if (!grid_sums<NT, 2>(P, epoch, {rr, rr}, s_vals, s_arr)) return;
@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(NT, 1) bicgstab_fused_kernel(OpArgs A, BicgVec
         if (jac) stw<W>(ph, i, precond_w<W>(A.diag, i, pi));
       });
     }
-    if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     // v = A phat, sigma = (rtilde, v)
     EpiStoreDot2 e1{v.v, v.rt, false, 0.0, 0.0};
     spmv_phase(A, ph, e1, s_prod, s_red);
@@ -633,7 +633,7 @@ __global__ void __launch_bounds__(NT, 1) cgs_fused_kernel(OpArgs A, CgsVecs v, I
     EpiResidual epi{v.b, v.r, nullptr, 0.0, 0.0};
     spmv_phase(A, v.x, epi, s_prod, s_red);
     rr = epi.rr;
-    if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     for (long long i = gt; i < n; i += gs) v.rt[i] = __ldcg(v.r + i);
   }
   if (!grid_sums<NT, 1>(P, epoch, {rr}, s_vals, s_arr)) return;
@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(NT, 1) cgs_fused_kernel(OpArgs A, CgsVecs v, I
         if (jac) stw<W>(ph, i, precond_w<W>(A.diag, i, pi));
       });
     }
-    if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     // vhat = A phat fused with delta = (rtilde, vhat)
     EpiStoreDot e1{v.vh, v.rt, 0.0};
     spmv_phase(A, ph, e1, s_prod, s_red);
@@ -707,7 +707,7 @@ __global__ void __launch_bounds__(NT, 1) cgs_fused_kernel(OpArgs A, CgsVecs v, I
         stw<W>(v.x, i, xi);
       }
     });
-    if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     // qhat = A uhat fused with Add(-alpha, qhat, r), ||r||^2 and (rtilde, r)
     EpiResidUpdate e2{v.r, v.rt, -alpha, 0.0, 0.0};
     spmv_phase(A, uh, e2, s_prod, s_red);
@@ -1003,7 +1003,7 @@ __global__ void __launch_bounds__(NT, 1) tfqmr_fused_kernel(OpArgs A, TfqmrVecs 
       }
     });
     if (done || fail) break;
-    if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     // 25.-26. g = M^{-1} A y1; v = beta^2 v + beta h + g; next sigma
     {
       EpiTfqmrNextV epi{A.diag, v.rt, v.h, v.g, v.v, beta, beta * beta, 0.0};
@@ -1096,7 +1096,7 @@ __global__ void __launch_bounds__(NT, 1) minres_fused_kernel(OpArgs A, MinresVec
       stw<W>(v.w_oold, i, zero);
     });
   }
-  if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+  if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
   double c = 1.0, s = 0.0, cold = 1.0, sold = 0.0;
   double np = normb;  // Norm2(b)
   double *u = v.u, *u_old = v.u_old, *vv = v.v, *v_old = v.v_old;
@@ -1215,7 +1215,7 @@ __global__ void __launch_bounds__(NT, 1) minres_fused_kernel(OpArgs A, MinresVec
       vv = v_old;
       v_old = t;
     }
-    if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     np = mul_rn(np, fabs(s));
     nb_iter++;
   }
@@ -1351,7 +1351,7 @@ __global__ void __launch_bounds__(NT, 1) gcr_fused_kernel(OpArgs A, GcrVecs v, I
         for (int k = 0; k < Wd; k++) ri.v[k] = mul_rn(ri.v[k], inv);
         stw<Wd>(v.P, i, ri);
       });
-      if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+      if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     }
     int j = 0;
     for (;;) {
@@ -1408,7 +1408,7 @@ __global__ void __launch_bounds__(NT, 1) gcr_fused_kernel(OpArgs A, GcrVecs v, I
             const double d = block_sum<NT>(epi.acc[k], s_red);
             if (tid == 0) s_vals[k] = d;
           }
-        if (!grid_sync<NT>(P, epoch, nd, s_vals, s_red)) return;
+        if (!grid_sync<NT>(P, epoch, nd, s_vals)) return;
       }
       if (tid < nd) s_delta[tid] = -s_vals[tid] / s_beta[tid];
       __syncthreads();
@@ -1428,7 +1428,7 @@ __global__ void __launch_bounds__(NT, 1) gcr_fused_kernel(OpArgs A, GcrVecs v, I
           }
           stw<Wd>(pn, i, pv);
         });
-        if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+        if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
       }
       nb_iter++;
       j++;
@@ -1563,7 +1563,7 @@ __global__ void __launch_bounds__(NT, 1) bicgstabl_fused_kernel(OpArgs A, BicglV
           if (jac && k == j) stw<W>(v.q, i, precond_w<W>(A.diag, i, u));
         }
       });
-      if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+      if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
       // u_{j+1} = A q; sigma = (u_{j+1}, r0)
       {
         EpiStoreDot epi{Uv(j + 1), v.rt, 0.0};
@@ -1595,7 +1595,7 @@ __global__ void __launch_bounds__(NT, 1) bicgstabl_fused_kernel(OpArgs A, BicglV
           if (jac && k == j) stw<W>(v.q, i, precond_w<W>(A.diag, i, r));
         }
       });
-      if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+      if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
       // r_{j+1} = A q; the next step's rho = (r_{j+1}, r0)
       {
         EpiStoreDot epi{Rv(j + 1), v.rt, 0.0};
@@ -1810,7 +1810,7 @@ __global__ void __launch_bounds__(NT, 1) qcgs_fused_kernel(OpArgs A, QcgsVecs v,
     EpiResidual epi{v.b, v.r, nullptr, 0.0, 0.0};
     spmv_phase(A, v.x, epi, s_prod, s_red);
   }
-  if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+  if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
   // rtilde = r_qcgs = r; x_qcgs = x; q = p = 0; ||r||^2 (= (rtilde, r))
   double rr = 0.0;
   for (long long i = gt; i < n; i += gs) {
@@ -1848,7 +1848,7 @@ __global__ void __launch_bounds__(NT, 1) qcgs_fused_kernel(OpArgs A, QcgsVecs v,
       stw<W>(v.p, i, pi);
       if (jac) stw<W>(ph, i, precond_w<W>(A.diag, i, pi));
     });
-    if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     // v = A phat with sigma = (rtilde, v) and (v, v)
     {
       EpiStoreDot2 epi{v.v, v.rt, true, 0.0, 0.0};
@@ -1882,7 +1882,7 @@ __global__ void __launch_bounds__(NT, 1) qcgs_fused_kernel(OpArgs A, QcgsVecs v,
       }
       if (jac) stw<W>(v.ph, i, precond_w<W>(A.diag, i, ui));
     });
-    if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     // u = A phat; Add(-alpha, u, r); u = r_qcgs - r; the four projections
     {
       EpiQcgsFit epi{v.r, v.uf, v.rq, v.v, -alpha, 0.0, 0.0, 0.0, 0.0};
@@ -2011,7 +2011,7 @@ __global__ void __launch_bounds__(NT, 1) bicg_fused_kernel(OpArgs A, BcgVecs v, 
     EpiResidual epi{v.b, v.r, nullptr, 0.0, 0.0};
     spmv_phase(A, v.x, epi, s_prod, s_red);
   }
-  if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+  if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
   // r~ = r; ||r||^2 and rho = (M^{-1} r, r~)
   double rr = 0.0, rz = 0.0;
   for (long long i = gt; i < n; i += gs) {
@@ -2053,7 +2053,7 @@ __global__ void __launch_bounds__(NT, 1) bicg_fused_kernel(OpArgs A, BcgVecs v, 
           stw<W>(v.pt, i, pti);
         }
       });
-      if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+      if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     }
     // q = A p with delta = (p~, q); q~ = A^T p~
     {
@@ -2184,7 +2184,7 @@ __global__ void __launch_bounds__(NT, 1) cgne_fused_kernel(OpArgs A, CgneVecs v,
   } else {
     EpiStore e1{v.p};
     spmv_phase(A, v.x, e1, s_prod, s_red);
-    if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     EpiCgneInit e2{v.r, v.q, A.diag, 0.0};
     spmv_phase(v.AT, v.p, e2, s_prod, s_red);
     rz = e2.rz;
@@ -2216,13 +2216,13 @@ __global__ void __launch_bounds__(NT, 1) cgne_fused_kernel(OpArgs A, CgneVecs v,
           stw<W>(v.p, i, pi);
         }
       });
-      if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+      if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     }
     // q = A p
     {
       EpiStore e{v.q};
       spmv_phase(A, v.p, e, s_prod, s_red);
-      if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+      if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     }
     // z = A^T q with delta = (p, z)
     {
@@ -2316,7 +2316,7 @@ __global__ void __launch_bounds__(NT, 1) symmlq_fused_kernel(OpArgs A, SymmlqVec
     EpiResidual epi{v.b, v.r, nullptr, 0.0, 0.0};
     spmv_phase(A, v.x, epi, s_prod, s_red);
   }
-  if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+  if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
   // z = M^{-1} r; dp = (r, z)
   {
     double a0 = 0.0;
@@ -2343,7 +2343,7 @@ __global__ void __launch_bounds__(NT, 1) symmlq_fused_kernel(OpArgs A, SymmlqVec
       u_old[i] = 0.0;
       v_old[i] = 0.0;
     }
-    if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
   }
   double ceta = 0.0, ceta_old = 0.0, ceta_oold = 0.0;
   double c = 1.0, cold = 1.0, s = 0.0, sold = 0.0;
@@ -2385,7 +2385,7 @@ __global__ void __launch_bounds__(NT, 1) symmlq_fused_kernel(OpArgs A, SymmlqVec
           stw<W>(v.x, i, xi);
         }
       });
-      if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+      if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
       ceta_oold = ceta_old;
       ceta_old = ceta;
     }
@@ -2510,7 +2510,7 @@ __global__ void __launch_bounds__(NT, 1) qmrsym_fused_kernel(OpArgs A, QmrsVecs 
     EpiResidual epi{v.b, v.r, nullptr, 0.0, 0.0};
     spmv_phase(A, v.x, epi, s_prod, s_red);
   }
-  if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+  if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
   // v = r; y = M^{-1} v; rho = ||y||; ||r||^2
   double rr, rho;
   {
@@ -2567,7 +2567,7 @@ __global__ void __launch_bounds__(NT, 1) qmrsym_fused_kernel(OpArgs A, QmrsVecs 
           stw<W>(v.p, i, pi);
         }
       });
-      if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+      if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     }
     // pt = A p with ep = (p, pt)
     {
@@ -2725,7 +2725,7 @@ __global__ void __launch_bounds__(NT, 1) lsqr_fused_kernel(OpArgs A, LsqrVecs v,
       v.u[i] = mul_rn(__ldg(v.b + i), tb);
       v.x[i] = 0.0;
     }
-    if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
   }
   // v = A^T u, alpha = ||v||; v /= alpha; w = v
   double alpha;
@@ -2740,7 +2740,7 @@ __global__ void __launch_bounds__(NT, 1) lsqr_fused_kernel(OpArgs A, LsqrVecs v,
       v.v[i] = vi;
       v.w[i] = vi;
     }
-    if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
   }
   double phi_bar = normb, rho_bar = alpha;
   double *u = v.u, *u1 = v.u1, *vv = v.v, *v1 = v.v1;
@@ -2769,7 +2769,7 @@ __global__ void __launch_bounds__(NT, 1) lsqr_fused_kernel(OpArgs A, LsqrVecs v,
         for (int j = 0; j < W; j++) ui.v[j] = mul_rn(ui.v[j], tb);
         stw<W>(u1, i, ui);
       });
-      if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+      if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     }
     // v1 = A^T u1; Add(-beta, v, v1); alpha = ||v1||
     {
@@ -2805,7 +2805,7 @@ __global__ void __launch_bounds__(NT, 1) lsqr_fused_kernel(OpArgs A, LsqrVecs v,
         for (int j = 0; j < W; j++) wi.v[j] = add_rn(mul_rn(wi.v[j], tw), vi.v[j]);
         stw<W>(v.w, i, wi);
       });
-      if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+      if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     }
     rnorm = fabs(phi_bar);
     double* t = u1; u1 = u; u = t;
@@ -2877,14 +2877,14 @@ __global__ void __launch_bounds__(NT, 1) bicgcr_fused_kernel(OpArgs A, BcrVecs v
     EpiResidual epi{v.b, v.v, nullptr, 0.0, 0.0};
     spmv_phase(A, v.x, epi, s_prod, s_red);
   }
-  if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+  if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
   // s = M^{-1} v; p = s
   for (long long i = gt; i < n; i += gs) {
     const double si = precond_val(A.diag, (int)i, __ldcg(v.v + i));
     v.s[i] = si;
     v.p[i] = si;
   }
-  if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+  if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
   // a = A p; w = M^{-1} a; ++iter
   double vv, wv, wa;
   {
@@ -2920,7 +2920,7 @@ __global__ void __launch_bounds__(NT, 1) bicgcr_fused_kernel(OpArgs A, BcrVecs v
         stw<W>(v.s, i, si);
       });
     }
-    if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     // z = A s with tau = (w, z)
     {
       EpiStoreDot e{v.z, v.w, 0.0};
@@ -3033,7 +3033,7 @@ __global__ void __launch_bounds__(NT, 1) gmres_fused_kernel(OpArgs A, GmresVecs 
   } else {
     EpiResidual epi{v.b, v.w, nullptr, 0.0, 0.0};
     spmv_phase(A, v.x, epi, s_prod, s_red);
-    if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     for (long long i = gt; i < n; i += gs) {
       const double ri = precond_val(A.diag, (int)i, __ldcg(v.w + i));
       v.r[i] = ri;
@@ -3065,7 +3065,7 @@ __global__ void __launch_bounds__(NT, 1) gmres_fused_kernel(OpArgs A, GmresVecs 
     }
     const int inner_max = nb_iter + m;
     int i = 0;
-    if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     for (;;) {
       double* Vi = v.V + (size_t)i * nn;
       // u = A V_i; w = M^{-1} u; h_{0,i} = (V_0, w)
@@ -3125,7 +3125,7 @@ __global__ void __launch_bounds__(NT, 1) gmres_fused_kernel(OpArgs A, GmresVecs 
       if (lead) hist_push(H, &hlen, nb_iter, rin);
       reste = rin;
       const bool stop = (rin < it.tol) || (nb_iter >= inner_max);
-      if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;  // V_{i} complete
+      if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;  // V_{i} complete
       if (stop) break;
     }
     // Solve(H, s): netlib DTRSV column sweep on the leading i x i block
@@ -3145,11 +3145,11 @@ __global__ void __launch_bounds__(NT, 1) gmres_fused_kernel(OpArgs A, GmresVecs 
         if (sv[k] != 0.0) xe = add_rn(xe, mul_rn(sv[k], __ldcg(v.V + (size_t)k * nn + e)));
       v.x[e] = xe;
     }
-    if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     // w = b - A x; r = M^{-1} w; beta = ||r||
     EpiResidual epi{v.b, v.w, nullptr, 0.0, 0.0};
     spmv_phase(A, v.x, epi, s_prod, s_red);
-    if (!grid_sync<NT>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NT>(P, epoch, 0, s_vals)) return;
     rr = 0.0;
     for (long long e = gt; e < n; e += gs) {
       const double re = precond_val(A.diag, (int)e, __ldcg(v.w + e));
@@ -3412,8 +3412,7 @@ static int fused_solve(int which, const sb2_csr* A, const double* diag, double* 
 // ----------------------------------------------------------------- vectors on chip
 
 // 512 threads with the matrix on chip, where a phase is short and its barriers
-// matter; 1024 where the matrix streams and more loads in flight do.  (Two
-// quads a thread of 512 are more rows than fit with their part of the matrix.)
+// matter; 1024 where the matrix streams and more loads in flight do.
 static const void* gmres_resident(bool ms, int quads, int* threads) {
   *threads = ms ? 512 : 1024;
   const int qr = (quads + *threads - 1) / *threads;

@@ -182,8 +182,7 @@ __device__ __forceinline__ bool grid_wait(const Persist& P, unsigned epoch, int 
 }
 
 template <int NT>
-__device__ __forceinline__ bool grid_sync(const Persist& P, unsigned& epoch, int K,
-                                          double* s_vals, double*) {
+__device__ __forceinline__ bool grid_sync(const Persist& P, unsigned& epoch, int K, double* s_vals) {
   grid_arrive<NT>(P, epoch, K, s_vals);
   return grid_wait<NT>(P, epoch, K, s_vals, true);
 }

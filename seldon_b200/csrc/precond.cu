@@ -72,6 +72,15 @@ static void tri_levels(int n, const int* ptr, const int* ind, bool lower,
   }
 }
 
+// Levels of the mirrored entries of symmetric storage (row j, stored columns
+// >= j): row c depends on each j < c that stores column c.
+static void mirrored_levels(int n, const int* ptr, const int* ind, std::vector<int>& level) {
+  level.assign(n, 0);
+  for (int j = 0; j < n; j++)
+    for (int k = ptr[j]; k < ptr[j + 1]; k++)
+      if (ind[k] > j) level[ind[k]] = std::max(level[ind[k]], level[j] + 1);
+}
+
 // ------------------------------------------------------------------ row ops
 
 #ifdef __CUDACC__
@@ -191,7 +200,6 @@ struct sb2_precond {
   double* d_tmp = nullptr;    // SOR, several launches: their other target
   double* d_sdiag = nullptr;  // SOR, symmetric storage: diagonal of each stored row
   std::mutex mu;
-  bool planned = false;
   // ILUT: order, storage, permutations (and the inverse of the row one),
   // 1/U(i,i) or 1/D(i), and the sweeps (unsymmetric: L forward, U backward,
   // U^T forward, L^T backward; symmetric: L forward through the transposed
@@ -206,60 +214,65 @@ struct sb2_precond {
 
 namespace sb2 {
 
-static int plan_sor(sb2_precond* M) {
+static int place_rows(const SweepGrid& G, const SweepPlan& P, int4* span, const int* ptr, const int* uptr) {
+  if (G.n == 0) return SB2_OK;
+  sweep_place_kernel<<<std::min((G.n + 255) / 256, 1184), 256>>>(G.n, P.d_rows, P.d_pos, span, ptr, uptr);
+  SB2_CUDA_TRY(cudaGetLastError());
+  return SB2_OK;
+}
+
+// Plans the sweeps not planned yet of those asked for.
+static int plan_sor(sb2_precond* M, bool fwd, bool bwd) {
   std::lock_guard<std::mutex> g(M->mu);
-  if (M->planned) return SB2_OK;
+  fwd = fwd && !M->fwd.d_buf;
+  bwd = bwd && !M->bwd.d_buf;
+  if (!fwd && !bwd) return SB2_OK;
   const sb2_csr* A = M->A;
   const int n = A->m;
-  const CsrArrays& f = A->full;
-  std::vector<int> ptr(n + 1), ind(f.nnz), uptr, uind;
-  SB2_CUDA_TRY(cudaMemcpy(ptr.data(), f.d_ptr, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost));
-  if (f.nnz) SB2_CUDA_TRY(cudaMemcpy(ind.data(), f.d_ind, sizeof(int) * f.nnz, cudaMemcpyDeviceToHost));
-  if (A->sym) {
-    const CsrArrays& u = A->upper;
-    uptr.resize(n + 1);
-    uind.resize(u.nnz);
-    SB2_CUDA_TRY(cudaMemcpy(uptr.data(), u.d_ptr, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost));
-    if (u.nnz) SB2_CUDA_TRY(cudaMemcpy(uind.data(), u.d_ind, sizeof(int) * u.nnz, cudaMemcpyDeviceToHost));
-  }
-  SB2_TRY(make_sweep_grid(n, &M->grid));
-  auto span = [&](int, int j) {
-    if (!A->sym) return make_int4(ptr[j], ptr[j + 1], 0, 0);
-    // the mirrored entries come first in the expanded row
-    const int stored = uptr[j + 1] - uptr[j];
-    return make_int4(uptr[j], uptr[j + 1], ptr[j], ptr[j + 1] - stored);
-  };
-  std::vector<int> level, order, pos;
-  tri_levels(n, ptr.data(), ind.data(), true, level);
-  SB2_TRY(make_sweep_plan(M->grid, level, &M->fwd, order, pos, span));
-  if (A->sym) tri_levels(n, uptr.data(), uind.data(), false, level);
-  else tri_levels(n, ptr.data(), ind.data(), false, level);
-  SB2_TRY(make_sweep_plan(M->grid, level, &M->bwd, order, pos, span));
-  if (A->sym) {
+  const CsrArrays &f = A->full, &src = A->sym ? A->upper : A->full;
+  std::vector<int> ptr(n + 1), ind(std::max<long long>(src.nnz, 1));
+  SB2_CUDA_TRY(cudaMemcpy(ptr.data(), src.d_ptr, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost));
+  if (src.nnz) SB2_CUDA_TRY(cudaMemcpy(ind.data(), src.d_ind, sizeof(int) * src.nnz, cudaMemcpyDeviceToHost));
+  if (!M->grid.d_state) SB2_TRY(make_sweep_grid(n, &M->grid));
+  if (A->sym && !M->d_sdiag) {
     // values of symmetric storage never change (sb2_csr_set_values)
-    const CsrArrays& u = A->upper;
     SB2_CUDA_TRY(cudaMalloc(&M->d_sdiag, sizeof(double) * std::max(n, 1)));
-    if (n > 0) {
-      sym_diag_kernel<<<std::min((n + 255) / 256, 1184), 256>>>(n, u.d_ptr, u.d_ind, u.d_val, M->d_sdiag);
-      SB2_CUDA_TRY(cudaGetLastError());
-      SB2_CUDA_TRY(cudaDeviceSynchronize());
-    }
+    if (n > 0)
+      sym_diag_kernel<<<std::min((n + 255) / 256, 1184), 256>>>(n, src.d_ptr, src.d_ind, src.d_val, M->d_sdiag);
+    SB2_CUDA_TRY(cudaGetLastError());
   }
-  M->planned = true;
-  return SB2_OK;
+  std::vector<int> level;
+  SweepOrder order;
+  SweepPlan made[2];
+  int st = SB2_OK;
+  for (int k = 0; k < 2 && st == SB2_OK; k++) {
+    if (!(k ? bwd : fwd)) continue;
+    if (k == 0 && A->sym) mirrored_levels(n, ptr.data(), ind.data(), level);
+    else tri_levels(n, ptr.data(), ind.data(), k == 0, level);
+    make_sweep_order(M->grid, level, &order);
+    st = upload_sweep_plan(M->grid, order, nullptr, &made[k]);
+    if (st == SB2_OK) st = place_rows(M->grid, made[k], made[k].d_span, f.d_ptr, A->sym ? src.d_ptr : nullptr);
+  }
+  // complete before any stream reads it
+  if (st == SB2_OK) st = map_cuda_error(cudaStreamSynchronize(nullptr));
+  for (int k = 0; k < 2; k++) {
+    if (st != SB2_OK) made[k].release();
+    else if (made[k].d_buf) (k ? M->bwd : M->fwd) = made[k];
+  }
+  return st;
 }
 
 // SOR(A, X, B, omega, iter, type_ssor) on the device: the sweeps from x0
 // (null: zero) into x, two a launch.  x0 is null or x itself.
 static int sor_apply(sb2_precond* M, const double* x0, double* x, const double* b, double omega,
                      int iter, int type_ssor, int late, cudaStream_t s) {
-  SB2_TRY(plan_sor(M));
+  const int nf = type_ssor % 2 == 0 ? std::max(iter, 0) : 0;
+  const int total = nf + (type_ssor % 3 == 0 ? std::max(iter, 0) : 0);
+  SB2_TRY(plan_sor(M, nf > 0, total > nf));
   const sb2_csr* A = M->A;
   const int n = A->m;
   if (!A->sym) SB2_TRY(ensure_diag(A));
   const SweepGrid& G = M->grid;
-  const int nf = type_ssor % 2 == 0 ? std::max(iter, 0) : 0;
-  const int total = nf + (type_ssor % 3 == 0 ? std::max(iter, 0) : 0);
   const int launches = (total + 1) / 2;
   // targets alternate between x and a work vector, so that none is the
   // vector its launch starts from; from zero the last one is x
@@ -309,19 +322,25 @@ static void gather_levels(int n, const std::vector<int>& ptr, const std::vector<
 static int upload_sweep(const SweepGrid& G, const std::vector<int>& ptr,
                         const std::vector<int>& ind, const std::vector<double>& val,
                         bool ascending, GatherSweep* S) {
-  std::vector<int> level, order, pos;
+  std::vector<int> level, pos(std::max(G.n, 1));
   gather_levels(G.n, ptr, ind, ascending, level);
+  SweepOrder order;
+  make_sweep_order(G, level, &order);
+  for (int i = 0; i < G.n; i++) pos[order.rows[i]] = i;
   // the lists in the order the rows are taken, columns as positions
   std::vector<int> pind;
   std::vector<double> pval;
+  std::vector<int4> span(std::max(G.n, 1));
   pind.reserve(ind.size());
   pval.reserve(val.size());
-  SB2_TRY(make_sweep_plan(G, level, &S->plan, order, pos, [&](int, int j) {
-    const int k0 = (int)pind.size();
+  for (int i = 0; i < G.n; i++) {
+    const int j = order.rows[i], k0 = (int)pind.size();
     for (int k = ptr[j]; k < ptr[j + 1]; k++) pind.push_back(pos[ind[k]]);
     pval.insert(pval.end(), val.begin() + ptr[j], val.begin() + ptr[j + 1]);
-    return make_int4(k0, (int)pind.size(), 0, 0);
-  }));
+    span[i] = make_int4(k0, (int)pind.size(), 0, 0);
+  }
+  SB2_TRY(upload_sweep_plan(G, order, span.data(), &S->plan));
+  SB2_TRY(place_rows(G, S->plan, nullptr, nullptr, nullptr));
   const size_t nz = pind.size();
   SB2_CUDA_TRY(cudaMalloc(&S->d_ind, sizeof(int) * std::max<size_t>(nz, 1)));
   SB2_CUDA_TRY(cudaMalloc(&S->d_val, sizeof(double) * std::max<size_t>(nz, 1)));
@@ -335,24 +354,27 @@ static int upload_sweep(const SweepGrid& G, const std::vector<int>& ptr,
 // Update lists of a column scatter: entry (i -> c, v) for the rows i in the
 // order the sequential loop visits them, each row's entries in stored order.
 struct ListBuilder {
-  std::vector<std::vector<int>> src;
-  std::vector<std::vector<double>> v;
-  explicit ListBuilder(int n) : src(n), v(n) {}
+  int n;
+  std::vector<int> to, from;
+  std::vector<double> v;
+  explicit ListBuilder(int order) : n(order) {}
   void add(int target, int source, double value) {
-    src[target].push_back(source);
-    v[target].push_back(value);
+    to.push_back(target);
+    from.push_back(source);
+    v.push_back(value);
   }
+  // the lists one after the other, each in the order of its entries' arrival
   void flatten(std::vector<int>& ptr, std::vector<int>& ind, std::vector<double>& val) const {
-    const int n = (int)src.size();
     ptr.assign(n + 1, 0);
-    for (int j = 0; j < n; j++) ptr[j + 1] = ptr[j] + (int)src[j].size();
-    ind.clear();
-    val.clear();
-    ind.reserve(ptr[n]);
-    val.reserve(ptr[n]);
-    for (int j = 0; j < n; j++) {
-      ind.insert(ind.end(), src[j].begin(), src[j].end());
-      val.insert(val.end(), v[j].begin(), v[j].end());
+    for (int j : to) ptr[j + 1]++;
+    for (int j = 0; j < n; j++) ptr[j + 1] += ptr[j];
+    ind.resize(to.size());
+    val.resize(to.size());
+    std::vector<int> at(ptr.begin(), ptr.end() - 1);
+    for (size_t e = 0; e < to.size(); e++) {
+      const int q = at[to[e]]++;
+      ind[q] = from[e];
+      val[q] = v[e];
     }
   }
 };
@@ -443,6 +465,7 @@ static int plan_ilut(sb2_precond* M, int n, const int* fp, const int* fi, const 
     SB2_CUDA_TRY(cudaMalloc(&M->d_pcol, sizeof(int) * std::max(n, 1)));
     SB2_CUDA_TRY(cudaMemcpy(M->d_pcol, pcol, sizeof(int) * n, cudaMemcpyHostToDevice));
   }
+  SB2_CUDA_TRY(cudaStreamSynchronize(nullptr));  // complete before any stream reads it
   return SB2_OK;
 }
 

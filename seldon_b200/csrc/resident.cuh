@@ -68,7 +68,6 @@ struct ResVec {
   double* p;
   int NQ;
   __device__ __forceinline__ double& at(int q, int j) const { return p[j * NQ + q]; }
-  __device__ __forceinline__ double row(int i) const { return p[(i & 3) * NQ + (i >> 2)]; }
   __device__ __forceinline__ void get(int q, double (&v)[4]) const {
 #pragma unroll
     for (int j = 0; j < 4; j++) v[j] = p[j * NQ + q];
@@ -280,7 +279,7 @@ __device__ __noinline__ void res_product(const ResOp& A, int s0, int s1, const i
   double* mval = nullptr;                              \
   const bool lead = (blockIdx.x == 0 && tid == 0);     \
   const bool jac = A.diag != nullptr;                  \
-  constexpr std::integral_constant<int, NTR == 512 ? (MS ? 4 : 3) : (MS ? 2 : 1)> kRound; \
+  constexpr std::integral_constant<int, MS ? 4 : 1> kRound; \
   unsigned epoch = 0;                                  \
   int hlen = 0;                                        \
   /* fence: another CTA's vector is read before the next barrier */ \
@@ -554,7 +553,7 @@ __global__ void __launch_bounds__(NTR, 1) bicgstab_resident_kernel(ResOp A, Bicg
       if (jac) phs.set(q, pv);
       vst4(v.ph + row, pv);
     });
-    if (!grid_sync<NTR>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NTR>(P, epoch, 0, s_vals)) return;
     // v = A phat, sigma = (rtilde, v)
     product(kRound, ResGather{phs.p, C.NQ, v.ph, C.r0, C.rows}, vs);
     double d = 0.0;
@@ -778,7 +777,7 @@ __global__ void __launch_bounds__(NTR, 1) gmres_resident_kernel(ResOp A, GmresRe
     }
     const int inner_max = nb_iter + m;
     int i = 0;
-    if (!grid_sync<NTR>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NTR>(P, epoch, 0, s_vals)) return;
     for (;;) {
       // w = M^{-1} A V_i
       product(kRound, ResGather{us.p, C.NQ, v.V + (size_t)i * v.ld, C.r0, C.rows}, ws, A.diag);
@@ -912,7 +911,7 @@ __global__ void __launch_bounds__(NTR, 1) gmres_resident_kernel(ResOp A, GmresRe
         }
       res_store(v.x, row, A.n, xv);
     });
-    if (!grid_sync<NTR>(P, epoch, 0, s_vals, s_red)) return;
+    if (!grid_sync<NTR>(P, epoch, 0, s_vals)) return;
     // w = b - A x; r = M^{-1} w; beta = ||r||
     rr = 0.0;
     product(kRound, ResGatherAll{v.x}, ws);

@@ -56,42 +56,33 @@ constexpr int kStLeave = 0, kStLateSolve = 1, kStLateApply = 2, kStProgress = 3;
 // was copied from the caller with these very bits is stored as the quiet NaN.
 constexpr unsigned long long kSweepFill = 0x7ff4b2005e1d0001ull;
 
-// The rows of one sweep in the order they are taken.
+// The rows of one sweep in the order they are taken (one allocation).
 struct SweepPlan {
-  int* d_rows = nullptr;      // [n] row of each position
+  void* d_buf = nullptr;
   int4* d_span = nullptr;     // [n] entry ranges of each position's row
   int4* d_item = nullptr;     // [items] first position, rows, step, arrivals (below)
+  int* d_rows = nullptr;      // [n] row of each position
+  int* d_pos = nullptr;       // [n] position of each row
   int* d_cta_item = nullptr;  // [ctas + 1] first item of each CTA
   int* d_steps = nullptr;     // [ctas] steps of each CTA
-  int* d_pos = nullptr;       // [n] position of each row
   void release() {
-    cudaFree(d_rows);
-    cudaFree(d_span);
-    cudaFree(d_item);
-    cudaFree(d_cta_item);
-    cudaFree(d_steps);
-    cudaFree(d_pos);
-    d_rows = d_cta_item = d_steps = d_pos = nullptr;
-    d_span = nullptr;
-    d_item = nullptr;
+    cudaFree(d_buf);
+    *this = SweepPlan();
   }
 };
 
 // The row blocks shared by all sweeps of one preconditioner, and the vectors
-// the sweeps write.
+// the sweeps write (one allocation).
 struct SweepGrid {
   int n = 0, ctas = 0, max_rows = 0;
   std::vector<int> h_blk;     // [ctas + 1] first row of each block
-  int* d_blk = nullptr;
   double* d_new[2] = {nullptr, nullptr};
+  int* d_blk = nullptr;
   unsigned* d_state = nullptr;  // [kStProgress + kSweepMaxCtas]
   void release() {
-    cudaFree(d_blk);
     cudaFree(d_new[0]);
-    cudaFree(d_new[1]);
-    cudaFree(d_state);
-    d_blk = nullptr;
     d_new[0] = d_new[1] = nullptr;
+    d_blk = nullptr;
     d_state = nullptr;
   }
 };
@@ -134,67 +125,85 @@ inline int make_sweep_grid(int n, SweepGrid* G) {
   G->max_rows = per;
   G->h_blk.resize(G->ctas + 1);
   for (int c = 0; c <= G->ctas; c++) G->h_blk[c] = (int)std::min<long long>((long long)c * per, n);
-  SB2_CUDA_TRY(cudaMalloc(&G->d_blk, sizeof(int) * (G->ctas + 1)));
-  SB2_CUDA_TRY(cudaMemcpy(G->d_blk, G->h_blk.data(), sizeof(int) * (G->ctas + 1), cudaMemcpyHostToDevice));
-  for (int k = 0; k < 2; k++) SB2_CUDA_TRY(cudaMalloc(&G->d_new[k], sizeof(double) * std::max(n, 1)));
-  SB2_CUDA_TRY(cudaMalloc(&G->d_state, sizeof(unsigned) * (kStProgress + kSweepMaxCtas)));
-  SB2_CUDA_TRY(cudaMemset(G->d_state, 0, sizeof(unsigned) * (kStProgress + kSweepMaxCtas)));
+  // d_new, then d_blk and d_state
+  const size_t len = std::max(n, 1), words = G->ctas + 1 + kStProgress + kSweepMaxCtas;
+  SB2_CUDA_TRY(cudaMalloc(&G->d_new[0], 2 * sizeof(double) * len + sizeof(int) * words));
+  G->d_new[1] = G->d_new[0] + len;
+  G->d_blk = reinterpret_cast<int*>(G->d_new[1] + len);
+  G->d_state = reinterpret_cast<unsigned*>(G->d_blk + G->ctas + 1);
+  std::vector<int> head(words, 0);
+  std::copy(G->h_blk.begin(), G->h_blk.end(), head.begin());
+  SB2_CUDA_TRY(cudaMemcpy(G->d_blk, head.data(), sizeof(int) * words, cudaMemcpyHostToDevice));
   return SB2_OK;
 }
 
-// Positions, items and spans of one sweep from the rows' levels.  span(i, j)
-// gives the entry ranges of row j at position i, once `order` (the row of each
-// position) and `pos` (the position of each row) are complete.
-template <class Span>
-int make_sweep_plan(const SweepGrid& G, const std::vector<int>& level, SweepPlan* P,
-                    std::vector<int>& order, std::vector<int>& pos, const Span& span) {
-  const int n = G.n;
-  int nlev = 0;
-  for (int i = 0; i < n; i++) nlev = std::max(nlev, level[i] + 1);
-  std::vector<int> first(nlev + 1, 0), by_level(std::max(n, 1));
-  for (int i = 0; i < n; i++) first[level[i] + 1]++;
-  for (int l = 0; l < nlev; l++) first[l + 1] += first[l];
-  for (int i = 0; i < n; i++) by_level[first[level[i]]++] = i;
-  // dealt to the blocks in level order
-  const int per = std::max(1, G.max_rows);
-  std::vector<int> at(G.h_blk.begin(), G.h_blk.end());
-  order.assign(std::max(n, 1), 0);
-  for (int q = 0; q < n; q++) order[at[by_level[q] / per]++] = by_level[q];
-  pos.assign(std::max(n, 1), 0);
-  for (int i = 0; i < n; i++) pos[order[i]] = i;
+// The order of one sweep on the host.
+struct SweepOrder {
+  std::vector<int> rows, cta_item, steps;
   std::vector<int4> item;
-  std::vector<int> cta_item(G.ctas + 1, 0), steps(G.ctas, 0);
-  std::vector<int4> sp(std::max(n, 1));
+};
+
+// Each block's rows by level (increasing row in a level) and the items they
+// make.  A call of SOR plans on the way, so that the passes stay within a block:
+// 885,000 rows take 3 ms (11 with one sort over all rows).
+inline void make_sweep_order(const SweepGrid& G, const std::vector<int>& level, SweepOrder* O) {
+  const int n = G.n;
+  O->rows.resize(std::max(n, 1));
+  O->cta_item.assign(G.ctas + 1, 0);
+  O->steps.assign(G.ctas, 0);
+  O->item.clear();
+  std::vector<int> at;
   for (int c = 0; c < G.ctas; c++) {
-    cta_item[c] = (int)item.size();
-    for (int i = G.h_blk[c]; i < G.h_blk[c + 1];) {
+    const int r0 = G.h_blk[c], r1 = G.h_blk[c + 1];
+    O->cta_item[c] = (int)O->item.size();
+    if (r0 == r1) continue;
+    int* rows = O->rows.data();
+    const auto range = std::minmax_element(level.begin() + r0, level.begin() + r1);
+    const int lo = *range.first;
+    const long long span = (long long)*range.second - lo + 1;
+    if (span <= 4LL * (r1 - r0)) {
+      at.assign(span + 1, 0);
+      for (int i = r0; i < r1; i++) at[level[i] - lo + 1]++;
+      for (long long l = 0; l < span; l++) at[l + 1] += at[l];
+      for (int i = r0; i < r1; i++) rows[r0 + at[level[i] - lo]++] = i;
+    } else {
+      for (int i = r0; i < r1; i++) rows[i] = i;
+      std::stable_sort(rows + r0, rows + r1, [&](int a, int b) { return level[a] < level[b]; });
+    }
+    for (int i = r0; i < r1;) {
       // a step: up to kSweepStep items of one level; its last item makes up
       // the barrier's count
-      const int lev = level[order[i]];
+      const int lev = level[rows[i]];
       int q = 0;
-      for (; q < kSweepStep && i < G.h_blk[c + 1] && level[order[i]] == lev; q++) {
+      for (; q < kSweepStep && i < r1 && level[rows[i]] == lev; q++) {
         const int s = i;
-        while (i < G.h_blk[c + 1] && i - s < 32 && level[order[i]] == lev) i++;
-        item.push_back(make_int4(s, i - s, steps[c], 1));
+        while (i < r1 && i - s < 32 && level[rows[i]] == lev) i++;
+        O->item.push_back(make_int4(s, i - s, O->steps[c], 1));
       }
-      item.back().w = kSweepStep - (q - 1);
-      steps[c]++;
+      O->item.back().w = kSweepStep - (q - 1);
+      O->steps[c]++;
     }
   }
-  cta_item[G.ctas] = (int)item.size();
-  for (int i = 0; i < n; i++) sp[i] = span(i, order[i]);
-  SB2_CUDA_TRY(cudaMalloc(&P->d_rows, sizeof(int) * std::max(n, 1)));
-  SB2_CUDA_TRY(cudaMalloc(&P->d_span, sizeof(int4) * std::max(n, 1)));
-  SB2_CUDA_TRY(cudaMalloc(&P->d_item, sizeof(int4) * std::max<size_t>(item.size(), 1)));
-  SB2_CUDA_TRY(cudaMalloc(&P->d_cta_item, sizeof(int) * cta_item.size()));
-  SB2_CUDA_TRY(cudaMemcpy(P->d_rows, order.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-  SB2_CUDA_TRY(cudaMemcpy(P->d_span, sp.data(), sizeof(int4) * n, cudaMemcpyHostToDevice));
-  SB2_CUDA_TRY(cudaMemcpy(P->d_item, item.data(), sizeof(int4) * item.size(), cudaMemcpyHostToDevice));
-  SB2_CUDA_TRY(cudaMalloc(&P->d_pos, sizeof(int) * std::max(n, 1)));
-  SB2_CUDA_TRY(cudaMemcpy(P->d_pos, pos.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-  SB2_CUDA_TRY(cudaMalloc(&P->d_steps, sizeof(int) * G.ctas));
-  SB2_CUDA_TRY(cudaMemcpy(P->d_steps, steps.data(), sizeof(int) * G.ctas, cudaMemcpyHostToDevice));
-  SB2_CUDA_TRY(cudaMemcpy(P->d_cta_item, cta_item.data(), sizeof(int) * cta_item.size(), cudaMemcpyHostToDevice));
+  O->cta_item[G.ctas] = (int)O->item.size();
+}
+
+// The order on the device.  d_pos and, without `span`, d_span are for the
+// caller to fill (sweep_place_kernel).
+inline int upload_sweep_plan(const SweepGrid& G, const SweepOrder& O, const int4* span, SweepPlan* P) {
+  const size_t n = std::max(G.n, 1), items = O.item.size(), words = 2 * (size_t)G.ctas + 1;
+  SB2_CUDA_TRY(cudaMalloc(&P->d_buf, sizeof(int4) * (n + items) + sizeof(int) * (2 * n + words)));
+  P->d_span = static_cast<int4*>(P->d_buf);
+  P->d_item = P->d_span + n;
+  P->d_rows = reinterpret_cast<int*>(P->d_item + items);
+  P->d_pos = P->d_rows + n;
+  P->d_cta_item = P->d_pos + n;
+  P->d_steps = P->d_cta_item + G.ctas + 1;
+  std::vector<int> tail(O.cta_item);
+  tail.insert(tail.end(), O.steps.begin(), O.steps.end());
+  if (span) SB2_CUDA_TRY(cudaMemcpy(P->d_span, span, sizeof(int4) * G.n, cudaMemcpyHostToDevice));
+  SB2_CUDA_TRY(cudaMemcpy(P->d_item, O.item.data(), sizeof(int4) * items, cudaMemcpyHostToDevice));
+  SB2_CUDA_TRY(cudaMemcpy(P->d_rows, O.rows.data(), sizeof(int) * G.n, cudaMemcpyHostToDevice));
+  SB2_CUDA_TRY(cudaMemcpy(P->d_cta_item, tail.data(), sizeof(int) * words, cudaMemcpyHostToDevice));
   return SB2_OK;
 }
 
@@ -757,6 +766,27 @@ __global__ void sym_diag_kernel(int n, const int* __restrict__ ptr, const int* _
     for (int k = ptr[j]; k < ptr[j + 1]; k++)
       if (ind[k] == j) ajj = add_rn(ajj, val[k]);
     d[j] = ajj;
+  }
+}
+
+// Positions of the rows, and with `span` the entry ranges of rows of the pattern
+// `ptr` (with `uptr` of symmetric storage: the stored row, then the mirrored
+// entries, which come first in the expanded one).
+__global__ void __launch_bounds__(256) sweep_place_kernel(int n, const int* __restrict__ rows, int* pos,
+                                                          int4* span, const int* __restrict__ ptr,
+                                                          const int* __restrict__ uptr) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x) {
+    const int j = __ldg(rows + i);
+    pos[j] = (int)i;
+    if (!span) continue;
+    const int a = __ldg(ptr + j), e = __ldg(ptr + j + 1);
+    if (uptr) {
+      const int u = __ldg(uptr + j), ue = __ldg(uptr + j + 1);
+      span[i] = make_int4(u, ue, a, e - (ue - u));
+    } else {
+      span[i] = make_int4(a, e, 0, 0);
+    }
   }
 }
 
