@@ -138,3 +138,25 @@ def test_gmres_where_the_forms_change(api, oracle, n, restart):
     """Up to 8192 rows a CTA and one more, at the restarts where the fused kernel
     hands over."""
     test_resident_vs_oracle(api, oracle, "gmres", "ragged", n, restart, 20, True, False)
+
+
+@pytest.mark.parametrize("which,name,n", [("cg", "lap", 301 * 301), ("bicgstab", "ragged_sym", 19001),
+                                          ("gmres", "ragged_sym", 70001)])
+@pytest.mark.parametrize("jacobi", [False, True])
+def test_resident_symmetric_storage(api, oracle, which, name, n, jacobi):
+    """The expanded rows of symmetric storage, against the oracle's general ones."""
+    import torch
+    ptr, ind, val = _matrix(name, n)
+    b = matgen.matvec(ptr, ind, val, np.random.default_rng(n).uniform(-1, 1, n))
+    A = api.RowSymSparse(n, *matgen.upper(ptr, ind, val))
+    X = torch.zeros(n, dtype=torch.float64, device="cuda")
+    it = api.Iteration(5000, 1e-10)
+    it.SetRestart(20)
+    it.HideMessages()
+    M = api.JacobiPreconditioner() if jacobi else api.Preconditioner_Base()
+    code = {"cg": api.Cg, "bicgstab": api.BiCgStab, "gmres": api.Gmres}[which](A, X, to_dev(b), M, it)
+    xo, co, no, _, _ = oracle.solve(which, ptr, ind, val, b, precond=1 if jacobi else 0, tol=1e-10,
+                                    max_iter=5000, restart=20)
+    assert code == co == 0
+    assert abs(it.GetNumberIteration() - no) <= max(2, no // 20)
+    assert np.linalg.norm(to_host(X) - xo) <= 1e-5 * np.linalg.norm(xo)

@@ -62,7 +62,7 @@ def breaker(cuda):
     import os
     import subprocess
     here = os.path.join(os.path.dirname(os.path.abspath(__file__)), "cuda")
-    subprocess.run(["make", "-C", here], check=True, capture_output=True)
+    subprocess.run(["make", "-C", here, "sweep_wait.so"], check=True, capture_output=True)
     lib = ctypes.CDLL(os.path.join(here, "sweep_wait.so"))
 
     def point(handle, sweep, entry, at):
