@@ -438,12 +438,13 @@ k_emit_segment(const unsigned long long* __restrict__ key, long long b, long lon
 // every bucket is sorted in shared memory and written out.  A tile of keys is
 // grouped by bucket in shared memory before it goes to global memory, then its
 // values through the same shared memory, so that a bucket's part of a tile is
-// written as one run and no access of either pass is a lone 8-byte one.  (With
-// the values gathered by the second pass, a 32-byte sector each, that pass
-// alone took 458 us for 14.6M triplets of 7 a row, against 161 us.)  The form after it scatters one
-// key at a time to its row and gathers one value at a time; it stays for what
-// does not fit here: more than kBktMax buckets, buckets beyond a CTA's shared
-// memory (rows of very uneven length), keys beyond 64 bits.
+// written as one run: two entries on the mean with 4096 buckets, more with
+// fewer.  (With the values gathered by the second pass, a 32-byte sector each,
+// that pass alone took 458 us for 14.6M triplets of 7 a row, against 161 us.)
+// The form after it scatters one key at a time to its row and gathers one value
+// at a time; it stays for what does not fit here: more than kBktMax buckets,
+// buckets beyond a CTA's shared memory (rows of very uneven length), keys beyond
+// 64 bits, scratch beyond the memory there is.
 //   k_bkt_count  entries per bucket
 //   k_bkt_scan   first entry of each bucket; whether one is too large
 //   k_bkt_deal   tiles of keys (row in the bucket, column, input position) and

@@ -19,11 +19,11 @@
 // The arithmetic is the fused kernels' (and so the reference's), operation by
 // operation; only the grouping of the reductions differs.
 //
-// Measured against the fused kernels on the same barrier (us per iteration,
-// 7- or 5-point operators): Cg 512^2 16.4 -> 8.4, 64^3 18.8 -> 10.8;
-// BiCgStab with Jacobi 32^3 17.0 -> 9.0; Gmres(30) with Jacobi 32^3 65.9 ->
-// 49.5, 64^3 74.9 -> 56.7, and with the matrix streamed 96^3 119 -> 91, 128^3
-// 190 -> 174.  Cg and BiCgStab with the matrix streamed gained nothing (80^3
+// Measured in turn with the fused kernels, on the same barrier and with Jacobi (us
+// per iteration, 7- or 5-point operators): Cg 512^2 18.7 -> 10.7, 48^3 16.7 -> 10.8;
+// BiCgStab 32^3 13.8 -> 10.4, 512^2 16.0 -> 11.9; Gmres(30) 32^3 66 -> 52, 64^3 74 ->
+// 60, and with the matrix streamed 96^3 117 -> 93, 112^3 152 -> 139, 128^3 188 ->
+// 183 (short restarts lose there: see resident_solve).  Cg and BiCgStab with the matrix streamed gained nothing (80^3
 // 20.8 -> 21.4, 90^3 32 -> 33): there the product sets the pace, and with the
 // shared memory taken its gathers lose the L1.
 #pragma once
