@@ -17,8 +17,9 @@
 // reference's own operations with separately rounded products, so the result
 // is the reference's bit for bit.
 //
-// Both run as persistent launches whose rows wait for the values they read
-// (sweep.cuh).  Only the device factorization of ILU(0) runs level by level.
+// Both run as persistent launches whose rows wait for the values they read, or
+// level by level where levels are few and wide or rows long (sweep.cuh:
+// SweepForm).  The device factorization of ILU(0) runs level by level.
 #include <algorithm>
 #include <vector>
 
@@ -79,6 +80,32 @@ static void mirrored_levels(int n, const int* ptr, const int* ind, std::vector<i
   for (int j = 0; j < n; j++)
     for (int k = ptr[j]; k < ptr[j + 1]; k++)
       if (ind[k] > j) level[ind[k]] = std::max(level[ind[k]], level[j] + 1);
+}
+
+// Levels of a sweep that works in place: row j comes after the rows whose new
+// value it reads and before the rows that it reads old.
+static void in_place_levels(int n, const int* ptr, const int* ind, bool forward, std::vector<int>& level) {
+  level.assign(n, 0);
+  std::vector<int> least(n, 0);
+  for (int q = 0; q < n; q++) {
+    const int j = forward ? q : n - 1 - q;
+    int lev = least[j];
+    for (int k = ptr[j]; k < ptr[j + 1]; k++) {
+      const int c = ind[k];
+      if (forward ? c < j : c > j) lev = std::max(lev, level[c] + 1);
+    }
+    level[j] = lev;
+    for (int k = ptr[j]; k < ptr[j + 1]; k++) {
+      const int c = ind[k];
+      if (forward ? c > j : c < j) least[c] = std::max(least[c], lev + 1);
+    }
+  }
+}
+
+static int count_levels(const std::vector<int>& level) {
+  int most = 0;
+  for (int l : level) most = std::max(most, l + 1);
+  return std::max(most, 1);
 }
 
 // ------------------------------------------------------------------ row ops
@@ -156,7 +183,7 @@ __global__ void jacobi_kernel(int n, const double* __restrict__ r,
 constexpr int kSingleCtaMaxN = 65536;
 
 template <class Op>
-static int run_levels(const LevelPlan& P, int n, const Op& op, cudaStream_t s) {
+static int run_factor_levels(const LevelPlan& P, int n, const Op& op, cudaStream_t s) {
   if (n == 0 || P.nlev == 0) return SB2_OK;
   if (n <= kSingleCtaMaxN) {
     level_single_cta<Op><<<1, 1024, 0, s>>>(P.nlev, P.d_lvl, P.d_rows, op);
@@ -198,6 +225,7 @@ struct sb2_precond {
   sb2::SweepGrid grid;      // row blocks and work vectors of the sweeps
   sb2::SweepPlan fwd, bwd;  // SOR
   double* d_tmp = nullptr;    // SOR, several launches: their other target
+  int form = -1;              // SweepForm (-1: not planned yet)
   double* d_sdiag = nullptr;  // SOR, symmetric storage: diagonal of each stored row
   std::mutex mu;
   // ILUT: order, storage, permutations (and the inverse of the row one),
@@ -244,14 +272,37 @@ static int plan_sor(sb2_precond* M, bool fwd, bool bwd) {
   std::vector<int> level;
   SweepOrder order;
   SweepPlan made[2];
+  int longest = 0;
+  if (A->sym) {
+    std::vector<int> len(n);  // stored and mirrored entries
+    for (int j = 0; j < n; j++) {
+      len[j] += ptr[j + 1] - ptr[j];
+      for (int k = ptr[j]; k < ptr[j + 1]; k++)
+        if (ind[k] > j) len[ind[k]]++;
+    }
+    for (int l : len) longest = std::max(longest, l);
+  } else {
+    for (int j = 0; j < n; j++) longest = std::max(longest, ptr[j + 1] - ptr[j]);
+  }
   int st = SB2_OK;
   for (int k = 0; k < 2 && st == SB2_OK; k++) {
     if (!(k ? bwd : fwd)) continue;
     if (k == 0 && A->sym) mirrored_levels(n, ptr.data(), ind.data(), level);
     else tri_levels(n, ptr.data(), ind.data(), k == 0, level);
-    make_sweep_order(M->grid, level, &order);
-    st = upload_sweep_plan(M->grid, order, nullptr, &made[k]);
-    if (st == SB2_OK) st = place_rows(M->grid, made[k], made[k].d_span, f.d_ptr, A->sym ? src.d_ptr : nullptr);
+    if (M->form < 0)
+      M->form = sweep_form(n, count_levels(level), (double)f.nnz / std::max(n, 1), A->sym ? 1 : 0);
+    if (M->form == kFormSweep) {
+      make_sweep_order(M->grid, level, &order);
+      st = upload_sweep_plan(M->grid, order, nullptr, &made[k]);
+    } else {
+      if (M->form == kFormInPlace && !A->sym) in_place_levels(n, ptr.data(), ind.data(), k == 0, level);
+      std::vector<int> rows, lvl;
+      make_level_order(n, level, &rows, &lvl);
+      st = upload_level_plan(n, rows, lvl, nullptr, &made[k]);
+    }
+    made[k].max_len = longest;
+    if (st == SB2_OK && M->form == kFormSweep)
+      st = place_rows(M->grid, made[k], made[k].d_span, f.d_ptr, A->sym ? src.d_ptr : nullptr);
   }
   // complete before any stream reads it
   if (st == SB2_OK) st = map_cuda_error(cudaStreamSynchronize(nullptr));
@@ -276,26 +327,58 @@ static int sor_apply(sb2_precond* M, const double* x0, double* x, const double* 
   const int launches = (total + 1) / 2;
   // targets alternate between x and a work vector, so that none is the
   // vector its launch starts from; from zero the last one is x
-  if (launches > (x0 ? 0 : 1) && !M->d_tmp) {
+  if ((M->form == kFormSweep ? launches : M->form == kFormLevels ? total : 2 * (int)A->sym) > (x0 ? 0 : 1) && !M->d_tmp) {
     std::lock_guard<std::mutex> g(M->mu);
     if (!M->d_tmp) SB2_CUDA_TRY(cudaMalloc(&M->d_tmp, sizeof(double) * std::max(n, 1)));
   }
   const double* cur = x0;
-  for (int l = 0, done = 0; l < launches; l++, done += 2) {
+  const CsrArrays &u = A->upper, &f = A->full;
+  const double rest = 1.0 - omega, ratio = rest / omega;
+  if (M->form == kFormLevels) {
+    // the same, a sweep at a time
+    const LevelSpan span{nullptr, f.d_ptr, A->sym ? u.d_ptr : nullptr};
+    for (int q = 0; q < total; q++) {
+      const bool fwd = q < nf;
+      double* out = (x0 ? q % 2 == 1 : (total - 1 - q) % 2 == 0) ? x : M->d_tmp;
+      const SweepPlan& P = fwd ? M->fwd : M->bwd;
+      if (A->sym)
+        SB2_TRY(run_levels(P, n, 0, fwd, span, cur, out,
+                           SymmetricSor{u.d_ind, u.d_val, f.d_ind, f.d_val, M->d_sdiag, b, cur, omega, ratio}, s));
+      else
+        SB2_TRY(run_levels(P, n, 0, fwd, span, cur, out,
+                           GeneralSor{f.d_ind, f.d_val, A->d_diag, b, cur, omega, rest}, s));
+      cur = out;
+    }
+  } else if (M->form == kFormInPlace) {
+    if (!x0) SB2_CUDA_TRY(cudaMemsetAsync(x, 0, sizeof(double) * n, s));
+    for (int q = 0; q < total; q++) {
+      const bool fwd = q < nf;
+      const SweepPlan& P = fwd ? M->fwd : M->bwd;
+      if (A->sym) {
+        InPlaceSymmetricSor op{u.d_ptr, u.d_ind, u.d_val, f.d_ptr, f.d_ind, f.d_val, M->d_sdiag,
+                           b, x, M->d_tmp, omega, ratio, fwd, true};
+        all_rows_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, op);
+        SB2_CUDA_TRY(cudaGetLastError());
+        op.start = false;
+        SB2_TRY(run_in_place(P, n, op, s));
+      } else {
+        SB2_TRY(run_in_place(P, n, InPlaceSor{f.d_ptr, f.d_ind, f.d_val, A->d_diag, b, x, omega, rest}, s));
+      }
+    }
+    cur = x;
+  }
+  for (int l = 0, done = 0; l < launches && M->form == kFormSweep; l++, done += 2) {
     const int sweeps = done + 1 < total ? 2 : 1;
     const bool fwd[2] = {done < nf, done + 1 < nf};
     const SweepPlan* const plan[2] = {fwd[0] ? &M->fwd : &M->bwd, fwd[1] ? &M->fwd : &M->bwd};
     const bool into_x = x0 ? l % 2 == 1 : (launches - 1 - l) % 2 == 0;
     double* last = into_x ? x : M->d_tmp;
     if (A->sym) {
-      const CsrArrays &u = A->upper, &f = A->full;
       SB2_TRY(launch_sweeps(G, sweeps, plan, fwd, last,
-                            SymmetricSor{u.d_ind, u.d_val, f.d_ind, f.d_val, M->d_sdiag, b, cur, omega,
-                                         (1.0 - omega) / omega}, late, s));
+                            SymmetricSor{u.d_ind, u.d_val, f.d_ind, f.d_val, M->d_sdiag, b, cur, omega, ratio}, late, s));
     } else {
-      const CsrArrays& f = A->full;
       SB2_TRY(launch_sweeps(G, sweeps, plan, fwd, last,
-                            GeneralSor{f.d_ind, f.d_val, A->d_diag, b, cur, omega, 1.0 - omega}, late, s));
+                            GeneralSor{f.d_ind, f.d_val, A->d_diag, b, cur, omega, rest}, late, s));
     }
     cur = last;
   }
@@ -319,15 +402,21 @@ static void gather_levels(int n, const std::vector<int>& ptr, const std::vector<
   }
 }
 
-static int upload_sweep(const SweepGrid& G, const std::vector<int>& ptr,
+static int upload_sweep(sb2_precond* M, const std::vector<int>& ptr,
                         const std::vector<int>& ind, const std::vector<double>& val,
                         bool ascending, GatherSweep* S) {
+  const SweepGrid& G = M->grid;
   std::vector<int> level, pos(std::max(G.n, 1));
   gather_levels(G.n, ptr, ind, ascending, level);
+  if (M->form < 0) M->form = sweep_form(G.n, count_levels(level), (double)ind.size() / std::max(G.n, 1), 2);
+  const bool levels = M->form == kFormLevels;
   SweepOrder order;
-  make_sweep_order(G, level, &order);
-  for (int i = 0; i < G.n; i++) pos[order.rows[i]] = i;
-  // the lists in the order the rows are taken, columns as positions
+  std::vector<int> lvl;
+  if (levels) make_level_order(G.n, level, &order.rows, &lvl);
+  else make_sweep_order(G, level, &order);
+  // the values are by position, or by row when run by levels
+  for (int i = 0; i < G.n; i++) pos[order.rows[i]] = levels ? order.rows[i] : i;
+  // the lists in the order the rows are taken
   std::vector<int> pind;
   std::vector<double> pval;
   std::vector<int4> span(std::max(G.n, 1));
@@ -339,8 +428,15 @@ static int upload_sweep(const SweepGrid& G, const std::vector<int>& ptr,
     pval.insert(pval.end(), val.begin() + ptr[j], val.begin() + ptr[j + 1]);
     span[i] = make_int4(k0, (int)pind.size(), 0, 0);
   }
-  SB2_TRY(upload_sweep_plan(G, order, span.data(), &S->plan));
-  SB2_TRY(place_rows(G, S->plan, nullptr, nullptr, nullptr));
+  if (levels) {
+    std::vector<int> lists(G.n + 1, 0);
+    for (int i = 0; i < G.n; i++) lists[i + 1] = span[i].y;
+    SB2_TRY(upload_level_plan(G.n, order.rows, lvl, lists.data(), &S->plan));
+  } else {
+    SB2_TRY(upload_sweep_plan(G, order, span.data(), &S->plan));
+    SB2_TRY(place_rows(G, S->plan, nullptr, nullptr, nullptr));
+  }
+  for (int i = 0; i < G.n; i++) S->plan.max_len = std::max(S->plan.max_len, span[i].y - span[i].x);
   const size_t nz = pind.size();
   SB2_CUDA_TRY(cudaMalloc(&S->d_ind, sizeof(int) * std::max<size_t>(nz, 1)));
   SB2_CUDA_TRY(cudaMalloc(&S->d_val, sizeof(double) * std::max<size_t>(nz, 1)));
@@ -397,7 +493,6 @@ static int plan_ilut(sb2_precond* M, int n, const int* fp, const int* fi, const 
   if (!is_permutation(n, prow) || (!M->ilu_sym && !is_permutation(n, pcol)))
     return SB2_ERR_INVALID_VALUE;
   SB2_TRY(make_sweep_grid(n, &M->grid));
-  const SweepGrid& G = M->grid;
   std::vector<double> dinv(n);
   std::vector<int> ptr, ind;
   std::vector<double> val;
@@ -418,8 +513,8 @@ static int plan_ilut(sb2_precond* M, int n, const int* fp, const int* fi, const 
       bptr[i + 1] = (int)bind.size();
     }
     fwd.flatten(ptr, ind, val);
-    SB2_TRY(upload_sweep(G, ptr, ind, val, true, &M->s_lf));
-    SB2_TRY(upload_sweep(G, bptr, bind, bval, false, &M->s_ub));
+    SB2_TRY(upload_sweep(M, ptr, ind, val, true, &M->s_lf));
+    SB2_TRY(upload_sweep(M, bptr, bind, bval, false, &M->s_ub));
   } else {
     // row i: L part (columns < i), then 1/U(i,i), then the U part
     std::vector<int> lptr(n + 1, 0), lind, uptr(n + 1, 0), uind;
@@ -448,12 +543,12 @@ static int plan_ilut(sb2_precond* M, int n, const int* fp, const int* fi, const 
     }
     for (int i = n - 1; i >= 0; i--)  // L^T: x(k) -= L(i,k) x(i), i decreasing
       for (int k = fp[i]; k < dpos[i]; k++) ltb.add(fi[k], i, fv[k]);
-    SB2_TRY(upload_sweep(G, lptr, lind, lval, true, &M->s_lf));
-    SB2_TRY(upload_sweep(G, uptr, uind, uval, false, &M->s_ub));
+    SB2_TRY(upload_sweep(M, lptr, lind, lval, true, &M->s_lf));
+    SB2_TRY(upload_sweep(M, uptr, uind, uval, false, &M->s_ub));
     utf.flatten(ptr, ind, val);
-    SB2_TRY(upload_sweep(G, ptr, ind, val, true, &M->s_utf));
+    SB2_TRY(upload_sweep(M, ptr, ind, val, true, &M->s_utf));
     ltb.flatten(ptr, ind, val);
-    SB2_TRY(upload_sweep(G, ptr, ind, val, false, &M->s_ltb));
+    SB2_TRY(upload_sweep(M, ptr, ind, val, false, &M->s_ltb));
   }
   std::vector<int> iprow(n);
   for (int i = 0; i < n; i++) iprow[prow[i]] = i;
@@ -513,7 +608,7 @@ static int ilu0_factor(const sb2_csr* A, int modified, std::vector<int>& ptr,
   if (st == SB2_OK) st = map_cuda_error(e);
   int status = 0;
   if (st == SB2_OK)
-    st = run_levels(plan, n, Ilu0Row{f.d_ptr, f.d_ind, d_val, d_dpos, d_status, modified}, s);
+    st = run_factor_levels(plan, n, Ilu0Row{f.d_ptr, f.d_ind, d_val, d_dpos, d_status, modified}, s);
   if (st == SB2_OK) {
     e = cudaMemcpyAsync(&status, d_status, sizeof(int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess && f.nnz)
@@ -547,6 +642,13 @@ static int ilut_apply(sb2_precond* M, bool trans, const double* r, double* z, in
                  z, !sym && !trans ? M->d_pcol : M->d_iprow};
   const SweepPlan* const plan[2] = {&first.plan, &second.plan};
   const bool fwd[2] = {true, false};
+  if (M->form == kFormLevels) {
+    const SweepGrid& G = M->grid;
+    SB2_TRY(run_levels(first.plan, G.n, 0, true, LevelSpan{first.plan.d_lists, nullptr, nullptr}, nullptr, G.d_new[0],
+                       op, s));
+    return run_levels(second.plan, G.n, 1, false, LevelSpan{second.plan.d_lists, nullptr, nullptr}, G.d_new[0],
+                      G.d_new[1], op, s);
+  }
   return launch_sweeps(M->grid, 2, plan, fwd, nullptr, op, late, s);
 }
 

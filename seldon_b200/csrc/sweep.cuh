@@ -28,6 +28,9 @@
 // 384 threads for three-entry and symmetric rows: with 256 the small grids lose
 // (ILU(0) 16^3 54 us against 45), with 768 and more the registers spill on the
 // chain (83 us); general rows hold more and spill at 384 already (64^3 307 us).
+// Rows of more entries than a lane holds have a kernel of their own (LONG): the
+// others' is faster without its code (ILU(0) 64^3 199 us, 211 with), and it loads
+// ahead: ILU(0) of 27-entry rows, 40^3 657 us, 1697 entry by entry.
 //
 // Progress: all CTAs are resident (cooperative launch), a warp's items are in
 // level order and a row reads rows of smaller levels only.  Every wait is
@@ -47,6 +50,7 @@ constexpr int kSweepMaxCtas = 148;
 constexpr int kSweepStep = 32;   // items of one step at most
 constexpr int kSweepRing = 64;   // step barriers (more than the warps of a CTA)
 constexpr int kSweepSmem = 224 * 1024;  // most shared memory a CTA takes for its values
+constexpr int kSweepLong = 256;   // threads of a CTA where rows hold more entries than a lane does
 constexpr int kSweepNote = 4096;  // entries of a long row between two notes of progress
 // Words of SweepGrid::d_state: the grid leaves; a wait ran out since the word
 // was last read, in a solver's apply and in a caller's own; then one word a
@@ -65,6 +69,11 @@ struct SweepPlan {
   int* d_pos = nullptr;       // [n] position of each row
   int* d_cta_item = nullptr;  // [ctas + 1] first item of each CTA
   int* d_steps = nullptr;     // [ctas] steps of each CTA
+  int max_len = 0;            // entries of the longest row
+  // by levels (SweepForm): d_rows in level order, and
+  std::vector<int> h_lvl;     // [levels + 1] first position of each level
+  int* d_lvl = nullptr;       // the same on the device
+  int* d_lists = nullptr;     // [n + 1] first entry of each position's list
   void release() {
     cudaFree(d_buf);
     *this = SweepPlan();
@@ -204,6 +213,72 @@ inline int upload_sweep_plan(const SweepGrid& G, const SweepOrder& O, const int4
   SB2_CUDA_TRY(cudaMemcpy(P->d_item, O.item.data(), sizeof(int4) * items, cudaMemcpyHostToDevice));
   SB2_CUDA_TRY(cudaMemcpy(P->d_rows, O.rows.data(), sizeof(int) * G.n, cudaMemcpyHostToDevice));
   SB2_CUDA_TRY(cudaMemcpy(P->d_cta_item, tail.data(), sizeof(int) * words, cudaMemcpyHostToDevice));
+  return SB2_OK;
+}
+
+// ------------------------------------------------------------------ by levels
+
+constexpr int kLevelCta = 65536;  // rows up to which one CTA takes all levels of a sweep in place
+
+// How a sweep runs.  Bit for bit the same; what differs is what they wait for.
+enum SweepForm {
+  kFormSweep = 0,   // rows that wait for their values, above
+  kFormLevels = 1,  // a launch per level
+  kFormInPlace = 2  // x in place (SOR): all levels in one CTA, or a plain launch each
+};
+
+// The form for n rows of `entries` on the average in `levels`, kind 0 SOR, 1 SOR
+// on symmetric storage, 2 a factor's solves.
+//  - Few wide levels leave the sweep's one CTA per SM waiting for memory, where a
+//    launch per level (2.4 us, its own loads ahead of the one before) fills the
+//    GPU.  Forward SOR, sweep / launches: 1000^2 grid in red-black order, 2 levels,
+//    189 / 26 us; 300^2 in random order, 14 levels, 73 / 37; 1000^2 so, 15 levels, 262 /
+//    66; 10^6 diagonal rows 68 / 13.  Many levels: 40^3 convection-diffusion, 118, 94 /
+//    288.  A sweep moves 5 rows a ns, which is a launch's time at 12,000 rows a
+//    level.
+//  - Rows of many entries in narrow levels are bound by the instructions of the
+//    few lanes that have a row; one CTA whose operand stays in L1 needs the fewest.
+//    SSOR, sweep / one CTA: 20^3 grid of 27-entry rows, symmetric storage, 1.80 / 1.01
+//    ms, 40^3 4.0 / 3.2; bands of 31 entries, 2000 rows 6.6 / 4.9, of 81, 20,000 rows
+//    412 / 196.  General storage with 60 and 234 rows a level 1.0 / 0.96, 2.3 / 4.4 ms;
+//    with 262,144 rows more than one CTA is needed.
+//  - Very wide levels are bound by their bytes, of which x in place takes the
+//    fewest: SSOR, launches / in place: red-black 1000^2 54 / 34 us, 10^6 diagonal rows
+//    29 / 19; random order, 66,667 rows a level, 144 / 183.
+inline SweepForm sweep_form(int n, int levels, double entries, int kind) {
+  if (kind != 2 && n >= 200000LL * levels) return kFormInPlace;
+  if ((levels <= 16 && n >= 4096) || n >= 16000LL * levels) return kFormLevels;
+  if (kind != 2 && n <= kLevelCta && entries >= 16.0 && (kind == 1 || n <= 32LL * levels)) return kFormInPlace;
+  return kFormSweep;
+}
+
+// All rows by level (increasing row in a level), and the levels' offsets.
+inline void make_level_order(int n, const std::vector<int>& level, std::vector<int>* rows,
+                             std::vector<int>* lvl) {
+  int levels = 0;
+  for (int l : level) levels = std::max(levels, l + 1);
+  lvl->assign(levels + 1, 0);
+  for (int l : level) (*lvl)[l + 1]++;
+  for (int l = 0; l < levels; l++) (*lvl)[l + 1] += (*lvl)[l];
+  rows->resize(std::max(n, 1));
+  std::vector<int> at(lvl->begin(), lvl->end());
+  for (int i = 0; i < n; i++) (*rows)[at[level[i]]++] = i;
+}
+
+// lists: [n + 1] first entry of each position's list (null: the rows' own).
+inline int upload_level_plan(int n, const std::vector<int>& rows, const std::vector<int>& lvl,
+                             const int* lists, SweepPlan* P) {
+  const size_t len = std::max(n, 1);
+  SB2_CUDA_TRY(cudaMalloc(&P->d_buf, sizeof(int) * (2 * len + 1 + lvl.size())));
+  P->d_rows = static_cast<int*>(P->d_buf);
+  P->d_lvl = P->d_rows + len;
+  P->h_lvl = lvl;
+  SB2_CUDA_TRY(cudaMemcpy(P->d_rows, rows.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
+  SB2_CUDA_TRY(cudaMemcpy(P->d_lvl, lvl.data(), sizeof(int) * lvl.size(), cudaMemcpyHostToDevice));
+  if (lists) {
+    P->d_lists = P->d_lvl + lvl.size();
+    SB2_CUDA_TRY(cudaMemcpy(P->d_lists, lists, sizeof(int) * (n + 1), cudaMemcpyHostToDevice));
+  }
   return SB2_OK;
 }
 
@@ -354,7 +429,8 @@ struct Divisor {
 
 // RowSparse sweep (Relaxation_MatVect.cxx:69-77 / :83-91).  span.x..y: row j.
 struct GeneralSor {
-  static constexpr int kAhead = 8, kThreads = 256;
+  static constexpr int kAhead = 8, kThreads = 256, kAheadLong = 8;
+  static constexpr bool kTwoAhead = false, kTail = false;
   static constexpr bool kPositions = false;
   const int* ind; const double* val; const double* diag;
   const double* b; const double* x0; double omega, rest;  // rest = 1 - omega
@@ -399,7 +475,8 @@ struct GeneralSor {
 // (((1-w)/w * ajj) * x_j + b_j) - y; x_j = ((t - sum_{p != j} a_jp x_p) * w) /
 // ajj, the x_p new: the mirrored entries, then the stored ones.
 struct SymmetricSor {
-  static constexpr int kAhead = 8, kThreads = 384;
+  static constexpr int kAhead = 8, kThreads = 384, kAheadLong = 6;
+  static constexpr bool kTwoAhead = true, kTail = true;
   static constexpr bool kPositions = false;
   const int* uind; const double* uval; const int* find; const double* fval;
   const double* diag; const double* b; const double* x0;
@@ -469,7 +546,8 @@ struct SymmetricSor {
 // input permutation, the second from the first's values; its results also go
 // to z through the output permutation.  span.x..y: the row's update list.
 struct FactorSolve {
-  static constexpr int kAhead = 4, kThreads = 384;
+  static constexpr int kAhead = 4, kThreads = 384, kAheadLong = 8;
+  static constexpr bool kTwoAhead = true, kTail = false;
   static constexpr bool kPositions = true;
   const int* ind[2]; const double* val[2];
   const double* pre[2]; const double* post[2];
@@ -540,11 +618,11 @@ static __device__ __noinline__ void sweep_mark(const int4* items, const int* row
 
 // ------------------------------------------------------------------ the kernel
 
-template <class Op, bool OWN>
-__global__ void __launch_bounds__(Op::kThreads, 1) sweep_kernel(SweepArgs a, Op op) {
+template <class Op, bool OWN, bool LONG>
+__global__ void __launch_bounds__(LONG ? kSweepLong : Op::kThreads, 1) sweep_kernel(SweepArgs a, Op op) {
   extern __shared__ double s_own[];
   __shared__ unsigned long long s_bar[kSweepRing];  // step s completes s_bar[s % ring]
-  constexpr int U = Op::kAhead, W = Op::kThreads / 32;
+  constexpr int U = LONG ? Op::kAheadLong : Op::kAhead, W = (LONG ? kSweepLong : Op::kThreads) / 32;
   static_assert(W + 2 < kSweepRing, "a warp may be W items ahead of the oldest unfinished step");
   const int c0 = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int r0 = __ldg(a.blk + c0), rows = __ldg(a.blk + c0 + 1) - r0;
@@ -687,6 +765,23 @@ __global__ void __launch_bounds__(Op::kThreads, 1) sweep_kernel(SweepArgs a, Op 
         from[u] = fresh.own + ((near >> u & 1u) ? 8u * (unsigned)(at[u] - r0) : 0u);
       }
       double sum = live ? op.running(R, s) : 0.0;
+      // the first entries beyond, before the row's turn
+      int c1[U], q1[U], c2[U];
+      double f1[U], f2[U];
+      if (LONG) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          c1[u] = c2[u] = q1[u] = 0;
+          f1[u] = f2[u] = 0.0;
+          if (U + u < len) op.entry(R, U + u, c1[u], f1[u]);
+          if (Op::kTwoAhead && 2 * U + u < len) op.entry(R, 2 * U + u, c2[u], f2[u]);
+        }
+        if (Op::kTwoAhead) {
+#pragma unroll
+          for (int u = 0; u < U; u++)
+            if (U + u < len) q1[u] = place(c1[u], op.is_new(R, U + u, c1[u]));
+        }
+      }
       // wait for the other CTAs' new values and for this CTA's earlier steps
       while (ok) {
         const bool more = poll(~0u);
@@ -709,7 +804,71 @@ __global__ void __launch_bounds__(Op::kThreads, 1) sweep_kernel(SweepArgs a, Op 
         for (int u = 0; u < U; u++)
           if (adds >> u & 1u) sum = add_rn(sum, x[u]);
         if (adds) op.run_to(R, s, sum);
-        // rows longer than the entries held in registers
+        // rows longer than the entries held in registers, U at a time: while the
+        // values of U entries come, so do the places of the next U and the
+        // entries after those
+        if (LONG) {
+          for (int k0 = U; k0 < len && ok; k0 += U) {
+            if (k0 % kSweepNote == 0) *((volatile unsigned*)a.state + kStProgress + c0) = ~(unsigned)k0;
+            unsigned wait = 0u;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+              x[u] = 0.0;
+              if (k0 + u < len) {
+                if (!Op::kTwoAhead) q1[u] = place(c1[u], op.is_new(R, k0 + u, c1[u]));
+                if (op.is_new(R, k0 + u, c1[u]) || ph == 1) {
+                  if (OWN && (unsigned)(q1[u] - r0) < (unsigned)rows)
+                    x[u] = ld_shared((op.is_new(R, k0 + u, c1[u]) ? fresh : old).own + 8u * (unsigned)(q1[u] - r0));
+                  else
+                    wait |= 1u << u;
+                } else if (x0) {
+                  x[u] = __ldcg(x0 + q1[u]);
+                }
+              }
+            }
+            int c3[U], q2[U];
+            double f3[U];
+            if (Op::kTwoAhead) {
+#pragma unroll
+              for (int u = 0; u < U; u++) {
+                q2[u] = 0;
+                if (k0 + U + u < len) q2[u] = place(c2[u], op.is_new(R, k0 + U + u, c2[u]));
+              }
+            }
+            constexpr int kNext = (Op::kTwoAhead ? 2 : 1) * U;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+              c3[u] = 0;
+              f3[u] = 0.0;
+              if (k0 + kNext + u < len) op.entry(R, k0 + kNext + u, c3[u], f3[u]);
+            }
+            for (unsigned n = 1; wait && ok; n++) {
+              double y[U];
+#pragma unroll
+              for (int u = 0; u < U; u++)
+                if (wait >> u & 1u) y[u] = ld_volatile((op.is_new(R, k0 + u, c1[u]) ? fresh : old).g + q1[u]);
+#pragma unroll
+              for (int u = 0; u < U; u++)
+                if ((wait >> u & 1u) && !is_fill(y[u])) {
+                  x[u] = y[u];
+                  wait &= ~(1u << u);
+                }
+              if ((n & 255u) == 0u && wait && !w.go_on(t0, seen)) ok = false;
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+              if (k0 + u < len) op.take(R, s, k0 + u, c1[u], f1[u], x[u]);
+              c1[u] = Op::kTwoAhead ? c2[u] : c3[u];
+              f1[u] = Op::kTwoAhead ? f2[u] : f3[u];
+              if (Op::kTwoAhead) {
+                q1[u] = q2[u];
+                c2[u] = c3[u];
+                f2[u] = f3[u];
+              }
+            }
+          }
+        }
+        if (!LONG && Op::kTail) {
         for (int k = U; k < len && ok; k++) {
           if (k % kSweepNote == 0) *((volatile unsigned*)a.state + kStProgress + c0) = ~(unsigned)k;
           int cc;
@@ -732,6 +891,7 @@ __global__ void __launch_bounds__(Op::kThreads, 1) sweep_kernel(SweepArgs a, Op 
             y = __ldcg(x0 + cc);
           }
           op.take(R, s, k, cc, ff, y);
+        }
         }
         if (ok) {
           const double v = not_fill(op.last(R, s));
@@ -802,6 +962,203 @@ __global__ void __launch_bounds__(256) sweep_fill_kernel(int n, double* x, doubl
   }
 }
 
+// One sweep by levels: a row reads new values in `out` and the others in `old`
+// (null: zero), both by row.  What does not depend on other rows is loaded by
+// load(), before the level before is complete, the rest by finish().
+template <class Op, bool LONG>
+struct LevelRow {
+  static constexpr int U = 8;
+  typename Op::Row R;
+  int j, c[U];
+  double f[U];
+  __device__ __forceinline__ void load(const Op& op, int ph, bool fwd, int row, const int4& span) {
+    j = row;
+    R = op.load(ph, fwd, row, span);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      c[u] = 0;
+      f[u] = 0.0;
+      if (u < R.len) op.entry(R, u, c[u], f[u]);
+    }
+  }
+  __device__ __forceinline__ void finish(const Op& op, const double* old, double* out) {
+    typename Op::Sum s;
+    op.first(R, s, old ? old[j] : 0.0);
+    int k0 = 0;
+    do {
+      int c2[U];
+      double f2[U], x[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        x[u] = 0.0;
+        if (k0 + u < R.len) {
+          const double* p = op.is_new(R, k0 + u, c[u]) ? out : old;
+          if (p) x[u] = p[c[u]];
+        }
+      }
+      if (LONG) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          c2[u] = 0;
+          f2[u] = 0.0;
+          if (k0 + U + u < R.len) op.entry(R, k0 + U + u, c2[u], f2[u]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        if (k0 + u < R.len) op.take(R, s, k0 + u, c[u], f[u], x[u]);
+        if (LONG) {
+          c[u] = c2[u];
+          f[u] = f2[u];
+        }
+      }
+      k0 += U;
+    } while (LONG && k0 < R.len);
+    const double v = op.last(R, s);
+    out[j] = v;
+    op.store(R, v);
+  }
+};
+
+// Where a row's entries are: lists by position, or the rows' own with, for
+// symmetric storage, the stored half.
+struct LevelSpan {
+  const int *lists, *ptr, *uptr;
+  __device__ __forceinline__ int4 operator()(int i, int j) const {
+    if (lists) return make_int4(__ldg(lists + i), __ldg(lists + i + 1), 0, 0);
+    const int a = __ldg(ptr + j), e = __ldg(ptr + j + 1);
+    if (!uptr) return make_int4(a, e, 0, 0);
+    const int u = __ldg(uptr + j), ue = __ldg(uptr + j + 1);
+    return make_int4(u, ue, a, e - (ue - u));
+  }
+};
+
+// One level: what it needs of the level before is awaited by the hardware
+// (programmatic dependent launch), after its own loads are under way.
+template <class Op, bool LONG>
+__global__ void __launch_bounds__(256) level_rows_kernel(int begin, int end, int ph, bool fwd, const int* rows,
+                                                         LevelSpan span, const double* old, double* out, Op op) {
+  const int i = begin + blockIdx.x * blockDim.x + threadIdx.x;
+  LevelRow<Op, LONG> r;
+  if (i < end) {
+    const int j = __ldg(rows + i);
+    r.load(op, ph, fwd, j, span(i, j));
+  }
+  pdl_release();
+  pdl_wait();
+  if (i < end) r.finish(op, old, out);
+}
+
+// One sweep, a launch per level.
+template <class Op>
+int run_levels(const SweepPlan& P, int n, int ph, bool fwd, const LevelSpan& span, const double* old, double* out,
+               const Op& op, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(256);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  auto* kern = P.max_len > LevelRow<Op, true>::U ? level_rows_kernel<Op, true> : level_rows_kernel<Op, false>;
+  for (int l = 0; l + 1 < (int)P.h_lvl.size(); l++) {
+    const int begin = P.h_lvl[l], end = P.h_lvl[l + 1];
+    cfg.gridDim = dim3((end - begin + 255) / 256);
+    cfg.numAttrs = l > 0 ? 1 : 0;  // the first follows all that the caller queued
+    SB2_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, begin, end, ph, fwd, (const int*)P.d_rows, span, old, out, op));
+  }
+  return SB2_OK;
+}
+
+// x in place: levels then separate a row from the rows that read its new value and
+// from those that read its old one.  f(j): row j.
+template <class Row>
+__global__ void __launch_bounds__(1024) level_cta_kernel(int levels, const int* __restrict__ lvl,
+                                                         const int* __restrict__ rows, Row f) {
+  for (int l = 0; l < levels; l++) {
+    for (int i = lvl[l] + threadIdx.x; i < lvl[l + 1]; i += 1024) f(rows[i]);
+    __syncthreads();
+  }
+}
+
+// A row of GeneralSor, x in place.
+struct InPlaceSor {
+  const int *ptr, *ind;
+  const double *val, *diag, *b;
+  double* x;
+  double omega, rest;
+  __device__ __forceinline__ void operator()(int j) const {
+    double t = 0.0;
+    for (int k = ptr[j], e = ptr[j + 1]; k < e; k++) t = add_rn(t, mul_rn(val[k], x[ind[k]]));
+    const double xj = x[j], ajj = diag[j];
+    t = add_rn(__dsub_rn(b[j], t), mul_rn(ajj, xj));
+    x[j] = add_rn(mul_rn(rest, xj), __ddiv_rn(mul_rn(omega, t), ajj));
+  }
+};
+
+// Rows of SymmetricSor in two passes: `start` makes t of every row from old
+// values, `finish` takes the new ones.  Forward the stored entries are old and the
+// mirrored ones (which lead the expanded row) new, backward the other way round.
+struct InPlaceSymmetricSor {
+  const int *uptr, *uind;
+  const double* uval;
+  const int *ptr, *ind;
+  const double *val, *diag, *b;
+  double *x, *t;
+  double omega, ratio;
+  bool fwd, start;
+  __device__ __forceinline__ void operator()(int j) const {
+    const double ajj = diag[j];
+    double v = start || !fwd ? 0.0 : t[j];
+    if (fwd == start) {
+      for (int k = uptr[j], e = uptr[j + 1]; k < e; k++)
+        if (uind[k] != j) v = add_rn(v, mul_rn(uval[k], x[uind[k]]));
+    } else {
+      const int e = ptr[j + 1] - (uptr[j + 1] - uptr[j]);
+      for (int k = ptr[j]; k < e; k++) {
+        const double p = mul_rn(val[k], x[ind[k]]);
+        v = start ? add_rn(v, p) : __dsub_rn(v, p);
+      }
+    }
+    if (start) {
+      const double q = mul_rn(mul_rn(ratio, ajj), x[j]);
+      t[j] = fwd ? add_rn(q, __dsub_rn(b[j], v)) : __dsub_rn(add_rn(q, b[j]), v);
+    } else if (fwd) {
+      x[j] = mul_rn(v, __ddiv_rn(omega, ajj));
+    } else {
+      x[j] = __ddiv_rn(mul_rn(__dsub_rn(t[j], v), omega), ajj);
+    }
+  }
+};
+
+template <class Row>
+__global__ void __launch_bounds__(256) level_in_place_kernel(int begin, int end, const int* __restrict__ rows,
+                                                             Row f) {
+  const int i = begin + blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < end) f(rows[i]);
+}
+
+template <class Row>
+int run_in_place(const SweepPlan& P, int n, const Row& f, cudaStream_t s) {
+  const int levels = (int)P.h_lvl.size() - 1;
+  if (n <= kLevelCta) {
+    level_cta_kernel<<<1, 1024, 0, s>>>(levels, P.d_lvl, P.d_rows, f);
+  } else {
+    for (int l = 0; l < levels; l++) {
+      const int begin = P.h_lvl[l], end = P.h_lvl[l + 1];
+      level_in_place_kernel<<<(end - begin + 255) / 256, 256, 0, s>>>(begin, end, P.d_rows, f);
+    }
+  }
+  SB2_CUDA_TRY(cudaGetLastError());
+  return SB2_OK;
+}
+
+template <class Row>
+__global__ void __launch_bounds__(256) all_rows_kernel(int n, Row f) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < n) f(j);
+}
+
 // One launch of `sweeps` (1 or 2) sweeps; the last one's values go to `result`
 // by row (null: the operation stores them).  late: kStLateSolve or kStLateApply.
 template <class Op>
@@ -830,11 +1187,13 @@ int launch_sweeps(const SweepGrid& G, int sweeps, const SweepPlan* const (&plan)
   sweep_fill_kernel<<<g, 256, 0, s>>>(n, G.d_new[0], sweeps > 1 ? G.d_new[1] : nullptr, G.d_state,
                                    late);
   SB2_CUDA_TRY(cudaGetLastError());
-  const void* kern = own ? (const void*)sweep_kernel<Op, true> : (const void*)sweep_kernel<Op, false>;
+  const bool lng = plan[0]->max_len > Op::kAhead || plan[sweeps - 1]->max_len > Op::kAhead;
+  const void* kern = lng ? (own ? (const void*)sweep_kernel<Op, true, true> : (const void*)sweep_kernel<Op, false, true>)
+                         : (own ? (const void*)sweep_kernel<Op, true, false> : (const void*)sweep_kernel<Op, false, false>);
   if (own && smem > 48 * 1024) SB2_CUDA_TRY(allow_shared(kern, kSweepSmem));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(G.ctas);
-  cfg.blockDim = dim3(Op::kThreads);
+  cfg.blockDim = dim3(lng ? kSweepLong : Op::kThreads);
   cfg.dynamicSmemBytes = own ? smem : 0;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];

@@ -158,17 +158,15 @@ def test_long_row_is_progress(short_limit, oracle):
     """A row whose sum takes one lane longer than the wait limit: the row that
     waits for it goes on waiting."""
     from seldon_b200 import api
-    n = 6_000_000
+    n, chain = 6_000_000, 420  # (a chain of rows: with few levels each would be a launch)
     long = n - 2
-    ptr = np.arange(n + 1, dtype=np.int64)
-    ptr[long + 1:] += long
-    ptr[long + 2:] += 1
-    ind = np.concatenate([np.arange(long), np.arange(long + 1), [long, n - 1]]).astype(np.int32)
-    val = np.full(ind.size, 1e-7)
-    val[:long] = 2.0
-    val[ptr[long + 1] - 1] = 3.0
-    val[-2:] = [0.5, 2.0]
-    ptr = ptr.astype(np.int32)
+    one = np.arange(long)
+    rows = np.concatenate([one, one[1:chain], np.full(long + 1, long), [n - 1, n - 1]])
+    cols = np.concatenate([one, one[:chain - 1], np.arange(long + 1), [long, n - 1]])
+    ptr = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=n))]).astype(np.int32)
+    at = np.lexsort((cols, rows))
+    ind = cols[at].astype(np.int32)
+    val = np.where(rows[at] == ind, 2.0, np.where(rows[at] == long, 1e-7, 0.5))
     rng = np.random.default_rng(2)
     x0, b = rng.standard_normal(n), rng.standard_normal(n)
     x = to_dev(x0)
