@@ -23,8 +23,8 @@
 // division; everything that reads only old values comes before, while the
 // warp's predecessors still work.  From one CTA to the next a value takes about
 // a microsecond.  Two sweeps on a 7-point grid, against a graph of one launch
-// per level before: ILU(0) apply 96^3 424 us (2070), 128^3 694 us (2970); SSOR on
-// 64^3 with symmetric storage 289 us (1446), with general storage 271 us (1547).
+// per level before: ILU(0) apply 96^3 408 us (2070), 128^3 673 us (2970); SSOR on
+// 64^3 with symmetric storage 288 us (1446), with general storage 265 us (1547).
 // 384 threads for three-entry and symmetric rows: with 256 the small grids lose
 // (ILU(0) 16^3 54 us against 45), with 768 and more the registers spill on the
 // chain (83 us); general rows hold more and spill at 384 already (64^3 307 us).
@@ -243,8 +243,8 @@ enum SweepForm {
 //    412 / 196.  General storage with 60 and 234 rows a level 1.0 / 0.96, 2.3 / 4.4 ms;
 //    with 262,144 rows more than one CTA is needed.
 //  - Very wide levels are bound by their bytes, of which x in place takes the
-//    fewest: SSOR, launches / in place: red-black 1000^2 54 / 34 us, 10^6 diagonal rows
-//    29 / 19; random order, 66,667 rows a level, 144 / 183.
+//    fewest: SSOR, launches / in place: red-black 1000^2 54 / 42 us, 10^6 diagonal rows
+//    29 / 21; random order, 66,667 rows a level, 144 / 183.
 inline SweepForm sweep_form(int n, int levels, double entries, int kind) {
   if (kind != 2 && n >= 200000LL * levels) return kFormInPlace;
   if ((levels <= 16 && n >= 4096) || n >= 16000LL * levels) return kFormLevels;
@@ -964,10 +964,12 @@ __global__ void __launch_bounds__(256) sweep_fill_kernel(int n, double* x, doubl
 
 // One sweep by levels: a row reads new values in `out` and the others in `old`
 // (null: zero), both by row.  What does not depend on other rows is loaded by
-// load(), before the level before is complete, the rest by finish().
+// load(), before the level before is complete, the rest by finish().  (U entries
+// in flight: with eight, a factor's solves hold 48 registers for 32, and 10^6
+// diagonal rows take 23 us for 19.)
 template <class Op, bool LONG>
 struct LevelRow {
-  static constexpr int U = 8;
+  static constexpr int U = Op::kAhead;
   typename Op::Row R;
   int j, c[U];
   double f[U];
