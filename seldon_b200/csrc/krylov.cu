@@ -60,6 +60,7 @@ struct OpArgs {
   int n;
   const double* diag;  // nullptr: identity preconditioner, else Jacobi
   SellOp<double> sell; // binned SELL-32 (nslice < 0: use the row blocks)
+  int pack;            // warps that go to a CTA together (sell_pack)
 };
 
 struct IterArgs {
@@ -213,7 +214,7 @@ __device__ __forceinline__ void spmv_phase(const OpArgs& A, const double* x, Epi
                                            double* s_prod, double* s_red) {
   XLoadCa<double> xl{x};
   if (A.sell.nslice >= 0) {
-    sell_spmv_wide<NT, double, double>(A.sell, xl, epi, s_red);
+    sell_spmv_wide<NT, double, double>(A.sell, A.pack, xl, epi, s_red);
     return;
   }
   for (int b = blockIdx.x; b < A.nblk; b += gridDim.x)
@@ -3257,10 +3258,24 @@ static int finish_solve(SolveScratch& S, cudaStream_t s, sb2_iter_result* res, d
 
 SellOp<double> sell_op(const CsrArrays& a);
 
-static OpArgs op_args(const sb2_csr* A, const double* diag) {
+// Warps that go to a CTA together in a product by `grid` CTAs (log2; sell_spmv_wide).
+// Eight, as with CTAs of 256 threads: with all 32 warps of a CTA on consecutive
+// slices, a product of fewer slices than the grid has warps left most SMs idle
+// (200,000 rows of power-law lengths: Cg 185 us an iteration, 119 so).  Packs of 8
+// against 1 and 4: the same to 5 %, ahead where rows are wide, as a pack's slices
+// share their operand in L1.  Where slices are alike and one round of half the
+// warps or more, whole CTAs take as long (BiCgStab on 80^3 19.2 us an iteration, 19.0
+// in packs); with more rounds the last one is what packs spread.
+static int sell_pack(const CsrArrays& a, int grid) {
+  const bool even = !a.sell.sorted && !a.sell.nwarp && !a.sell.ncta;
+  const long long warps = (long long)grid * (NT / 32);
+  return even && 2LL * a.sell.nslice >= warps && a.sell.nslice <= warps ? 5 : 3;
+}
+
+static OpArgs op_args(const sb2_csr* A, const double* diag, int grid) {
   const CsrArrays& f = A->full;
   return OpArgs{f.d_ptr, f.d_ind, f.d_val, f.part.d_blk, f.part.d_kind, f.part.nblk, A->m, diag,
-                sell_op(f)};
+                sell_op(f), sell_pack(f, grid)};
 }
 
 enum Solver {
@@ -3322,7 +3337,7 @@ static int fused_solve(int which, const sb2_csr* A, const double* diag, double* 
   IterArgs it{prm->tol, prm->max_iter,
               which == kGcr ? std::max(prm->restart, 0) : which == kBicgl ? prm->restart : m,
               prm->init_guess_null};
-  OpArgs op = op_args(A, diag);
+  OpArgs op = op_args(A, diag, grid);
   const size_t nn = vector_stride(n, sizeof(double));
   double* V = S.vec;
   void* args[6];
@@ -3390,7 +3405,7 @@ static int fused_solve(int which, const sb2_csr* A, const double* diag, double* 
     // Seldon's transpose of RowSymSparse storage is the matrix itself
     const CsrArrays& t = A->sym ? A->full : A->trans;
     const OpArgs at{t.d_ptr, t.d_ind, t.d_val, t.part.d_blk, t.part.d_kind, t.part.nblk, A->m,
-                    diag, sell_op(t)};
+                    diag, sell_op(t), sell_pack(t, grid)};
     if (which == kBcg) {
       gcv = BcgVecs{b, x, V, V + nn, V + 2 * nn, V + 3 * nn, V + 4 * nn, V + 5 * nn, at};
       args[1] = &gcv;
@@ -5143,7 +5158,7 @@ static int cg_noalloc(const sb2_csr* A, double* x, const double* b, const sb2_it
   Persist P{sync, partials, barrier_wait_ns()};
   History H{hist, hist_it, 1};
   IterArgs it{prm->tol, prm->max_iter, std::max(prm->restart, 1), prm->init_guess_null};
-  OpArgs op = op_args(A, nullptr);
+  OpArgs op = op_args(A, nullptr, grid);
   CgVecs cv{b, x, vec, vec + n, vec + 2 * n};
   void* args[6] = {&op, &cv, &it, &P, &H, &out};
   SB2_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)cg_fused_kernel, dim3(grid), dim3(NT),

@@ -223,29 +223,24 @@ __device__ __forceinline__ void sell_group_row(const SellOp<VT>& S, int row, int
   asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(GT) : "memory");
 }
 
-// All bins by a grid of one large CTA per SM (s_red: NT / 32).
-// Eight warps at a time go to the next CTA, as with CTAs of 256 threads: with
-// all 32 warps of a CTA on consecutive slices, a product of fewer slices than
-// the grid has warps left most SMs idle (200,000 rows of power-law lengths: Cg
-// 185 us an iteration, 119 so).  Packs of 8 against 1 and 4: the same to 5 %,
-// ahead where rows are wide, as a pack's slices share their operand in L1.
-// Rows of the CTA bin go to groups of 256 threads where there are more of them
-// than CTAs; a single row takes the whole CTA (a row of 25,000 entries: Cg 20 us
-// an iteration, 32 with CTAs of 256 threads).
+// All bins by a grid of one large CTA per SM (s_red: NT / 32): 2^pack warps at a
+// time go to the next CTA.  Rows of the CTA bin go to groups of 256 threads where
+// there are more of them than CTAs; a single row takes the whole CTA (a row of
+// 25,000 entries: Cg 20 us an iteration, 32 with CTAs of 256 threads).
 template <int NT, typename VT, typename AT, class XLoad, class Epi>
-__device__ __forceinline__ void sell_spmv_wide(const SellOp<VT>& S, const XLoad& xl, Epi& epi,
+__device__ __forceinline__ void sell_spmv_wide(const SellOp<VT>& S, int pack, const XLoad& xl, Epi& epi,
                                                AT* s_red) {
-  constexpr int W = NT / 32, PACK = 8, GT = 32 * PACK;
+  constexpr int W = NT / 32, GT = 256;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ncta = gridDim.x;
   const long long nw = (long long)ncta * W;
-  const long long gw = ((long long)(warp / PACK) * ncta + blockIdx.x) * PACK + warp % PACK;
+  const long long gw = (((warp >> pack) * ncta + (int)blockIdx.x) << pack) + (warp & ((1 << pack) - 1));
   for (long long s = gw; s < S.nslice; s += nw) sell_slice<VT, AT, XLoad, Epi>(S, (int)s, lane, xl, epi);
   for (long long r = gw; r < S.nwarp_rows; r += nw)
     sell_warp_row<VT, AT>(S, __ldg(S.wrows + r), lane, xl, epi);
   if (S.ncta_rows > ncta) {
     const int group = threadIdx.x / GT;
     for (int r = group * ncta + blockIdx.x; r < S.ncta_rows; r += ncta * (NT / GT))
-      sell_group_row<GT, VT, AT>(S, __ldg(S.crows + r), group, xl, epi, s_red + group * PACK);
+      sell_group_row<GT, VT, AT>(S, __ldg(S.crows + r), group, xl, epi, s_red + group * (GT / 32));
   } else {
     for (int r = blockIdx.x; r < S.ncta_rows; r += ncta)
       sell_cta_row<NT, VT, AT>(S, __ldg(S.crows + r), xl, epi, s_red);
